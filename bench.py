@@ -461,7 +461,7 @@ def continuation_compare(nel: int, wi_end: float = 1.0, device: int = 0, log=Non
 
 def _solver_desc(solver) -> str:
     if type(solver).__name__ == "FrontalLU":
-        return (f"GPU panel-frontal LU, FP64 ({solver.npan} panels of {solver.G} elements, "
+        return (f"GPU frontal LU, FP64 ({solver.npan} fronts, "
                 f"{solver.flops / 1e12:.2f} TFLOP per factorisation)")
     return "host SuperLU (nested dissection)"
 
@@ -678,7 +678,7 @@ def frontal_solve_timing(nel: int, steps: int, warmup: int, device: int = 0):
                        f"Oldroyd-B Wi=0.5 SQRT, perturbed fully developed state; "
                        f"{_solver_desc(lu)}",
            "factor_s": t_fac, "factor_mode": lu.mode, "min_relative_pivot": lu.min_pivot,
-           "solve_ms": ev0.elapsed_time(ev1) / steps, "launches_per_solve": 2 * lu.npan + 2,
+           "solve_ms": ev0.elapsed_time(ev1) / steps, "launches_per_solve": lu.launches_per_solve,
            "solve_path": {1: "programmatic dependent launch", 2: "plain stream order"}.get(
                lu.solve_path, None),
            "solve_rel_residual": rel, "reproducible": bool(torch.equal(xs, xr))}

@@ -245,6 +245,36 @@ void vefem_frontal_destroy(vefem_frontal *f);
 const char *vefem_frontal_last_error(const vefem_frontal *f);
 int vefem_frontal_solve_path(const vefem_frontal *f);
 
+/* ---- Linear solver: multifrontal elimination over a tree of element sets --
+ * The same solve with the fronts of a nested dissection (the package's
+ * dissection.py is the symbolic phase): nlevel levels, deepest first, level l
+ * holding fronts level_ptr[l] .. level_ptr[l+1]; front t is an n[t] x n[t]
+ * matrix, row-major with leading dimension ld[t] (a multiple of 4, >= n[t]) at
+ * buf + off[t] (a multiple of 4), its p[t] pivots first.  ids [idx_off[t] ..):
+ * the global unknown of every row/column of front t.  child [2*t + s]: its
+ * children (in the level before it) or -1; src [s * idx_off[nfront] +
+ * idx_off[t] + j]: the row in child s's front of entry j of front t, or -1.
+ * Every unknown is a pivot of exactly one front.  All of these are host arrays,
+ * read by create only.
+ * vefem_tree_factor: vals [nnz] (device) go to buf[dest[k]] (device, int64,
+ * distinct), everything else in buf [buf_len] starts from zero; the elimination
+ * leaves A^-1 and A^-1 B in the pivot rows.  tol, min_pivot and
+ * VEFEM_ERR_SINGULAR as in vefem_frontal_factor.  Synchronises the stream.
+ * vefem_tree_solve: x = A^-1 b, device vectors of N doubles; asynchronous on
+ * the stream, vefem_tree_launches kernels replayed from a CUDA graph. */
+typedef struct vefem_tree vefem_tree;
+
+int vefem_tree_create(int device, int nfront, int nlevel, const int32_t *level_ptr,
+                      const int64_t *off, const int32_t *n, const int32_t *p, const int32_t *ld,
+                      const int32_t *child, const int64_t *ids, const int64_t *idx_off,
+                      const int32_t *src, int64_t N, vefem_tree **out);
+int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_t *dest, int64_t nnz,
+                      double *buf, int64_t buf_len, void *stream, double tol, double *min_pivot);
+int vefem_tree_solve(vefem_tree *f, const double *buf, const double *b, double *x, void *stream);
+int vefem_tree_launches(const vefem_tree *f);
+void vefem_tree_destroy(vefem_tree *f);
+const char *vefem_tree_last_error(const vefem_tree *f);
+
 /* ---- Linear stability: batched A/B assembly --------------------------------
  * setEquationsBulkStability (Stability/Equations_Stability_mod.F90:20-226):
  * the matrices of the generalised eigenproblem A x = lambda B x for

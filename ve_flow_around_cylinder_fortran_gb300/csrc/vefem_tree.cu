@@ -1,0 +1,671 @@
+// Multifrontal elimination of the bordered Newton Jacobian over a nested
+// dissection of the mesh: the Newton and continuation drivers' linear solver,
+// in place of the MUMPS factorisation and solve behind KSPSolve
+// (Petsc_mod.F90:850).
+//
+// The fronts are those of a complete binary tree of element sets (the
+// package's dissection.py); front t is an n x n matrix with leading dimension
+// ld (n rounded up to 4), its p pivots first.  All fronts of one depth are
+// factorised together, deepest first:
+//
+//   k_assemble  M += the children's Schur complements (pulled entry by entry,
+//               first child before second: no atomics, the same bits every run);
+//   k_pivot     per 16 pivots K: D^-1 and T = D^-1 M[K,:], and a copy of the
+//   k_update    columns C = M[P,K]; then M[i,:] -= C_i T for the other pivot
+//               rows i (M[i,K] = -C_i D^-1), M[K,:] = T: blocked Gauss-Jordan
+//               without pivoting on the pivot rows only, which leaves
+//               M[P,P] = A^-1 and M[P,F] = X = A^-1 B;
+//   k_schur     M[F,F] -= C X, one tiled product.
+//
+// What bounds it on GB300: the FP64 pipe, 2 multiply-adds per clock and SM
+// (0.63 T/s).  A sweep of element columns (vefem_frontal.cu) does 270 G
+// multiply-adds for 20,000 quads in 30,600 dependent steps; this tree does 63 G
+// in 273 (the pivots of the deepest path over 16), so the steps' latency
+// matters only near the root and the rest is FP64 throughput.  Eliminating the
+// pivot rows only and leaving the Schur complement to one product is 18% fewer
+// operations than Gauss-Jordan over the whole front, and a product has no
+// serial part.  Measured, factorise and solve: 1,184 ms (panels) -> 152 ms at
+// 20,000 quads, 89.5 -> 12.1 ms at 2,000; a solve checked to 1e-14 43.2 -> 2.6 ms
+// at 20,000 (2,500 panels are 5,000 dependent launches, the tree 41), and one
+// sweep already leaves a residual of 1e-15, where the panels' longer chain of
+// pivots left 1e-12 and took a refinement.
+//
+// Solve: per depth, deepest first, y_P = A^-1 b_P and the update -C y_P a
+// front hands to its parent; then, root first, x_P = y_P - X x_F.  A row's dot
+// product is spread over 8 lanes: with 32, the five shuffle additions per row
+// cost more of the FP64 pipe than the products of a small front.
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <cstring>
+#include <numeric>
+#include <string>
+#include <vector>
+
+#include "vefem.h"
+#include "vefem_gj.cuh"
+
+namespace {
+
+struct Front {
+    int64_t off;       // first entry of the matrix in the factor buffer
+    int64_t cpan;      // first entry of the pivot-column copy (16 per pivot row)
+    int64_t tpan;      // first entry of T (16 rows of ld)
+    int32_t base;      // first entry of the front's unknowns, maps and vectors
+    int32_t n, p, ld;
+    int32_t child[2];  // front index, or -1
+};
+
+// ---------------------------------------------------------------- factorisation
+
+// original entries into their fronts (every entry has a place of its own)
+__global__ void k_scatter(int64_t nnz, const int64_t *__restrict__ dest, const double *__restrict__ vals,
+                          double *__restrict__ buf)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nnz) buf[dest[i]] = vals[i];
+}
+
+constexpr int AS_ROWS = 8;
+// M[i,j] += S_child0[src0[i], src0[j]], then the same for the second child
+__global__ void __launch_bounds__(32 * AS_ROWS)
+k_assemble(const Front *__restrict__ fr, const int32_t *__restrict__ perm, const int32_t *__restrict__ src0,
+           const int32_t *__restrict__ src1, double *__restrict__ buf)
+{
+    const Front f = fr[perm[blockIdx.x]];
+    const int i = blockIdx.y * AS_ROWS + threadIdx.y;
+    if (i >= f.n) return;
+    const int a0 = src0[f.base + i], a1 = src1[f.base + i];
+    if (a0 < 0 && a1 < 0) return;
+    const double *r0 = nullptr, *r1 = nullptr;
+    if (a0 >= 0) r0 = buf + fr[f.child[0]].off + (int64_t)a0 * fr[f.child[0]].ld;
+    if (a1 >= 0) r1 = buf + fr[f.child[1]].off + (int64_t)a1 * fr[f.child[1]].ld;
+    double *m = buf + f.off + (int64_t)i * f.ld;
+    for (int j = threadIdx.x; j < f.n; j += 32) {
+        const int b0 = r0 ? src0[f.base + j] : -1, b1 = r1 ? src1[f.base + j] : -1;
+        if (b0 < 0 && b1 < 0) continue;
+        double v = m[j];
+        if (b0 >= 0) v += r0[b0];
+        if (b1 >= 0) v += r1[b1];
+        m[j] = v;
+    }
+}
+
+// Step on pivots K = [k0, k0 + kb): every CTA inverts D = M[K,K] (the same
+// bits in each) and forms T for its W columns; columns K of T hold D^-1.
+// W = 32 spreads the T of a few large fronts over many SMs, W = 128 inverts
+// less often where there are many fronts.
+template <int W>
+__global__ void __launch_bounds__(128)
+k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
+        double *__restrict__ cpan, double *__restrict__ tpan, int *err, unsigned long long *minpiv, double tol)
+{
+    __shared__ double sA[2 * NB][NB + 1];
+    __shared__ double s_red[4];
+    const Front f = fr[perm[blockIdx.x]];
+    const int j0 = blockIdx.y * W;
+    if (j0 >= f.ld) return;
+    const int kb = min(NB, f.p - k0), t = threadIdx.x;
+    const double *M = buf + f.off;
+    for (int u = t; u < 2 * NB * NB; u += 128) {
+        const int c = u / NB, r = u % NB;
+        double v;
+        if (c < NB)
+            v = (r < kb && c < kb) ? M[(int64_t)(k0 + r) * f.ld + k0 + c] : (r == c ? 1.0 : 0.0);
+        else
+            v = (r == c - NB) ? 1.0 : 0.0;
+        sA[c][r] = v;
+    }
+    // this CTA's share of the pivot-column copy
+    for (int u = t; u < W * NB; u += 128) {
+        const int r = j0 + u / NB, l = u % NB;
+        if (r < f.p) cpan[f.cpan + (int64_t)r * NB + l] = l < kb ? M[(int64_t)r * f.ld + k0 + l] : 0.0;
+    }
+    __syncthreads();
+    const double rel = block_invert(sA, kb, tol, s_red);
+    if (blockIdx.y == 0 && t == 0) {
+        if (rel < 0.0) atomicExch(err, 1);
+        else atomic_min_pos(minpiv, rel);
+    }
+    constexpr int PER = NB * W / 128;                 // rows of T per thread
+    const int j = j0 + t % W, g = t / W;
+    if (j < f.ld) {
+        const bool own = j >= k0 && j < k0 + kb;
+        double m[NB];
+#pragma unroll
+        for (int l = 0; l < NB; l++) m[l] = l < kb ? M[(int64_t)(k0 + l) * f.ld + j] : 0.0;
+        double *T = tpan + f.tpan + j;
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const int k = g * PER + q;
+            double acc = 0.0;
+            if (own) {
+                acc = sA[NB + j - k0][k];
+            } else {
+#pragma unroll
+                for (int l = 0; l < NB; l++) acc = fma(sA[NB + l][k], m[l], acc);
+            }
+            T[(int64_t)k * f.ld] = acc;
+        }
+    }
+}
+
+constexpr int TILE = 64;   // rows and columns of a CTA's tile, 8 warps of 16 x 32
+
+// acc[a][b] += sum over 16 k of A[k][row a] B[k][col b] for a warp's 16 x 32
+// part of the tile: lane = (row quad, column pair), columns 2 apart by 16
+__device__ __forceinline__ void tile_fma(double (&acc)[4][4], const double (*sa)[TILE + 2],
+                                         const double (*sb)[TILE], int r, int c)
+{
+#pragma unroll
+    for (int l = 0; l < NB; l++) {
+        double a[4], b[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) a[u] = sa[l][r + u];
+        const double2 b0 = *reinterpret_cast<const double2 *>(&sb[l][c]);
+        const double2 b1 = *reinterpret_cast<const double2 *>(&sb[l][c + 16]);
+        b[0] = b0.x; b[1] = b0.y; b[2] = b1.x; b[3] = b1.y;
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+#pragma unroll
+            for (int v = 0; v < 4; v++) acc[u][v] = fma(a[u], b[v], acc[u][v]);
+    }
+}
+
+// M[i,:] -= C_i T for the pivot rows outside K, M[K,:] = T (in place: C and T
+// are copies, an entry is read and written by its own thread)
+__global__ void __launch_bounds__(256, 2)
+k_update(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, int ntc,
+         const double *__restrict__ cpan, const double *__restrict__ tpan, double *__restrict__ buf)
+{
+    __shared__ double sa[NB][TILE + 2];
+    __shared__ __align__(16) double sb[NB][TILE];
+    const Front f = fr[perm[blockIdx.x]];
+    const int i0 = (blockIdx.y / ntc) * TILE, j0 = (blockIdx.y % ntc) * TILE;
+    if (i0 >= f.p || j0 >= f.ld) return;
+    const int t = threadIdx.x;
+    for (int u = t; u < TILE * NB; u += 256) {
+        const int r = u / NB, l = u % NB;
+        sa[l][r] = i0 + r < f.p ? cpan[f.cpan + (int64_t)(i0 + r) * NB + l] : 0.0;
+        const int k = u / TILE, c = u % TILE;
+        sb[k][c] = j0 + c < f.ld ? tpan[f.tpan + (int64_t)k * f.ld + j0 + c] : 0.0;
+    }
+    __syncthreads();
+    const int w = t >> 5, lane = t & 31;
+    const int wr = (w >> 1) * 16, wc = (w & 1) * 32;
+    if (i0 + wr >= f.p || j0 + wc >= f.ld) return;
+    const int r = wr + (lane >> 3) * 4, c = wc + (lane & 7) * 2;
+    const int kb = min(NB, f.p - k0);
+    double acc[4][4] = {};
+    const bool copy = i0 + wr == k0;                  // the warp's rows are K
+    if (!copy) tile_fma(acc, sa, sb, r, c);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int i = i0 + r + u;
+        if (i >= f.p) continue;
+        double *row = buf + f.off + (int64_t)i * f.ld + j0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int cc = c + 16 * h, j = j0 + cc;
+            if (j >= f.ld) continue;
+            double2 v;
+            if (copy) {
+                v = *reinterpret_cast<const double2 *>(&sb[i - k0][cc]);
+            } else {
+                v = *reinterpret_cast<const double2 *>(row + cc);
+                if (j >= k0 && j < k0 + kb) v.x = 0.0;
+                if (j + 1 >= k0 && j + 1 < k0 + kb) v.y = 0.0;
+                v.x -= acc[u][2 * h];
+                v.y -= acc[u][2 * h + 1];
+            }
+            *reinterpret_cast<double2 *>(row + cc) = v;
+        }
+    }
+}
+
+// M[F,F] -= M[F,P] M[P,F]
+__global__ void __launch_bounds__(256, 2)
+k_schur(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int nt, double *__restrict__ buf)
+{
+    __shared__ double sa[2][NB][TILE + 2];
+    __shared__ __align__(16) double sb[2][NB][TILE];
+    const Front f = fr[perm[blockIdx.x]];
+    const int q = f.n - f.p;
+    const int i0 = (blockIdx.y / nt) * TILE, j0 = (blockIdx.y % nt) * TILE;
+    if (i0 >= q || j0 >= q || f.p == 0) return;
+    double *M = buf + f.off;
+    const int t = threadIdx.x;
+    // a thread stages 4 entries of A (one row, 4 consecutive k) and 4 of B (one k, 4 columns)
+    const int ar = t >> 2, ak = (t & 3) * 4, bk = t >> 4, bc = (t & 15) * 4;
+    const double *pa = M + (int64_t)(f.p + min(i0 + ar, q - 1)) * f.ld;
+    const double *pb = M + f.p + j0;
+    double va[4], vb[4];
+    auto fetch = [&](int k) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            va[u] = k + ak + u < f.p ? pa[k + ak + u] : 0.0;
+            vb[u] = (k + bk < f.p && j0 + bc + u < q) ? pb[(int64_t)(k + bk) * f.ld + bc + u] : 0.0;
+        }
+    };
+    auto stage = [&](int s) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            sa[s][ak + u][ar] = va[u];
+            sb[s][bk][bc + u] = vb[u];
+        }
+    };
+    const int w = t >> 5, lane = t & 31;
+    const int wr = (w >> 1) * 16, wc = (w & 1) * 32;
+    const int r = wr + (lane >> 3) * 4, c = wc + (lane & 7) * 2;
+    const bool live = i0 + wr < q && j0 + wc < q;
+    double acc[4][4] = {};
+    fetch(0);
+    stage(0);
+    __syncthreads();
+    int s = 0;
+    for (int k = 0; k < f.p; k += NB, s ^= 1) {
+        const bool more = k + NB < f.p;
+        if (more) fetch(k + NB);
+        if (live) tile_fma(acc, sa[s], sb[s], r, c);
+        if (more) stage(s ^ 1);
+        __syncthreads();
+    }
+    if (!live) return;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int i = i0 + r + u;
+        if (i >= q) continue;
+        double *row = M + (int64_t)(f.p + i) * f.ld + f.p + j0;
+#pragma unroll
+        for (int v = 0; v < 4; v++) {
+            const int cc = c + (v & 1) + 16 * (v >> 1);
+            if (j0 + cc < q) row[cc] -= acc[u][v];
+        }
+    }
+}
+
+// ---------------------------------------------------------------- solve
+
+constexpr int SV_THREADS = 256;
+constexpr int SV_LANES = 8;                            // lanes per row
+constexpr int SV_ROWS = SV_THREADS / SV_LANES;         // rows per pass of a CTA
+
+// dot product of a row with the staged vector over 8 lanes (fixed order)
+__device__ __forceinline__ double row_dot(const double *__restrict__ row, const double *s_vec, int m, int lane)
+{
+    double s = 0.0;
+#pragma unroll 4
+    for (int k = lane; k < m; k += SV_LANES) s = fma(row[k], s_vec[k], s);
+#pragma unroll
+    for (int o = SV_LANES / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
+// what the children hand to position j of front f
+__device__ __forceinline__ double handed(const Front &f, const Front *__restrict__ fr, int j,
+                                         const int32_t *__restrict__ src0, const int32_t *__restrict__ src1,
+                                         const double *__restrict__ y)
+{
+    double v = 0.0;
+    const int a0 = src0[f.base + j], a1 = src1[f.base + j];
+    if (a0 >= 0) v += y[fr[f.child[0]].base + a0];
+    if (a1 >= 0) v += y[fr[f.child[1]].base + a1];
+    return v;
+}
+
+// y_P = A^-1 (b_P + handed)
+__global__ void __launch_bounds__(SV_THREADS)
+k_tree_fwd(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int rows, const int32_t *__restrict__ ids,
+           const int32_t *__restrict__ src0, const int32_t *__restrict__ src1, const double *__restrict__ buf,
+           const double *__restrict__ b, double *__restrict__ y)
+{
+    extern __shared__ double s_vec[];
+    const Front f = fr[perm[blockIdx.x]];
+    const int r0 = blockIdx.y * rows, r1 = min(r0 + rows, f.p);
+    if (r0 >= f.p) return;
+    for (int j = threadIdx.x; j < f.p; j += SV_THREADS)
+        s_vec[j] = b[ids[f.base + j]] + handed(f, fr, j, src0, src1, y);
+    __syncthreads();
+    const int lane = threadIdx.x % SV_LANES;
+    for (int rr = r0; rr < r1; rr += SV_ROWS) {
+        const int r = rr + threadIdx.x / SV_LANES;
+        const double s = row_dot(buf + f.off + (int64_t)min(r, f.p - 1) * f.ld, s_vec, f.p, lane);
+        if (r < r1 && lane == 0) y[f.base + r] = s;
+    }
+}
+
+// the update for the parent: handed - C y_P
+__global__ void __launch_bounds__(SV_THREADS)
+k_tree_up(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int rows, const int32_t *__restrict__ src0,
+          const int32_t *__restrict__ src1, const double *__restrict__ buf, double *__restrict__ y)
+{
+    extern __shared__ double s_vec[];
+    const Front f = fr[perm[blockIdx.x]];
+    const int r0 = f.p + blockIdx.y * rows, r1 = min(r0 + rows, f.n);
+    if (r0 >= f.n) return;
+    for (int j = threadIdx.x; j < f.p; j += SV_THREADS) s_vec[j] = y[f.base + j];
+    __syncthreads();
+    const int lane = threadIdx.x % SV_LANES;
+    for (int rr = r0; rr < r1; rr += SV_ROWS) {
+        const int r = rr + threadIdx.x / SV_LANES;
+        const double s = row_dot(buf + f.off + (int64_t)min(r, f.n - 1) * f.ld, s_vec, f.p, lane);
+        if (r < r1 && lane == 0) y[f.base + r] = handed(f, fr, r, src0, src1, y) - s;
+    }
+}
+
+// x_P = y_P - X x_F
+__global__ void __launch_bounds__(SV_THREADS)
+k_tree_bwd(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int rows, const int32_t *__restrict__ ids,
+           const double *__restrict__ buf, const double *__restrict__ y, double *__restrict__ x)
+{
+    extern __shared__ double s_vec[];
+    const Front f = fr[perm[blockIdx.x]];
+    const int r0 = blockIdx.y * rows, r1 = min(r0 + rows, f.p);
+    if (r0 >= f.p) return;
+    const int q = f.n - f.p;
+    for (int j = threadIdx.x; j < q; j += SV_THREADS) s_vec[j] = x[ids[f.base + f.p + j]];
+    __syncthreads();
+    const int lane = threadIdx.x % SV_LANES;
+    for (int rr = r0; rr < r1; rr += SV_ROWS) {
+        const int r = rr + threadIdx.x / SV_LANES;
+        const double s = row_dot(buf + f.off + (int64_t)min(r, f.p - 1) * f.ld + f.p, s_vec, q, lane);
+        if (r < r1 && lane == 0) x[ids[f.base + r]] = y[f.base + r] - s;
+    }
+}
+
+struct Guard {
+    int prev = -1;
+    explicit Guard(int d)
+    {
+        if (cudaGetDevice(&prev) != cudaSuccess) prev = -1;
+        cudaSetDevice(d);
+    }
+    ~Guard()
+    {
+        if (prev >= 0) cudaSetDevice(prev);
+    }
+};
+
+struct Level {
+    int first, count;           // fronts, and their places in perm (most pivots first)
+    int nmax, pmax, qmax, ldmax;
+    std::vector<int> active;    // fronts with more than 16 s pivots, per step s
+    std::vector<int> ld_active; // largest leading dimension among them
+};
+
+}  // namespace
+
+struct vefem_tree {
+    int device = 0, nfront = 0, sms = 0;
+    int64_t N = 0, total = 0;
+    std::vector<Level> levels;
+    int pmax = 0, qmax = 0;
+    Front *fr = nullptr;
+    int32_t *perm = nullptr, *ids = nullptr, *src0 = nullptr, *src1 = nullptr;
+    double *cpan = nullptr, *tpan = nullptr;
+    double *y = nullptr, *b = nullptr, *x = nullptr;
+    int *err = nullptr;
+    unsigned long long *minpiv = nullptr;
+    unsigned long long h_one = 0;      // staging of the initial minimum (outlives the async copy)
+    cudaStream_t cs = nullptr;
+    cudaGraphExec_t graph = nullptr;   // the sweeps of a solve, captured per factor buffer
+    const double *graph_buf = nullptr;
+    std::string msg;
+};
+
+namespace {
+
+int tfail(vefem_tree *f, int code, const std::string &m)
+{
+    if (f) f->msg = m;
+    return code;
+}
+
+#define TCK(call)                                                                        \
+    do {                                                                                 \
+        cudaError_t _e = (call);                                                         \
+        if (_e != cudaSuccess)                                                           \
+            return tfail(f, VEFEM_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(_e)); \
+    } while (0)
+
+unsigned up(int a, int b) { return (unsigned)((a + b - 1) / b); }
+
+// rows per CTA of a sweep launch: one CTA per front where the fronts fill the
+// GPU twice over, else as many as spread the rows over it
+int rows_per_cta(const vefem_tree *f, int fronts, int rmax)
+{
+    if (fronts >= 2 * f->sms) return std::max(SV_ROWS, rmax);
+    const int parts = std::max(1, 4 * f->sms / fronts);
+    return std::max(SV_ROWS, (int)up((int)up(rmax, parts), SV_ROWS) * SV_ROWS);
+}
+
+cudaError_t launch_sweeps(vefem_tree *f, const double *buf, cudaStream_t s)
+{
+    for (const Level &l : f->levels) {
+        const int32_t *perm = f->perm + l.first;
+        const size_t sm = (size_t)std::max(1, l.pmax) * sizeof(double);
+        if (l.pmax > 0) {
+            const int r = rows_per_cta(f, l.count, l.pmax);
+            k_tree_fwd<<<dim3(l.count, up(l.pmax, r)), SV_THREADS, sm, s>>>(f->fr, perm, r, f->ids, f->src0, f->src1,
+                                                                           buf, f->b, f->y);
+        }
+        if (l.qmax > 0) {
+            const int r = rows_per_cta(f, l.count, l.qmax);
+            k_tree_up<<<dim3(l.count, up(l.qmax, r)), SV_THREADS, sm, s>>>(f->fr, perm, r, f->src0, f->src1, buf, f->y);
+        }
+    }
+    for (auto it = f->levels.rbegin(); it != f->levels.rend(); ++it) {
+        const Level &l = *it;
+        if (l.pmax == 0) continue;
+        const int r = rows_per_cta(f, l.count, l.pmax);
+        k_tree_bwd<<<dim3(l.count, up(l.pmax, r)), SV_THREADS, (size_t)std::max(1, l.qmax) * sizeof(double), s>>>(
+            f->fr, f->perm + l.first, r, f->ids, buf, f->y, f->x);
+    }
+    return cudaGetLastError();
+}
+
+}  // namespace
+
+extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32_t *level_ptr, const int64_t *off,
+                                 const int32_t *n, const int32_t *p, const int32_t *ld, const int32_t *child,
+                                 const int64_t *ids, const int64_t *idx_off, const int32_t *src, int64_t N,
+                                 vefem_tree **out)
+{
+    if (!out || nfront <= 0 || nlevel <= 0 || !level_ptr || !off || !n || !p || !ld || !child || !ids || !idx_off ||
+        !src || N <= 0 || N >= INT32_MAX || idx_off[nfront] >= INT32_MAX)
+        return VEFEM_ERR_ARG;
+    *out = nullptr;
+    if (level_ptr[0] != 0 || level_ptr[nlevel] != nfront) return VEFEM_ERR_ARG;
+    const int64_t tot = idx_off[nfront];
+    // every unknown a pivot once; every map inside its child's boundary; children one level below
+    std::vector<int> level(nfront);
+    for (int l = 0; l < nlevel; l++) {
+        if (level_ptr[l + 1] <= level_ptr[l]) return VEFEM_ERR_ARG;
+        for (int t = level_ptr[l]; t < level_ptr[l + 1]; t++) level[t] = l;
+    }
+    std::vector<char> seen((size_t)N, 0);
+    int64_t pivots = 0;
+    for (int t = 0; t < nfront; t++) {
+        if (n[t] < 0 || p[t] < 0 || p[t] > n[t] || ld[t] < n[t] || ld[t] % 4 || off[t] % 4 ||
+            off[t + 1] - off[t] < (int64_t)n[t] * ld[t] || idx_off[t + 1] - idx_off[t] != n[t])
+            return VEFEM_ERR_ARG;
+        for (int j = 0; j < n[t]; j++) {
+            const int64_t u = ids[idx_off[t] + j];
+            if (u < 0 || u >= N || (j < p[t] && seen[(size_t)u])) return VEFEM_ERR_ARG;
+            if (j < p[t]) seen[(size_t)u] = 1;
+        }
+        pivots += p[t];
+        for (int s = 0; s < 2; s++) {
+            const int c = child[2 * t + s];
+            if (c >= nfront || (c >= 0 && level[c] != level[t] - 1)) return VEFEM_ERR_ARG;
+            for (int j = 0; j < n[t]; j++) {
+                const int a = src[s * tot + idx_off[t] + j];
+                if (a >= 0 && (c < 0 || a < p[c] || a >= n[c])) return VEFEM_ERR_ARG;
+            }
+        }
+    }
+    if (pivots != N) return VEFEM_ERR_ARG;
+
+    vefem_tree *f = new vefem_tree();
+    f->device = device;
+    f->nfront = nfront;
+    f->N = N;
+    f->total = tot;
+    std::vector<Front> fr(nfront);
+    std::vector<int32_t> perm(nfront);
+    std::iota(perm.begin(), perm.end(), 0);
+    int64_t cmax = 0, tmax = 0;
+    for (int l = 0; l < nlevel; l++) {
+        Level v{level_ptr[l], level_ptr[l + 1] - level_ptr[l], 0, 0, 0, 0, {}, {}};
+        std::stable_sort(perm.begin() + v.first, perm.begin() + v.first + v.count,
+                         [&](int a, int c) { return p[a] > p[c]; });
+        int64_t cp = 0, tp = 0;
+        for (int k = v.first; k < v.first + v.count; k++) {
+            const int t = perm[k];
+            fr[t] = Front{off[t], cp, tp, (int32_t)idx_off[t], n[t], p[t], ld[t], {child[2 * t], child[2 * t + 1]}};
+            cp += (int64_t)p[t] * NB;
+            tp += (int64_t)ld[t] * NB;
+            v.nmax = std::max(v.nmax, n[t]);
+            v.pmax = std::max(v.pmax, p[t]);
+            v.qmax = std::max(v.qmax, n[t] - p[t]);
+            v.ldmax = std::max(v.ldmax, ld[t]);
+        }
+        for (int k0 = 0; k0 < v.pmax; k0 += NB) {
+            int a = 0, m = 0;
+            while (a < v.count && p[perm[v.first + a]] > k0) m = std::max(m, (int)ld[perm[v.first + a++]]);
+            v.active.push_back(a);
+            v.ld_active.push_back(m);
+        }
+        cmax = std::max(cmax, cp);
+        tmax = std::max(tmax, tp);
+        f->pmax = std::max(f->pmax, v.pmax);
+        f->qmax = std::max(f->qmax, v.qmax);
+        f->levels.push_back(std::move(v));
+    }
+    std::vector<int32_t> ids32(ids, ids + tot);
+    Guard g(device);
+    auto put = [](auto **dst, const auto *from, size_t count) {
+        return cudaMalloc((void **)dst, std::max<size_t>(1, count) * sizeof(**dst)) == cudaSuccess &&
+               (!from || cudaMemcpy(*dst, from, count * sizeof(**dst), cudaMemcpyHostToDevice) == cudaSuccess);
+    };
+    const double *none = nullptr;
+    const bool ok =
+        cudaDeviceGetAttribute(&f->sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
+        cudaStreamCreateWithFlags(&f->cs, cudaStreamNonBlocking) == cudaSuccess && put(&f->fr, fr.data(), fr.size()) &&
+        put(&f->perm, perm.data(), perm.size()) && put(&f->ids, ids32.data(), ids32.size()) &&
+        put(&f->src0, src, (size_t)tot) && put(&f->src1, src + tot, (size_t)tot) && put(&f->cpan, none, (size_t)cmax) &&
+        put(&f->tpan, none, (size_t)tmax) && put(&f->y, none, (size_t)tot) && put(&f->b, none, (size_t)N) &&
+        put(&f->x, none, (size_t)N) && put(&f->err, (const int *)nullptr, 1) &&
+        put(&f->minpiv, (const unsigned long long *)nullptr, 1);
+    const int sm_p = f->pmax * (int)sizeof(double), sm_q = f->qmax * (int)sizeof(double);
+    if (!ok || (sm_p > 48 * 1024 &&
+                (cudaFuncSetAttribute(k_tree_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess ||
+                 cudaFuncSetAttribute(k_tree_up, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess)) ||
+        (sm_q > 48 * 1024 &&
+         cudaFuncSetAttribute(k_tree_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_q) != cudaSuccess)) {
+        cudaGetLastError();
+        vefem_tree_destroy(f);
+        return VEFEM_ERR_NOMEM;
+    }
+    *out = f;
+    return VEFEM_OK;
+}
+
+extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_t *dest, int64_t nnz, double *buf,
+                                 int64_t buf_len, void *stream, double tol, double *min_pivot)
+{
+    if (!f || !vals || !dest || nnz <= 0 || !buf) return VEFEM_ERR_ARG;
+    Guard g(f->device);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const double one = 1.0;
+    std::memcpy(&f->h_one, &one, sizeof(one));
+    TCK(cudaMemsetAsync(f->err, 0, sizeof(int), s));
+    TCK(cudaMemcpyAsync(f->minpiv, &f->h_one, sizeof(f->h_one), cudaMemcpyHostToDevice, s));
+    TCK(cudaMemsetAsync(buf, 0, (size_t)buf_len * sizeof(double), s));
+    k_scatter<<<(unsigned)((nnz + 255) / 256), 256, 0, s>>>(nnz, dest, vals, buf);
+    for (size_t li = 0; li < f->levels.size(); li++) {
+        const Level &l = f->levels[li];
+        const int32_t *perm = f->perm + l.first;
+        if (li > 0 && l.nmax > 0)
+            k_assemble<<<dim3(l.count, up(l.nmax, AS_ROWS)), dim3(32, AS_ROWS), 0, s>>>(f->fr, perm, f->src0, f->src1,
+                                                                                       buf);
+        for (size_t st = 0; st < l.active.size(); st++) {
+            const int k0 = (int)st * NB, a = l.active[st], ld = l.ld_active[st];
+            if ((int64_t)a * up(ld, 128) >= 4 * f->sms)
+                k_pivot<128><<<dim3(a, up(ld, 128)), 128, 0, s>>>(f->fr, perm, k0, buf, f->cpan, f->tpan, f->err,
+                                                                  f->minpiv, tol);
+            else
+                k_pivot<32><<<dim3(a, up(ld, 32)), 128, 0, s>>>(f->fr, perm, k0, buf, f->cpan, f->tpan, f->err,
+                                                                f->minpiv, tol);
+            const int ntc = (int)up(ld, TILE);
+            k_update<<<dim3(a, ntc * up(l.pmax, TILE)), 256, 0, s>>>(f->fr, perm, k0, ntc, f->cpan, f->tpan, buf);
+        }
+        if (l.qmax > 0 && l.pmax > 0) {
+            const int nt = (int)up(l.qmax, TILE);
+            k_schur<<<dim3(l.count, nt * nt), 256, 0, s>>>(f->fr, perm, nt, buf);
+        }
+    }
+    TCK(cudaGetLastError());
+    int herr = 0;
+    unsigned long long hmin = 0;
+    TCK(cudaMemcpyAsync(&herr, f->err, sizeof(int), cudaMemcpyDeviceToHost, s));
+    TCK(cudaMemcpyAsync(&hmin, f->minpiv, sizeof(hmin), cudaMemcpyDeviceToHost, s));
+    TCK(cudaStreamSynchronize(s));
+    if (min_pivot) std::memcpy(min_pivot, &hmin, sizeof(double));
+    if (herr) return tfail(f, VEFEM_ERR_SINGULAR, "a pivot below the tolerance (unpivoted elimination)");
+    return VEFEM_OK;
+}
+
+extern "C" int vefem_tree_solve(vefem_tree *f, const double *buf, const double *b, double *x, void *stream)
+{
+    if (!f || !buf || !b || !x) return VEFEM_ERR_ARG;
+    Guard g(f->device);
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (!f->graph || f->graph_buf != buf) {
+        if (f->graph) cudaGraphExecDestroy(f->graph);
+        f->graph = nullptr;
+        cudaGraph_t gr = nullptr;
+        TCK(cudaStreamBeginCapture(f->cs, cudaStreamCaptureModeThreadLocal));
+        const cudaError_t le = launch_sweeps(f, buf, f->cs);
+        const cudaError_t ce = cudaStreamEndCapture(f->cs, &gr);
+        cudaError_t e = le != cudaSuccess ? le : ce;
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&f->graph, gr, 0);
+        if (gr) cudaGraphDestroy(gr);
+        if (e != cudaSuccess) {
+            f->graph = nullptr;
+            cudaGetLastError();
+            return tfail(f, VEFEM_ERR_CUDA, std::string("solve graph: ") + cudaGetErrorString(e));
+        }
+        f->graph_buf = buf;
+    }
+    TCK(cudaMemcpyAsync(f->b, b, (size_t)f->N * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    TCK(cudaGraphLaunch(f->graph, s));
+    TCK(cudaMemcpyAsync(x, f->x, (size_t)f->N * sizeof(double), cudaMemcpyDeviceToDevice, s));
+    return VEFEM_OK;
+}
+
+extern "C" int vefem_tree_launches(const vefem_tree *f)
+{
+    if (!f) return -1;
+    int n = 0;
+    for (const Level &l : f->levels) n += 2 * (l.pmax > 0) + (l.qmax > 0);
+    return n;
+}
+
+extern "C" void vefem_tree_destroy(vefem_tree *f)
+{
+    if (!f) return;
+    {
+        Guard g(f->device);
+        if (f->graph) cudaGraphExecDestroy(f->graph);
+        if (f->cs) cudaStreamDestroy(f->cs);
+        void *p[] = {f->fr, f->perm, f->ids, f->src0, f->src1, f->cpan, f->tpan, f->y, f->b, f->x, f->err, f->minpiv};
+        for (void *q : p) cudaFree(q);
+    }
+    delete f;
+}
+
+extern "C" const char *vefem_tree_last_error(const vefem_tree *f) { return f ? f->msg.c_str() : "null tree handle"; }

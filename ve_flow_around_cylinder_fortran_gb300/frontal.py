@@ -1,25 +1,30 @@
-"""Panel-frontal LU of the bordered Newton Jacobian on the GPU (stand-in for
-the reference's MUMPS direct solve, ``KSPSolve`` in Petsc_mod.F90:850).
+"""Frontal LU of the bordered Newton Jacobian on the GPU (stand-in for the
+reference's MUMPS direct solve, ``KSPSolve`` in Petsc_mod.F90:850).
 
 The host SuperLU of ``linsolve.py`` needs ~32 s per factorisation of the
 20,000-quad Jacobian; this solver factorises the same matrix on the device in
-dense FP64 blocks.
-
-Symbolic phase (once per mesh and AIJ pattern).  Elements are swept
-downstream in order of their centroid x and grouped into panels of ``G``
-elements (by default about one element column of the channel).  A node is
-*fully summed* after the last panel that touches it; the *front* after panel
-q is the set of nodes touched by panels <= q and by a later panel.  Panel q's
-frontal matrix covers, in this order, its pivots P_q (the unknowns of the
-nodes fully summed at q) and the front F_q; the border unknowns (the
+dense FP64 fronts.  Each CSR entry (i, j) is added exactly once, to the front
+where the first of its two unknowns is eliminated; the border unknowns (the
 arclength lambda: a dense row and column) stay at the end of every front and
-are eliminated with the last panel's pivots, so a Jacobian that is singular
-at a fold (where the bordered matrix is not) never has to be factorised
-without its border.  Each CSR entry (i, j) is added exactly once, to the
-frontal matrix of panel min(last(i), last(j)); both ends are in that panel's
-pivots or front.
+are eliminated last, so a Jacobian that is singular at a fold (where the
+bordered matrix is not) never has to be factorised without its border.
 
-Numeric phase (every factorisation), for q = 0, 1, ...:
+Two orderings of the fronts:
+
+* Nested dissection (the default on a CUDA device): the fronts of a binary
+  tree of element sets (``dissection.py``), all fronts of one depth at a time
+  in the library's kernels (``csrc/vefem_tree.cu``).  63 G multiply-adds and
+  273 dependent steps for 20,000 quads.
+* Panels (``panel`` given, the pivoted method, the CPU): elements are swept
+  downstream in order of their centroid x and grouped into panels of ``G``
+  elements.  A node is *fully summed* after the last panel that touches it;
+  the *front* after panel q is the set of nodes touched by panels <= q and by a
+  later panel.  Panel q's frontal matrix covers, in this order, its pivots P_q
+  (the unknowns of the nodes fully summed at q) and the front F_q.  270 G
+  multiply-adds in 30,600 dependent steps for 20,000 quads
+  (``csrc/vefem_frontal.cu``).
+
+Numeric phase of the pivoted method, for panels q = 0, 1, ...:
 
     M_q  = original entries of panel q + extend-add of S_(q-1)
     LU_q = lu(M_q[P, P]) with partial pivoting            (cuSOLVER getrf)
@@ -30,19 +35,14 @@ A pivot the unpivoted elimination refuses (below 1e-12 of its 16 x 16 block)
 is met by delaying pressures: a pressure row couples to the velocities of
 its element-mates, and where those are all still in the front its entries
 inside the pivot block can cancel; the symbolic phase is then redone once
-with every pressure eliminated with the last panel that touches any of its
-element-mates (fronts ~1.3x, work ~1.55x), and the solver stays so.
+with every pressure eliminated no earlier than its element-mates, and the
+solver stays so; a matrix refused again goes to the pivoted method.
 
-Solve: forward y_P = LU_q^-1 b_P, b_F -= M_q[F, P] y_P; backward
-x_P = y_P - X_q x_F.  Each solve is checked against the CSR matrix (FP64
-SpMV) and refined (x += solve(b - A x)) up to ``refine`` times; a zero pivot
-or a solve that stays inaccurate hands the matrix to the host SuperLU
-(``linsolve.SparseLU``) for that factorisation.
-
-On the cylinder meshes the fronts are one node column of the channel plus the
-border (~500 unknowns on average at 20,000 quads, ~1,300 at most around the
-cylinder); a factorisation is ~0.9 TFLOP at 20,000 quads, 2.6 TFLOP at 40,000.
-Everything is FP64.
+Solve of the pivoted method: forward y_P = LU_q^-1 b_P, b_F -= M_q[F, P] y_P;
+backward x_P = y_P - X_q x_F.  Each solve is checked against the CSR matrix
+(FP64 SpMV) and refined (x += solve(b - A x)) up to ``refine`` times; a zero
+pivot or a solve that stays inaccurate hands the matrix to the host SuperLU
+(``linsolve.SparseLU``) for that factorisation.  Everything is FP64.
 """
 from __future__ import annotations
 
@@ -51,13 +51,16 @@ import warnings
 
 import numpy as np
 
+from . import dissection
+
 
 def default_panel(nel: int) -> int:
     """Elements per panel: about a quarter of an element column of the
     cylinder meshes (their channel is m elements high with nel ~ 20 m^2).
     Smaller panels mean smaller pivot blocks, hence less elimination work per
     unknown (the front, one node column, stays the same), but more steps;
-    a quarter column measured fastest on GB300 at 20,000 and 40,000 quads."""
+    a quarter column measured fastest of the panel sizes on GB300 at 20,000 and
+    40,000 quads."""
     return max(4, int(round(math.sqrt(nel / 20.0) / 4.0)))
 
 
@@ -104,11 +107,12 @@ class FrontalLU:
             raise ValueError("the native frontal elimination needs a CUDA device")
         self.method = method
         self.pivot_tol = pivot_tol
-        self.G = int(panel) if panel else default_panel(en.shape[0])
+        # nested dissection unless the caller asks for panels or for pivoting
+        self.tree = method == "native" and not panel
+        self.G = dissection.LEAF if self.tree else int(panel) if panel else default_panel(en.shape[0])
         self._handle = None
-        self._symbolic(en, mesh.xyz[0][en].mean(axis=1))
-        if method == "native":
-            self._create_native()
+        self._piv = None            # panel solver for a matrix the tree's pivots fail on
+        self._analyse(en)
         self.device_values = True   # factor() takes the AIJ values on the device
         self.fallbacks = 0          # factorisations handed to the host SuperLU
         self.pivoted_factorisations = 0   # native elimination refused a pivot
@@ -126,6 +130,87 @@ class FrontalLU:
         self._factors = None
 
     # ------------------------------------------------------------------ symbolic
+    def _analyse(self, en):
+        """Symbolic phase (mesh and pattern only) and the native handle."""
+        if self.tree:
+            self._symbolic_tree(en)
+            self._create_tree()
+            return
+        self._symbolic(en, self.mesh.xyz[0][en].mean(axis=1))
+        if self.method == "native":
+            self._create_native()
+
+    def _symbolic_tree(self, en):
+        torch, dev, N = self.torch, self.dev, self.N
+        t = dissection.Tree(en, self.mesh.xyz[:2][:, en].mean(axis=2), self.nn, self.neq, self.nb, self.G,
+                            self.p_field if self.delay_pressure else None)
+        self._t = t
+        self.npan, self.p_sz, self.n_sz, self.f_sz = t.nfront, t.p, t.n, t.n - t.p
+        self.idx_off = t.idx_off
+        self.ld = (t.n + 3) // 4 * 4         # rows start on 32-byte boundaries
+        self.off = np.concatenate([[0], np.cumsum(t.n * self.ld)])
+        # (front, unknown) -> position in the front
+        front = torch.repeat_interleave(torch.arange(t.nfront, device=dev), torch.from_numpy(t.n).to(dev))
+        ids = torch.from_numpy(t.ids).to(dev)
+        base = torch.from_numpy(t.idx_off).to(dev)
+        pos = torch.arange(len(ids), device=dev) - base[front]
+        keys, order = torch.sort(front * N + ids)
+        pos_sorted = pos[order]
+
+        def lookup(f, u):
+            k = f * N + u
+            i = torch.clamp(torch.searchsorted(keys, k), max=len(keys) - 1)
+            if not bool((keys[i] == k).all()):
+                raise RuntimeError("frontal symbolic phase: an entry outside its front")
+            return pos_sorted[i]
+
+        # each CSR entry goes to the deeper (larger heap id) of its unknowns' fronts
+        owner = torch.from_numpy(t.owner).to(dev)
+        front_of = torch.from_numpy(t.front_of).to(dev)
+        rp = torch.from_numpy(self.rowptr).to(dev)
+        ci = torch.from_numpy(self.colind.astype(np.int64)).to(dev)
+        rows = torch.repeat_interleave(torch.arange(N, device=dev), rp[1:] - rp[:-1])
+        q = front_of[torch.maximum(owner[rows], owner[ci])]
+        self.dest = lookup(q, rows)
+        self.dest *= torch.from_numpy(self.ld).to(dev)[q]
+        self.dest += lookup(q, ci)
+        self.dest += torch.from_numpy(self.off[:-1]).to(dev)[q]
+        del rows, q
+        # position in each child's front of every entry of a front (-1: not there)
+        heap = torch.from_numpy(t.heap).to(dev)
+        p = torch.from_numpy(t.p).to(dev)
+        up = torch.nonzero((pos >= p[front]) & (heap[front] > 1)).squeeze(1)
+        parent = front_of[heap[front[up]] >> 1]
+        at = base[parent] + lookup(parent, ids[up])
+        src = torch.full((2, len(ids)), -1, dtype=torch.int32, device=dev)
+        src[heap[front[up]] & 1, at] = pos[up].to(torch.int32)
+        self._src = src.cpu().numpy()
+        child = np.full((t.nfront, 2), -1, dtype=np.int32)
+        inner = t.heap < (1 << t.depth)
+        for s in range(2):
+            child[inner, s] = t.front_of[2 * t.heap[inner] + s]
+        self._child = child
+        self.buf = torch.empty(int(self.off[-1]), dtype=torch.float64, device=dev)
+        self.crow, self.col = rp, ci
+        pf, nf, ff = self.p_sz.astype(float), self.n_sz.astype(float), self.f_sz.astype(float)
+        self.flops = float((2.0 * (pf * pf * nf + pf * ff * ff)).sum())
+
+    def _create_tree(self):
+        import ctypes
+        from . import vefem as V
+        self._L = V.load()
+        t = self._t
+        lv = np.array([a for a, _ in t.levels] + [t.nfront], dtype=np.int32)
+        n, p, ld = (a.astype(np.int32) for a in (t.n, t.p, self.ld))
+        h = ctypes.c_void_p()
+        rc = self._L.vefem_tree_create(self.dev.index or 0, t.nfront, len(t.levels), lv.ctypes.data,
+                                       self.off.ctypes.data, n.ctypes.data, p.ctypes.data, ld.ctypes.data,
+                                       self._child.ctypes.data, t.ids.ctypes.data, t.idx_off.ctypes.data,
+                                       self._src.ctypes.data, self.N, ctypes.byref(h))
+        if rc != 0:
+            raise V.VefemError(f"vefem_tree_create failed ({rc})")
+        self._handle = h
+
     def _symbolic(self, en: np.ndarray, xcen: np.ndarray):
         torch, dev = self.torch, self.dev
         nel, nbf = en.shape
@@ -258,11 +343,18 @@ class FrontalLU:
         dependent launch, 2 plain stream order, -1 no solve yet."""
         if self._handle is None:
             return -1
+        if self.tree:
+            return 2 if self.mode == "native" else -1
         return int(self._L.vefem_frontal_solve_path(self._handle))
+
+    @property
+    def launches_per_solve(self):
+        """Kernel launches and device copies of one native solve."""
+        return 2 + (int(self._L.vefem_tree_launches(self._handle)) if self.tree else 2 * self.npan)
 
     def close(self):
         if self._handle is not None:
-            self._L.vefem_frontal_destroy(self._handle)
+            (self._L.vefem_tree_destroy if self.tree else self._L.vefem_frontal_destroy)(self._handle)
             self._handle = None
 
     def __del__(self):
@@ -300,9 +392,7 @@ class FrontalLU:
                 self.resymbolised = True
                 self.close()
                 self.buf = None
-                en = self.mesh.element_nodes()
-                self._symbolic(en, self.mesh.xyz[0][en].mean(axis=1))
-                self._create_native()
+                self._analyse(self.mesh.element_nodes())
                 if self._factor_native(v):
                     return self
         return self._factor_pivoted(v)
@@ -317,26 +407,48 @@ class FrontalLU:
         import ctypes
         from . import vefem as V
         torch = self.torch
-        self._scatter(v)
         mp = ctypes.c_double(0.0)
         stream = torch.cuda.current_stream(self.dev).cuda_stream
-        rc = self._L.vefem_frontal_factor(self._handle, self.buf.data_ptr(), stream,
-                                          self.pivot_tol, ctypes.byref(mp))
+        if self.tree:
+            rc = self._L.vefem_tree_factor(self._handle, v.data_ptr(), self.dest.data_ptr(), v.numel(),
+                                           self.buf.data_ptr(), self.buf.numel(), stream,
+                                           self.pivot_tol, ctypes.byref(mp))
+        else:
+            self._scatter(v)
+            rc = self._L.vefem_frontal_factor(self._handle, self.buf.data_ptr(), stream,
+                                              self.pivot_tol, ctypes.byref(mp))
         self.min_pivot = mp.value
         if rc == V.VEFEM_ERR_SINGULAR:
             self.pivoted_factorisations += 1
             return False
         if rc != 0:
-            raise V.VefemError("vefem_frontal_factor: " +
-                               self._L.vefem_frontal_last_error(self._handle).decode())
+            raise V.VefemError("frontal factorisation: " + self._native_error())
         self.mode = "native"
         return True
 
+    def _native_error(self):
+        err = self._L.vefem_tree_last_error if self.tree else self._L.vefem_frontal_last_error
+        return err(self._handle).decode()
+
     def _factor_pivoted(self, v):
+        self.mode = "pivoted"
+        if self.tree:                        # the panels' symbolic phase, built when first needed
+            if self._piv is None:
+                self._piv = FrontalLU(self.rowptr, self.colind, self.mesh, neq=self.neq, device=self.dev,
+                                      method="pivoted", p_field=self.p_field,
+                                      delay_pressure=self.delay_pressure)
+            bad = self._piv._eliminate_pivoted(v)
+        else:
+            bad = self._eliminate_pivoted(v)
+        if bad:
+            self._to_host()
+        return self
+
+    def _eliminate_pivoted(self, v) -> bool:
+        """Partial pivoting inside each panel's pivot block; True for a zero pivot."""
         torch = self.torch
         buf = self.buf
         self._scatter(v)
-        self.mode = "pivoted"
         facs, infos = [], []
         S = None
         for q in range(self.npan):
@@ -356,10 +468,7 @@ class FrontalLU:
             S = torch.addmm(M[p:, p:], M[p:, :p], X, beta=1.0, alpha=-1.0) if f else None
             facs.append((LU, piv, X, M[p:, :p] if f else None))
         self._factors = facs
-        bad = int(torch.stack(infos).max().item()) if infos else 0
-        if bad > 0:
-            self._to_host()
-        return self
+        return bool(infos) and int(torch.stack(infos).max().item()) > 0
 
     HOST_MAX_UNKNOWNS = 300_000
 
@@ -383,13 +492,18 @@ class FrontalLU:
             b = b.contiguous()
             x = torch.empty_like(b)
             stream = torch.cuda.current_stream(self.dev).cuda_stream
-            rc = self._L.vefem_frontal_solve(self._handle, self.buf.data_ptr(), b.data_ptr(),
-                                             x.data_ptr(), stream)
+            sweep = self._L.vefem_tree_solve if self.tree else self._L.vefem_frontal_solve
+            rc = sweep(self._handle, self.buf.data_ptr(), b.data_ptr(), x.data_ptr(), stream)
             if rc != 0:
                 from . import vefem as V
-                raise V.VefemError("vefem_frontal_solve: " +
-                                   self._L.vefem_frontal_last_error(self._handle).decode())
+                raise V.VefemError("frontal solve: " + self._native_error())
             return x
+        if self._piv is not None:
+            return self._piv._sweep_pivoted(b)
+        return self._sweep_pivoted(b)
+
+    def _sweep_pivoted(self, b):
+        torch = self.torch
         y = b.clone()
         ys = []
         for q, fac in enumerate(self._factors):

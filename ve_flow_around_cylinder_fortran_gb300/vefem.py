@@ -41,7 +41,9 @@ EXPORTED = ["vefem_abi_version", "vefem_create", "vefem_set_params", "vefem_asse
             "vefem_batch_last_timing", "vefem_batch_destroy", "vefem_batch_last_error",
             "vefem_stability_pattern", "vefem_stability_assemble",
             "vefem_frontal_create", "vefem_frontal_factor", "vefem_frontal_solve",
-            "vefem_frontal_destroy", "vefem_frontal_last_error", "vefem_frontal_solve_path"]
+            "vefem_frontal_destroy", "vefem_frontal_last_error", "vefem_frontal_solve_path",
+            "vefem_tree_create", "vefem_tree_factor", "vefem_tree_solve", "vefem_tree_launches",
+            "vefem_tree_destroy", "vefem_tree_last_error"]
 VEFEM_ERR_SINGULAR = 6
 BATCH_CLASSES = 6
 
@@ -125,6 +127,14 @@ def load(path: str = LIB_PATH):
     L.vefem_frontal_last_error.argtypes = [P]
     L.vefem_frontal_last_error.restype = ctypes.c_char_p
     L.vefem_frontal_solve_path.argtypes = [P]
+    L.vefem_tree_create.argtypes = [I, I, I, P, P, P, P, P, P, P, P, P, I64, ctypes.POINTER(P)]
+    L.vefem_tree_factor.argtypes = [P, P, P, I64, P, I64, P, ctypes.c_double, P]
+    L.vefem_tree_solve.argtypes = [P, P, P, P, P]
+    L.vefem_tree_launches.argtypes = [P]
+    L.vefem_tree_destroy.argtypes = [P]
+    L.vefem_tree_destroy.restype = None
+    L.vefem_tree_last_error.argtypes = [P]
+    L.vefem_tree_last_error.restype = ctypes.c_char_p
     _lib = L
     return L
 
