@@ -57,5 +57,7 @@ struct vefem_ctx {
     double *d_ses = nullptr, *d_tlb = nullptr, *d_kw = nullptr;
     double **d_Aptr = nullptr;
     double *d_Astage = nullptr, *d_Bstage = nullptr;
+    double *d_prec = nullptr, *d_pes = nullptr;   // planar base: Gauss-point records, pair outputs
+    int *d_nonplanar = nullptr;
     int stab_nk = 0, stab_nk_stage = 0;
 };

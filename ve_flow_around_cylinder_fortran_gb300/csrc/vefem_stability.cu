@@ -32,6 +32,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -598,6 +599,490 @@ __global__ void k_stability_gather(const GatherArgs g, const int64_t *__restrict
     }
 }
 
+// ---------------------------------------------------------------------------
+// Planar base states (W = Txz = Tyz = Tzz = 0, what updateStabilityArrays
+// embeds).  Most of the 10 x 10 x 33 x 3 coefficients above are then
+// structural zeros: in-plane and out-of-plane unknowns couple only through
+// the wavenumber, A's linear and quadratic parts in K and B act on values
+// only.  128 (equation, unknown) pairs are left of 400 for B and the three
+// coefficients A0, A1, A2 of A(K) = A0 + K A1 + K^2 A2.
+//
+// The general kernel is bound by the FP64 pipe (76% active) on 4.4 M
+// instructions per element: coefficients evaluated at 33 unit quantities and
+// three wavenumbers, 4 x 8100 outputs.  Here they are written down once per
+// Gauss point (k_planar_coef, a thread per point) and contracted pair by pair
+// (k_planar_contract: 0.24 M multiply-adds per element), and the scatter reads
+// 83 KB per element instead of 259.  20,000 quads, 16 wavenumbers and B:
+// 184.6 -> 18.6 ms.  The line between the routes is the check of the four
+// out-of-plane base fields (k_nonplanar, one pass over 2.6 MB): the pairs left
+// out are exact zeros for a planar base and for no other.
+
+constexpr int PL_NV = 17, PL_NS = 41, PL_NM = 70;        // pairs of velocity, stress/pressure, value type
+constexpr int PL_NP = PL_NV + PL_NS + PL_NM;             // 128
+// pairs that are nonzero without FENE (velocity, stress) and with Re = 0 besides (value type)
+constexpr int PL_NV0 = 15, PL_NS0 = 38, PL_NM0 = 46;
+// record of a Gauss point: coefficients [4 s][3 k][17], [3][3][41], [3 k][70],
+// each pair-fastest, then dphi/dx, dphi/dy and the Laplacian of the 9 nodes
+constexpr int PL_OS = 12 * PL_NV, PL_OM = PL_OS + 9 * PL_NS, PL_OG = PL_OM + 3 * PL_NM;
+constexpr int PL_REC = PL_OG + 27;                       // 810 doubles
+constexpr int PL_OUT = 81 * PL_NP;                       // outputs per element
+
+struct PlPair {
+    signed char m, e, f;    // matrix 0 B, 1 A0, 2 A1, 3 A2; equation; unknown
+};
+// Order of the pairs: those that need FENE (or Re, value type) come last.
+static const PlPair PL_PAIRS[PL_NP] = {
+    // velocity type, A0: u1, u2 in m1 m2 c 11 12 22; u3 in m3 13 23; FENE: u1, u2 in 33
+    {1, 0, 0}, {1, 1, 0}, {1, 3, 0}, {1, 4, 0}, {1, 5, 0}, {1, 6, 0},
+    {1, 0, 1}, {1, 1, 1}, {1, 3, 1}, {1, 4, 1}, {1, 5, 1}, {1, 6, 1},
+    {1, 2, 2}, {1, 7, 2}, {1, 8, 2}, {1, 9, 0}, {1, 9, 1},
+    // stress type, A0: p, s11, s12, s22 in m1 m2 c 11 12 22; s33 in m1 m2 11 12 22 33; s13, s23
+    // in m3 13 23; A1: u3 in m1, m2; FENE: s11, s12, s22 in 33
+    {1, 0, 3}, {1, 1, 3}, {1, 3, 3}, {1, 4, 3}, {1, 5, 3}, {1, 6, 3},
+    {1, 0, 4}, {1, 1, 4}, {1, 3, 4}, {1, 4, 4}, {1, 5, 4}, {1, 6, 4},
+    {1, 0, 5}, {1, 1, 5}, {1, 3, 5}, {1, 4, 5}, {1, 5, 5}, {1, 6, 5},
+    {1, 0, 6}, {1, 1, 6}, {1, 3, 6}, {1, 4, 6}, {1, 5, 6}, {1, 6, 6},
+    {1, 0, 9}, {1, 1, 9}, {1, 4, 9}, {1, 5, 9}, {1, 6, 9}, {1, 9, 9},
+    {1, 2, 7}, {1, 7, 7}, {1, 8, 7}, {1, 2, 8}, {1, 7, 8}, {1, 8, 8},
+    {2, 0, 2}, {2, 1, 2}, {1, 9, 4}, {1, 9, 5}, {1, 9, 6},
+    // value type: A1
+    {2, 0, 7}, {2, 1, 8}, {2, 2, 0}, {2, 2, 1}, {2, 2, 3}, {2, 2, 9}, {2, 3, 2}, {2, 3, 7}, {2, 3, 8},
+    {2, 4, 7}, {2, 4, 2}, {2, 5, 7}, {2, 5, 8}, {2, 5, 2}, {2, 6, 8}, {2, 6, 2}, {2, 9, 2},
+    {2, 7, 0}, {2, 7, 3}, {2, 7, 9}, {2, 8, 1}, {2, 8, 3}, {2, 8, 9},
+    // A2
+    {3, 0, 0}, {3, 1, 1}, {3, 2, 2}, {3, 3, 0}, {3, 3, 1}, {3, 4, 0}, {3, 5, 0}, {3, 5, 1}, {3, 6, 1},
+    {3, 7, 2}, {3, 8, 2},
+    // B
+    {0, 0, 4}, {0, 0, 5}, {0, 1, 5}, {0, 1, 6}, {0, 2, 7}, {0, 2, 8}, {0, 4, 4}, {0, 5, 5}, {0, 6, 6},
+    {0, 7, 7}, {0, 8, 8}, {0, 9, 9},
+    // B, Re only
+    {0, 0, 0}, {0, 1, 1}, {0, 2, 2}, {0, 3, 0}, {0, 3, 1}, {0, 4, 0}, {0, 5, 0}, {0, 5, 1}, {0, 6, 1},
+    {0, 7, 2}, {0, 8, 2},
+    // B, FENE only
+    {0, 0, 6}, {0, 0, 9}, {0, 1, 4}, {0, 1, 9}, {0, 4, 6}, {0, 4, 9}, {0, 5, 4}, {0, 5, 6}, {0, 5, 9},
+    {0, 6, 4}, {0, 6, 9}, {0, 9, 4}, {0, 9, 6}};
+
+// Values the coefficients of one unit quantity are made of.
+struct PlUnit {
+    double C11, C12, C22, C33;       // constitutive residual
+    double M1, M2;                   // momentum residual
+    double P11, P12, P22, div, conv1, conv2;
+};
+
+// flag = 1 when any base value lies out of the plane (a NaN counts)
+__global__ void k_nonplanar(int nnodes, const double *__restrict__ TLb, int *flag)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nnodes) return;
+    bool any = TLb[(size_t)2 * nnodes + i] != 0.0;
+    for (int f = 7; f < 10; f++) any |= TLb[(size_t)f * nnodes + i] != 0.0;
+    if (any) *flag = 1;
+}
+
+constexpr int PC_EL = 14, PC_THREADS = 128;   // 14 elements x 9 points: 126 of 128 lanes
+
+__global__ void __launch_bounds__(PC_THREADS)
+k_planar_coef(const StabArgs a, const KParams prm, double *__restrict__ rec)
+{
+    __shared__ double s_tlb[PC_EL][9 * ST_NEQ];
+    const int t = threadIdx.x, e0 = blockIdx.x * PC_EL;
+    for (int u = t; u < PC_EL * 9 * ST_NEQ; u += PC_THREADS) {
+        const int el = u / (9 * ST_NEQ), q = u % (9 * ST_NEQ);
+        if (e0 + el < a.nel)
+            s_tlb[el][q] = a.TLb[(size_t)(q % ST_NEQ) * a.nnodes + a.conn[(q / ST_NEQ) * a.nel + e0 + el]];
+    }
+    __syncthreads();
+    const int el = t / 9, gp = t % 9, e = e0 + el;
+    if (el >= PC_EL || e >= a.nel) return;
+    double *r = rec + ((size_t)e * 9 + gp) * PL_REC;
+    StabBase b;
+    {
+        double x[9], y[9], fx[9], fy[9], sx[9], sy[9];
+        for (int n = 0; n < 9; n++) {
+            const int gn = a.conn[n * a.nel + e];
+            x[n] = a.xy[gn];
+            y[n] = a.xy[a.nnodes + gn];
+        }
+        const auto go = geometry(s_bfn[gp], s_dfdc[gp], s_dfde[gp], s_d2c[gp], s_d2e[gp], s_d2ce[gp], s_w[gp], x, y,
+                                 fx, fy, sx, sy);
+        for (int n = 0; n < 9; n++) {
+            r[PL_OG + n] = fx[n];
+            r[PL_OG + 9 + n] = fy[n];
+            r[PL_OG + 18 + n] = sx[n] + sy[n];
+        }
+        stab_base(prm, s_tlb[el], fx, fy, sx, sy, go.H2, go.WET, gp, b);
+    }
+    const double W = b.WET, Wi = prm.WiN, be = prm.BvN, om = 1.0 - prm.BvN, Re = prm.ReN, Df = prm.DfN, VeN = prm.VeN;
+    const double z = a.kz ? 1.0 : 0.0;
+    const double U1 = b.U[0], U2 = b.U[1];
+    const double g11 = b.GU[0][0], g21 = b.GU[1][0], g12 = b.GU[0][1], g22 = b.GU[1][1];
+    const double S11 = b.S[0][0], S12 = b.S[0][1], S22 = b.S[1][1];
+    const double X11 = b.dT[0][0][0], X12 = b.dT[0][1][0], X22 = b.dT[1][1][0];
+    const double Y11 = b.dT[0][0][1], Y12 = b.dT[0][1][1], Y22 = b.dT[1][1][1];
+    const double f0 = b.f[0], f1 = b.f[1], f2 = b.f[2];
+    const double tm = b.tlsme, tc = b.tlsce, a1 = tm * Re * U1, a2 = tm * Re * U2;
+    const double b1 = tc * Wi * U1, b2 = tc * Wi * U2, to = tm * om;
+    const double md = b.tdcs / (2.0 * b.mag + 1.0e-12);   // tdcs x magnitude derivative per CE : CE'
+    const double c33 = -2.0 * om * f0;                    // CE'(3,3) per K u3
+    // f_T and what follows from it per unit trace of the stress perturbation
+    const bool fene = prm.model == FENE_CR || prm.model == FENE_P;
+    double cT = 0.0;
+    if (prm.model == L_PTT || prm.model == M_L_PTT) cT = VeN * Wi / om;
+    else if (prm.model == E_PTT || prm.model == M_E_PTT) cT = b.fT * VeN * Wi / om;
+    else if (prm.model == FENE_CR) cT = Wi / om / (VeN - 2.0);
+    else if (prm.model == FENE_P) cT = Wi / om / VeN;
+    const bool mod = prm.model == M_L_PTT || prm.model == M_E_PTT || prm.model == FENE_CR;
+    const double h0 = mod ? cT : 0.0;                     // f_0' per trace
+    double h1 = prm.model == GIESEKUS ? 0.0 : cT;         // f_1' per trace, trace_x, trace_y, u1, u2
+    double h1x = 0.0, h1y = 0.0, h1u = 0.0, h1v = 0.0;
+    double tI = 0.0, tIx = 0.0, tIy = 0.0, tIu = 0.0, tIv = 0.0, tIt = 0.0;
+    if (fene) {
+        const double kap = Wi / om / (prm.model == FENE_P ? VeN : VeN - 2.0);
+        const double d1 = kap * (X11 + X22), d2 = kap * (Y11 + Y22);      // grad f_T of the base
+        const double mv = -(cT / b.fT) * (U1 * d1 + U2 * d2);
+        h1 -= Wi * mv / b.fT;
+        h1x = -Wi * (U1 * kap) / b.fT;
+        h1y = -Wi * (U2 * kap) / b.fT;
+        h1u = -Wi * d1 / b.fT;
+        h1v = -Wi * d2 / b.fT;
+        if (prm.model == FENE_P) {
+            tI = mv / b.fT;
+            tIx = U1 * kap / b.fT;
+            tIy = U2 * kap / b.fT;
+            tIu = d1 / b.fT;
+            tIv = d2 / b.fT;
+            tIt = -om * cT / b.fT;
+        }
+    }
+    // coefficients of the in-plane equations for one unit quantity: component s
+    // of unknown f; dx, dy: the quantity is the x or y derivative of stress
+    // component dc (diffusion term)
+    auto emit = [&](int f, int s, const PlUnit &u, int dc, double dx, double dy) {
+        const double mg = md * (b.CE[0][0] * u.C11 + (b.CE[0][1] + b.CE[1][0]) * u.C12 + b.CE[1][1] * u.C22
+                                + b.CE[2][2] * u.C33);
+        auto put = [&](int e, double k0, double k1, double k2) {
+            double *d;
+            int np;
+            const int eq = e < 2 ? e : e - 1;                           // 0 1 3 4 5 6 -> 0..5
+            if (f < 2) {
+                d = r + s * 3 * PL_NV + (e == 9 ? 15 + f : f * 6 + eq);
+                np = PL_NV;
+            } else {
+                int at;
+                if (e == 9) at = f == 9 ? 29 : 38 + (f - 4);
+                else if (f == 9) at = 24 + (e < 2 ? e : e - 2);         // 0 1 4 5 6 -> 0..4
+                else at = (f - 3) * 6 + eq;
+                d = r + PL_OS + s * 3 * PL_NS + at;
+                np = PL_NS;
+            }
+            d[0] = W * k0;
+            d[np] = W * k1;
+            d[2 * np] = W * k2;
+        };
+        put(0, Re * u.conv1, u.P11 + a1 * u.M1 + b.tlsic * u.div - tc * u.C11, u.P12 + a2 * u.M1 - tc * u.C12);
+        put(1, Re * u.conv2, u.P12 + a1 * u.M2 - tc * u.C12, u.P22 + a2 * u.M2 + b.tlsic * u.div - tc * u.C22);
+        if (f != 9) put(3, u.div, tm * u.M1, tm * u.M2);
+        put(4, u.C11, (dc == 4 ? Df * dx : 0.0) - to * u.M1 + b1 * u.C11 + X11 * mg,
+            (dc == 4 ? Df * dy : 0.0) + b2 * u.C11 + Y11 * mg);
+        put(5, u.C12, (dc == 5 ? Df * dx : 0.0) - to * u.M2 + b1 * u.C12 + X12 * mg,
+            (dc == 5 ? Df * dy : 0.0) - to * u.M1 + b2 * u.C12 + Y12 * mg);
+        put(6, u.C22, (dc == 6 ? Df * dx : 0.0) + b1 * u.C22 + X22 * mg,
+            (dc == 6 ? Df * dy : 0.0) - to * u.M2 + b2 * u.C22 + Y22 * mg);
+        if (f != 3) put(9, u.C33, (dc == 9 ? Df * dx : 0.0) + b1 * u.C33, (dc == 9 ? Df * dy : 0.0) + b2 * u.C33);
+    };
+    {   // u1: value, x, y, Laplacian
+        PlUnit u = {Wi * X11 + h1u * S11 - om * tIu, Wi * X12 + h1u * S12, Wi * X22 + h1u * S22 - om * tIu, -om * tIu,
+                    Re * g11, Re * g12, 0.0, 0.0, 0.0, 0.0, g11, g12};
+        emit(0, 0, u, -1, 0.0, 0.0);
+        u = {-2.0 * (Wi * S11 + om * f0), -Wi * S12, 0.0, 0.0, Re * U1, 0.0, 2.0 * be, 0.0, 0.0, 1.0, U1, 0.0};
+        emit(0, 1, u, -1, 0.0, 0.0);
+        u = {-2.0 * Wi * S12, -Wi * S22 - om * f0, 0.0, 0.0, Re * U2, 0.0, 0.0, be, 0.0, 0.0, U2, 0.0};
+        emit(0, 2, u, -1, 0.0, 0.0);
+        u = {0.0, 0.0, 0.0, 0.0, -be, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        emit(0, 3, u, -1, 0.0, 0.0);
+        // u2
+        u = {Wi * Y11 + h1v * S11 - om * tIv, Wi * Y12 + h1v * S12, Wi * Y22 + h1v * S22 - om * tIv, -om * tIv,
+             Re * g21, Re * g22, 0.0, 0.0, 0.0, 0.0, g21, g22};
+        emit(1, 0, u, -1, 0.0, 0.0);
+        u = {0.0, -Wi * S11 - om * f0, -2.0 * Wi * S12, 0.0, 0.0, Re * U1, 0.0, be, 0.0, 0.0, 0.0, U1};
+        emit(1, 1, u, -1, 0.0, 0.0);
+        u = {0.0, -Wi * S12, -2.0 * (Wi * S22 + om * f0), 0.0, 0.0, Re * U2, 0.0, 0.0, 2.0 * be, 1.0, 0.0, U2};
+        emit(1, 2, u, -1, 0.0, 0.0);
+        u = {0.0, 0.0, 0.0, 0.0, 0.0, -be, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        emit(1, 3, u, -1, 0.0, 0.0);
+        // p
+        u = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, -1.0, 0.0, -1.0, 0.0, 0.0, 0.0};
+        emit(3, 0, u, -1, 0.0, 0.0);
+        u = {0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        emit(3, 1, u, -1, 0.0, 0.0);
+        u = {0.0, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        emit(3, 2, u, -1, 0.0, 0.0);
+        // stresses: the trace part of s11, s22, s33 first
+        const double t11 = h1 * S11 - om * (2.0 * h0 * g11 + tI), t12 = h1 * S12 - om * h0 * (g12 + g21);
+        const double t22 = h1 * S22 - om * (2.0 * h0 * g22 + tI), t33 = -om * tI;
+        u = {t11 - 2.0 * Wi * g11 + 2.0 * f2 * S11 + f1, t12 - Wi * g12 + f2 * S12, t22, t33, 0.0, 0.0, 1.0, 0.0, 0.0,
+             0.0, 0.0, 0.0};
+        emit(4, 0, u, -1, 0.0, 0.0);
+        u = {-2.0 * Wi * g21 + 2.0 * f2 * S12, -Wi * (g11 + g22) + f2 * (S11 + S22) + f1,
+             -2.0 * Wi * g12 + 2.0 * f2 * S12, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 0.0};
+        emit(5, 0, u, -1, 0.0, 0.0);
+        u = {t11, t12 - Wi * g21 + f2 * S12, t22 - 2.0 * Wi * g22 + 2.0 * f2 * S22 + f1, t33, 0.0, 0.0, 0.0, 0.0, 1.0,
+             0.0, 0.0, 0.0};
+        emit(6, 0, u, -1, 0.0, 0.0);
+        u = {t11, t12, t22, t33 + f1, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        emit(9, 0, u, -1, 0.0, 0.0);
+        // their x and y derivatives
+        for (int s = 1; s <= 2; s++) {
+            const double wu = Wi * (s == 1 ? U1 : U2), hx = s == 1 ? h1x : h1y, ix = om * (s == 1 ? tIx : tIy);
+            const double q11 = hx * S11 - ix, q12 = hx * S12, q22 = hx * S22 - ix;
+            const double dx = s == 1 ? 1.0 : 0.0, dy = 1.0 - dx;
+            u = {wu + q11, q12, q22, -ix, -dx, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            emit(4, s, u, 4, dx, dy);
+            u = {0.0, wu, 0.0, 0.0, -dy, -dx, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            emit(5, s, u, 5, dx, dy);
+            u = {q11, q12, wu + q22, -ix, 0.0, -dy, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            emit(6, s, u, 6, dx, dy);
+            u = {q11, q12, q22, wu - ix, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+            emit(9, s, u, 9, dx, dy);
+        }
+    }
+    // out-of-plane unknowns in A0: m3, 13, 23 per (C13, C23, M3, P13, P23, conv3)
+    auto emit3 = [&](double *d, int np, int stride, double C13, double C23, double M3, double P13, double P23,
+                     double conv3, double d13x, double d13y, double d23x, double d23y) {
+        const double k[3][3] = {{Re * conv3, P13 + a1 * M3 - tc * C13, P23 + a2 * M3 - tc * C23},
+                                {C13, Df * d13x - to * M3 + b1 * C13, Df * d13y + b2 * C13},
+                                {C23, Df * d23x + b1 * C23, Df * d23y - to * M3 + b2 * C23}};
+        for (int e = 0; e < 3; e++)
+            for (int c = 0; c < 3; c++) d[c * np + e * stride] = W * k[e][c];
+    };
+    {
+        double *v = r + 12;                              // u3
+        emit3(v, PL_NV, 1, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+        emit3(v + 3 * PL_NV, PL_NV, 1, -Wi * S11 - om * f0, -Wi * S12, Re * U1, be, 0.0, U1, 0.0, 0.0, 0.0, 0.0);
+        emit3(v + 6 * PL_NV, PL_NV, 1, -Wi * S12, -Wi * S22 - om * f0, Re * U2, 0.0, be, U2, 0.0, 0.0, 0.0, 0.0);
+        emit3(v + 9 * PL_NV, PL_NV, 1, 0.0, 0.0, -be, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+        double *q = r + PL_OS + 30;                      // s13, then s23
+        emit3(q, PL_NS, 1, -Wi * g11 + f2 * S11 + f1, -Wi * g12 + f2 * S12, 0.0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+        emit3(q + 3 * PL_NS, PL_NS, 1, Wi * U1, 0.0, -1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0);
+        emit3(q + 6 * PL_NS, PL_NS, 1, Wi * U2, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0);
+        q += 3;
+        emit3(q, PL_NS, 1, -Wi * g21 + f2 * S12, -Wi * g22 + f2 * S22 + f1, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 0.0, 0.0);
+        emit3(q + 3 * PL_NS, PL_NS, 1, 0.0, Wi * U1, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0, 0.0);
+        emit3(q + 6 * PL_NS, PL_NS, 1, 0.0, Wi * U2, -1.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 1.0);
+        // A1: u3 in m1 and m2 (its x or y derivative in the value term, its value in the gradient terms)
+        for (int i = 0; i < 2; i++) {
+            double *d = r + PL_OS + 36 + i;
+            for (int c = 0; c < 9; c++) d[c * PL_NS] = 0.0;
+            d[(1 + i) * 3 * PL_NS] = -W * be;
+            d[(1 + i) * PL_NS] = W * z * b.tlsic;
+        }
+    }
+    // value type
+    auto val = [&](int i, double k0, double k1, double k2) {
+        double *d = r + PL_OM + i;
+        d[0] = W * k0;
+        d[PL_NM] = W * k1;
+        d[2 * PL_NM] = W * k2;
+    };
+    const double mg3 = md * b.CE[2][2] * c33, of = om * f0;
+    val(0, -1.0, -z * a1, -z * a2);
+    val(1, -1.0, -z * a1, -z * a2);
+    val(2, 0.0, -z * (be + tc * of), 0.0);
+    val(3, 0.0, 0.0, -z * (be + tc * of));
+    val(4, -1.0, -z * a1, -z * a2);
+    val(5, 1.0, z * a1, z * a2);
+    val(6, z, 0.0, 0.0);
+    val(7, 0.0, -z * tm, 0.0);
+    val(8, 0.0, 0.0, -z * tm);
+    val(9, 0.0, z * to, 0.0);
+    val(10, 0.0, z * X11 * mg3, z * Y11 * mg3);
+    val(11, 0.0, 0.0, z * to);
+    val(12, 0.0, z * to, 0.0);
+    val(13, 0.0, z * X12 * mg3, z * Y12 * mg3);
+    val(14, 0.0, 0.0, z * to);
+    val(15, 0.0, z * X22 * mg3, z * Y22 * mg3);
+    val(16, z * c33, z * b1 * c33, z * b2 * c33);
+    val(17, z * of, z * b1 * of, z * b2 * of);
+    val(18, 0.0, z * to, 0.0);
+    val(19, 0.0, -z * to, 0.0);
+    val(20, z * of, z * b1 * of, z * b2 * of);
+    val(21, 0.0, 0.0, z * to);
+    val(22, 0.0, 0.0, -z * to);
+    const double zb = z * be, zt = -z * to * be;
+    val(23, zb, a1 * zb, a2 * zb);
+    val(24, zb, a1 * zb, a2 * zb);
+    val(25, 2.0 * zb, a1 * zb, a2 * zb);
+    val(26, 0.0, tm * zb, 0.0);
+    val(27, 0.0, 0.0, tm * zb);
+    val(28, 0.0, zt, 0.0);
+    val(29, 0.0, 0.0, zt);
+    val(30, 0.0, zt, 0.0);
+    val(31, 0.0, 0.0, zt);
+    val(32, 0.0, zt, 0.0);
+    val(33, 0.0, 0.0, zt);
+    // B (its sign: TERM_RES_b = -TERM_RES_b); w: the FENE part per trace
+    const double w0 = fene ? -Wi * cT / b.fT : 0.0;
+    const double w11 = w0 * S11 + tIt, w12 = w0 * S12, w22 = w0 * S22 + tIt;
+    auto mom = [&](int i, double c1, double c2) { val(i, 0.0, tc * c1, tc * c2); };
+    auto str = [&](int i, double c) { val(i, -c, -b1 * c, -b2 * c); };
+    mom(34, Wi + w11, w12);
+    mom(35, 0.0, Wi);
+    mom(36, Wi, 0.0);
+    mom(37, w12, Wi + w22);
+    mom(38, Wi, 0.0);
+    mom(39, 0.0, Wi);
+    str(40, Wi + w11);
+    str(41, Wi);
+    str(42, Wi + w22);
+    str(43, Wi);
+    str(44, Wi);
+    str(45, Wi + tIt);
+    val(46, -Re, -a1 * Re, -a2 * Re);
+    val(47, -Re, -a1 * Re, -a2 * Re);
+    val(48, -Re, -a1 * Re, -a2 * Re);
+    val(49, 0.0, -tm * Re, 0.0);
+    val(50, 0.0, 0.0, -tm * Re);
+    val(51, 0.0, to * Re, 0.0);
+    val(52, 0.0, 0.0, to * Re);
+    val(53, 0.0, to * Re, 0.0);
+    val(54, 0.0, 0.0, to * Re);
+    val(55, 0.0, to * Re, 0.0);
+    val(56, 0.0, 0.0, to * Re);
+    mom(57, w11, w12);
+    mom(58, w11, w12);
+    mom(59, w12, w22);
+    mom(60, w12, w22);
+    str(61, w11);
+    str(62, w11);
+    str(63, w12);
+    str(64, w12);
+    str(65, w12);
+    str(66, w22);
+    str(67, w22);
+    str(68, tIt);
+    str(69, tIt);
+}
+
+constexpr int PK_WARPS = 8;
+
+// One (test node, pair) of an element: 9 trial nodes, NS components
+template <int NS>
+__device__ __forceinline__ void planar_pair(const double *__restrict__ rec, const double *__restrict__ phi,
+                                            int off, int np, int pair, int i, double *__restrict__ out)
+{
+    double acc[9];
+#pragma unroll
+    for (int j = 0; j < 9; j++) acc[j] = 0.0;
+#pragma unroll 1
+    for (int gp = 0; gp < 9; gp++) {
+        const double *r = rec + gp * PL_REC, *d = r + off + pair, *g = r + PL_OG, *p = phi + gp * 9;
+        const double p0 = p[i], p1 = g[i], p2 = g[9 + i];
+        double c[NS];
+#pragma unroll
+        for (int s = 0; s < NS; s++)
+            c[s] = p0 * d[(3 * s) * np] + p1 * d[(3 * s + 1) * np] + p2 * d[(3 * s + 2) * np];
+#pragma unroll
+        for (int j = 0; j < 9; j++) {
+            acc[j] += c[0] * p[j];
+            if constexpr (NS > 1) acc[j] += c[1] * g[j];
+            if constexpr (NS > 2) acc[j] += c[2] * g[9 + j];
+            if constexpr (NS > 3) acc[j] += c[3] * g[18 + j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 9; j++) out[(size_t)(i * 9 + j) * PL_NP] = acc[j];
+}
+
+// A CTA per element: its records in shared memory, a lane per (test node,
+// pair), the lanes of a warp on one type.  40 multiply-adds per Gauss point and
+// lane against ~50 shared loads, most of them broadcasts: an FP64 instruction
+// holds the pipe for 16 clocks of the SM, so the loads hide.
+__global__ void __launch_bounds__(PK_WARPS * 32)
+k_planar_contract(const double *__restrict__ rec_all, double *__restrict__ es, int nv, int ns, int nm)
+{
+    extern __shared__ __align__(16) double rec[];
+    __shared__ double phi[81];
+    const double2 *src = reinterpret_cast<const double2 *>(rec_all + (size_t)blockIdx.x * 9 * PL_REC);
+    for (int u = threadIdx.x; u < 9 * PL_REC / 2; u += PK_WARPS * 32) reinterpret_cast<double2 *>(rec)[u] = src[u];
+    if (threadIdx.x < 81) phi[threadIdx.x] = s_bfn[threadIdx.x / 9][threadIdx.x % 9];
+    __syncthreads();
+    double *out = es + (size_t)blockIdx.x * PL_OUT;
+    const int lane = threadIdx.x & 31;
+    const int wv = (nv * 9 + 31) / 32, ws = (ns * 9 + 31) / 32, wm = (nm * 9 + 31) / 32;
+    for (int w = threadIdx.x >> 5; w < wv + ws + wm; w += PK_WARPS) {
+        if (w < wv) {
+            const int k = w * 32 + lane;
+            if (k < nv * 9) planar_pair<4>(rec, phi, 0, PL_NV, k % nv, k / nv, out + k % nv);
+        } else if (w < wv + ws) {
+            const int k = (w - wv) * 32 + lane;
+            if (k < ns * 9) planar_pair<3>(rec, phi, PL_OS, PL_NS, k % ns, k / ns, out + PL_NV + k % ns);
+        } else {
+            const int k = (w - wv - ws) * 32 + lane;
+            if (k < nm * 9) planar_pair<1>(rec, phi, PL_OM, PL_NM, k % nm, k / nm, out + PL_NV + PL_NS + k % nm);
+        }
+    }
+}
+
+struct PlMap {
+    signed char at[4][100];     // pair of (matrix, equation x unknown), -1: zero
+};
+
+constexpr int PG_THREADS = 256;
+
+// Scatter: the element-ordered sums of the pairs, then B and A(K) of every
+// wavenumber.  COVER (the stability pattern is exactly the node-pair blocks): a
+// CTA per row node walks its 10 rows in the order they are stored, so a warp
+// writes consecutive entries of every matrix; store leaves out reading them.
+template <bool COVER>
+__global__ void __launch_bounds__(PG_THREADS)
+k_planar_gather(const GatherArgs g, const PlMap map, const int64_t *__restrict__ rowptr10,
+                const int32_t *__restrict__ boff10, const double *__restrict__ es, int nk,
+                const double *__restrict__ kw, double *const *A, double *B, int store)
+{
+    __shared__ signed char s_at[4][100];
+    for (int u = threadIdx.x; u < 400; u += PG_THREADS) s_at[u / 100][u % 100] = map.at[u / 100][u % 100];
+    __syncthreads();
+    int64_t first = 0, count = 0, base = 0;
+    int wide = 0;
+    if (COVER) {
+        base = rowptr10[(int64_t)blockIdx.x * ST_NEQ];
+        count = rowptr10[(int64_t)(blockIdx.x + 1) * ST_NEQ] - base;
+        wide = (int)(count / ST_NEQ);
+    } else {
+        first = (int64_t)blockIdx.x * PG_THREADS;
+        count = min((int64_t)PG_THREADS, (int64_t)g.nblocks * 100 - first);
+    }
+    for (int64_t t = threadIdx.x; t < count; t += PG_THREADS) {
+        int blk, r;
+        int64_t slot;
+        if (COVER) {
+            const int jeq = (int)t / wide, c = (int)t - jeq * wide;
+            blk = (int)(base / 100) + c / ST_NEQ;
+            r = jeq * ST_NEQ + c % ST_NEQ;
+            slot = base + t;
+        } else {
+            blk = (int)((first + t) / 100);
+            r = (int)((first + t) % 100);
+            slot = rowptr10[(int64_t)g.brow[blk] * ST_NEQ + r / ST_NEQ] + boff10[blk] + r % ST_NEQ;
+        }
+        const int iB = s_at[0][r], i0 = s_at[1][r], i1 = s_at[2][r], i2 = s_at[3][r];
+        double sb = 0.0, s0 = 0.0, s1 = 0.0, s2 = 0.0;
+        const int c1 = g.bptr[blk + 1];
+        for (int c = g.bptr[blk]; c < c1; c++) {
+            const double *src = es + (size_t)g.bcon[c] * PL_NP;
+            if (iB >= 0) sb += src[iB];
+            if (i0 >= 0) s0 += src[i0];
+            if (i1 >= 0) s1 += src[i1];
+            if (i2 >= 0) s2 += src[i2];
+        }
+        if (B) B[slot] = store ? sb : B[slot] + sb;
+        for (int k = 0; k < nk; k++) {
+            const double K = kw[k], v = __fma_rn(K, __fma_rn(K, s2, s1), s0);
+            A[k][slot] = store ? v : A[k][slot] + v;
+        }
+    }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -708,8 +1193,8 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
     if (int rc = stab_pattern(ctx)) return rc;
     cudaStream_t s = ctx->stream;
     const int64_t N10 = (int64_t)ctx->nnodes * ST_NEQ, nnz10 = (int64_t)ctx->h_colind10.size();
-    if (!ctx->d_ses) {
-        SCK(cudaMalloc((void **)&ctx->d_ses, (size_t)ctx->nel * 4 * ST_BLK * sizeof(double)));
+    if (!ctx->d_nonplanar) SCK(cudaMalloc((void **)&ctx->d_nonplanar, sizeof(int)));
+    if (!ctx->d_tlb) {
         SCK(cudaMalloc((void **)&ctx->d_tlb, (size_t)N10 * sizeof(double)));
         GaussTables gt;
         gauss_tables_host(&gt);
@@ -744,7 +1229,16 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
         for (int k = 0; k < nk; k++) dA[k] = A[k];
         SCK(cudaMemcpyAsync(ctx->d_tlb, TLb, N10 * sizeof(double), cudaMemcpyDeviceToDevice, s));
     }
-    if (flags & VEFEM_ZERO_FIRST) {
+    // a base state in the plane takes the sparse kernels, any other the general one
+    int nonplanar = 0;
+    SCK(cudaMemsetAsync(ctx->d_nonplanar, 0, sizeof(int), s));
+    k_nonplanar<<<(ctx->nnodes + 255) / 256, 256, 0, s>>>(ctx->nnodes, ctx->d_tlb, ctx->d_nonplanar);
+    SCK(cudaGetLastError());
+    SCK(cudaMemcpyAsync(&nonplanar, ctx->d_nonplanar, sizeof(int), cudaMemcpyDeviceToHost, s));
+    SCK(cudaStreamSynchronize(s));
+    const bool cover = nnz10 == (int64_t)ctx->nblocks * 100;
+    const bool store = (flags & VEFEM_ZERO_FIRST) && !nonplanar && cover;   // every entry written, none read
+    if ((flags & VEFEM_ZERO_FIRST) && !store) {
         for (int k = 0; k < nk; k++) SCK(cudaMemsetAsync(dA[k], 0, nnz10 * sizeof(double), s));
         if (dB) SCK(cudaMemsetAsync(dB, 0, nnz10 * sizeof(double), s));
     }
@@ -760,21 +1254,8 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
     a.conn = ctx->d_conn;
     a.xy = ctx->d_xy;
     a.TLb = ctx->d_tlb;
-    a.es = ctx->d_ses;
+    a.es = nullptr;
     a.kz = (flags & VEFEM_STAB_AS_WRITTEN) ? 0 : 1;
-    const size_t smem = sizeof(double) * st_smem_doubles() + 9 * sizeof(StabBase);
-    SCK(cudaFuncSetAttribute(k_stability, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    int occ = 0;
-    SCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_stability, ST_THREADS, smem));
-    int sms = 0;
-    SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    const int grid = std::min<int>(ctx->nel, sms * std::max(1, occ));
-    ctx->launches = 0;
-    if (ctx->nel > 0) {
-        k_stability<<<grid, ST_THREADS, smem, s>>>(a, ctx->prm);
-        SCK(cudaGetLastError());
-        ctx->launches++;
-    }
     GatherArgs g;
     g.nnodes = ctx->nnodes;
     g.nblocks = ctx->nblocks;
@@ -786,12 +1267,55 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
     g.boff = ctx->d_boff;
     g.bptr = ctx->d_bptr;
     g.bcon = ctx->d_bcon;
+    ctx->launches = 1;
     const int64_t nthr = (int64_t)ctx->nblocks * 100;
-    if (nthr > 0) {
-        k_stability_gather<<<(unsigned)((nthr + 255) / 256), 256, 0, s>>>(
-            g, ctx->d_rowptr10, ctx->d_boff10, ctx->d_ses, nk, ctx->d_kw, ctx->d_Aptr, dB);
+    if (!nonplanar) {
+        const bool fene = ctx->prm.model == FENE_CR || ctx->prm.model == FENE_P;
+        const int nv = fene ? PL_NV : PL_NV0, ns = fene ? PL_NS : PL_NS0;
+        const int nm = fene || ctx->prm.ReN != 0.0 ? PL_NM : PL_NM0;
+        if (!ctx->d_prec) SCK(cudaMalloc((void **)&ctx->d_prec, (size_t)ctx->nel * 9 * PL_REC * sizeof(double)));
+        if (!ctx->d_pes) SCK(cudaMalloc((void **)&ctx->d_pes, (size_t)ctx->nel * PL_OUT * sizeof(double)));
+        PlMap map;
+        std::memset(map.at, -1, sizeof(map.at));
+        for (int q = 0; q < PL_NP; q++) {
+            const bool on = q < PL_NV ? q < nv : (q < PL_NV + PL_NS ? q - PL_NV < ns : q - PL_NV - PL_NS < nm);
+            if (on) map.at[PL_PAIRS[q].m][PL_PAIRS[q].e * 10 + PL_PAIRS[q].f] = (signed char)q;
+        }
+        k_planar_coef<<<(ctx->nel + PC_EL - 1) / PC_EL, PC_THREADS, 0, s>>>(a, ctx->prm, ctx->d_prec);
         SCK(cudaGetLastError());
-        ctx->launches++;
+        const int smem = 9 * PL_REC * (int)sizeof(double);
+        SCK(cudaFuncSetAttribute(k_planar_contract, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        k_planar_contract<<<ctx->nel, PK_WARPS * 32, smem, s>>>(ctx->d_prec, ctx->d_pes, nv, ns, nm);
+        SCK(cudaGetLastError());
+        if (cover)
+            k_planar_gather<true><<<ctx->nnodes, PG_THREADS, 0, s>>>(
+                g, map, ctx->d_rowptr10, ctx->d_boff10, ctx->d_pes, nk, ctx->d_kw, ctx->d_Aptr, dB, store);
+        else
+            k_planar_gather<false><<<(unsigned)((nthr + PG_THREADS - 1) / PG_THREADS), PG_THREADS, 0, s>>>(
+                g, map, ctx->d_rowptr10, ctx->d_boff10, ctx->d_pes, nk, ctx->d_kw, ctx->d_Aptr, dB, store);
+        SCK(cudaGetLastError());
+        ctx->launches += 3;
+    } else {
+        if (!ctx->d_ses) SCK(cudaMalloc((void **)&ctx->d_ses, (size_t)ctx->nel * 4 * ST_BLK * sizeof(double)));
+        a.es = ctx->d_ses;
+        const size_t smem = sizeof(double) * st_smem_doubles() + 9 * sizeof(StabBase);
+        SCK(cudaFuncSetAttribute(k_stability, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        int occ = 0;
+        SCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_stability, ST_THREADS, smem));
+        int sms = 0;
+        SCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
+        const int grid = std::min<int>(ctx->nel, sms * std::max(1, occ));
+        if (ctx->nel > 0) {
+            k_stability<<<grid, ST_THREADS, smem, s>>>(a, ctx->prm);
+            SCK(cudaGetLastError());
+            ctx->launches++;
+        }
+        if (nthr > 0) {
+            k_stability_gather<<<(unsigned)((nthr + 255) / 256), 256, 0, s>>>(
+                g, ctx->d_rowptr10, ctx->d_boff10, ctx->d_ses, nk, ctx->d_kw, ctx->d_Aptr, dB);
+            SCK(cudaGetLastError());
+            ctx->launches++;
+        }
     }
     if (!on_device) {
         for (int k = 0; k < nk; k++)
