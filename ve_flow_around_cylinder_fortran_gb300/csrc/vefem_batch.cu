@@ -347,6 +347,7 @@ extern "C" int vefem_batch_create(int ninst, const vefem_mesh *meshes, const vef
             I.ea.nnodes = c->nnodes;
             I.ea.conn = c->d_conn;
             I.ea.xy = c->d_xy;
+            I.ea.geo = c->d_geo;
             I.prm = c->prm;
             I.ga.nnodes = c->nnodes;
             I.ga.nblocks = c->nblocks;

@@ -429,6 +429,8 @@ extern "C" int vefem_create(const vefem_mesh *mesh, const vefem_csr *pat,
     }
 #undef UPL
     if ((ce = upload_tables(tab, s)) != cudaSuccess || (ce = upload_tables_exact(tab, s)) != cudaSuccess ||
+        (ce = cudaMalloc((void **)&ctx->d_geo, (size_t)nel * 9 * GEO_REC * sizeof(double))) != cudaSuccess ||
+        (ce = launch_geometry(nel, nn, ctx->d_conn, ctx->d_xy, ctx->d_geo, s)) != cudaSuccess ||
         (ce = cudaStreamSynchronize(s)) != cudaSuccess) {
         std::string m = std::string("tables: ") + cudaGetErrorString(ce);
         vefem_destroy(ctx);
@@ -552,6 +554,7 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     ea.nnodes = ctx->nnodes;
     ea.conn = ctx->d_conn;
     ea.xy = ctx->d_xy;
+    ea.geo = ctx->d_geo;
     ea.TL = dTL;
     ea.EU = dEU;
     ea.rs = ctx->d_rs;
@@ -749,7 +752,7 @@ extern "C" int vefem_destroy(vefem_ctx *ctx)
     if (!ctx) return VEFEM_OK;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    void *ptrs[] = {ctx->d_conn, ctx->d_xy, ctx->d_rowptr, ctx->d_nptr, ctx->d_ncon, ctx->d_brow,
+    void *ptrs[] = {ctx->d_conn, ctx->d_xy, ctx->d_geo, ctx->d_rowptr, ctx->d_nptr, ctx->d_ncon, ctx->d_brow,
                     ctx->d_boff, ctx->d_bptr, ctx->d_bcon, ctx->d_edge_elem, ctx->d_edge_id,
                     ctx->d_edge_row, ctx->d_edge_off, ctx->d_rs, ctx->d_es, ctx->d_as,
                     ctx->d_ers, ctx->d_ees, ctx->d_eas, ctx->d_TL, ctx->d_EU, ctx->d_b,

@@ -28,6 +28,7 @@ struct vefem_ctx {
     // device tables
     int32_t *d_conn = nullptr;
     double *d_xy = nullptr;
+    double *d_geo = nullptr;    // geometry table (launch_geometry), filled at create
     int64_t *d_rowptr = nullptr;
     int32_t *d_nptr = nullptr, *d_ncon = nullptr;
     int32_t *d_brow = nullptr, *d_boff = nullptr, *d_bptr = nullptr, *d_bcon = nullptr;

@@ -23,7 +23,8 @@
 //    take the full path).  Terms that are exact zeros for Re = 0 or DfN = 0
 //    are left out by template specialisation.
 //  * k_res64: residual only ('MNR'): one thread per (element, Gauss point),
-//    followed by an in-order sum over the Gauss points in shared memory.
+//    followed by an in-order sum over the Gauss points in shared memory;
+//    k_res64_wide: an element spread over a CTA, for small meshes.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -237,16 +238,24 @@ __global__ void __launch_bounds__(FD_THREADS) k_fd64(const ElemArgs a, const KPa
 
 // ---------------------------------------------------------------------------
 // Residual-only kernel: thread = (element, Gauss point)
-
-// residual kernel: one thread per (element, Gauss point), RES_EPB elements per
-// CTA (vefem_internal.h)
+//
+// A CTA of RES_EPB = 7 elements is 63 of 64 lanes; 8 elements (72 threads) left
+// 24 of 96 lanes idle, and an FP64 instruction holds the pipe for a whole warp
+// whatever its lanes do.  The geometry of the Gauss points comes from the
+// mesh's table (11% of the instructions, once per mesh instead of per call).
+// The 54 terms of a Gauss point go through shared memory three test nodes at a
+// time, which keeps a CTA at 31 KB, 6 or 7 of them per SM.  40,000 elements:
+// 2.43 ms -> RES_MS_AFTER.
 constexpr int RS_EPB = RES_EPB;
-constexpr int RS_THREADS = RS_EPB * 9;
-// 3 CTAs per SM requested: the compiler then keeps the SQRT form at 168
-// registers (a few spilled values) instead of 252, and 4 CTAs fit per SM;
-// measured 2.58 ms instead of 2.61 ms per 40,000 elements (the kernel is
-// bound by the FP64 pipe, not by latency)
-constexpr int RS_MIN_CTAS = 3;
+constexpr int RS_THREADS = 64;
+constexpr int RS_MIN_CTAS = 6;
+constexpr int RS_CHUNK = 3;                 // test nodes per pass through shared memory
+static_assert(RS_EPB * 9 <= RS_THREADS, "a thread per element and Gauss point");
+
+__device__ __forceinline__ double wi_of(const ElemArgs &a, const KParams &prm)
+{
+    return prm.nex > 0 ? prm.Wi0 * a.EU[prm.nex - 1] : prm.WiN;
+}
 
 // elements [e0, e0 + count) of one mesh, count <= RS_EPB; SPEC leaves out the
 // exact-zero terms of ReN = 0 / DfN = 0 as the FD kernel does (same values)
@@ -255,15 +264,16 @@ __device__ __forceinline__ void res64_block(const ElemArgs &a, const KParams &pr
                                             int count)
 {
     __shared__ double s_tl[RS_EPB][54];
-    __shared__ double s_part[RS_EPB][9][54];
+    __shared__ __align__(16) double s_geo[RS_EPB * 9 * GEO_REC];
+    __shared__ double s_bfn[9][9];
+    __shared__ double s_part[RS_EPB][9][RS_CHUNK * 6];
     const int t = threadIdx.x;
     const int el = t / 9;
     const int ig = t - el * 9;
-    const int e = e0 + el;
     const int e_end = min(e0 + count, a.nel);
-    const bool live = (t < RS_THREADS) && e < e_end;
-    // stage element states: 54 values per element, spread over the CTA
-    for (int i = t; i < RS_EPB * 54; i += blockDim.x) {
+    const bool live = t < RS_EPB * 9 && e0 + el < e_end;
+    // stage element states (54 values each, spread over the CTA) and geometry records
+    for (int i = t; i < RS_EPB * 54; i += RS_THREADS) {
         const int ee = e0 + i / 54;
         const int pos = i - (i / 54) * 54;
         if (ee < e_end) {
@@ -271,38 +281,40 @@ __device__ __forceinline__ void res64_block(const ElemArgs &a, const KParams &pr
             s_tl[i / 54][pos] = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + ee]];
         }
     }
+    const double2 *gsrc = reinterpret_cast<const double2 *>(a.geo + (size_t)e0 * 9 * GEO_REC);
+    const int ng = (e_end - e0) * 9 * GEO_REC / 2;
+    for (int i = t; i < ng; i += RS_THREADS) reinterpret_cast<double2 *>(s_geo)[i] = gsrc[i];
+    for (int i = t; i < 81; i += RS_THREADS) s_bfn[i / 9][i % 9] = c_bfn[i / 9][i % 9];
     __syncthreads();
+    const double *geo = s_geo + (live ? t : 0) * GEO_REC;
+    const double *dFx = geo, *dFy = geo + 9, *bfn = s_bfn[ig];
+    const double WET = geo[37];
+    double dotU[9];
+    GpCoef<double> g;
     if (live) {
-        double x[9], y[9], dFx[9], dFy[9], d2x[9], d2y[9];
-#pragma unroll
-        for (int n = 0; n < 9; n++) {
-            const int gn = a.conn[n * a.nel + e];
-            x[n] = a.xy[gn];
-            y[n] = a.xy[a.nnodes + gn];
-        }
-        auto go = geometry(c_bfn[ig], c_dfdc[ig], c_dfde[ig], c_d2fdc2[ig], c_d2fde2[ig],
-                             c_d2fdce[ig], c_w[ig], x, y, dFx, dFy, d2x, d2y);
-        double WiN = prm.WiN;
-        if (prm.nex > 0) WiN = prm.Wi0 * a.EU[prm.nex - 1];
         SmemView V{s_tl[el]};
-        auto I = interpolate(V, c_bfn[ig], dFx, dFy, d2x, d2y);
-        double dotU[9];
-        auto g = gauss_point<FORM, SPEC>(I, prm, WiN, go.H2, dFx, dFy, dotU);
-#pragma unroll
-        for (int n = 0; n < 9; n++)
-            test_node<FORM, SPEC>(g, prm, c_bfn[ig][n], dFx[n], dFy[n], dotU[n], go.WET,
-                                  &s_part[el][ig][n * 6]);
+        const auto I = interpolate(V, bfn, dFx, dFy, geo + 18, geo + 27);
+        g = gauss_point<FORM, SPEC>(I, prm, wi_of(a, prm), geo[36], dFx, dFy, dotU);
     }
-    __syncthreads();
-    // in-order sum over the Gauss points (Res = Res + TERM*WET, ig = 1..9)
-    for (int i = t; i < RS_EPB * 54; i += blockDim.x) {
-        const int le = i / 54, pos = i - (i / 54) * 54;
-        const int ee = e0 + le;
-        if (ee >= e_end) continue;
-        double s = 0.0;
 #pragma unroll
-        for (int q = 0; q < 9; q++) s = s + s_part[le][q][pos];
-        a.rs[(size_t)ee * 54 + pos] = s;
+    for (int n0 = 0; n0 < 9; n0 += RS_CHUNK) {
+        if (live) {
+#pragma unroll
+            for (int n = n0; n < n0 + RS_CHUNK; n++)
+                test_node<FORM, SPEC>(g, prm, bfn[n], dFx[n], dFy[n], dotU[n], WET,
+                                      &s_part[el][ig][(n - n0) * 6]);
+        }
+        __syncthreads();
+        // in-order sum over the Gauss points (Res = Res + TERM*WET, ig = 1..9)
+        for (int i = t; i < RS_EPB * RS_CHUNK * 6; i += RS_THREADS) {
+            const int le = i / (RS_CHUNK * 6), pos = i - le * (RS_CHUNK * 6);
+            if (e0 + le >= e_end) continue;
+            double s = 0.0;
+#pragma unroll
+            for (int q = 0; q < 9; q++) s = s + s_part[le][q][pos];
+            a.rs[(size_t)(e0 + le) * 54 + n0 * 6 + pos] = s;
+        }
+        __syncthreads();
     }
 }
 
@@ -310,6 +322,74 @@ template <int FORM, int SPEC>
 __global__ void __launch_bounds__(RS_THREADS, RS_MIN_CTAS) k_res64(const ElemArgs a, const KParams prm)
 {
     res64_block<FORM, SPEC>(a, prm, blockIdx.x * RS_EPB, RS_EPB);
+}
+
+// The same residual for a mesh that leaves the GPU short of warps: the time is
+// then one thread's chain of FP64 instructions, so E elements are spread over a
+// CTA: a thread per interpolated sum (22 at each Gauss point), per Gauss point,
+// and per (Gauss point, test node).  Every sum is the one of k_res64, in its
+// order.  The Gauss points' warp differs from CTA to CTA, so that the longest
+// phase of the CTAs of an SM spreads over its four FP64 pipes.
+template <int FORM, int SPEC, int E, int THREADS>
+__global__ void __launch_bounds__(THREADS, E == 1 ? 4 : 2) k_res64_wide(const ElemArgs a, const KParams prm)
+{
+    __shared__ double s_tl[E][54];
+    __shared__ __align__(16) double s_geo[E * 9 * GEO_REC];
+    __shared__ double s_bfn[9][9];
+    __shared__ double s_ip[E * 9][22];
+    __shared__ GpCoef<double> s_g[E * 9];
+    __shared__ double s_du[E * 9][9];
+    __shared__ double s_part[E * 9][54];
+    const int t = threadIdx.x, e0 = blockIdx.x * E, ne = min(E, a.nel - e0);
+    for (int i = t; i < ne * 54; i += THREADS) {
+        const int el = i / 54, pos = i - 54 * el, inod = pos / 6, f = pos - 6 * inod;
+        s_tl[el][pos] = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e0 + el]];
+    }
+    for (int i = t; i < ne * 9 * GEO_REC; i += THREADS) s_geo[i] = a.geo[(size_t)e0 * 9 * GEO_REC + i];
+    for (int i = t; i < 81; i += THREADS) s_bfn[i / 9][i % 9] = c_bfn[i / 9][i % 9];
+    __syncthreads();
+    // sums 0..4 and 5..9: u and v against phi, dphi/dx, dphi/dy, d2x, d2y;
+    // 10..21: p and the stresses against phi, dphi/dx, dphi/dy
+    for (int i = t; i < ne * 9 * 22; i += THREADS) {
+        const int gp = i / 22, q = i - 22 * gp;
+        const int f = q < 10 ? q / 5 : 2 + (q - 10) / 3, k = q < 10 ? q % 5 : (q - 10) % 3;
+        const double *w = k == 0 ? s_bfn[gp % 9] : s_geo + gp * GEO_REC + 9 * (k - 1);
+        double s = 0.0;
+#pragma unroll
+        for (int n = 0; n < 9; n++) s = s + s_tl[gp / 9][n * 6 + f] * w[n];
+        s_ip[gp][q] = s;
+    }
+    __syncthreads();
+    const int gp = t - 32 * (blockIdx.x % (THREADS / 32));
+    if (gp >= 0 && gp < ne * 9) {
+        const double *q = s_ip[gp], *geo = s_geo + gp * GEO_REC;
+        Interp<double> I;
+        I.U1 = q[0]; I.GU11 = q[1]; I.GU21 = q[2]; I.lap1 = q[3] + q[4];
+        I.U2 = q[5]; I.GU12 = q[6]; I.GU22 = q[7]; I.lap2 = q[8] + q[9];
+        I.P = q[10]; I.dPx = q[11]; I.dPy = q[12];
+        I.S11 = q[13]; I.dS11x = q[14]; I.dS11y = q[15];
+        I.S12 = q[16]; I.dS12x = q[17]; I.dS12y = q[18];
+        I.S22 = q[19]; I.dS22x = q[20]; I.dS22y = q[21];
+        double dotU[9];
+        s_g[gp] = gauss_point<FORM, SPEC>(I, prm, wi_of(a, prm), geo[36], geo, geo + 9, dotU);
+#pragma unroll
+        for (int n = 0; n < 9; n++) s_du[gp][n] = dotU[n];
+    }
+    __syncthreads();
+    for (int i = t; i < ne * 81; i += THREADS) {
+        const int ig = i / 9, n = i - 9 * ig;
+        const double *geo = s_geo + ig * GEO_REC;
+        test_node<FORM, SPEC>(s_g[ig], prm, s_bfn[ig % 9][n], geo[n], geo[9 + n], s_du[ig][n], geo[37],
+                              &s_part[ig][n * 6]);
+    }
+    __syncthreads();
+    for (int i = t; i < ne * 54; i += THREADS) {
+        const int el = i / 54, pos = i - 54 * el;
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < 9; q++) s = s + s_part[el * 9 + q][pos];
+        a.rs[(size_t)(e0 + el) * 54 + pos] = s;
+    }
 }
 
 // persistent form over the work items of many meshes
@@ -354,10 +434,58 @@ static int spec_of(const KParams &p)
 cudaError_t launch_residual64(const ElemArgs &a, const KParams &p, cudaStream_t s)
 {
     if (a.nel <= 0) return cudaSuccess;
+    if (a.nel <= RES_WIDE1_MAX) {
+#define GO(F, SP) k_res64_wide<F, SP, 1, 96><<<a.nel, 96, 0, s>>>(a, p)
+        RES_DISPATCH(p.form, spec_of(p), GO);
+#undef GO
+        return cudaGetLastError();
+    }
+    if (a.nel <= RES_WIDE3_MAX) {
+#define GO(F, SP) k_res64_wide<F, SP, 3, 256><<<(a.nel + 2) / 3, 256, 0, s>>>(a, p)
+        RES_DISPATCH(p.form, spec_of(p), GO);
+#undef GO
+        return cudaGetLastError();
+    }
     const int grid = (a.nel + RS_EPB - 1) / RS_EPB;
 #define GO(F, SP) k_res64<F, SP><<<grid, RS_THREADS, 0, s>>>(a, p)
     RES_DISPATCH(p.form, spec_of(p), GO);
 #undef GO
+    return cudaGetLastError();
+}
+
+// Geometry table of a mesh: per element and Gauss point dphi/dx, dphi/dy,
+// d2phi/dx2, d2phi/dy2 of the 9 nodes, H^2 and the weight
+__global__ void __launch_bounds__(128) k_geometry(int nel, int nnodes, const int32_t *__restrict__ conn,
+                                                  const double *__restrict__ xy, double *__restrict__ geo)
+{
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= (int64_t)nel * 9) return;
+    const int e = (int)(t / 9), ig = (int)(t - (int64_t)e * 9);
+    double x[9], y[9], dFx[9], dFy[9], d2x[9], d2y[9];
+#pragma unroll
+    for (int n = 0; n < 9; n++) {
+        const int gn = conn[n * nel + e];
+        x[n] = xy[gn];
+        y[n] = xy[nnodes + gn];
+    }
+    const auto go = geometry(c_bfn[ig], c_dfdc[ig], c_dfde[ig], c_d2fdc2[ig], c_d2fde2[ig], c_d2fdce[ig], c_w[ig],
+                             x, y, dFx, dFy, d2x, d2y);
+    double *r = geo + t * GEO_REC;
+#pragma unroll
+    for (int n = 0; n < 9; n++) {
+        r[n] = dFx[n];
+        r[9 + n] = dFy[n];
+        r[18 + n] = d2x[n];
+        r[27 + n] = d2y[n];
+    }
+    r[36] = go.H2;
+    r[37] = go.WET;
+}
+
+cudaError_t launch_geometry(int nel, int nnodes, const int32_t *conn, const double *xy, double *geo, cudaStream_t s)
+{
+    if (nel <= 0) return cudaSuccess;
+    k_geometry<<<(unsigned)(((int64_t)nel * 9 + 127) / 128), 128, 0, s>>>(nel, nnodes, conn, xy, geo);
     return cudaGetLastError();
 }
 

@@ -12,7 +12,15 @@ namespace vefem {
 enum { FORM_T = 0, FORM_SQRT = 1 };
 
 // FP64 residual kernel: elements per CTA and per batched work item
-constexpr int RES_EPB = 8;
+constexpr int RES_EPB = 7;
+// Meshes up to these sizes take the kernel that spreads 1 or 3 elements over a
+// CTA: as many as are resident at once on 152 SMs (4 CTAs of 1, 2 of 3).  SQRT
+// form, residual call on 300 / 500 / 600 / 900 quads: 46 / 60 / 60 / 98 us with
+// 1, 51 / 65 / 65 / 65 with 3, 98 throughout with k_res64; one wave more costs
+// 94 (1, 800 quads) and 96 us (3, 1,000).
+constexpr int RES_WIDE1_MAX = 4 * 152, RES_WIDE3_MAX = 6 * 152;
+// doubles per Gauss point of a mesh's geometry table
+constexpr int GEO_REC = 38;
 
 // Specialisations that leave out terms which are exact zeros for the given
 // parameters; a sum that drops an exact-zero addend keeps its value, so the
@@ -43,6 +51,7 @@ struct ElemArgs {
     int nel, nnodes;
     const int32_t *conn;   // [9][nel], 0-based
     const double *xy;      // [2][nnodes]
+    const double *geo;     // [nel][9][GEO_REC] geometry table
     const double *TL;      // [6][nnodes]
     const double *EU;      // [nex] (device)
     double *rs;            // residual scratch [(e*9 + jnod)*6 + jeq]
@@ -51,6 +60,8 @@ struct ElemArgs {
 };
 
 cudaError_t upload_tables(const GaussTables &t, cudaStream_t s);
+cudaError_t launch_geometry(int nel, int nnodes, const int32_t *conn, const double *xy, double *geo,
+                            cudaStream_t s);
 cudaError_t launch_residual64(const ElemArgs &a, const KParams &p, cudaStream_t s);
 cudaError_t launch_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s);
 

@@ -49,7 +49,10 @@ VF_HD R div_r(R x, R y, R r)
 #ifdef __CUDA_ARCH__
     if constexpr (std::is_same<R, double>::value) {
         const double q0 = x * r;
-        if (q0 == 0.0) return q0;                   // keeps the sign of a zero quotient
+        // A zero quotient keeps its sign.  The test is on the bits: an FP64
+        // comparison would be one more of the four instructions on the FP64
+        // pipe (2 lanes per clock and SM), integer ones run beside it.
+        if ((__double_as_longlong(q0) << 1) == 0) return q0;
         const double e = __fma_rn(-q0, y, x);
         return __fma_rn(e, r, q0);
     }
