@@ -139,8 +139,8 @@ struct vefem_batch {
     // descriptors and index spaces
     std::vector<BatchInst> h_inst;
     BatchInst *d_inst = nullptr;
-    WorkItem *d_res_work = nullptr, *d_ex_work = nullptr;
-    int n_res_work = 0, n_ex_work = 0;
+    WorkItem *d_res_work = nullptr, *d_ex_work[2] = {nullptr, nullptr};   // Jacobian: FP32, FP64
+    int n_res_work = 0, n_ex_work[2] = {0, 0};
     ScatterItem *d_sc_work = nullptr;
     int n_sc_work = 0;
     int64_t total_el = 0;
@@ -177,24 +177,37 @@ int bfail(vefem_batch *b, int code, const std::string &msg)
 
 int spec_of(const KParams &p) { return (p.ReN == 0.0 ? SPEC_RE0 : 0) | (p.DfN == 0.0 ? SPEC_DF0 : 0); }
 
+// a run of `tile` elements holds whole groups of the elements the Jacobian
+// kernel works on at a time: a smaller tile would leave its lanes idle
+int whole_tile(int tile, int elem_size)
+{
+    const int ne = exact_elements_at_a_time(elem_size);
+    return (tile + ne - 1) / ne * ne;
+}
+
 int build_work(vefem_batch *bt)
 {
-    std::vector<WorkItem> rw, xw;
+    std::vector<WorkItem> rw, xw[2];
     for (int i = 0; i < bt->ninst; i++) {
         const int nel = bt->ctx[i]->nel;
         for (int e0 = 0; e0 < nel; e0 += RES_EPB) rw.push_back({i, e0, std::min(RES_EPB, nel - e0), 0});
-        const int tile = bt->tiles[size_class(nel)];
-        for (int e0 = 0; e0 < nel; e0 += tile) xw.push_back({i, e0, std::min(tile, nel - e0), 0});
+        for (int k = 0; k < 2; k++) {
+            const int tile = whole_tile(bt->tiles[size_class(nel)], k == 0 ? 4 : 8);
+            for (int e0 = 0; e0 < nel; e0 += tile) xw[k].push_back({i, e0, std::min(tile, nel - e0), 0});
+        }
     }
     cudaFree(bt->d_res_work);
-    cudaFree(bt->d_ex_work);
-    bt->d_res_work = bt->d_ex_work = nullptr;
+    bt->d_res_work = nullptr;
     BCK(cudaMalloc(&bt->d_res_work, rw.size() * sizeof(WorkItem)));
-    BCK(cudaMalloc(&bt->d_ex_work, xw.size() * sizeof(WorkItem)));
     BCK(cudaMemcpy(bt->d_res_work, rw.data(), rw.size() * sizeof(WorkItem), cudaMemcpyHostToDevice));
-    BCK(cudaMemcpy(bt->d_ex_work, xw.data(), xw.size() * sizeof(WorkItem), cudaMemcpyHostToDevice));
     bt->n_res_work = (int)rw.size();
-    bt->n_ex_work = (int)xw.size();
+    for (int k = 0; k < 2; k++) {
+        cudaFree(bt->d_ex_work[k]);
+        bt->d_ex_work[k] = nullptr;
+        BCK(cudaMalloc(&bt->d_ex_work[k], xw[k].size() * sizeof(WorkItem)));
+        BCK(cudaMemcpy(bt->d_ex_work[k], xw[k].data(), xw[k].size() * sizeof(WorkItem), cudaMemcpyHostToDevice));
+        bt->n_ex_work[k] = (int)xw[k].size();
+    }
     if (!bt->d_sc_work) {
         std::vector<ScatterItem> sw;
         for (int i = 0; i < bt->ninst; i++) {
@@ -269,10 +282,10 @@ void launch_all(vefem_batch *bt, int flags, bool timing, cudaError_t *err)
         bt->launches++;
     }
     if (jmode && e == cudaSuccess) {
-        const int g = std::min(ex_grid, bt->n_ex_work);
-        e = f32 ? launch_exact_batched<float>(bt->d_inst, bt->d_ex_work, bt->n_ex_work, bt->form,
+        const int k = f32 ? 0 : 1, g = std::min(ex_grid, bt->n_ex_work[k]);
+        e = f32 ? launch_exact_batched<float>(bt->d_inst, bt->d_ex_work[0], bt->n_ex_work[0], bt->form,
                                               bt->spec, g, s)
-                : launch_exact_batched<double>(bt->d_inst, bt->d_ex_work, bt->n_ex_work, bt->form,
+                : launch_exact_batched<double>(bt->d_inst, bt->d_ex_work[1], bt->n_ex_work[1], bt->form,
                                                bt->spec, g, s);
         bt->launches++;
     }
@@ -590,12 +603,16 @@ extern "C" int vefem_batch_autotune(vefem_batch *bt, int flags, int reps, int *t
         for (int i = 0; i < bt->ninst; i++) present |= size_class(bt->ctx[i]->nel) == c;
         if (!present) continue;
         float best = 1e30f;
+        int tried = 0;
         for (int tile : EX_TILES) {
+            const int run = whole_tile(tile, (int)vsize);
+            if (run == tried) continue;      // the same work items as a smaller tile's
+            tried = run;
             std::vector<WorkItem> w;
             for (int i = 0; i < bt->ninst; i++) {
                 const int nel = bt->ctx[i]->nel;
                 if (size_class(nel) != c) continue;
-                for (int e0 = 0; e0 < nel; e0 += tile) w.push_back({i, e0, std::min(tile, nel - e0), 0});
+                for (int e0 = 0; e0 < nel; e0 += run) w.push_back({i, e0, std::min(run, nel - e0), 0});
             }
             WorkItem *dw = nullptr;
             BCK(cudaMalloc(&dw, w.size() * sizeof(WorkItem)));
@@ -636,8 +653,8 @@ extern "C" int vefem_batch_info(const vefem_batch *bt, int64_t out[6])
     if (!bt || !out) return VEFEM_ERR_ARG;
     out[0] = bt->ninst;
     out[1] = bt->total_el;
-    out[2] = bt->n_ex_work;
     const size_t vs = bt->es_elem ? bt->es_elem : sizeof(float);
+    out[2] = bt->n_ex_work[vs == sizeof(float) ? 0 : 1];
     out[3] = (int64_t)bt->sms * std::max(1, exact_batched_ctas_per_sm((int)vs, bt->form, bt->spec));
     out[4] = bt->launches;
     out[5] = bt->replays;
@@ -658,7 +675,7 @@ extern "C" int vefem_batch_destroy(vefem_batch *bt)
     if (bt->s) cudaStreamSynchronize(bt->s);
     if (bt->graph) cudaGraphExecDestroy(bt->graph);
     for (vefem_ctx *c : bt->ctx) vefem_destroy(c);
-    void *p[] = {bt->d_inst, bt->d_res_work, bt->d_ex_work, bt->d_sc_work,
+    void *p[] = {bt->d_inst, bt->d_res_work, bt->d_ex_work[0], bt->d_ex_work[1], bt->d_sc_work,
                  bt->d_rs, bt->d_es, bt->d_as};
     for (void *q : p)
         if (q) cudaFree(q);

@@ -582,11 +582,15 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
         if (jmode == VEFEM_JAC_EXACT64 || jac32) {
             if (!ctx->d_self) {
                 CK(cudaMalloc((void **)&ctx->d_self, sizeof(BatchInst)));
-                std::vector<WorkItem> w(nel);
-                for (int e = 0; e < (int)nel; e++) w[e] = {0, e, 1, 0};
-                CK(cudaMalloc((void **)&ctx->d_work, nel * sizeof(WorkItem)));
-                CK(cudaMemcpy(ctx->d_work, w.data(), nel * sizeof(WorkItem), cudaMemcpyHostToDevice));
                 CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
+            }
+            const int ne = exact_elements_at_a_time(jac32 ? 4 : 8), nwork = ((int)nel + ne - 1) / ne;
+            WorkItem *&d_work = ctx->d_work[jac32 ? 0 : 1];
+            if (!d_work) {
+                std::vector<WorkItem> w(nwork);
+                for (int i = 0; i < nwork; i++) w[i] = {0, i * ne, std::min(ne, (int)nel - i * ne), 0};
+                CK(cudaMalloc((void **)&d_work, nwork * sizeof(WorkItem)));
+                CK(cudaMemcpy(d_work, w.data(), nwork * sizeof(WorkItem), cudaMemcpyHostToDevice));
             }
             BatchInst &I = ctx->h_self;
             I.ea = ea;
@@ -596,11 +600,11 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
             CK(cudaMemcpyAsync(ctx->d_self, &I, sizeof(BatchInst), cudaMemcpyHostToDevice, s));
             const int spec = (ctx->prm.ReN == 0.0 ? SPEC_RE0 : 0) | (ctx->prm.DfN == 0.0 ? SPEC_DF0 : 0);
             const int occ = exact_batched_ctas_per_sm(jac32 ? 4 : 8, ctx->prm.form, spec);
-            const int grid = std::min<int>((int)nel, ctx->sms * std::max(1, occ));
+            const int grid = std::min(nwork, ctx->sms * std::max(1, occ));
             if (jac32)
-                CK(launch_exact_batched<float>(ctx->d_self, ctx->d_work, (int)nel, ctx->prm.form, spec, grid, s));
+                CK(launch_exact_batched<float>(ctx->d_self, d_work, nwork, ctx->prm.form, spec, grid, s));
             else
-                CK(launch_exact_batched<double>(ctx->d_self, ctx->d_work, (int)nel, ctx->prm.form, spec, grid, s));
+                CK(launch_exact_batched<double>(ctx->d_self, d_work, nwork, ctx->prm.form, spec, grid, s));
             ctx->launches++;
         }
         if (side) CK(cudaStreamWaitEvent(s, ctx->join, 0));
@@ -757,7 +761,7 @@ extern "C" int vefem_destroy(vefem_ctx *ctx)
                     ctx->d_edge_row, ctx->d_edge_off, ctx->d_rs, ctx->d_es, ctx->d_as,
                     ctx->d_ers, ctx->d_ees, ctx->d_eas, ctx->d_TL, ctx->d_EU, ctx->d_b,
                     ctx->d_vals, ctx->d_es32, ctx->d_as32, ctx->d_vals32, ctx->d_colind,
-                    ctx->d_self, ctx->d_work, ctx->d_rowptr10, ctx->d_boff10, ctx->d_ses,
+                    ctx->d_self, ctx->d_work[0], ctx->d_work[1], ctx->d_rowptr10, ctx->d_boff10, ctx->d_ses,
                     ctx->d_tlb, ctx->d_kw, ctx->d_Aptr, ctx->d_Astage, ctx->d_Bstage,
                     ctx->d_prec, ctx->d_pes, ctx->d_nonplanar};
     for (void *p : ptrs)

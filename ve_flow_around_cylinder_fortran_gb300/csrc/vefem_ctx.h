@@ -48,7 +48,7 @@ struct vefem_ctx {
     // for bit): its descriptor and one work item per element
     vefem::BatchInst h_self{};
     vefem::BatchInst *d_self = nullptr;
-    vefem::WorkItem *d_work = nullptr;
+    vefem::WorkItem *d_work[2] = {nullptr, nullptr};
     int sms = 0;
     // linear-stability assembly (10 unknowns per node): pattern and scratch
     std::vector<int64_t> h_rowptr10;
