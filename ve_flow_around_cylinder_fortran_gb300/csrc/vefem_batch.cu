@@ -25,6 +25,7 @@
 
 #include "vefem.h"
 #include "vefem_ctx.h"
+#include "vefem_gather.cuh"
 #include "vefem_internal.h"
 
 using namespace vefem;
@@ -41,8 +42,8 @@ struct ScatterItem {
     int count, pad;
 };
 constexpr int SC_RES_RUN = 2048;     // residual / arclength entries per item
-constexpr int SC_JAC_RUN = 64 * 36;  // Jacobian entries (64 node-pair blocks) per item
-constexpr int SC_THREADS = 256;
+constexpr int SC_JAC_RUN = 128;      // node-pair blocks per item
+constexpr int SC_THREADS = GB_THREADS;
 
 // One launch for the scatter of every instance: per item the instance's
 // tables, then the element-ordered sums of the single-mesh gathers
@@ -66,35 +67,23 @@ k_scatter_batched(const BatchInst *__restrict__ insts, const ScatterItem *__rest
             double *b = I.b;
             for (int64_t t = it.first + threadIdx.x; t < end; t += SC_THREADS) {
                 const int node = (int)(t / 6), jeq = (int)(t - (int64_t)node * 6);
-                double acc = store ? 0.0 : b[t];
-                const int c0 = g.nptr[node], c1 = g.nptr[node + 1];
-                for (int c = c0; c < c1; c++) acc = acc + rs[(int64_t)g.ncon[c] * 6 + jeq];
-                b[t] = acc;
+                b[t] = ordered_sum(store ? 0.0 : b[t], g.ncon, g.nptr[node], g.nptr[node + 1],
+                                   [&](int c) { return rs[(int64_t)c * 6 + jeq]; });
             }
         } else if (it.kind == SC_JAC) {
-            const T *es = static_cast<const T *>(I.es);
-            T *vals = static_cast<T *>(I.vals);
-            for (int64_t t = it.first + threadIdx.x; t < end; t += SC_THREADS) {
-                const int blk = (int)(t / 36);
-                const int r = (int)(t - (int64_t)blk * 36);
-                const int jeq = r / 6, ieq = r - 6 * (r / 6);
-                const int64_t slot = g.rowptr[(int64_t)g.brow[blk] * 6 + jeq] + g.boff[blk] + ieq;
-                T acc = store ? (T)0 : vals[slot];
-                const int c0 = g.bptr[blk], c1 = g.bptr[blk + 1];
-                for (int c = c0; c < c1; c++) acc = acc + es[(int64_t)g.bcon[c] * 36 + r];
-                vals[slot] = acc;
+            GatherArgs blocks = g;
+            blocks.store = store;
+            for (int p = threadIdx.x; p < it.count * GB_PAIRS; p += SC_THREADS) {
+                const int blk = p / GB_PAIRS;
+                gather_pair(blocks, (int)it.first + blk, p - blk * GB_PAIRS, static_cast<const T *>(I.es),
+                            static_cast<T *>(I.vals));
             }
         } else if (it.kind == SC_ARC) {
-            const T *as = static_cast<const T *>(I.as);
-            T *vals = static_cast<T *>(I.vals);
-            for (int64_t t = it.first + threadIdx.x; t < end; t += SC_THREADS) {
-                const int node = (int)(t / 6), jeq = (int)(t - (int64_t)node * 6);
-                const int64_t slot = g.rowptr[t + 1] - 1;
-                T acc = store ? (T)0 : vals[slot];
-                const int c0 = g.nptr[node], c1 = g.nptr[node + 1];
-                for (int c = c0; c < c1; c++) acc = acc + as[(int64_t)g.ncon[c] * 6 + jeq];
-                vals[slot] = acc;
-            }
+            GatherArgs rows = g;
+            rows.store = store;
+            for (int64_t t = it.first + threadIdx.x; t < end; t += SC_THREADS)
+                gather_arclength(rows, (int)(t / 6), (int)(t % 6), static_cast<const T *>(I.as),
+                                 static_cast<T *>(I.vals));
         } else {
             // the rows after the node unknowns: the lambda row of the values
             // (entries first .. end) and the lambda entries of b
@@ -212,11 +201,11 @@ int build_work(vefem_batch *bt)
         std::vector<ScatterItem> sw;
         for (int i = 0; i < bt->ninst; i++) {
             const vefem_ctx *c = bt->ctx[i];
-            const int64_t n6 = (int64_t)c->nnodes * 6, nj = (int64_t)c->nblocks * 36;
+            const int64_t n6 = (int64_t)c->nnodes * 6;
             for (int64_t f = 0; f < n6; f += SC_RES_RUN)
                 sw.push_back({i, SC_RES, f, (int)std::min<int64_t>(SC_RES_RUN, n6 - f), 0});
-            for (int64_t f = 0; f < nj; f += SC_JAC_RUN)
-                sw.push_back({i, SC_JAC, f, (int)std::min<int64_t>(SC_JAC_RUN, nj - f), 0});
+            for (int f = 0; f < c->nblocks; f += SC_JAC_RUN)
+                sw.push_back({i, SC_JAC, f, std::min(SC_JAC_RUN, c->nblocks - f), 0});
             if (c->nex) {
                 for (int64_t f = 0; f < n6; f += SC_RES_RUN)
                     sw.push_back({i, SC_ARC, f, (int)std::min<int64_t>(SC_RES_RUN, n6 - f), 0});
@@ -293,7 +282,7 @@ void launch_all(vefem_batch *bt, int flags, bool timing, cudaError_t *err)
     if (timing && e == cudaSuccess) e = cudaEventRecord(bt->ev[2], s);
     // scatter: one persistent launch over the scatter work list
     if (e == cudaSuccess) {
-        const int grid = std::min(bt->n_sc_work, bt->sms * 8);
+        const int grid = std::min(bt->n_sc_work, bt->sms * (2048 / SC_THREADS));
         if (f32)
             k_scatter_batched<float><<<grid, SC_THREADS, 0, s>>>(bt->d_inst, bt->d_sc_work, bt->n_sc_work,
                                                                 want_res, jmode != 0, store);
@@ -372,6 +361,7 @@ extern "C" int vefem_batch_create(int ninst, const vefem_mesh *meshes, const vef
             I.ga.boff = c->d_boff;
             I.ga.bptr = c->d_bptr;
             I.ga.bcon = c->d_bcon;
+            I.ga.brec = c->d_brec;
         }
         return build_work(bt);
     };

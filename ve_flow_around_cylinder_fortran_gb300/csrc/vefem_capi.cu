@@ -431,6 +431,9 @@ extern "C" int vefem_create(const vefem_mesh *mesh, const vefem_csr *pat,
     if ((ce = upload_tables(tab, s)) != cudaSuccess || (ce = upload_tables_exact(tab, s)) != cudaSuccess ||
         (ce = cudaMalloc((void **)&ctx->d_geo, (size_t)nel * 9 * GEO_REC * sizeof(double))) != cudaSuccess ||
         (ce = launch_geometry(nel, nn, ctx->d_conn, ctx->d_xy, ctx->d_geo, s)) != cudaSuccess ||
+        (ce = cudaMalloc((void **)&ctx->d_brec, (size_t)nblocks * sizeof(BlockRec))) != cudaSuccess ||
+        (ce = launch_block_records(nblocks, ctx->d_brow, ctx->d_boff, ctx->d_bptr, ctx->d_bcon, ctx->d_brec, s)) !=
+            cudaSuccess ||
         (ce = cudaStreamSynchronize(s)) != cudaSuccess) {
         std::string m = std::string("tables: ") + cudaGetErrorString(ce);
         vefem_destroy(ctx);
@@ -622,6 +625,7 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     ga.boff = ctx->d_boff;
     ga.bptr = ctx->d_bptr;
     ga.bcon = ctx->d_bcon;
+    ga.brec = ctx->d_brec;
     ga.store = zero_first ? 1 : 0;
     if (want_res) {
         CK(launch_gather_residual(ga, ctx->d_rs, db, s));
@@ -629,21 +633,12 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     }
     if (timing) CK(cudaEventRecord(ctx->ev[3], s));
     ga.store = zero_first && ctx->blocks_cover ? 1 : 0;
-    if (want_jac && !jac32) {
-        CK(launch_gather_jacobian(ga, ctx->d_es, dvals, s));
-        ctx->launches++;
-        if (ctx->nex) {
-            CK(launch_gather_arclength(ga, ctx->d_as, dvals, s));
-            ctx->launches++;
-        }
-    }
-    if (jac32) {
-        CK(launch_gather_jacobian32(ga, ctx->d_es32, dvals32, s));
-        ctx->launches++;
-        if (ctx->nex) {
-            CK(launch_gather_arclength32(ga, ctx->d_as32, dvals32, s));
-            ctx->launches++;
-        }
+    if (want_jac) {
+        if (jac32)
+            CK(launch_gather_rows<float>(ga, ctx->d_es32, ctx->d_as32, dvals32, s));
+        else
+            CK(launch_gather_rows<double>(ga, ctx->d_es, ctx->d_as, dvals, s));
+        ctx->launches += ctx->nex ? 2 : 1;
     }
     if (timing) CK(cudaEventRecord(ctx->ev[4], s));
     if (edges) {
@@ -757,7 +752,7 @@ extern "C" int vefem_destroy(vefem_ctx *ctx)
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     void *ptrs[] = {ctx->d_conn, ctx->d_xy, ctx->d_geo, ctx->d_rowptr, ctx->d_nptr, ctx->d_ncon, ctx->d_brow,
-                    ctx->d_boff, ctx->d_bptr, ctx->d_bcon, ctx->d_edge_elem, ctx->d_edge_id,
+                    ctx->d_boff, ctx->d_bptr, ctx->d_bcon, ctx->d_brec, ctx->d_edge_elem, ctx->d_edge_id,
                     ctx->d_edge_row, ctx->d_edge_off, ctx->d_rs, ctx->d_es, ctx->d_as,
                     ctx->d_ers, ctx->d_ees, ctx->d_eas, ctx->d_TL, ctx->d_EU, ctx->d_b,
                     ctx->d_vals, ctx->d_es32, ctx->d_as32, ctx->d_vals32, ctx->d_colind,

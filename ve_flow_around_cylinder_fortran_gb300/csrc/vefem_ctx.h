@@ -32,6 +32,7 @@ struct vefem_ctx {
     int64_t *d_rowptr = nullptr;
     int32_t *d_nptr = nullptr, *d_ncon = nullptr;
     int32_t *d_brow = nullptr, *d_boff = nullptr, *d_bptr = nullptr, *d_bcon = nullptr;
+    vefem::BlockRec *d_brec = nullptr;          // launch_block_records, filled at create
     int32_t *d_edge_elem = nullptr, *d_edge_id = nullptr;
     int32_t *d_edge_row = nullptr, *d_edge_off = nullptr;   // [nedge][81]
     int32_t *d_colind = nullptr;                            // for MatZeroRows on the device

@@ -602,50 +602,4 @@ template cudaError_t launch_exact_batched<float>(const BatchInst *, const WorkIt
 template cudaError_t launch_exact_batched<double>(const BatchInst *, const WorkItem *, int, int,
                                                   int, int, cudaStream_t);
 
-
-// FP32 scatter of the exact Jacobian (element order, as the FP64 one)
-__global__ void k_gather_jacobian32(const GatherArgs g, const float *__restrict__ es,
-                                    float *__restrict__ vals)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)g.nblocks * 36) return;
-    const int blk = (int)(t / 36);
-    const int r = (int)(t - (int64_t)blk * 36);
-    const int jeq = r / 6, ieq = r - 6 * (r / 6);
-    const int64_t slot = g.rowptr[(int64_t)g.brow[blk] * 6 + jeq] + g.boff[blk] + ieq;
-    const float acc0 = g.store ? 0.0f : vals[slot];
-    vals[slot] = ordered_sum(acc0, g.bcon, g.bptr[blk], g.bptr[blk + 1],
-                             [&](int c) { return es[(int64_t)c * 36 + r]; });
-}
-
-__global__ void k_gather_arclength32(const GatherArgs g, const float *__restrict__ as,
-                                     float *__restrict__ vals)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)g.nnodes * 6) return;
-    const int node = (int)(t / 6), jeq = (int)(t - (int64_t)node * 6);
-    const int64_t slot = g.rowptr[t + 1] - 1;
-    const float acc0 = g.store ? 0.0f : vals[slot];
-    vals[slot] = ordered_sum(acc0, g.ncon, g.nptr[node], g.nptr[node + 1],
-                             [&](int c) { return as[(int64_t)c * 6 + jeq]; });
-}
-
-cudaError_t launch_gather_jacobian32(const GatherArgs &g, const float *es, float *vals,
-                                     cudaStream_t s)
-{
-    const int64_t n = (int64_t)g.nblocks * 36;
-    if (n == 0) return cudaSuccess;
-    k_gather_jacobian32<<<(unsigned)((n + 287) / 288), 288, 0, s>>>(g, es, vals);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gather_arclength32(const GatherArgs &g, const float *as, float *vals,
-                                      cudaStream_t s)
-{
-    const int64_t n = (int64_t)g.nnodes * 6;
-    if (n == 0 || g.nex == 0) return cudaSuccess;
-    k_gather_arclength32<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(g, as, vals);
-    return cudaGetLastError();
-}
-
 }  // namespace vefem

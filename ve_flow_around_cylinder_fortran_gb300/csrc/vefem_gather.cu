@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "vefem_gather.cuh"
 #include "vefem_internal.h"
 
 namespace vefem {
@@ -28,32 +29,47 @@ __global__ void k_gather_residual(const GatherArgs g, const double *__restrict__
                        [&](int c) { return rs[(int64_t)c * 6 + jeq]; });
 }
 
-// one thread per (node-pair block, jeq, ieq)
-__global__ void k_gather_jacobian(const GatherArgs g, const double *__restrict__ es,
-                                  double *__restrict__ vals)
+// two entries of a node-pair block per thread (vefem_gather.cuh)
+template <class T>
+__global__ void __launch_bounds__(GB_THREADS)
+k_gather_blocks(const GatherArgs g, const T *__restrict__ es, T *__restrict__ vals)
 {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)g.nblocks * 36) return;
-    const int blk = (int)(t / 36);
-    const int r = (int)(t - (int64_t)blk * 36);
-    const int jeq = r / 6, ieq = r - 6 * (r / 6);
-    const int64_t slot = g.rowptr[(int64_t)g.brow[blk] * 6 + jeq] + g.boff[blk] + ieq;
-    const double acc0 = g.store ? 0.0 : vals[slot];
-    vals[slot] = ordered_sum(acc0, g.bcon, g.bptr[blk], g.bptr[blk + 1],
-                             [&](int c) { return es[(int64_t)c * 36 + r]; });
+    const int64_t t = (int64_t)blockIdx.x * GB_THREADS + threadIdx.x;
+    if (t >= (int64_t)g.nblocks * GB_PAIRS) return;
+    const int blk = (int)(t / GB_PAIRS);
+    gather_pair(g, blk, (int)(t - (int64_t)blk * GB_PAIRS), es, vals);
 }
 
 // arclength column: the last entry of every node row (column N - 1)
-__global__ void k_gather_arclength(const GatherArgs g, const double *__restrict__ as,
-                                   double *__restrict__ vals)
+template <class T>
+__global__ void k_gather_arclength(const GatherArgs g, const T *__restrict__ as, T *__restrict__ vals)
 {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)g.nnodes * 6) return;
-    const int node = (int)(t / 6), jeq = (int)(t - (int64_t)node * 6);
-    const int64_t slot = g.rowptr[t + 1] - 1;
-    const double acc0 = g.store ? 0.0 : vals[slot];
-    vals[slot] = ordered_sum(acc0, g.ncon, g.nptr[node], g.nptr[node + 1],
-                             [&](int c) { return as[(int64_t)c * 6 + jeq]; });
+    if (t < (int64_t)g.nnodes * 6) gather_arclength(g, (int)(t / 6), (int)(t % 6), as, vals);
+}
+
+__global__ void k_block_records(int nblocks, const int32_t *__restrict__ brow, const int32_t *__restrict__ boff,
+                                const int32_t *__restrict__ bptr, const int32_t *__restrict__ bcon,
+                                BlockRec *__restrict__ rec)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nblocks) return;
+    BlockRec r;
+    r.row = brow[i];
+    r.off = boff[i];
+    r.c0 = bptr[i];
+    r.n = bptr[i + 1] - r.c0;
+#pragma unroll
+    for (int k = 0; k < ORDERED_PREFETCH; k++) r.id[k] = k < r.n ? bcon[r.c0 + k] : 0;
+    rec[i] = r;
+}
+
+cudaError_t launch_block_records(int nblocks, const int32_t *brow, const int32_t *boff, const int32_t *bptr,
+                                 const int32_t *bcon, BlockRec *rec, cudaStream_t s)
+{
+    if (nblocks <= 0) return cudaSuccess;
+    k_block_records<<<(nblocks + 255) / 256, 256, 0, s>>>(nblocks, brow, boff, bptr, bcon, rec);
+    return cudaGetLastError();
 }
 
 // Dirichlet rows: b = TL - value, and the AIJ row zeroed with 1 on the diagonal
@@ -103,22 +119,18 @@ cudaError_t launch_gather_residual(const GatherArgs &g, const double *rs, double
     return cudaGetLastError();
 }
 
-cudaError_t launch_gather_jacobian(const GatherArgs &g, const double *es, double *vals,
-                                   cudaStream_t s)
+template <class T>
+cudaError_t launch_gather_rows(const GatherArgs &g, const T *es, const T *as, T *vals, cudaStream_t s)
 {
-    const int64_t n = (int64_t)g.nblocks * 36;
-    if (n == 0) return cudaSuccess;
-    k_gather_jacobian<<<grid_for(n, 288), 288, 0, s>>>(g, es, vals);
+    const int64_t n = (int64_t)g.nblocks * GB_PAIRS;
+    if (n > 0) k_gather_blocks<T><<<grid_for(n, GB_THREADS), GB_THREADS, 0, s>>>(g, es, vals);
+    if (g.nex > 0 && g.nnodes > 0)
+        k_gather_arclength<T><<<grid_for((int64_t)g.nnodes * 6, 256), 256, 0, s>>>(g, as, vals);
     return cudaGetLastError();
 }
 
-cudaError_t launch_gather_arclength(const GatherArgs &g, const double *as, double *vals,
-                                    cudaStream_t s)
-{
-    const int64_t n = (int64_t)g.nnodes * 6;
-    if (n == 0 || g.nex == 0) return cudaSuccess;
-    k_gather_arclength<<<grid_for(n, 256), 256, 0, s>>>(g, as, vals);
-    return cudaGetLastError();
-}
+template cudaError_t launch_gather_rows<double>(const GatherArgs &, const double *, const double *, double *,
+                                                cudaStream_t);
+template cudaError_t launch_gather_rows<float>(const GatherArgs &, const float *, const float *, float *, cudaStream_t);
 
 }  // namespace vefem

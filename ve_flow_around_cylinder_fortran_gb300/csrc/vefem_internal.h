@@ -78,6 +78,13 @@ struct EdgeArgs {
 };
 cudaError_t launch_edge64(const EdgeArgs &a, const KParams &p, int want_jac, cudaStream_t s);
 
+// What the scatter needs of a node-pair block, in one 32-byte load.
+struct __attribute__((aligned(16))) BlockRec {
+    int32_t row, off;          // row node, column offset of the block inside its rows
+    int32_t c0, n;             // its contributors bcon[c0 .. c0 + n)
+    int32_t id[4];             // the first of them
+};
+
 // Deterministic element-ordered scatter (pull form).
 struct GatherArgs {
     int nnodes;
@@ -90,6 +97,7 @@ struct GatherArgs {
     const int32_t *boff;       // [nblocks] column offset of the block inside its rows
     const int32_t *bptr;       // [nblocks+1]
     const int32_t *bcon;       // contributor = e*81 + jnod*9 + inod, element order
+    const BlockRec *brec;      // [nblocks]
     int store = 0;             // 1: the sums start from zero (VEFEM_ZERO_FIRST), the
                                // destination is written without being read
 };
@@ -119,19 +127,15 @@ __device__ __forceinline__ T ordered_sum(T acc, const int32_t *__restrict__ con,
 
 cudaError_t launch_gather_residual(const GatherArgs &g, const double *rs, double *b,
                                    cudaStream_t s);
-cudaError_t launch_gather_jacobian(const GatherArgs &g, const double *es, double *vals,
-                                   cudaStream_t s);
-cudaError_t launch_gather_arclength(const GatherArgs &g, const double *as, double *vals,
-                                    cudaStream_t s);
+// AIJ values of the node rows (blocks and, with nex, the arclength column)
+template <class T>
+cudaError_t launch_gather_rows(const GatherArgs &g, const T *es, const T *as, T *vals, cudaStream_t s);
+cudaError_t launch_block_records(int nblocks, const int32_t *brow, const int32_t *boff, const int32_t *bptr,
+                                 const int32_t *bcon, BlockRec *rec, cudaStream_t s);
 
 // Exact-Jacobian kernels (vefem_exact.cu): element Jacobian and arclength column in T,
 // launched through launch_exact_batched (declared below with the batched form).
 cudaError_t upload_tables_exact(const GaussTables &t, cudaStream_t s);
-cudaError_t launch_gather_jacobian32(const GatherArgs &g, const float *es, float *vals,
-                                     cudaStream_t s);
-cudaError_t launch_gather_arclength32(const GatherArgs &g, const float *as, float *vals,
-                                      cudaStream_t s);
-
 cudaError_t launch_dirichlet(int nrows, int nnodes, const int64_t *rows, const double *values,
                              const double *TL, double *b, const int64_t *rowptr,
                              const int32_t *colind, void *vals, int vals_float, cudaStream_t s);

@@ -1267,6 +1267,7 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
     g.boff = ctx->d_boff;
     g.bptr = ctx->d_bptr;
     g.bcon = ctx->d_bcon;
+    g.brec = ctx->d_brec;
     ctx->launches = 1;
     const int64_t nthr = (int64_t)ctx->nblocks * 100;
     if (!nonplanar) {
