@@ -38,7 +38,7 @@ def nvcc() -> str:
 
 def _flags(src: str = ""):
     fmad = "-fmad=true" if src in FMAD_ON else "-fmad=false"
-    return ARCH + ["-O3", "-lineinfo", "-std=c++17", fmad, "-Xcompiler", "-fPIC",
+    return ARCH + ["-split-compile=0", "-O3", "-lineinfo", "-std=c++17", fmad, "-Xcompiler", "-fPIC",
                    "-Xcompiler", "-ffp-contract=off", "-I", INCLUDE, "-I", CSRC]
 
 

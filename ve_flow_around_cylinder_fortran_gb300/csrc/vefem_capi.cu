@@ -564,8 +564,9 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     ea.es = ctx->d_es;
     ea.as = ctx->d_as;
     if (jmode == VEFEM_JAC_FD64) {
+        CK(launch_residual64(ea, ctx->prm, s));    // the columns' base residual
         CK(launch_fd64(ea, ctx->prm, s));
-        ctx->launches++;
+        ctx->launches += 2;
     } else {
         // The FP64 residual and an exact Jacobian are independent until the
         // scatter: the residual runs on a second stream, so the FP64 pipe works
@@ -638,7 +639,7 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
             CK(launch_gather_rows<float>(ga, ctx->d_es32, ctx->d_as32, dvals32, s));
         else
             CK(launch_gather_rows<double>(ga, ctx->d_es, ctx->d_as, dvals, s));
-        ctx->launches += ctx->nex ? 2 : 1;
+        ctx->launches++;
     }
     if (timing) CK(cudaEventRecord(ctx->ev[4], s));
     if (edges) {

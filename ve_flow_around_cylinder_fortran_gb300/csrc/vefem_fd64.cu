@@ -11,17 +11,10 @@
 //
 // Kernel layout (GB300: FP64 is the scarce unit, so the work is arranged to
 // spend FP64 operations only on what the algorithm needs):
-//  * k_fd64: one CTA = 4 elements x 56 threads; thread (element, k) evaluates
-//    residual number k of storeBulk (Equations_mod.F90:264-306): k = 0 the
-//    base residual, k = 1..54 the column (inod, ieq) = divmod(k-1, 6), k = 55
-//    the arclength column.  The element state each evaluation sees (with the
-//    (x+eps)-eps restore residue of the earlier columns) is staged once per
-//    element in shared memory; state-independent geometry (basis2D) and the
-//    interpolants of the unperturbed state are computed once per element and
-//    Gauss point, so an evaluation recomputes only its perturbed field's
-//    sums (the same sums in the same order; elements with a restore residue
-//    take the full path).  Terms that are exact zeros for Re = 0 or DfN = 0
-//    are left out by template specialisation.
+//  * k_fd64: a thread per column of storeBulk's forward difference
+//    (Equations_mod.F90:264-306), CTAs by the field that the columns perturb;
+//    the base residual is k_res64's.  Terms that are exact zeros for Re = 0 or
+//    DfN = 0 are left out by template specialisation.
 //  * k_res64: residual only ('MNR'): one thread per (element, Gauss point),
 //    followed by an in-order sum over the Gauss points in shared memory;
 //    k_res64_wide: an element spread over a CTA, for small meshes.
@@ -76,22 +69,14 @@ cudaError_t upload_tables(const GaussTables &t, cudaStream_t s)
 // ---------------------------------------------------------------------------
 // FD kernel
 
+__device__ __forceinline__ double wi_of(const ElemArgs &a, const KParams &prm)
+{
+    return prm.nex > 0 ? prm.Wi0 * a.EU[prm.nex - 1] : prm.WiN;
+}
+
 struct SmemView {
     const double *p;
     __device__ __forceinline__ double operator()(int pos) const { return p[pos]; }
-};
-
-constexpr int FD_EPB = 4;        // elements per CTA
-constexpr int FD_NEV = 56;       // evaluations per element (base + 54 + arclength)
-constexpr int FD_THREADS = FD_EPB * FD_NEV;
-
-struct FdSmem {
-    double tl[FD_EPB][3][54];    // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
-    double dFx[FD_EPB][9][9], dFy[FD_EPB][9][9], d2x[FD_EPB][9][9], d2y[FD_EPB][9][9];
-    double H2[FD_EPB][9], WET[FD_EPB][9];
-    Interp<double> base[FD_EPB][9];   // interpolants of the original state per Gauss point
-    double res0[FD_EPB][54];
-    int residue[FD_EPB];         // 1 if some (x+eps)-eps differs from x in the element
 };
 
 // the state evaluation k sees: positions before kk are restored, kk is perturbed
@@ -105,7 +90,140 @@ struct FdView {
     }
 };
 
-// the same state when no restore residue exists: original except position kk
+// Forward-difference columns by perturbed field.
+//
+// Column (inod, ieq) of storeBulk perturbs one unknown, and only part of the
+// physics sees its field: the velocity columns keep what the stresses alone
+// give (StressPart, TestStress: 22% of a test node's operations, 40% of a Gauss
+// point's), the pressure columns everything but P and the momentum residual
+// (45 of 154 operations at a test node), the stress columns what the velocity
+// alone gives.  The kept values are computed once per element, from the same
+// expressions in the same order, and every term, product and sum that follows
+// is the reference's: the columns' bits are those of 54 full evaluations.  A
+// CTA takes one kind of column of a run of elements:
+//   27 stress columns and the arclength column x 9 elements  (252 of 256 threads)
+//   18 velocity columns                        x 14 elements (252)
+//    9 pressure columns                        x 28 elements (252)
+// so that every lane of a warp runs the same code; 28 + 18 + 9 CTAs cover the
+// same 252 elements, next to each other in the grid, so their parts of an
+// element's rows meet in L2.  Small meshes take 64-thread CTAs (2, 3, 7 elements;
+// 56, 54, 63 lanes), which spread over more SMs.  The base residual is k_res64's (launched before).
+// An element with a restore residue ((x + eps) - eps differs from x, so later
+// columns see a changed state) is left to the last kind of CTA, which
+// evaluates it in full.
+//
+// Bound: the FP64 pipe.  Eight full warps per SM at 255 registers instead of
+// seven; the columns' operations are 78% of full evaluations'.  Residual and
+// Jacobian, SQRT form: 81.3 -> 63.6 ms on 40,000 quads, 4.95 -> 3.72 on 2,000;
+// T form 50.9 -> 40.8 on 40,000.
+constexpr int FS_COLS = 28, FU_COLS = 18, FP_COLS = 9;
+
+// Elements per CTA by kind (stress, velocity, pressure, residue check)
+template <int THREADS> struct FdRun;
+template <> struct FdRun<256> { static constexpr int S = 9, U = 14, P = 28, R = 64; };
+template <> struct FdRun<64> { static constexpr int S = 2, U = 3, P = 7, R = 16; };
+constexpr int FD_RUN = 252;       // elements of a group of 256-thread CTAs
+
+template <int EL>
+struct FdStressSmem {
+    double tl[EL][2][54];        // 0: original, 1: perturbed x + eps
+    Interp<double> base[EL][9];
+    FlowPart<double> flow[EL][9];
+    double dotU[EL][9][9];
+    int residue[EL];
+};
+
+template <int FORM, int EL>
+struct FdFlowSmem {
+    double tl[EL][2][54];
+    Interp<double> base[EL][9];
+    StressPart<double> stress[EL][9];
+    double test[EL][9][9][FORM == FORM_SQRT ? 11 : 3];       // TestStress (T form: grad S . grad phi only)
+    int residue[EL];
+};
+
+template <int EL>
+struct FdPressureSmem {
+    double tl[EL][54];
+    double pert[EL][9];
+    GpCoef<double> g[EL][9];
+    double keep[EL][9][6];       // stress + BvN G without p, div T, BvN Laplacian
+    TestPressure<double> test[EL][9];                         // of the current Gauss point
+    int residue[EL];
+};
+
+template <int THREADS>
+struct FdResidueSmem {
+    double tl[THREADS / 64][3][54];   // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
+    int list[FdRun<THREADS>::R], n;
+};
+
+template <int FORM, int THREADS>
+union FdSmem {
+    FdStressSmem<FdRun<THREADS>::S> s;
+    FdFlowSmem<FORM, FdRun<THREADS>::U> u;
+    FdPressureSmem<FdRun<THREADS>::P> p;
+    FdResidueSmem<THREADS> r;
+};
+
+// x / y with r the rounded reciprocal of y: div_r's steps, infinities and NaN
+// passed through (the quotient is the difference of two residuals over eps)
+__device__ __forceinline__ double div_by(double x, double y, double r)
+{
+    const double q0 = x * r;
+    const unsigned hi = (unsigned)__double2hiint(q0) & 0x7fffffffu;
+    if (hi >= 0x7ff00000u || (hi | (unsigned)__double2loint(q0)) == 0u) return q0;
+    const double e = __fma_rn(-q0, y, x);
+    return __fma_rn(e, r, q0);
+}
+
+// Programmatic dependent launch: the residual kernels let the FD kernel start
+// beside them, which waits for the residual only where it takes differences.
+__device__ __forceinline__ void pdl_launch_dependents()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// column `inod, ieq` of the element (ieq 6: the arclength column)
+__device__ __forceinline__ void store_column(const ElemArgs &a, const KParams &prm, int e, int inod, int ieq,
+                                             const double (&res)[54])
+{
+    pdl_wait();
+    const double *res0 = a.rs + (size_t)e * 54;
+    const double eps = prm.eps;
+    const bool plain = !(eps > 1.0e-300 && eps < 1.0e300);
+    const double r = plain ? 0.0 : recip_for_div(eps);
+    double *dst = ieq == 6 ? a.as + (size_t)e * 54 : a.es + (size_t)e * 2916 + inod * 36 + ieq;
+    const int sn = ieq == 6 ? 6 : 324, se = ieq == 6 ? 1 : 6;
+#pragma unroll
+    for (int jnod = 0; jnod < 9; jnod++)
+#pragma unroll
+        for (int jeq = 0; jeq < 6; jeq++) {
+            const double d = res[jnod * 6 + jeq] - res0[jnod * 6 + jeq];
+            dst[jnod * sn + jeq * se] = plain ? d / eps : div_by(d, eps, r);
+        }
+}
+
+// stage the states of elements e0 .. e0 + ne, and mark those with a restore residue
+template <int EL, int THREADS>
+__device__ __forceinline__ void stage_states(const ElemArgs &a, const KParams &prm, int e0, int ne,
+                                             double (*tl)[2][54], int *residue)
+{
+    for (int i = threadIdx.x; i < EL; i += THREADS) residue[i] = 0;
+    __syncthreads();
+    for (int i = threadIdx.x; i < ne * 54; i += THREADS) {
+        const int el = i / 54, pos = i - 54 * el, inod = pos / 6, f = pos - 6 * inod;
+        const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e0 + el]];
+        const double vp = v + prm.eps, back = vp - prm.eps;
+        tl[el][0][pos] = v;
+        tl[el][1][pos] = vp;
+        if (__double_as_longlong(back) != __double_as_longlong(v)) residue[el] = 1;
+    }
+    __syncthreads();
+}
+
+// the state of a column: original except position kk
 struct FdCleanView {
     const double *orig, *pert;
     int kk;
@@ -115,125 +233,334 @@ struct FdCleanView {
     }
 };
 
-template <int FORM, int SPEC>
-__global__ void __launch_bounds__(FD_THREADS) k_fd64(const ElemArgs a, const KParams prm)
+// value and gradient of field f of the perturbed state (interpolate's sums)
+__device__ __forceinline__ void perturbed(const FdCleanView &V, int f, const double *bfn, const double *dFx,
+                                          const double *dFy, double &val, double &gx, double &gy)
 {
-    __shared__ FdSmem sm;
-    const int t = threadIdx.x;
-    const int el = t / FD_NEV;
-    const int k = t - el * FD_NEV;
-    const int e = blockIdx.x * FD_EPB + el;
-    const bool live = e < a.nel;
-    const double eps = prm.eps;
-
-    // stage the element state and geometry
-    if (live && k < 54) {
-        const int inod = k / 6, f = k - inod * 6;
-        const int gn = a.conn[inod * a.nel + e];
-        const double v = a.TL[(size_t)f * a.nnodes + gn];
-        const double vp = v + eps;
-        sm.tl[el][0][k] = v;
-        sm.tl[el][2][k] = vp;
-        sm.tl[el][1][k] = vp - eps;
-    }
-    if (live && k >= 54 - 9 && k < 54) {
-        // nine threads per element: the nine Gauss points' geometry
-        const int ig = k - 45;
-        double x[9], y[9];
+    val = 0.0;
+    gx = 0.0;
+    gy = 0.0;
 #pragma unroll
-        for (int n = 0; n < 9; n++) {
-            const int gn = a.conn[n * a.nel + e];
-            x[n] = a.xy[gn];
-            y[n] = a.xy[a.nnodes + gn];
-        }
-        auto go = geometry(c_bfn[ig], c_dfdc[ig], c_dfde[ig], c_d2fdc2[ig], c_d2fde2[ig],
-                           c_d2fdce[ig], c_w[ig], x, y, sm.dFx[el][ig], sm.dFy[el][ig],
-                           sm.d2x[el][ig], sm.d2y[el][ig]);
-        sm.H2[el][ig] = go.H2;
-        sm.WET[el][ig] = go.WET;
+    for (int n = 0; n < 9; n++) {
+        const double t = V(n * 6 + f);
+        val = val + t * bfn[n];
+        gx = gx + t * dFx[n];
+        gy = gy + t * dFy[n];
     }
-    __syncthreads();
-    if (live && k < 9) {
-        // interpolants of the original state, once per element and Gauss point
-        SmemView V0{sm.tl[el][0]};
-        sm.base[el][k] = interpolate(V0, c_bfn[k], sm.dFx[el][k], sm.dFy[el][k], sm.d2x[el][k],
-                                     sm.d2y[el][k]);
-    }
-    if (live && k == 9) {
-        int r = 0;
-        for (int i = 0; i < 54; i++)
-            r |= __double_as_longlong(sm.tl[el][1][i]) != __double_as_longlong(sm.tl[el][0][i]);
-        sm.residue[el] = r;
-    }
-    __syncthreads();
+}
 
-    const bool is_ac = (k == 55);
-    const bool active = live && (k < 55 || (is_ac && prm.nex > 0));
+template <int FORM, int SPEC, int EL, int THREADS>
+__device__ __forceinline__ void fd_stress(const ElemArgs &a, const KParams &prm, int e0, FdStressSmem<EL> &sm)
+{
+    static_assert(EL * FS_COLS <= THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(EL, a.nel - e0);
+    if (ne <= 0) return;
+    stage_states<EL, THREADS>(a, prm, e0, ne, sm.tl, sm.residue);
+    for (int i = t; i < ne * 9; i += THREADS) {
+        const int el = i / 9, ig = i - 9 * el;
+        const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
+        SmemView V{sm.tl[el][0]};
+        const Interp<double> I = interpolate(V, c_bfn[ig], geo, geo + 9, geo + 18, geo + 27);
+        sm.base[el][ig] = I;
+        sm.flow[el][ig] = flow_part(I, kinematics(I), geo, geo + 9, sm.dotU[el][ig]);
+    }
+    __syncthreads();
+    const int el = t / FS_COLS, c = t - FS_COLS * el;
+    const bool ac = c == 27;
+    if (el >= ne || sm.residue[el] || (ac && prm.nex == 0)) return;
+    const int inod = c / 3, f = 3 + c - 3 * inod, kk = ac ? -1 : inod * 6 + f, e = e0 + el;
+    double WiN = prm.WiN;
+    if (prm.nex > 0) {
+        const double eu = a.EU[prm.nex - 1];
+        WiN = prm.Wi0 * (ac ? eu + prm.eps : eu);
+    }
     double res[54];
 #pragma unroll
     for (int i = 0; i < 54; i++) res[i] = 0.0;
-    if (active) {
-        const int kk = (k == 0) ? -1 : (is_ac ? 54 : k - 1);
-        const int fk = kk >= 0 && kk < 54 ? kk - 6 * (kk / 6) : -1;
-        double WiN = prm.WiN;
-        if (prm.nex > 0) {
-            const double eu = a.EU[prm.nex - 1];
-            WiN = prm.Wi0 * (is_ac ? eu + eps : eu);
+#pragma unroll 1
+    for (int ig = 0; ig < 9; ig++) {
+        const double *geo = a.geo + ((size_t)e * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
+        const double H2 = geo[36], WET = geo[37];
+        Interp<double> I = sm.base[el][ig];
+        if (!ac) {
+            FdCleanView V{sm.tl[el][0], sm.tl[el][1], kk};
+            double v, gx, gy;
+            perturbed(V, f, c_bfn[ig], dFx, dFy, v, gx, gy);
+            I.S11 = f == 3 ? v : I.S11;
+            I.dS11x = f == 3 ? gx : I.dS11x;
+            I.dS11y = f == 3 ? gy : I.dS11y;
+            I.S12 = f == 4 ? v : I.S12;
+            I.dS12x = f == 4 ? gx : I.dS12x;
+            I.dS12y = f == 4 ? gy : I.dS12y;
+            I.S22 = f == 5 ? v : I.S22;
+            I.dS22x = f == 5 ? gx : I.dS22x;
+            I.dS22y = f == 5 ? gy : I.dS22y;
         }
-        const bool residue = sm.residue[el] != 0;
-        for (int ig = 0; ig < 9; ig++) {
-            const double *dFx = sm.dFx[el][ig], *dFy = sm.dFy[el][ig];
-            Interp<double> I;
-            if (!residue) {
-                // unperturbed fields from the cache; the perturbed field recomputed
-                I = sm.base[el][ig];
-                if (fk >= 0) {
-                    FdCleanView V{sm.tl[el][0], sm.tl[el][2], kk};
-                    interpolate_field(V, fk, c_bfn[ig], dFx, dFy, sm.d2x[el][ig], sm.d2y[el][ig],
-                                      I);
-                }
-            } else {
-                FdView V;
-                V.orig = sm.tl[el][0];
-                V.rest = sm.tl[el][1];
-                V.pert = sm.tl[el][2];
-                V.kk = kk;
-                I = interpolate(V, c_bfn[ig], dFx, dFy, sm.d2x[el][ig], sm.d2y[el][ig]);
-            }
-            double dotU[9];
-            auto g = gauss_point<FORM, SPEC>(I, prm, WiN, sm.H2[el][ig], dFx, dFy, dotU);
-            const double WET = sm.WET[el][ig];
+        const StressPart<double> p = stress_part<FORM>(I, prm, WiN, H2);
+        const GpCoef<double> g =
+            combine_parts<FORM, SPEC>(I, prm, WiN, H2, p, kinematics(I), sm.flow[el][ig]);
 #pragma unroll
-            for (int n = 0; n < 9; n++) {
-                double o[6];
-                test_node<FORM, SPEC>(g, prm, c_bfn[ig][n], dFx[n], dFy[n], dotU[n], WET, o);
+        for (int n = 0; n < 9; n++) {
+            double o[6];
+            const TestStress<double> ts = test_stress<FORM>(I, p.den, p.rden, dFx[n], dFy[n]);
+            test_terms<FORM, SPEC>(g, prm, ts, c_bfn[ig][n], dFx[n], dFy[n], sm.dotU[el][ig][n], WET, o);
 #pragma unroll
-                for (int f = 0; f < 6; f++) res[n * 6 + f] = res[n * 6 + f] + o[f];
-            }
+            for (int q = 0; q < 6; q++) res[n * 6 + q] = res[n * 6 + q] + o[q];
         }
     }
-    if (active && k == 0) {
-#pragma unroll
-        for (int i = 0; i < 54; i++) {
-            sm.res0[el][i] = res[i];
-            a.rs[(size_t)e * 54 + i] = res[i];
+    store_column(a, prm, e, inod, ac ? 6 : f, res);
+}
+
+template <int FORM, int SPEC, int EL, int THREADS>
+__device__ __forceinline__ void fd_flow(const ElemArgs &a, const KParams &prm, int e0, FdFlowSmem<FORM, EL> &sm)
+{
+    static_assert(EL * FU_COLS <= THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(EL, a.nel - e0);
+    if (ne <= 0) return;
+    const double WiN = wi_of(a, prm);
+    stage_states<EL, THREADS>(a, prm, e0, ne, sm.tl, sm.residue);
+    for (int i = t; i < ne * 9; i += THREADS) {
+        const int el = i / 9, ig = i - 9 * el;
+        const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
+        SmemView V{sm.tl[el][0]};
+        const Interp<double> I = interpolate(V, c_bfn[ig], geo, geo + 9, geo + 18, geo + 27);
+        sm.base[el][ig] = I;
+        sm.stress[el][ig] = stress_part<FORM>(I, prm, WiN, geo[36]);
+    }
+    __syncthreads();
+    for (int i = t; i < ne * 81; i += THREADS) {
+        const int el = i / 81, ig = (i / 9) % 9, n = i % 9;
+        const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
+        const StressPart<double> &p = sm.stress[el][ig];
+        const TestStress<double> ts = test_stress<FORM>(sm.base[el][ig], p.den, p.rden, geo[n], geo[9 + n]);
+        double *d = sm.test[el][ig][n];
+        d[0] = ts.gd11;
+        d[1] = ts.gd12;
+        d[2] = ts.gd22;
+        if (FORM == FORM_SQRT) {
+            d[3] = ts.u11; d[4] = ts.u12; d[5] = ts.u21; d[6] = ts.u22;
+            d[7] = ts.v11; d[8] = ts.v12; d[9] = ts.v21; d[10] = ts.v22;
         }
     }
     __syncthreads();
-    if (!active || k == 0) return;
-    if (is_ac) {
+    const int el = t / FU_COLS, c = t - FU_COLS * el;
+    if (el >= ne || sm.residue[el]) return;
+    const int inod = c >> 1, f = c & 1, kk = inod * 6 + f, e = e0 + el;
+    double res[54];
 #pragma unroll
-        for (int i = 0; i < 54; i++) a.as[(size_t)e * 54 + i] = (res[i] - sm.res0[el][i]) / eps;
+    for (int i = 0; i < 54; i++) res[i] = 0.0;
+#pragma unroll 1
+    for (int ig = 0; ig < 9; ig++) {
+        const double *geo = a.geo + ((size_t)e * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
+        const double H2 = geo[36], WET = geo[37];
+        Interp<double> I = sm.base[el][ig];
+        {
+            FdCleanView V{sm.tl[el][0], sm.tl[el][1], kk};
+            interpolate_field(V, f, c_bfn[ig], dFx, dFy, geo + 18, geo + 27, I);
+        }
+        double dotU[9];
+        const Kinematics<double> k = kinematics(I);
+        const FlowPart<double> q = flow_part(I, k, dFx, dFy, dotU);
+        const GpCoef<double> g = combine_parts<FORM, SPEC>(I, prm, WiN, H2, sm.stress[el][ig], k, q);
+#pragma unroll
+        for (int n = 0; n < 9; n++) {
+            double o[6];
+            const double *d = sm.test[el][ig][n];
+            TestStress<double> ts;
+            ts.gd11 = d[0];
+            ts.gd12 = d[1];
+            ts.gd22 = d[2];
+            if (FORM == FORM_SQRT) {
+                ts.u11 = d[3]; ts.u12 = d[4]; ts.u21 = d[5]; ts.u22 = d[6];
+                ts.v11 = d[7]; ts.v12 = d[8]; ts.v21 = d[9]; ts.v22 = d[10];
+            }
+            test_terms<FORM, SPEC>(g, prm, ts, c_bfn[ig][n], dFx[n], dFy[n], dotU[n], WET, o);
+#pragma unroll
+            for (int w = 0; w < 6; w++) res[n * 6 + w] = res[n * 6 + w] + o[w];
+        }
+    }
+    store_column(a, prm, e, inod, f, res);
+}
+
+template <int FORM, int SPEC, int EL, int THREADS>
+__device__ __forceinline__ void fd_pressure(const ElemArgs &a, const KParams &prm, int e0, FdPressureSmem<EL> &sm)
+{
+    static_assert(EL * FP_COLS <= THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(EL, a.nel - e0);
+    if (ne <= 0) return;
+    const double WiN = wi_of(a, prm);
+    for (int i = t; i < EL; i += THREADS) sm.residue[i] = 0;
+    __syncthreads();
+    for (int i = t; i < ne * 54; i += THREADS) {
+        const int el = i / 54, pos = i - 54 * el, inod = pos / 6, f = pos - 6 * inod;
+        const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e0 + el]];
+        const double vp = v + prm.eps, back = vp - prm.eps;
+        sm.tl[el][pos] = v;
+        if (f == 2) sm.pert[el][inod] = vp;
+        if (__double_as_longlong(back) != __double_as_longlong(v)) sm.residue[el] = 1;
+    }
+    __syncthreads();
+    for (int i = t; i < ne * 9; i += THREADS) {
+        const int el = i / 9, ig = i - 9 * el;
+        const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
+        SmemView V{sm.tl[el]};
+        const Interp<double> I = interpolate(V, c_bfn[ig], geo, geo + 9, geo + 18, geo + 27);
+        const Kinematics<double> k = kinematics(I);
+        const StressPart<double> p = stress_part<FORM>(I, prm, WiN, geo[36]);
+        double dotU[9];
+        const FlowPart<double> q = flow_part(I, k, geo, geo + 9, dotU);
+        sm.g[el][ig] = combine_parts<FORM, SPEC>(I, prm, WiN, geo[36], p, k, q);
+        double *c = sm.keep[el][ig];
+        c[0] = p.T11 + prm.BvN * k.Gd11;
+        c[1] = p.T22 + prm.BvN * k.Gd22;
+        c[2] = p.divT1;
+        c[3] = p.divT2;
+        c[4] = prm.BvN * I.lap1;
+        c[5] = prm.BvN * I.lap2;
+    }
+    __syncthreads();
+    const int el = t / FP_COLS, inod = t - FP_COLS * el;    // also the test node in the kept terms
+    const bool staged = el < ne, live = staged && !sm.residue[el];
+    const int e = e0 + el;
+    double res[54];
+#pragma unroll
+    for (int i = 0; i < 54; i++) res[i] = 0.0;
+#pragma unroll 1
+    for (int ig = 0; ig < 9; ig++) {
+        const double *geo = a.geo + ((size_t)(staged ? e : e0) * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
+        if (staged) {
+            const GpCoef<double> &g = sm.g[el][ig];
+            Interp<double> I;
+            I.S11 = g.S11; I.S12 = g.S12; I.S22 = g.S22;
+            I.dS11x = g.dS11x; I.dS11y = g.dS11y; I.dS12x = g.dS12x; I.dS12y = g.dS12y;
+            I.dS22x = g.dS22x; I.dS22y = g.dS22y;
+            const double fx = dFx[inod], fy = dFy[inod];
+            const TestStress<double> ts = test_stress<FORM>(I, g.den, g.rden, fx, fy);
+            sm.test[el][inod] =
+                test_pressure<FORM, SPEC>(g, prm, ts, c_bfn[ig][inod], fx, fy, g.U1 * fx + g.U2 * fy);
+        }
+        __syncthreads();
+        if (live) {
+            const GpCoef<double> &g = sm.g[el][ig];
+            const double *c = sm.keep[el][ig];
+            double P = 0.0, dPx = 0.0, dPy = 0.0;
+#pragma unroll
+            for (int n = 0; n < 9; n++) {
+                const double v = n == inod ? sm.pert[el][n] : sm.tl[el][n * 6 + 2];
+                P = P + v * c_bfn[ig][n];
+                dPx = dPx + v * dFx[n];
+                dPy = dPy + v * dFy[n];
+            }
+            const double P11 = c[0] - P, P22 = c[1] - P;
+            const double divP1 = (-dPx + c[2]) + c[4], divP2 = (-dPy + c[3]) + c[5];
+            const double M1 = (SPEC & SPEC_RE0) ? -divP1 : g.rc1 - divP1;
+            const double M2 = (SPEC & SPEC_RE0) ? -divP2 : g.rc2 - divP2;
+            const double WET = geo[37], scale = FORM == FORM_T ? g.omb : g.WiN;
+#pragma unroll
+            for (int n = 0; n < 9; n++) {
+                double o[6];
+                const double fx = dFx[n], fy = dFy[n];
+                pressure_terms<FORM, SPEC>(sm.test[el][n], P11, P22, M1, M2, g.rc1, g.rc2, g.tR, g.tlsme, scale,
+                                           c_bfn[ig][n], fx, fy, (SPEC & SPEC_RE0) ? 0.0 : g.U1 * fx + g.U2 * fy, WET,
+                                           o);
+#pragma unroll
+                for (int w = 0; w < 6; w++) res[n * 6 + w] = res[n * 6 + w] + o[w];
+            }
+        }
+        __syncthreads();
+    }
+    if (live) store_column(a, prm, e, inod, 2, res);
+}
+
+// Elements with a restore residue: all 55 columns, each a full evaluation of the
+// state the sequential loop would have, 64 threads an element.
+template <int FORM, int SPEC, int THREADS>
+__device__ __forceinline__ void fd_residue(const ElemArgs &a, const KParams &prm, int e0, FdResidueSmem<THREADS> &sm)
+{
+    const int t = threadIdx.x, ne = min(FdRun<THREADS>::R, a.nel - e0);
+    if (t == 0) sm.n = 0;
+    __syncthreads();
+    const double eps = prm.eps;
+    for (int el = t >> 2; el < ne; el += THREADS >> 2) {
+        bool any = false;
+        for (int pos = t & 3; pos < 54; pos += 4) {
+            const int inod = pos / 6, f = pos - 6 * inod;
+            const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e0 + el]];
+            any |= __double_as_longlong((v + eps) - eps) != __double_as_longlong(v);
+        }
+        const unsigned quad = 0xfu << (threadIdx.x & 28);
+        any = __any_sync(quad, any);
+        if (any && (t & 3) == 0) sm.list[atomicAdd(&sm.n, 1)] = e0 + el;
+    }
+    __syncthreads();
+    const int count = sm.n, grp = t >> 6, k = t & 63;
+    for (int i = 0; i < count; i += THREADS / 64) {
+        const bool live = i + grp < count;
+        const int e = live ? sm.list[i + grp] : 0;
+        if (live && k < 54) {
+            const int inod = k / 6, f = k - 6 * inod;
+            const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e]];
+            const double vp = v + eps;
+            sm.tl[grp][0][k] = v;
+            sm.tl[grp][2][k] = vp;
+            sm.tl[grp][1][k] = vp - eps;
+        }
+        __syncthreads();
+        const bool ac = k == 54;
+        if (live && (k < 54 || (ac && prm.nex > 0))) {
+            FdView V;
+            V.orig = sm.tl[grp][0];
+            V.rest = sm.tl[grp][1];
+            V.pert = sm.tl[grp][2];
+            V.kk = k;
+            double WiN = prm.WiN;
+            if (prm.nex > 0) {
+                const double eu = a.EU[prm.nex - 1];
+                WiN = prm.Wi0 * (ac ? eu + eps : eu);
+            }
+            double res[54];
+#pragma unroll
+            for (int q = 0; q < 54; q++) res[q] = 0.0;
+#pragma unroll 1
+            for (int ig = 0; ig < 9; ig++) {
+                const double *geo = a.geo + ((size_t)e * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
+                const Interp<double> I = interpolate(V, c_bfn[ig], dFx, dFy, geo + 18, geo + 27);
+                double dotU[9];
+                const GpCoef<double> g = gauss_point<FORM, SPEC>(I, prm, WiN, geo[36], dFx, dFy, dotU);
+#pragma unroll
+                for (int n = 0; n < 9; n++) {
+                    double o[6];
+                    test_node<FORM, SPEC>(g, prm, c_bfn[ig][n], dFx[n], dFy[n], dotU[n], geo[37], o);
+#pragma unroll
+                    for (int w = 0; w < 6; w++) res[n * 6 + w] = res[n * 6 + w] + o[w];
+                }
+            }
+            store_column(a, prm, e, ac ? 0 : k / 6, ac ? 6 : k - 6 * (k / 6), res);
+        }
+        __syncthreads();
+    }
+}
+
+template <int FORM, int SPEC, int THREADS>
+__global__ void __launch_bounds__(THREADS, 256 / THREADS) k_fd64(const ElemArgs a, const KParams prm, int groups, int run)
+{
+    typedef FdRun<THREADS> Run;
+    extern __shared__ __align__(16) unsigned char fd_raw[];
+    FdSmem<FORM, THREADS> &sm = *reinterpret_cast<FdSmem<FORM, THREADS> *>(fd_raw);
+    // CTAs of each kind in a group of `run` elements, in this order
+    const int S = (run + Run::S - 1) / Run::S, U = (run + Run::U - 1) / Run::U, P = (run + Run::P - 1) / Run::P;
+    const int grp = blockIdx.x / (S + U + P);
+    if (grp >= groups) {
+        fd_residue<FORM, SPEC, THREADS>(a, prm, (blockIdx.x - groups * (S + U + P)) * Run::R, sm.r);
         return;
     }
-    // column (inod, ieq) of TEMP_A_f; row (jnod, jeq)
-    const int inod = (k - 1) / 6, ieq = (k - 1) - 6 * ((k - 1) / 6);
-    double *dst = a.es + (size_t)e * 2916 + inod * 36 + ieq;
-#pragma unroll
-    for (int jnod = 0; jnod < 9; jnod++)
-#pragma unroll
-        for (int jeq = 0; jeq < 6; jeq++)
-            dst[jnod * 324 + jeq * 6] = (res[jnod * 6 + jeq] - sm.res0[el][jnod * 6 + jeq]) / eps;
+    const int b = blockIdx.x - grp * (S + U + P), e0 = grp * run;
+    if (b < S)
+        fd_stress<FORM, SPEC, Run::S, THREADS>(a, prm, e0 + b * Run::S, sm.s);
+    else if (b < S + U)
+        fd_flow<FORM, SPEC, Run::U, THREADS>(a, prm, e0 + (b - S) * Run::U, sm.u);
+    else
+        fd_pressure<FORM, SPEC, Run::P, THREADS>(a, prm, e0 + (b - S - U) * Run::P, sm.p);
 }
 
 // ---------------------------------------------------------------------------
@@ -251,11 +578,6 @@ constexpr int RS_THREADS = 64;
 constexpr int RS_MIN_CTAS = 6;
 constexpr int RS_CHUNK = 3;                 // test nodes per pass through shared memory
 static_assert(RS_EPB * 9 <= RS_THREADS, "a thread per element and Gauss point");
-
-__device__ __forceinline__ double wi_of(const ElemArgs &a, const KParams &prm)
-{
-    return prm.nex > 0 ? prm.Wi0 * a.EU[prm.nex - 1] : prm.WiN;
-}
 
 // elements [e0, e0 + count) of one mesh, count <= RS_EPB; SPEC leaves out the
 // exact-zero terms of ReN = 0 / DfN = 0 as the FD kernel does (same values)
@@ -321,6 +643,7 @@ __device__ __forceinline__ void res64_block(const ElemArgs &a, const KParams &pr
 template <int FORM, int SPEC>
 __global__ void __launch_bounds__(RS_THREADS, RS_MIN_CTAS) k_res64(const ElemArgs a, const KParams prm)
 {
+    pdl_launch_dependents();
     res64_block<FORM, SPEC>(a, prm, blockIdx.x * RS_EPB, RS_EPB);
 }
 
@@ -333,6 +656,7 @@ __global__ void __launch_bounds__(RS_THREADS, RS_MIN_CTAS) k_res64(const ElemArg
 template <int FORM, int SPEC, int E, int THREADS>
 __global__ void __launch_bounds__(THREADS, E == 1 ? 4 : 2) k_res64_wide(const ElemArgs a, const KParams prm)
 {
+    pdl_launch_dependents();
     __shared__ double s_tl[E][54];
     __shared__ __align__(16) double s_geo[E * 9 * GEO_REC];
     __shared__ double s_bfn[9][9];
@@ -508,27 +832,38 @@ int residual_batched_ctas_per_sm(int form, int spec)
     return n;
 }
 
-template <int FORM>
-static void launch_fd64_form(const ElemArgs &a, const KParams &p, int grid, cudaStream_t s)
+template <int FORM, int SPEC, int THREADS>
+static cudaError_t go_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
 {
-    const int spec = (p.ReN == 0.0 ? SPEC_RE0 : 0) | (p.DfN == 0.0 ? SPEC_DF0 : 0);
-    switch (spec) {
-    case 0: k_fd64<FORM, 0><<<grid, FD_THREADS, 0, s>>>(a, p); break;
-    case SPEC_RE0: k_fd64<FORM, SPEC_RE0><<<grid, FD_THREADS, 0, s>>>(a, p); break;
-    case SPEC_DF0: k_fd64<FORM, SPEC_DF0><<<grid, FD_THREADS, 0, s>>>(a, p); break;
-    default: k_fd64<FORM, SPEC_RE0 | SPEC_DF0><<<grid, FD_THREADS, 0, s>>>(a, p); break;
-    }
+    // a small mesh is one group: all stress CTAs, the longest, are placed first
+    typedef FdRun<THREADS> Run;
+    const int run = THREADS == 64 ? a.nel : FD_RUN, groups = (a.nel + run - 1) / run;
+    const int per = (run + Run::S - 1) / Run::S + (run + Run::U - 1) / Run::U + (run + Run::P - 1) / Run::P;
+    const int residue = (a.nel + Run::R - 1) / Run::R;
+    const int smem = (int)sizeof(FdSmem<FORM, THREADS>);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_fd64<FORM, SPEC, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(groups * per + residue));
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_fd64<FORM, SPEC, THREADS>, a, p, groups, run);
 }
 
 cudaError_t launch_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
 {
     if (a.nel <= 0) return cudaSuccess;
-    const int grid = (a.nel + FD_EPB - 1) / FD_EPB;
-    if (p.form == FORM_SQRT)
-        launch_fd64_form<FORM_SQRT>(a, p, grid, s);
-    else
-        launch_fd64_form<FORM_T>(a, p, grid, s);
-    return cudaGetLastError();
+#define GO(F, SP) return a.nel <= FD_NARROW_MAX ? go_fd64<F, SP, 64>(a, p, s) : go_fd64<F, SP, 256>(a, p, s)
+    RES_DISPATCH(p.form, spec_of(p), GO);
+#undef GO
+    return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------

@@ -29,23 +29,22 @@ __global__ void k_gather_residual(const GatherArgs g, const double *__restrict__
                        [&](int c) { return rs[(int64_t)c * 6 + jeq]; });
 }
 
-// two entries of a node-pair block per thread (vefem_gather.cuh)
+// two entries of a node-pair block per thread, then (CTAs from nblk on) the
+// arclength column (vefem_gather.cuh)
 template <class T>
 __global__ void __launch_bounds__(GB_THREADS)
-k_gather_blocks(const GatherArgs g, const T *__restrict__ es, T *__restrict__ vals)
+k_gather_rows(const GatherArgs g, const T *__restrict__ es, const T *__restrict__ as, T *__restrict__ vals,
+              unsigned nblk)
 {
+    if (blockIdx.x >= nblk) {
+        const int64_t t = (int64_t)(blockIdx.x - nblk) * GB_THREADS + threadIdx.x;
+        if (t < (int64_t)g.nnodes * 6) gather_arclength(g, (int)(t / 6), (int)(t % 6), as, vals);
+        return;
+    }
     const int64_t t = (int64_t)blockIdx.x * GB_THREADS + threadIdx.x;
     if (t >= (int64_t)g.nblocks * GB_PAIRS) return;
     const int blk = (int)(t / GB_PAIRS);
     gather_pair(g, blk, (int)(t - (int64_t)blk * GB_PAIRS), es, vals);
-}
-
-// arclength column: the last entry of every node row (column N - 1)
-template <class T>
-__global__ void k_gather_arclength(const GatherArgs g, const T *__restrict__ as, T *__restrict__ vals)
-{
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < (int64_t)g.nnodes * 6) gather_arclength(g, (int)(t / 6), (int)(t % 6), as, vals);
 }
 
 __global__ void k_block_records(int nblocks, const int32_t *__restrict__ brow, const int32_t *__restrict__ boff,
@@ -122,10 +121,9 @@ cudaError_t launch_gather_residual(const GatherArgs &g, const double *rs, double
 template <class T>
 cudaError_t launch_gather_rows(const GatherArgs &g, const T *es, const T *as, T *vals, cudaStream_t s)
 {
-    const int64_t n = (int64_t)g.nblocks * GB_PAIRS;
-    if (n > 0) k_gather_blocks<T><<<grid_for(n, GB_THREADS), GB_THREADS, 0, s>>>(g, es, vals);
-    if (g.nex > 0 && g.nnodes > 0)
-        k_gather_arclength<T><<<grid_for((int64_t)g.nnodes * 6, 256), 256, 0, s>>>(g, as, vals);
+    const unsigned nblk = grid_for((int64_t)g.nblocks * GB_PAIRS, GB_THREADS);
+    const unsigned narc = g.nex > 0 ? grid_for((int64_t)g.nnodes * 6, GB_THREADS) : 0;
+    if (nblk + narc > 0) k_gather_rows<T><<<nblk + narc, GB_THREADS, 0, s>>>(g, es, as, vals, nblk);
     return cudaGetLastError();
 }
 

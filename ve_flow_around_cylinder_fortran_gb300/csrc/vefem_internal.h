@@ -19,6 +19,11 @@ constexpr int RES_EPB = 7;
 // 1, 51 / 65 / 65 / 65 with 3, 98 throughout with k_res64; one wave more costs
 // 94 (1, 800 quads) and 96 us (3, 1,000).
 constexpr int RES_WIDE1_MAX = 4 * 152, RES_WIDE3_MAX = 6 * 152;
+// Forward-difference kernel: meshes up to this size take 64-thread CTAs, four
+// of which are resident on each of 152 SMs.  SQRT form, 64 against 256 threads:
+// 0.69 / 1.33 ms on 200 quads, 1.30 / 1.35 on 600, 1.56 / 1.36 on 700; T form
+// 0.44 / 0.79 on 200, even on 500, 1.13 / 0.90 on 700.
+constexpr int FD_NARROW_MAX = 4 * 152;
 // doubles per Gauss point of a mesh's geometry table
 constexpr int GEO_REC = 38;
 
@@ -63,6 +68,7 @@ cudaError_t upload_tables(const GaussTables &t, cudaStream_t s);
 cudaError_t launch_geometry(int nel, int nnodes, const int32_t *conn, const double *xy, double *geo,
                             cudaStream_t s);
 cudaError_t launch_residual64(const ElemArgs &a, const KParams &p, cudaStream_t s);
+// the columns are differences from the residual in a.rs: launch_residual64 comes first
 cudaError_t launch_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s);
 
 // Outlet open-BC edges: residual and FD Jacobian of each listed edge into edge scratch.
