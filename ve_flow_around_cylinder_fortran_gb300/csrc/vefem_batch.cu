@@ -357,6 +357,7 @@ extern "C" int vefem_batch_create(int ninst, const vefem_mesh *meshes, const vef
             I.ga.rowptr = c->d_rowptr;
             I.ga.nptr = c->d_nptr;
             I.ga.ncon = c->d_ncon;
+            I.ga.nbptr = c->d_nbptr;
             I.ga.brow = c->d_brow;
             I.ga.boff = c->d_boff;
             I.ga.bptr = c->d_bptr;

@@ -417,6 +417,7 @@ extern "C" int vefem_create(const vefem_mesh *mesh, const vefem_csr *pat,
     UPL(d_colind, colind, (size_t)rowptr[N])
     UPL(d_nptr, nptr.data(), nptr.size())
     UPL(d_ncon, ncon.data(), ncon.size())
+    UPL(d_nbptr, nbptr.data(), nbptr.size())
     UPL(d_brow, brow.data(), brow.size())
     UPL(d_boff, boff.data(), boff.size())
     UPL(d_bptr, bptr.data(), bptr.size())
@@ -622,6 +623,7 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     ga.rowptr = ctx->d_rowptr;
     ga.nptr = ctx->d_nptr;
     ga.ncon = ctx->d_ncon;
+    ga.nbptr = ctx->d_nbptr;
     ga.brow = ctx->d_brow;
     ga.boff = ctx->d_boff;
     ga.bptr = ctx->d_bptr;
@@ -752,7 +754,7 @@ extern "C" int vefem_destroy(vefem_ctx *ctx)
     if (!ctx) return VEFEM_OK;
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    void *ptrs[] = {ctx->d_conn, ctx->d_xy, ctx->d_geo, ctx->d_rowptr, ctx->d_nptr, ctx->d_ncon, ctx->d_brow,
+    void *ptrs[] = {ctx->d_conn, ctx->d_xy, ctx->d_geo, ctx->d_rowptr, ctx->d_nptr, ctx->d_ncon, ctx->d_nbptr, ctx->d_brow,
                     ctx->d_boff, ctx->d_bptr, ctx->d_bcon, ctx->d_brec, ctx->d_edge_elem, ctx->d_edge_id,
                     ctx->d_edge_row, ctx->d_edge_off, ctx->d_rs, ctx->d_es, ctx->d_as,
                     ctx->d_ers, ctx->d_ees, ctx->d_eas, ctx->d_TL, ctx->d_EU, ctx->d_b,

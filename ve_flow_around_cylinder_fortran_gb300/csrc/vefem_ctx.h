@@ -31,6 +31,7 @@ struct vefem_ctx {
     double *d_geo = nullptr;    // geometry table (launch_geometry), filled at create
     int64_t *d_rowptr = nullptr;
     int32_t *d_nptr = nullptr, *d_ncon = nullptr;
+    int32_t *d_nbptr = nullptr;
     int32_t *d_brow = nullptr, *d_boff = nullptr, *d_bptr = nullptr, *d_bcon = nullptr;
     vefem::BlockRec *d_brec = nullptr;          // launch_block_records, filled at create
     int32_t *d_edge_elem = nullptr, *d_edge_id = nullptr;

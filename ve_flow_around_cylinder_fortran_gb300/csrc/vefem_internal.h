@@ -99,6 +99,7 @@ struct GatherArgs {
     const int64_t *rowptr;     // [N+1]
     const int32_t *nptr;       // [nnodes+1] node -> residual contributors
     const int32_t *ncon;       // contributor = e*9 + jnod, element order
+    const int32_t *nbptr;      // [nnodes+1] row node -> its node-pair blocks
     const int32_t *brow;       // [nblocks] row node of each node-pair block
     const int32_t *boff;       // [nblocks] column offset of the block inside its rows
     const int32_t *bptr;       // [nblocks+1]

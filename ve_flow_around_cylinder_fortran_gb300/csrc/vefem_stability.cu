@@ -613,7 +613,7 @@ __global__ void k_stability_gather(const GatherArgs g, const int64_t *__restrict
 // Gauss point (k_planar_coef, a thread per point) and contracted pair by pair
 // (k_planar_contract: 0.24 M multiply-adds per element), and the scatter reads
 // 83 KB per element instead of 259.  20,000 quads, 16 wavenumbers and B:
-// 184.6 -> 18.6 ms.  The line between the routes is the check of the four
+// 184.6 -> 14.5 ms.  The line between the routes is the check of the four
 // out-of-plane base fields (k_nonplanar, one pass over 2.6 MB): the pairs left
 // out are exact zeros for a planar base and for no other.
 
@@ -1023,62 +1023,104 @@ k_planar_contract(const double *__restrict__ rec_all, double *__restrict__ es, i
     }
 }
 
+// Where a pair's sum goes: B or A0 at equation x unknown `r`, or the K (pw 1) or
+// K^2 (pw 2) part of the `dep`-th of the 36 entries of a block that depend on K.
+constexpr int PL_DEP = 36;
 struct PlMap {
-    signed char at[4][100];     // pair of (matrix, equation x unknown), -1: zero
+    unsigned char n;                               // pairs that are not identically zero
+    unsigned char pair[PL_NP], m[PL_NP], at[PL_NP]; // pair; matrix; r or dep
+    unsigned char dr[PL_DEP], dpw[PL_DEP];
 };
 
-constexpr int PG_THREADS = 256;
+constexpr int PG_THREADS = 256, PG_BLK = 16;       // node-pair blocks at a time
+constexpr int PG_OWN = (PG_BLK * 100 + PG_THREADS - 1) / PG_THREADS;       // entries per thread
+constexpr int PG_DEP = (PG_BLK * PL_DEP + PG_THREADS - 1) / PG_THREADS;    // K-dependent ones
 
-// Scatter: the element-ordered sums of the pairs, then B and A(K) of every
-// wavenumber.  COVER (the stability pattern is exactly the node-pair blocks): a
-// CTA per row node walks its 10 rows in the order they are stored, so a warp
-// writes consecutive entries of every matrix; store leaves out reading them.
-template <bool COVER>
+// Scatter: a CTA per row node sums its blocks' pairs in element order and writes
+// its 10 rows of B and of A(K) for every wavenumber.  Only 36 of a block's 100
+// entries depend on K, in one power each: they are evaluated on full warps into
+// shared memory (a thread per entry, K in two multiply-adds whatever the entry
+// holds, spent 6.5 ms of FP64 pipe on 20,000 quads x 16 wavenumbers, more than
+// the 2.6 ms of writing 17.5 GB), and the rows are written from there in the
+// order they are stored.  store: leave out reading the matrices.
+// Scatter of that case 9.2 -> 5.1 ms, the call 18.6 -> 14.5 ms.
 __global__ void __launch_bounds__(PG_THREADS)
 k_planar_gather(const GatherArgs g, const PlMap map, const int64_t *__restrict__ rowptr10,
                 const int32_t *__restrict__ boff10, const double *__restrict__ es, int nk,
-                const double *__restrict__ kw, double *const *A, double *B, int store)
+                const double *__restrict__ kw, double *const *__restrict__ A, double *__restrict__ B, int store)
 {
-    __shared__ signed char s_at[4][100];
-    for (int u = threadIdx.x; u < 400; u += PG_THREADS) s_at[u / 100][u % 100] = map.at[u / 100][u % 100];
-    __syncthreads();
-    int64_t first = 0, count = 0, base = 0;
-    int wide = 0;
-    if (COVER) {
-        base = rowptr10[(int64_t)blockIdx.x * ST_NEQ];
-        count = rowptr10[(int64_t)(blockIdx.x + 1) * ST_NEQ] - base;
-        wide = (int)(count / ST_NEQ);
-    } else {
-        first = (int64_t)blockIdx.x * PG_THREADS;
-        count = min((int64_t)PG_THREADS, (int64_t)g.nblocks * 100 - first);
-    }
-    for (int64_t t = threadIdx.x; t < count; t += PG_THREADS) {
-        int blk, r;
-        int64_t slot;
-        if (COVER) {
-            const int jeq = (int)t / wide, c = (int)t - jeq * wide;
-            blk = (int)(base / 100) + c / ST_NEQ;
-            r = jeq * ST_NEQ + c % ST_NEQ;
-            slot = base + t;
-        } else {
-            blk = (int)((first + t) / 100);
-            r = (int)((first + t) % 100);
-            slot = rowptr10[(int64_t)g.brow[blk] * ST_NEQ + r / ST_NEQ] + boff10[blk] + r % ST_NEQ;
+    __shared__ PlMap s_map;
+    __shared__ double s_v[PG_BLK * 100], s_b[PG_BLK * 100], s_x[PG_BLK * PL_DEP];
+    __shared__ int s_id[PG_BLK][4], s_n[PG_BLK], s_c0[PG_BLK], s_off[PG_BLK];
+    __shared__ int64_t s_row[ST_NEQ];
+    const int t = threadIdx.x;
+    for (int u = t; u < (int)sizeof(PlMap); u += PG_THREADS)
+        reinterpret_cast<unsigned char *>(&s_map)[u] = reinterpret_cast<const unsigned char *>(&map)[u];
+    if (t < ST_NEQ) s_row[t] = rowptr10[(int64_t)blockIdx.x * ST_NEQ + t];
+    const int b1 = g.nbptr[blockIdx.x + 1];
+    for (int b0 = g.nbptr[blockIdx.x]; b0 < b1; b0 += PG_BLK) {
+        const int nb = min(PG_BLK, b1 - b0), wide = nb * ST_NEQ, count = nb * 100;
+        __syncthreads();
+        if (t < nb) {
+            const int4 *rp = reinterpret_cast<const int4 *>(g.brec + b0 + t);
+            const int4 head = rp[0], ids = rp[1];
+            s_c0[t] = head.z;
+            s_n[t] = head.w;
+            s_off[t] = boff10[b0 + t];
+            s_id[t][0] = ids.x; s_id[t][1] = ids.y; s_id[t][2] = ids.z; s_id[t][3] = ids.w;
         }
-        const int iB = s_at[0][r], i0 = s_at[1][r], i1 = s_at[2][r], i2 = s_at[3][r];
-        double sb = 0.0, s0 = 0.0, s1 = 0.0, s2 = 0.0;
-        const int c1 = g.bptr[blk + 1];
-        for (int c = g.bptr[blk]; c < c1; c++) {
-            const double *src = es + (size_t)g.bcon[c] * PL_NP;
-            if (iB >= 0) sb += src[iB];
-            if (i0 >= 0) s0 += src[i0];
-            if (i1 >= 0) s1 += src[i1];
-            if (i2 >= 0) s2 += src[i2];
+        for (int i = t; i < count; i += PG_THREADS) s_v[i] = s_b[i] = 0.0;
+        __syncthreads();
+        const int np = s_map.n;
+        for (int i = t; i < nb * np; i += PG_THREADS) {
+            const int b = i / np, q = i - b * np, n = s_n[b];
+            const double *src = es + s_map.pair[q];
+            double x = 0.0;
+            for (int k = 0; k < n; k++)
+                x += src[(size_t)(k < 4 ? s_id[b][k] : g.bcon[s_c0[b] + k]) * PL_NP];
+            const int m = s_map.m[q], at = s_map.at[q];
+            if (m >= 2)
+                s_x[b * PL_DEP + at] = x;
+            else
+                (m == 0 ? s_b : s_v)[at / ST_NEQ * wide + b * ST_NEQ + at % ST_NEQ] = x;
         }
-        if (B) B[slot] = store ? sb : B[slot] + sb;
+        __syncthreads();
+        int64_t slot[PG_OWN];
+#pragma unroll
+        for (int u = 0; u < PG_OWN; u++) {
+            const int i = t + u * PG_THREADS;
+            if (i >= count) continue;
+            const int jeq = i / wide, c = i - jeq * wide, b = c / ST_NEQ;
+            slot[u] = s_row[jeq] + s_off[b] + c - b * ST_NEQ;
+            if (B) B[slot[u]] = store ? s_b[i] : B[slot[u]] + s_b[i];
+        }
+        int at[PG_DEP];
+        double v0[PG_DEP], vx[PG_DEP];
+        bool sq[PG_DEP];
+#pragma unroll
+        for (int u = 0; u < PG_DEP; u++) {
+            const int d = t + u * PG_THREADS;
+            at[u] = -1;
+            if (d >= nb * PL_DEP) continue;
+            const int b = d / PL_DEP, j = d - b * PL_DEP, r = s_map.dr[j];
+            at[u] = r / ST_NEQ * wide + b * ST_NEQ + r % ST_NEQ;
+            v0[u] = s_v[at[u]];
+            vx[u] = s_x[d];
+            sq[u] = s_map.dpw[j] == 2;
+        }
         for (int k = 0; k < nk; k++) {
-            const double K = kw[k], v = __fma_rn(K, __fma_rn(K, s2, s1), s0);
-            A[k][slot] = store ? v : A[k][slot] + v;
+            const double K = kw[k], K2 = K * K;
+            double *Ak = A[k];
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < PG_DEP; u++)
+                if (at[u] >= 0) s_v[at[u]] = __fma_rn(sq[u] ? K2 : K, vx[u], v0[u]);
+            __syncthreads();
+#pragma unroll
+            for (int u = 0; u < PG_OWN; u++) {
+                const int i = t + u * PG_THREADS;
+                if (i < count) Ak[slot[u]] = store ? s_v[i] : Ak[slot[u]] + s_v[i];
+            }
         }
     }
 }
@@ -1263,6 +1305,7 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
     g.rowptr = ctx->d_rowptr;
     g.nptr = ctx->d_nptr;
     g.ncon = ctx->d_ncon;
+    g.nbptr = ctx->d_nbptr;
     g.brow = ctx->d_brow;
     g.boff = ctx->d_boff;
     g.bptr = ctx->d_bptr;
@@ -1276,11 +1319,20 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
         const int nm = fene || ctx->prm.ReN != 0.0 ? PL_NM : PL_NM0;
         if (!ctx->d_prec) SCK(cudaMalloc((void **)&ctx->d_prec, (size_t)ctx->nel * 9 * PL_REC * sizeof(double)));
         if (!ctx->d_pes) SCK(cudaMalloc((void **)&ctx->d_pes, (size_t)ctx->nel * PL_OUT * sizeof(double)));
-        PlMap map;
-        std::memset(map.at, -1, sizeof(map.at));
+        PlMap map = {};
+        int dep = 0;
         for (int q = 0; q < PL_NP; q++) {
             const bool on = q < PL_NV ? q < nv : (q < PL_NV + PL_NS ? q - PL_NV < ns : q - PL_NV - PL_NS < nm);
-            if (on) map.at[PL_PAIRS[q].m][PL_PAIRS[q].e * 10 + PL_PAIRS[q].f] = (signed char)q;
+            if (!on) continue;
+            const PlPair &pp = PL_PAIRS[q];
+            const int k = map.n++, r = pp.e * ST_NEQ + pp.f;
+            map.pair[k] = (unsigned char)q;
+            map.m[k] = (unsigned char)pp.m;
+            map.at[k] = (unsigned char)(pp.m >= 2 ? dep : r);
+            if (pp.m >= 2) {
+                map.dr[dep] = (unsigned char)r;
+                map.dpw[dep++] = (unsigned char)(pp.m - 1);
+            }
         }
         k_planar_coef<<<(ctx->nel + PC_EL - 1) / PC_EL, PC_THREADS, 0, s>>>(a, ctx->prm, ctx->d_prec);
         SCK(cudaGetLastError());
@@ -1288,12 +1340,8 @@ extern "C" int vefem_stability_assemble(vefem_ctx *ctx, const double *TLb, int n
         SCK(cudaFuncSetAttribute(k_planar_contract, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         k_planar_contract<<<ctx->nel, PK_WARPS * 32, smem, s>>>(ctx->d_prec, ctx->d_pes, nv, ns, nm);
         SCK(cudaGetLastError());
-        if (cover)
-            k_planar_gather<true><<<ctx->nnodes, PG_THREADS, 0, s>>>(
-                g, map, ctx->d_rowptr10, ctx->d_boff10, ctx->d_pes, nk, ctx->d_kw, ctx->d_Aptr, dB, store);
-        else
-            k_planar_gather<false><<<(unsigned)((nthr + PG_THREADS - 1) / PG_THREADS), PG_THREADS, 0, s>>>(
-                g, map, ctx->d_rowptr10, ctx->d_boff10, ctx->d_pes, nk, ctx->d_kw, ctx->d_Aptr, dB, store);
+        k_planar_gather<<<ctx->nnodes, PG_THREADS, 0, s>>>(g, map, ctx->d_rowptr10, ctx->d_boff10, ctx->d_pes, nk,
+                                                           ctx->d_kw, ctx->d_Aptr, dB, store);
         SCK(cudaGetLastError());
         ctx->launches += 3;
     } else {
