@@ -19,13 +19,13 @@
 //
 // What bounds it on GB300: the FP64 pipe, 2 multiply-adds per clock and SM
 // (0.63 T/s).  A sweep of element columns (vefem_frontal.cu) does 270 G
-// multiply-adds for 20,000 quads in 30,600 dependent steps; this tree does 63 G
-// in 273 (the pivots of the deepest path over 16), so the steps' latency
+// multiply-adds for 20,000 quads in 30,600 dependent steps; this tree does 50 G
+// in 260 (the pivots of the deepest path over 16), so the steps' latency
 // matters only near the root and the rest is FP64 throughput.  Eliminating the
 // pivot rows only and leaving the Schur complement to one product is 18% fewer
 // operations than Gauss-Jordan over the whole front, and a product has no
-// serial part.  Measured, factorise and solve: 1,184 ms (panels) -> 152 ms at
-// 20,000 quads, 89.5 -> 12.1 ms at 2,000; a solve checked to 1e-14 43.2 -> 2.6 ms
+// serial part.  Measured, factorise and solve: 1,185 ms (panels) -> 127 ms at
+// 20,000 quads, 89.9 -> 10.6 ms at 2,000; a solve checked to 1e-14 43.6 -> 1.6 ms
 // at 20,000 (2,500 panels are 5,000 dependent launches, the tree 41), and one
 // sweep already leaves a residual of 1e-15, where the panels' longer chain of
 // pivots left 1e-12 and took a refinement.

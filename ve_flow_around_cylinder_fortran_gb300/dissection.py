@@ -1,9 +1,9 @@
 """Nested-dissection fronts of the bordered Newton Jacobian: the symbolic phase
 of the tree elimination in ``frontal.py``.
 
-The elements are bisected recursively by their centroids, at every level along
-the axis that leaves fewer nodes on the cut, into a complete binary tree of
-element sets (heap numbering: root 1, children 2t and 2t + 1).  A node is
+The elements are bisected recursively by their centroids, at every level where
+a cut along x, y or a diagonal leaves the fewest nodes on it, into a complete
+binary tree of element sets (heap numbering: root 1, children 2t and 2t + 1).  A node is
 eliminated with the smallest set that holds all of its elements; the *front* of
 a set is made of the unknowns eliminated with it (its pivots) and those of its
 elements' nodes that are eliminated further up.  Fronts of one depth are
@@ -16,9 +16,37 @@ import math
 
 import numpy as np
 
-# elements per leaf: 2, 4, 8 cost 75.5, 76.8, 82.2 G multiply-adds at 20,000
-# quads; a leaf of 4 halves the fronts of 2 and stores 5% less
+# elements per leaf on average: 2, 4, 8 cost 62.0, 63.0, 66.9 G multiply-adds at
+# 20,000 quads (median cuts); a leaf of 4 halves the fronts of 2 and stores 5% less
 LEAF = 4
+
+
+# A cut may lie this far from the middle (of the elements), and larger sets than
+# MEDIAN also try the diagonals.  Multiply-adds of the elimination, 20,000 quads:
+# medians along x or y 63.0 G, and +-20% 54.1 G, and diagonals 49.2 G (2,000
+# quads: 2.3, 2.1, 1.8 G); +-30% 49.5 G.  Sets of up to MEDIAN elements take the
+# median along x or y: they are most of the sets and hardly any of the work.
+SLACK = 0.2
+MEDIAN = 24
+
+
+def _split(c: np.ndarray, sel: np.ndarray, en: np.ndarray, first: np.ndarray, last: np.ndarray):
+    """(score, lower, upper) of the best cut of the elements ``sel`` in the order
+    of ``c``: nodes on the cut, times 1 + its distance from the middle."""
+    n = len(sel)
+    order = sel[np.argsort(c[sel], kind="stable")]
+    v = en[order].reshape(-1)
+    pos = np.repeat(np.arange(n), en.shape[1])
+    first[v[::-1]] = pos[::-1]
+    last[v] = pos
+    own = first[v] == pos                               # every node once
+    cut = np.cumsum(np.bincount(pos[own] + 1, minlength=n + 2) - np.bincount(last[v[own]] + 1, minlength=n + 2))
+    slack = SLACK if n > MEDIAN else 0.0
+    k = np.arange(max(1, int(n * (0.5 - slack))), max(int(n * (0.5 + slack)), n // 2) + 1)
+    score = cut[k] * (1.0 + np.abs(k / n - 0.5))
+    j = int(np.argmin(score)) if slack else 0
+    k = int(k[j]) if slack else n // 2
+    return cut[k] * (1.0 + abs(k / n - 0.5)), order[:k], order[k:]
 
 
 def bisect(en: np.ndarray, cen: np.ndarray, leaf: int):
@@ -26,23 +54,18 @@ def bisect(en: np.ndarray, cen: np.ndarray, leaf: int):
     nel = en.shape[0]
     depth = max(0, math.ceil(math.log2(max(1.0, nel / leaf))))
     ids = np.ones(nel, dtype=np.int64)
-    mark = np.zeros(int(en.max()) + 1, dtype=bool)
+    first = np.empty(int(en.max()) + 1, dtype=np.int64)
+    last = np.empty_like(first)
+    axes = [cen[0], cen[1], cen[0] + cen[1], cen[0] - cen[1]]
     stack = [(np.arange(nel), 1, 0)]
     while stack:
         sel, node, d = stack.pop()
-        if d == depth:
-            ids[sel] = node
+        if d == depth or len(sel) < 2:
+            # a set too small to cut goes down the lower side
+            ids[sel] = node << (depth - d)
             continue
-        best = None
-        for c in cen:
-            o = np.argsort(c[sel], kind="stable")
-            lo, hi = sel[o[:len(sel) // 2]], sel[o[len(sel) // 2:]]
-            a, b = en[lo].ravel(), en[hi].ravel()
-            mark[a] = True
-            cut = np.unique(b[mark[b]]).size
-            mark[a] = False
-            if best is None or cut < best[0]:
-                best = (cut, lo, hi)
+        best = min((_split(c, sel, en, first, last) for c in axes[:2 if len(sel) <= MEDIAN else 4]),
+                   key=lambda s: s[0])
         stack.append((best[1], 2 * node, d + 1))
         stack.append((best[2], 2 * node + 1, d + 1))
     return ids, depth

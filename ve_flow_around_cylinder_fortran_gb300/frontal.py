@@ -13,8 +13,8 @@ Two orderings of the fronts:
 
 * Nested dissection (the default on a CUDA device): the fronts of a binary
   tree of element sets (``dissection.py``), all fronts of one depth at a time
-  in the library's kernels (``csrc/vefem_tree.cu``).  63 G multiply-adds and
-  273 dependent steps for 20,000 quads.
+  in the library's kernels (``csrc/vefem_tree.cu``).  50 G multiply-adds and
+  260 dependent steps for 20,000 quads.
 * Panels (``panel`` given, the pivoted method, the CPU): elements are swept
   downstream in order of their centroid x and grouped into panels of ``G``
   elements.  A node is *fully summed* after the last panel that touches it;
