@@ -1,0 +1,383 @@
+// FP64 matrix product on the bf16 tensor cores: a 128 x 48 tile of A B from
+// 64-bit fixed-point operands cut into eight digits.
+//
+// The FP64 pipe of this GPU does 2 multiply-adds per clock and SM, its tensor
+// cores 4,096 in bf16.  An entry of A becomes an integer of 63 bits relative to
+// the largest entry of its row (of B: of its column), written in eight balanced
+// digits of base 256, d in [-128, 127]: exact in bf16.  Digit a of A times digit
+// b of B has weight 256^(14-a-b); the products of equal a + b go to one FP32
+// accumulator, where sums over up to 128 k are at most 2^24 and therefore exact
+// integers.  The 43 pairs a + b <= 8 are kept.  The accumulators are added up in
+// 64-bit integers, so a result is rounded once, at the end.  (The error-free
+// splitting is that of Ozaki, Ogita, Oishi and Rump, "Error-free transformations
+// of matrix multiplication", Numer. Algorithms 59, 2012.)
+//
+// Error: quantisation and dropped pairs are below 2^-60 of (largest entry of the
+// row) x (largest entry of the column) per k.  The inner index is first scaled by
+// powers of two, exactly, so that every row of B has the same largest exponent
+// (inner_exponent): neither the units of the unknowns (stresses, velocities,
+// pressures) nor the size of a pivot then cost digits.  On the Schur
+// complements of a 2,000-quad Jacobian the error against extended precision is a
+// quarter of an FP64 product's (all its fronts and rows no larger); with the
+// pairs a + b <= 7 alone, or A's columns evened too, single rows were 2 to 14
+// times worse and the residual of a solve grew by 40%.
+//
+// One tcgen05.mma takes a digit of A (128 x 16) against several digits of B,
+// laid out as one operand of up to 256 columns: 14 instructions per 16 k.
+// Operands are cut by the CTA's 16 warps straight into the core-matrix layout
+// (8 rows x 16 bytes, no swizzle), two stages of 32 k, so the tensor core works
+// on one while the next is cut; the nine accumulators take 432 of the SM's 512
+// tensor memory columns, which is why a tile has 48 columns and not 64.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+namespace split {
+
+constexpr int TM = 128, TN = 48;       // tile
+constexpr int KS = 32;                 // k per stage
+constexpr int EXACT_K = 128;           // k per exact FP32 sum: 8 pairs x 128 x 2^14 = 2^24
+constexpr int ND = 8;                  // digits
+constexpr int NA = 9;                  // accumulators: sums of digit numbers kept
+constexpr int TMEM = 512;              // columns taken (a power of two)
+static_assert(NA * TN <= TMEM, "tensor memory");
+constexpr int THREADS = 512;
+constexpr int LBO_A = ND * TM * 16;    // bytes between k-neighbouring core matrices
+constexpr int LBO_B = ND * TN * 16;
+constexpr int STAGE_A = (KS / 8) * LBO_A, STAGE_B = (KS / 8) * LBO_B;
+constexpr int STAGE = STAGE_A + STAGE_B;
+constexpr int SMEM = 2 * STAGE;
+constexpr int OUT_LD = TN + 1;         // the result tile, in the stages' place
+static_assert(TM * OUT_LD * 8 <= SMEM, "result tile");
+constexpr int NOT_FINITE = 1 << 20;    // exponent of a row or column with an infinity or NaN
+constexpr int EMPTY = -(1 << 20);      // ... of one with zeros only
+
+// exponent field of the high word of |x|: 1 for subnormal numbers too
+__device__ __forceinline__ int field_of(int hi) { return max((hi >> 20) & 0x7ff, 1); }
+
+// high word of |x|, 0 for infinities and NaN
+__device__ __forceinline__ int finite_high(double x)
+{
+    const int hi = __double2hiint(x) & 0x7fffffff;
+    return hi < 0x7ff00000 ? hi : 0;
+}
+
+// power of two applied to column k of A (its inverse to row k of B) from the
+// largest high word of |B[k,:]|
+__device__ __forceinline__ int inner_exponent(int hi_b) { return hi_b ? field_of(hi_b) - 1023 : 0; }
+
+// exponent of x 2^s for a row's or column's largest
+__device__ __forceinline__ int scaled_exponent(double x, int s)
+{
+    const int hi = __double2hiint(x) & 0x7fffffff;
+    if (hi >= 0x7ff00000) return NOT_FINITE;
+    return (hi | __double2loint(x)) == 0 ? EMPTY : field_of(hi) + s;
+}
+
+// x 2^s 2^(1084 - top) to the nearest integer, biased by 128 in every byte
+__device__ __forceinline__ uint64_t fixed_point(double x, int s, int top)
+{
+    const int hi = __double2hiint(x);
+    const uint64_t m = ((uint64_t)((hi & 0xfffff) | ((hi & 0x7ff00000) ? 0x100000 : 0)) << 32) |
+                       (uint32_t)__double2loint(x);
+    const int sh = min(max(top - (field_of(hi) + s), 0), 63);
+    const uint64_t v = (((m << 10) >> sh) + 1) >> 1;
+    return (hi < 0 ? 0 - v : v) + 0x8080808080808080ull;
+}
+
+// the digits of eight k of one row, 16 bytes per digit
+template <int ROWS>
+__device__ __forceinline__ void put_digits(char *dst, const uint64_t (&w)[8])
+{
+#pragma unroll
+    for (int a = 0; a < ND; a++) {
+        uint32_t r[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const uint32_t w0 = (uint32_t)(w[2 * u] >> (a < 4 ? 32 : 0)), w1 = (uint32_t)(w[2 * u + 1] >> (a < 4 ? 32 : 0));
+            // 2^23 + byte, less 2^23 + 128: a small integer, its bf16 the upper half
+            const float f0 = __uint_as_float(__byte_perm(w0, 0x4b000000u, 0x7440u | (3 - (a & 3)))) - 8388736.0f;
+            const float f1 = __uint_as_float(__byte_perm(w1, 0x4b000000u, 0x7440u | (3 - (a & 3)))) - 8388736.0f;
+            r[u] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
+        }
+        *reinterpret_cast<uint4 *>(dst + a * ROWS * 16) = make_uint4(r[0], r[1], r[2], r[3]);
+    }
+}
+
+__device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// K-major operand without swizzle: leading offset along k, stride offset along rows
+__device__ __forceinline__ uint64_t operand(uint32_t addr, int lbo)
+{
+    return (uint64_t)((addr >> 4) & 0x3fff) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(128 >> 4) << 32) | (1ull << 46);
+}
+
+__device__ __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, int n, uint32_t accumulate)
+{
+    const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n / 8) << 17) | ((uint32_t)(TM / 16) << 24);
+    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d), "l"(a), "l"(b), "r"(idesc),
+                 "r"(accumulate)
+                 : "memory");
+}
+
+// bounded: the products of a stage take microseconds
+__device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity)
+{
+    for (int i = 0; i < (1 << 20); i++) {
+        uint32_t ok;
+        asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok)
+                     : "r"(bar), "r"(parity)
+                     : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+
+// W columns of a warp's 32 rows, as integers
+template <int W>
+__device__ __forceinline__ void tmem_load(uint32_t addr, int (&v)[W])
+{
+    static_assert(W == 4 || W == 8, "columns");
+    uint32_t r[8];
+    if constexpr (W == 8)
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                     : "r"(addr));
+    else
+        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                     : "r"(addr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < W; i++) v[i] = __float2int_rn(__uint_as_float(r[i]));
+}
+
+// hi 2^40 + lo += W columns of the nine accumulators, N columns apart (the one
+// of a + b = d is at most (d + 1) 2^21 in size, and 2^24)
+template <int N, int W>
+__device__ __forceinline__ void add_sums(uint32_t addr, int64_t *hi, int64_t *lo)
+{
+    int p[W], v[W];
+    tmem_load<W>(addr, p);
+    tmem_load<W>(addr + N, v);
+#pragma unroll
+    for (int i = 0; i < W; i++) hi[i] += (int64_t)(p[i] * 256 + v[i]) * 65536;
+    tmem_load<W>(addr + 2 * N, p);
+    tmem_load<W>(addr + 3 * N, v);
+#pragma unroll
+    for (int i = 0; i < W; i++) hi[i] += (int64_t)(p[i] * 256 + v[i]);
+    tmem_load<W>(addr + 4 * N, p);
+    tmem_load<W>(addr + 5 * N, v);
+#pragma unroll
+    for (int i = 0; i < W; i++) lo[i] += ((int64_t)p[i] * 256 + v[i]) * 16777216;
+    tmem_load<W>(addr + 6 * N, p);
+    tmem_load<W>(addr + 7 * N, v);
+#pragma unroll
+    for (int i = 0; i < W; i++) lo[i] += ((int64_t)p[i] * 256 + v[i]) * 256;
+    tmem_load<W>(addr + 8 * N, p);
+#pragma unroll
+    for (int i = 0; i < W; i++) lo[i] += p[i];
+}
+
+// (hi 2^40 + lo) 2^e rounded to a double, e from the largest exponents of row
+// and column.  In integers: two conversions, a multiply-add and a scaling would
+// be 64 clocks each per warp on the FP64 pipe, two thirds of a short tile.
+__device__ __forceinline__ double rounded(int64_t hi, int64_t lo, int ta, int tb)
+{
+    if (max(ta, tb) >= NOT_FINITE / 2) return __longlong_as_double(0x7ff8000000000000ll);
+    const int e = ta + tb - (2 * 1084 - 48);
+    int64_t top = hi + (lo >> 40);                                 // with rem, a fraction of 64 bits
+    uint64_t rem = (uint64_t)lo << 24;
+    const bool neg = top < 0;
+    if (neg) {
+        rem = 0 - rem;
+        top = ~top + (rem == 0);
+    }
+    uint64_t y;
+    int n;
+    if (top != 0) {
+        n = __clzll(top);
+        y = ((uint64_t)top << n) | (rem >> (64 - n));
+    } else {
+        if (rem == 0) return 0.0;
+        n = __clzll((long long)rem);
+        y = rem << n;
+        n += 64;
+    }
+    const uint64_t mant = (y >> 11) + ((y >> 10) & 1);             // 2^52 .. 2^53, times 2^(51 - n + e)
+    const int be = e + 51 - n + 52 + 1023;
+    double v;
+    if (be >= 1 && be < 2046)
+        v = __longlong_as_double((long long)(((uint64_t)(be - 1) << 52) + mant));
+    else
+        v = ldexp((double)mant, e + 51 - n);
+    return neg ? -v : v;
+}
+
+// 16 k: every digit of A with the digits of B it meets, N columns per digit.
+// accumulate = 0 starts the sums: digit 0 of A writes a + b = 0 .. 7, digit 1
+// with digit 7 of B writes a + b = 8.
+template <int N>
+__device__ __forceinline__ void mma_step(uint32_t tmem, uint32_t sa, uint32_t sb, int lbo_a, int lbo_b, uint32_t accumulate)
+{
+    constexpr int PER = 256 / N;                       // digits of B in one instruction
+    const uint64_t da = operand(sa, lbo_a), db = operand(sb, lbo_b);
+    auto go = [&](int a, int b, int count, uint32_t acc) { mma(tmem + (a + b) * N, da + a * TM, db + b * N, count * N, acc); };
+#pragma unroll
+    for (int a = 0; a < ND; a++) {
+        const int digits = a == 1 ? ND - 1 : a == 0 ? ND : NA - a;
+#pragma unroll
+        for (int b = 0; b < digits; b += PER) go(a, b, digits - b < PER ? digits - b : PER, a == 0 ? accumulate : 1u);
+        if (a == 1) go(a, ND - 1, 1, accumulate);
+    }
+}
+
+__device__ __forceinline__ void tmem_alloc(uint32_t *slot)
+{
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(slot)), "n"(TMEM) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void tmem_free(uint32_t tmem)
+{
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(TMEM) : "memory");
+}
+
+struct Operands {
+    const double *a;        // rows of A, k contiguous, 16-byte aligned rows
+    const double *b;        // rows k of B
+    int64_t lda, ldb;
+    int m, n, k;            // rows and columns left from the tile's corner, inner length
+    const int32_t *s;       // inner exponents
+    const int32_t *ta, *tb; // largest exponents of the tile's rows and columns
+};
+
+// out[row * OUT_LD + column] (shared) = the tile of A B; false (to all threads)
+// if a wait ran out.  smem: SMEM bytes, 1024-byte aligned; all 512 threads call.
+__device__ __forceinline__ bool product(char *smem, const Operands &o)
+{
+    __shared__ uint32_t s_tmem;
+    __shared__ __align__(8) uint64_t s_bar[2];
+    const int t = threadIdx.x, warp = t >> 5;
+    const uint32_t bar0 = smem_addr(&s_bar[0]);
+    if (warp == 0) tmem_alloc(&s_tmem);
+    if (t == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+
+    const int ra = t & (TM - 1), ga = t / TM;          // row and 8-k group of A (4 groups)
+    const int cb = t % TN, gb = t / TN;                // column and group of B (the first threads)
+    const int top_a = ra < o.m ? o.ta[ra] : EMPTY, top_b = cb < o.n ? o.tb[cb] : EMPTY;
+    const double *pa = o.a + (int64_t)min(ra, o.m - 1) * o.lda;
+    constexpr int PART = TN / 4;                       // columns of a warp's share
+    int64_t hi[PART], lo[PART];
+#pragma unroll
+    for (int i = 0; i < PART; i++) hi[i] = lo[i] = 0;
+    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * PART);
+    auto drain = [&]() {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        add_sums<TN, 8>(mine, hi, lo);
+        add_sums<TN, 4>(mine + 8, hi + 8, lo + 8);
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    };
+
+    const int steps = (o.k + KS - 1) / KS;
+    bool ok = true;
+    int sent = 0;                                      // stages handed to the tensor core
+    for (int st = 0; st < steps; st++) {
+        char *const stage = smem + (st & 1) * STAGE;
+        if (st >= 2) ok = wait(bar0 + 8 * (st & 1), ((st - 2) >> 1) & 1);
+        if (ra < o.m) {                                // rows beyond m stay undefined, and unread
+            const int k0 = st * KS + ga * 8;
+            double x[8];
+            int e[8];
+            if (k0 + 8 <= o.k) {
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const double2 v = __ldg(reinterpret_cast<const double2 *>(pa + k0) + u);
+                    x[2 * u] = v.x;
+                    x[2 * u + 1] = v.y;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; u++) e[u] = __ldg(o.s + k0 + u);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 8; u++) {
+                    const bool in = k0 + u < o.k;
+                    x[u] = in ? pa[k0 + u] : 0.0;
+                    e[u] = in ? o.s[k0 + u] : 0;
+                }
+            }
+            uint64_t w[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) w[u] = fixed_point(x[u], e[u], top_a);
+            put_digits<TM>(stage + ga * LBO_A + ra * 16, w);
+        }
+        if (t < TN * (KS / 8) && cb < o.n) {
+            const int k0 = st * KS + gb * 8;
+            uint64_t w[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const bool in = k0 + u < o.k;
+                const double x = in ? o.b[(int64_t)(k0 + u) * o.ldb + cb] : 0.0;
+                w[u] = fixed_point(x, in ? -o.s[k0 + u] : 0, top_b);
+            }
+            put_digits<TN>(stage + STAGE_A + gb * LBO_B + cb * 16, w);
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        if (st > 0 && st % (EXACT_K / KS) == 0) {      // the exact sums are full
+            ok = wait(bar0 + 8 * ((st - 1) & 1), ((st - 1) >> 1) & 1) && ok;
+            __syncwarp();
+            if (__all_sync(0xffffffffu, ok)) drain();
+        }
+        if (__syncthreads_or(!ok)) {
+            ok = false;
+            break;
+        }
+        if (t == 0) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t sa = smem_addr(stage), sb = sa + STAGE_A;
+            const int halves = min(KS / 16, (o.k - st * KS + 15) / 16);
+            for (int h = 0; h < halves; h++)
+                mma_step<TN>(tmem, sa + h * 2 * LBO_A, sb + h * 2 * LBO_B, LBO_A, LBO_B,
+                             (st % (EXACT_K / KS) != 0 || h > 0) ? 1u : 0u);
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                             bar0 + 8 * (st & 1))
+                         : "memory");
+        }
+        __syncwarp();
+        sent = st + 1;
+    }
+    // the last two stages' products (also after a failed wait, again bounded)
+    bool done = true;
+    if (sent > 1) done = wait(bar0 + 8 * ((sent - 2) & 1), ((sent - 2) >> 1) & 1);
+    if (sent > 0) done = wait(bar0 + 8 * ((sent - 1) & 1), ((sent - 1) >> 1) & 1) && done;
+    ok = !__syncthreads_or(!(ok && done));
+    if (ok) {
+        drain();
+        double *out = reinterpret_cast<double *>(smem);
+        const int row = (warp & 3) * 32 + (t & 31), col = (warp >> 2) * PART;
+        const int ta = row < o.m ? o.ta[row] : EMPTY;
+#pragma unroll
+        for (int i = 0; i < PART; i++) {
+            const int tb = col + i < o.n ? o.tb[col + i] : EMPTY;
+            out[row * OUT_LD + col + i] = rounded(hi[i], lo[i], ta, tb);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) tmem_free(tmem);
+    return ok;
+}
+
+}  // namespace split

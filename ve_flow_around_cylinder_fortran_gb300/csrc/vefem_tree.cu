@@ -15,17 +15,21 @@
 //               rows i (M[i,K] = -C_i D^-1), M[K,:] = T: blocked Gauss-Jordan
 //               without pivoting on the pivot rows only, which leaves
 //               M[P,P] = A^-1 and M[P,F] = X = A^-1 B;
-//   k_schur     M[F,F] -= C X, one tiled product.
+//   k_schur     M[F,F] -= C X, one tiled product on the tensor cores
+//               (vefem_split.cuh), for which k_split_inner and k_split_outer
+//               find the exponents.
 //
 // What bounds it on GB300: the FP64 pipe, 2 multiply-adds per clock and SM
-// (0.63 T/s).  A sweep of element columns (vefem_frontal.cu) does 270 G
+// (0.63 T/s), up to the Schur complements.  A sweep of element columns (vefem_frontal.cu) does 270 G
 // multiply-adds for 20,000 quads in 30,600 dependent steps; this tree does 50 G
 // in 260 (the pivots of the deepest path over 16), so the steps' latency
 // matters only near the root and the rest is FP64 throughput.  Eliminating the
 // pivot rows only and leaving the Schur complement to one product is 18% fewer
 // operations than Gauss-Jordan over the whole front, and a product has no
-// serial part.  Measured, factorise and solve: 1,185 ms (panels) -> 127 ms at
-// 20,000 quads, 89.9 -> 10.6 ms at 2,000; a solve checked to 1e-14 43.6 -> 1.6 ms
+// serial part: 35 G of the 50 G multiply-adds, 70 ms on the FP64 pipe and 20 ms
+// (exponents included) in bf16 digits.  Measured, factorise and solve: 1,185 ms
+// (panels) -> 127 (all on the FP64 pipe) -> 76 ms at 20,000 quads, 89.9 -> 10.6
+// -> 8.1 ms at 2,000; a solve checked to 1e-14 43.6 -> 1.6 ms
 // at 20,000 (2,500 panels are 5,000 dependent launches, the tree 41), and one
 // sweep already leaves a residual of 1e-15, where the panels' longer chain of
 // pivots left 1e-12 and took a refinement.
@@ -47,6 +51,7 @@
 
 #include "vefem.h"
 #include "vefem_gj.cuh"
+#include "vefem_split.cuh"
 
 namespace {
 
@@ -226,64 +231,87 @@ k_update(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0,
     }
 }
 
-// M[F,F] -= M[F,P] M[P,F]
-__global__ void __launch_bounds__(256, 2)
-k_schur(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int nt, double *__restrict__ buf)
+// Scaling of the split product: the power of two that evens row k of X (e0 at
+// the pivots' places); then, per 32 boundary unknowns, the largest exponent of
+// their row of C (e0) and column of X (e1).
+__global__ void __launch_bounds__(256)
+k_split_inner(const Front *__restrict__ fr, const int32_t *__restrict__ perm, const double *__restrict__ buf,
+              int32_t *__restrict__ e0)
 {
-    __shared__ double sa[2][NB][TILE + 2];
-    __shared__ __align__(16) double sb[2][NB][TILE];
+    const Front f = fr[perm[blockIdx.x]];
+    const int k0 = blockIdx.y * 32, x = threadIdx.x & 31;
+    for (int r = k0 + (threadIdx.x >> 5); r < min(k0 + 32, f.p); r += 8) {
+        const double *row = buf + f.off + (int64_t)r * f.ld;
+        int b = 0;
+        for (int j = f.p + x; j < f.n; j += 32) b = max(b, split::finite_high(row[j]));
+        b = __reduce_max_sync(0xffffffffu, b);
+        if (x == 0) e0[f.base + r] = split::inner_exponent(b);
+    }
+}
+
+__global__ void __launch_bounds__(256)
+k_split_outer(const Front *__restrict__ fr, const int32_t *__restrict__ perm, const double *__restrict__ buf, int32_t *e0,
+              int32_t *__restrict__ e1)
+{
+    __shared__ int s_b[8][32];
+    const Front f = fr[perm[blockIdx.x]];
+    const int i0 = blockIdx.y * 32, q = f.n - f.p;
+    if (i0 >= q) return;
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const double *M = buf + f.off;
+    const int32_t *sk = e0 + f.base;
+    for (int r = y; r < 32 && i0 + r < q; r += 8) {
+        const double *row = M + (int64_t)(f.p + i0 + r) * f.ld;
+        int a = split::EMPTY;
+        for (int k = x; k < f.p; k += 32) a = max(a, split::scaled_exponent(row[k], sk[k]));
+        a = __reduce_max_sync(0xffffffffu, a);
+        if (x == 0) e0[f.base + f.p + i0 + r] = a;
+    }
+    int b = split::EMPTY;
+    if (i0 + x < q)
+        for (int k = y; k < f.p; k += 8) b = max(b, split::scaled_exponent(M[(int64_t)k * f.ld + f.p + i0 + x], -sk[k]));
+    s_b[y][x] = b;
+    __syncthreads();
+    if (y == 0 && i0 + x < q) {
+#pragma unroll
+        for (int r = 1; r < 8; r++) b = max(b, s_b[r][x]);
+        e1[f.base + f.p + i0 + x] = b;
+    }
+}
+
+// M[F,F] -= M[F,P] M[P,F] on the tensor cores, for every p: fronts with fewer
+// than 16, 32 or 64 pivots left to a tiled FP64 product made 20,000 quads 0.2,
+// 2.1 and 9.4 ms slower.  Bound by the cutting of the operands
+// (integer instructions) and, in the deepest levels, by a tile's fixed cost.
+__global__ void __launch_bounds__(split::THREADS, 1)
+k_schur(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int ntc, const int32_t *__restrict__ e0,
+              const int32_t *__restrict__ e1, double *__restrict__ buf, int *err)
+{
+    extern __shared__ __align__(1024) char s_stage[];
     const Front f = fr[perm[blockIdx.x]];
     const int q = f.n - f.p;
-    const int i0 = (blockIdx.y / nt) * TILE, j0 = (blockIdx.y % nt) * TILE;
+    const int i0 = (blockIdx.y / ntc) * split::TM, j0 = (blockIdx.y % ntc) * split::TN;
     if (i0 >= q || j0 >= q || f.p == 0) return;
     double *M = buf + f.off;
-    const int t = threadIdx.x;
-    // a thread stages 4 entries of A (one row, 4 consecutive k) and 4 of B (one k, 4 columns)
-    const int ar = t >> 2, ak = (t & 3) * 4, bk = t >> 4, bc = (t & 15) * 4;
-    const double *pa = M + (int64_t)(f.p + min(i0 + ar, q - 1)) * f.ld;
-    const double *pb = M + f.p + j0;
-    double va[4], vb[4];
-    auto fetch = [&](int k) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            va[u] = k + ak + u < f.p ? pa[k + ak + u] : 0.0;
-            vb[u] = (k + bk < f.p && j0 + bc + u < q) ? pb[(int64_t)(k + bk) * f.ld + bc + u] : 0.0;
-        }
-    };
-    auto stage = [&](int s) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            sa[s][ak + u][ar] = va[u];
-            sb[s][bk][bc + u] = vb[u];
-        }
-    };
-    const int w = t >> 5, lane = t & 31;
-    const int wr = (w >> 1) * 16, wc = (w & 1) * 32;
-    const int r = wr + (lane >> 3) * 4, c = wc + (lane & 7) * 2;
-    const bool live = i0 + wr < q && j0 + wc < q;
-    double acc[4][4] = {};
-    fetch(0);
-    stage(0);
-    __syncthreads();
-    int s = 0;
-    for (int k = 0; k < f.p; k += NB, s ^= 1) {
-        const bool more = k + NB < f.p;
-        if (more) fetch(k + NB);
-        if (live) tile_fma(acc, sa[s], sb[s], r, c);
-        if (more) stage(s ^ 1);
-        __syncthreads();
+    split::Operands o;
+    o.a = M + (int64_t)(f.p + i0) * f.ld;
+    o.b = M + f.p + j0;
+    o.lda = o.ldb = f.ld;
+    o.m = min(q - i0, split::TM);
+    o.n = min(q - j0, split::TN);
+    o.k = f.p;
+    o.s = e0 + f.base;
+    o.ta = e0 + f.base + f.p + i0;
+    o.tb = e1 + f.base + f.p + j0;
+    if (!split::product(s_stage, o)) {
+        if (threadIdx.x == 0) atomicExch(err, 2);
+        return;
     }
-    if (!live) return;
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int i = i0 + r + u;
-        if (i >= q) continue;
-        double *row = M + (int64_t)(f.p + i) * f.ld + f.p + j0;
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            const int cc = c + (v & 1) + 16 * (v >> 1);
-            if (j0 + cc < q) row[cc] -= acc[u][v];
-        }
+    const double *out = reinterpret_cast<const double *>(s_stage);
+    double *S = M + (int64_t)(f.p + i0) * f.ld + f.p + j0;
+    for (int u = threadIdx.x; u < o.m * split::TN; u += split::THREADS) {
+        const int r = u / split::TN, c = u % split::TN;
+        if (c < o.n) S[(int64_t)r * f.ld + c] -= out[r * split::OUT_LD + c];
     }
 }
 
@@ -405,6 +433,7 @@ struct vefem_tree {
     int pmax = 0, qmax = 0;
     Front *fr = nullptr;
     int32_t *perm = nullptr, *ids = nullptr, *src0 = nullptr, *src1 = nullptr;
+    int32_t *e0 = nullptr, *e1 = nullptr;   // exponents of the split products
     double *cpan = nullptr, *tpan = nullptr;
     double *y = nullptr, *b = nullptr, *x = nullptr;
     int *err = nullptr;
@@ -556,12 +585,15 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
         cudaDeviceGetAttribute(&f->sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&
         cudaStreamCreateWithFlags(&f->cs, cudaStreamNonBlocking) == cudaSuccess && put(&f->fr, fr.data(), fr.size()) &&
         put(&f->perm, perm.data(), perm.size()) && put(&f->ids, ids32.data(), ids32.size()) &&
-        put(&f->src0, src, (size_t)tot) && put(&f->src1, src + tot, (size_t)tot) && put(&f->cpan, none, (size_t)cmax) &&
+        put(&f->src0, src, (size_t)tot) && put(&f->src1, src + tot, (size_t)tot) &&
+        put(&f->e0, (const int32_t *)nullptr, (size_t)tot) && put(&f->e1, (const int32_t *)nullptr, (size_t)tot) && put(&f->cpan, none, (size_t)cmax) &&
         put(&f->tpan, none, (size_t)tmax) && put(&f->y, none, (size_t)tot) && put(&f->b, none, (size_t)N) &&
         put(&f->x, none, (size_t)N) && put(&f->err, (const int *)nullptr, 1) &&
         put(&f->minpiv, (const unsigned long long *)nullptr, 1);
     const int sm_p = f->pmax * (int)sizeof(double), sm_q = f->qmax * (int)sizeof(double);
-    if (!ok || (sm_p > 48 * 1024 &&
+    if (!ok ||
+        cudaFuncSetAttribute(k_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SMEM) != cudaSuccess ||
+        (sm_p > 48 * 1024 &&
                 (cudaFuncSetAttribute(k_tree_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess ||
                  cudaFuncSetAttribute(k_tree_up, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess)) ||
         (sm_q > 48 * 1024 &&
@@ -604,8 +636,11 @@ extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_
             k_update<<<dim3(a, ntc * up(l.pmax, TILE)), 256, 0, s>>>(f->fr, perm, k0, ntc, f->cpan, f->tpan, buf);
         }
         if (l.qmax > 0 && l.pmax > 0) {
-            const int nt = (int)up(l.qmax, TILE);
-            k_schur<<<dim3(l.count, nt * nt), 256, 0, s>>>(f->fr, perm, nt, buf);
+            const int ntc = (int)up(l.qmax, split::TN);
+            k_split_inner<<<dim3(l.count, up(l.pmax, 32)), 256, 0, s>>>(f->fr, perm, buf, f->e0);
+            k_split_outer<<<dim3(l.count, up(l.qmax, 32)), 256, 0, s>>>(f->fr, perm, buf, f->e0, f->e1);
+            k_schur<<<dim3(l.count, ntc * up(l.qmax, split::TM)), split::THREADS, split::SMEM, s>>>(
+                f->fr, perm, ntc, f->e0, f->e1, buf, f->err);
         }
     }
     TCK(cudaGetLastError());
@@ -615,6 +650,7 @@ extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_
     TCK(cudaMemcpyAsync(&hmin, f->minpiv, sizeof(hmin), cudaMemcpyDeviceToHost, s));
     TCK(cudaStreamSynchronize(s));
     if (min_pivot) std::memcpy(min_pivot, &hmin, sizeof(double));
+    if (herr == 2) return tfail(f, VEFEM_ERR_CUDA, "a wait for the tensor core ran out");
     if (herr) return tfail(f, VEFEM_ERR_SINGULAR, "a pivot below the tolerance (unpivoted elimination)");
     return VEFEM_OK;
 }
@@ -662,7 +698,7 @@ extern "C" void vefem_tree_destroy(vefem_tree *f)
         Guard g(f->device);
         if (f->graph) cudaGraphExecDestroy(f->graph);
         if (f->cs) cudaStreamDestroy(f->cs);
-        void *p[] = {f->fr, f->perm, f->ids, f->src0, f->src1, f->cpan, f->tpan, f->y, f->b, f->x, f->err, f->minpiv};
+        void *p[] = {f->fr, f->perm, f->ids, f->src0, f->src1, f->e0, f->e1, f->cpan, f->tpan, f->y, f->b, f->x, f->err, f->minpiv};
         for (void *q : p) cudaFree(q);
     }
     delete f;
