@@ -1,5 +1,5 @@
-"""The Schur complement of a front on the tensor cores (csrc/vefem_split.cuh):
-one front of p pivots and q boundary unknowns whose pivot block is the
+"""The elimination of a front on the tensor cores (csrc/vefem_split.cuh): one front
+of given entries, its inverse and solution by their residuals, and one front of p pivots and q boundary unknowns whose pivot block is the
 identity, so that it is D - C B with the entries given, against the same in
 extended precision, at sizes around the tile (128 x 48), the stage (32), the
 exact sum (128)."""
@@ -21,7 +21,8 @@ def _built():
     V.load()
 
 
-def _schur(C, X, D):
+def _eliminate(A, C, X, D):
+    """The front [A X; C D] after its p pivots: [A^-1, A^-1 X; C, D - C A^-1 X]."""
     q, p = C.shape
     n = np.array([p + q, q], np.int32)
     ld = (n + 3) // 4 * 4
@@ -38,7 +39,7 @@ def _schur(C, X, D):
     lev = np.array([0, 1, 2], np.int32)
     assert lib.vefem_tree_create(0, 2, 2, ptr(lev), ptr(off), ptr(n), ptr(piv), ptr(ld), ptr(child), ptr(ids),
                                  ptr(idx_off), ptr(src), ct.c_int64(p + q), ct.byref(h)) == 0
-    M = np.block([[np.eye(p), X], [C, D]])
+    M = np.block([[A, X], [C, D]])
     dest = (np.arange(p + q)[:, None] * int(ld[0]) + np.arange(p + q)).ravel()
     vals = torch.from_numpy(M.ravel()).cuda()
     dest = torch.from_numpy(dest.astype(np.int64)).cuda()
@@ -50,9 +51,14 @@ def _schur(C, X, D):
                           ct.c_void_p(buf.data_ptr()), ct.c_int64(buf.numel()), ct.c_void_p(0), ct.c_double(1e-12),
                           ct.byref(mp))
     torch.cuda.synchronize()
-    got = buf[:int(off[1])].cpu().numpy().reshape(p + q, int(ld[0]))[p:, p:p + q]
+    got = buf[:int(off[1])].cpu().numpy().reshape(p + q, int(ld[0]))[:, :p + q]
     lib.vefem_tree_destroy(h)
     return got
+
+
+def _schur(C, X, D):
+    p = C.shape[1]
+    return _eliminate(np.eye(p), C, X, D)[p:, p:]
 
 
 def _operands(p, q, seed):
@@ -82,6 +88,22 @@ def test_units_cost_no_digits(p, q):
     exact = D - C.astype(np.longdouble) @ X.astype(np.longdouble)
     err = np.abs(_schur(C, X, D) - exact).astype(float)
     assert np.all(err <= 2.0 ** -53 * (p + 2) * (np.abs(C) @ np.abs(X) + np.abs(D)))
+
+
+@pytest.mark.parametrize("p,q", [(1, 3), (15, 20), (16, 31), (17, 33), (31, 97), (32, 96), (33, 15), (64, 64), (97, 31),
+                                 (128, 16), (129, 47), (161, 200)])
+def test_inverse_and_solution(p, q):
+    r = np.random.default_rng(p)
+    C, X, D = _operands(p, q, q)
+    scale = 2.0 ** r.integers(-40, 41, p)                # equations and unknowns of any unit
+    A = (r.uniform(-1, 1, (p, p)) + 2.0 * p * np.eye(p)) * scale / scale[::-1, None]
+    X = X / scale[::-1, None]
+    M = _eliminate(A, C, X, D).astype(np.longdouble)
+    inv, sol = M[:p, :p], M[:p, p:]
+    # diagonally dominant up to its scaling: no growth, at most 2 p roundings of |A| |A^-1| per entry
+    bound = lambda Y: 2.0 ** -53 * 4 * (p + 2) * (np.abs(A) @ np.abs(Y))
+    assert np.all(np.abs(A @ inv - np.eye(p)) <= bound(inv))
+    assert np.all(np.abs(A @ sol - X) <= bound(sol))
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])

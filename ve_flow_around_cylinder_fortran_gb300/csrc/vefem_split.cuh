@@ -380,4 +380,127 @@ __device__ __forceinline__ bool product(char *smem, const Operands &o)
     return ok;
 }
 
+// ---- products of up to 32 inner indices: one stage, exponents found by the CTA
+
+constexpr int SHORT_THREADS = 256;
+template <int N>
+constexpr int SHORT_SMEM = (KS / 8) * ND * (TM + N) * 16;
+
+// out[row * (N + 1) + column] (shared) = sum over k < 32 of A[row, k] fb(k, column)
+// for m rows and n columns; fa(row, k, x) gives A[row, k .. k + 7], and fa and
+// fb give 0 for k outside.  EVEN_A: the columns of A, not the rows of B, are the
+// ones evened (the transpose of a product evens its right factor so).  The tensor memory
+// is taken after the operands are cut: with two CTAs on an SM one cuts while
+// the other multiplies.
+template <int N, bool EVEN_A, class FA, class FB>
+__device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, FB fb)
+{
+    constexpr int LA = ND * TM * 16, LB = ND * N * 16;
+    static_assert(TM * (N + 1) * 8 <= SHORT_SMEM<N>, "result tile");
+    __shared__ uint32_t s_tmem;
+    __shared__ __align__(8) uint64_t s_bar;
+    __shared__ int s_k[KS], s_ta[TM], s_tb[N];
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const uint32_t bar = smem_addr(&s_bar);
+    if (t < KS) s_k[t] = 0;
+    if (t < TM) s_ta[t] = EMPTY;
+    if (t < N) s_tb[t] = EMPTY;
+    if (t == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    const int ra = t & (TM - 1), ga = t / TM;          // row, and 8-k groups ga and ga + 2 of A
+    // columns 16 to a half warp, so that one maximum per half warp is one k's
+    const int hw = t / 16, gb = hw / (N / 16), cb = hw % (N / 16) * 16 + (t & 15);
+    const bool in_a = ra < m, in_b = gb < KS / 8 && cb < n;
+    double xa[2][8], xb[8];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+#pragma unroll
+        for (int u = 0; u < 8; u++) xa[h][u] = 0.0;
+        if (in_a) fa(ra, (ga + 2 * h) * 8, xa[h]);
+    }
+#pragma unroll
+    for (int u = 0; u < 8; u++) xb[u] = in_b ? fb(gb * 8 + u, cb) : 0.0;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        if (EVEN_A) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int r = __reduce_max_sync(0xffffffffu, finite_high(xa[h][u]));
+                if (lane == 0) atomicMax(&s_k[(ga + 2 * h) * 8 + u], r);
+            }
+        } else {
+            const int r = __reduce_max_sync(0xffffu << (lane & 16), finite_high(xb[u]));
+            if ((t & 15) == 0 && gb < KS / 8) atomicMax(&s_k[gb * 8 + u], r);
+        }
+    }
+    __syncthreads();
+    auto inner = [&](int k) { return EVEN_A ? -inner_exponent(s_k[k]) : inner_exponent(s_k[k]); };
+    int ta = EMPTY, tb = EMPTY;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) ta = max(ta, scaled_exponent(xa[h][u], inner((ga + 2 * h) * 8 + u)));
+        if (in_b) tb = max(tb, scaled_exponent(xb[u], -inner(gb * 8 + u)));
+    }
+    if (in_a) atomicMax(&s_ta[ra], ta);
+    if (in_b) atomicMax(&s_tb[cb], tb);
+    __syncthreads();
+    uint64_t w[8];
+    if (in_a) {
+        ta = s_ta[ra];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int g = ga + 2 * h;
+#pragma unroll
+            for (int u = 0; u < 8; u++) w[u] = fixed_point(xa[h][u], inner(g * 8 + u), ta);
+            put_digits<TM>(smem + g * LA + ra * 16, w);
+        }
+    }
+    if (in_b) {
+        tb = s_tb[cb];
+#pragma unroll
+        for (int u = 0; u < 8; u++) w[u] = fixed_point(xb[u], -inner(gb * 8 + u), tb);
+        put_digits<N>(smem + (KS / 8) * LA + gb * LB + cb * 16, w);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (warp == 0) tmem_alloc(&s_tmem);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    if (t == 0) {
+        const uint32_t sa = smem_addr(smem), sb = sa + (KS / 8) * LA;
+        for (int h = 0; h < KS / 16; h++) mma_step<N>(tmem, sa + h * 2 * LA, sb + h * 2 * LB, LA, LB, h > 0 ? 1u : 0u);
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    }
+    __syncwarp();
+    bool ok = wait(bar, 0);
+    if (!ok) ok = wait(bar, 0);
+    ok = !__syncthreads_or(!ok);
+    if (ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        double *out = reinterpret_cast<double *>(smem);
+        const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * (N / 2);
+        ta = s_ta[row];
+#pragma unroll 1
+        for (int c = c0; c < c0 + N / 2; c += 8) {
+            int64_t hi[8], lo[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) hi[i] = lo[i] = 0;
+            add_sums<N, 8>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c, hi, lo);
+            if (row < m)
+#pragma unroll
+                for (int i = 0; i < 8; i++) out[row * (N + 1) + c + i] = rounded(hi[i], lo[i], ta, s_tb[c + i]);
+            __syncwarp();
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0) tmem_free(tmem);
+    return ok;
+}
+
 }  // namespace split

@@ -10,29 +10,29 @@
 //
 //   k_assemble  M += the children's Schur complements (pulled entry by entry,
 //               first child before second: no atomics, the same bits every run);
-//   k_pivot     per 16 pivots K: D^-1 and T = D^-1 M[K,:], and a copy of the
-//   k_update    columns C = M[P,K]; then M[i,:] -= C_i T for the other pivot
-//               rows i (M[i,K] = -C_i D^-1), M[K,:] = T: blocked Gauss-Jordan
-//               without pivoting on the pivot rows only, which leaves
-//               M[P,P] = A^-1 and M[P,F] = X = A^-1 B;
-//   k_schur     M[F,F] -= C X, one tiled product on the tensor cores
-//               (vefem_split.cuh), for which k_split_inner and k_split_outer
-//               find the exponents.
+//   k_invert    per 32 pivots K: D^-1, D = M[K,K];
+//   k_pivot     T = D^-1 M[K,:], and a copy of the columns C = M[P,K];
+//   k_update    M[i,:] -= C_i T for the other pivot rows i (M[i,K] = -C_i D^-1),
+//               M[K,:] = T: blocked Gauss-Jordan without pivoting on the pivot
+//               rows only, which leaves M[P,P] = A^-1 and M[P,F] = X = A^-1 B;
+//   k_schur     M[F,F] -= C X, for which k_split_inner and k_split_outer find
+//               the exponents.
 //
-// What bounds it on GB300: the FP64 pipe, 2 multiply-adds per clock and SM
-// (0.63 T/s), up to the Schur complements.  A sweep of element columns (vefem_frontal.cu) does 270 G
-// multiply-adds for 20,000 quads in 30,600 dependent steps; this tree does 50 G
-// in 260 (the pivots of the deepest path over 16), so the steps' latency
-// matters only near the root and the rest is FP64 throughput.  Eliminating the
-// pivot rows only and leaving the Schur complement to one product is 18% fewer
-// operations than Gauss-Jordan over the whole front, and a product has no
-// serial part: 35 G of the 50 G multiply-adds, 70 ms on the FP64 pipe and 20 ms
-// (exponents included) in bf16 digits.  Measured, factorise and solve: 1,185 ms
-// (panels) -> 127 (all on the FP64 pipe) -> 76 ms at 20,000 quads, 89.9 -> 10.6
-// -> 8.1 ms at 2,000; a solve checked to 1e-14 43.6 -> 1.6 ms
-// at 20,000 (2,500 panels are 5,000 dependent launches, the tree 41), and one
-// sweep already leaves a residual of 1e-15, where the panels' longer chain of
-// pivots left 1e-12 and took a refinement.
+// What bounds it on GB300: on the FP64 pipe (2 multiply-adds per clock and SM,
+// 0.63 T/s) the 50 G multiply-adds of 20,000 quads are 80 ms, so every product
+// goes to the tensor cores in bf16 digits (vefem_split.cuh) and only the
+// inversion of the 32 x 32 pivot blocks stays on that pipe.  What is left is the
+// fixed cost of a tile in the deep levels and the chain of 133 steps near the
+// root.  A sweep of element columns (vefem_frontal.cu) does 270 G multiply-adds
+// in 30,600 dependent steps.  Eliminating the pivot rows only and leaving the
+// Schur complement to one product is 18% fewer operations than Gauss-Jordan
+// over the whole front.  Measured, factorise and solve, 20,000 and 2,000 quads:
+// panels 1,185 and 89.9 ms; the tree on the FP64 pipe, 16 pivots a step, 127 and
+// 10.6; Schur complements in digits 76 and 8.1; all products in digits, 32
+// pivots a step, 55.8 and 7.0.  A solve checked to 1e-14 went from 43.6 to 1.6
+// ms at 20,000 (2,500 panels are 5,000 dependent launches, the tree 41): one
+// sweep leaves a residual of 1e-15, where the panels' longer chain of pivots
+// left 1e-12 and took a refinement.
 //
 // Solve: per depth, deepest first, y_P = A^-1 b_P and the update -C y_P a
 // front hands to its parent; then, root first, x_P = y_P - X x_F.  A row's dot
@@ -57,8 +57,8 @@ namespace {
 
 struct Front {
     int64_t off;       // first entry of the matrix in the factor buffer
-    int64_t cpan;      // first entry of the pivot-column copy (16 per pivot row)
-    int64_t tpan;      // first entry of T (16 rows of ld)
+    int64_t cpan;      // first entry of the pivot-column copy (32 per pivot row)
+    int64_t tpan;      // first entry of T (32 rows of ld)
     int32_t base;      // first entry of the front's unknowns, maps and vectors
     int32_t n, p, ld;
     int32_t child[2];  // front index, or -1
@@ -99,135 +99,153 @@ k_assemble(const Front *__restrict__ fr, const int32_t *__restrict__ perm, const
     }
 }
 
-// Step on pivots K = [k0, k0 + kb): every CTA inverts D = M[K,K] (the same
-// bits in each) and forms T for its W columns; columns K of T hold D^-1.
-// W = 32 spreads the T of a few large fronts over many SMs, W = 128 inverts
-// less often where there are many fronts.
-template <int W>
+constexpr int KB = 2 * NB;   // pivots per step
+
+// The inverse of D = M[K,K], K = [k0, k0 + kb), transposed to dinv: blocked
+// Gauss-Jordan in two steps of 16 pivots, a CTA per front.  Bound by its own
+// chain, 2 x 16 pivots, where the fronts are few, and by the FP64 pipe (32^3
+// multiply-adds) where they are many.
 __global__ void __launch_bounds__(128)
-k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
-        double *__restrict__ cpan, double *__restrict__ tpan, int *err, unsigned long long *minpiv, double tol)
+k_invert(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
+         double *__restrict__ dinv, int *err, unsigned long long *minpiv, double tol)
 {
-    __shared__ double sA[2 * NB][NB + 1];
+    __shared__ double sW[KB][KB + 1], sT[NB][KB + 1], sA[2 * NB][NB + 1];
     __shared__ double s_red[4];
     const Front f = fr[perm[blockIdx.x]];
-    const int j0 = blockIdx.y * W;
-    if (j0 >= f.ld) return;
-    const int kb = min(NB, f.p - k0), t = threadIdx.x;
-    const double *M = buf + f.off;
-    for (int u = t; u < 2 * NB * NB; u += 128) {
-        const int c = u / NB, r = u % NB;
-        double v;
-        if (c < NB)
-            v = (r < kb && c < kb) ? M[(int64_t)(k0 + r) * f.ld + k0 + c] : (r == c ? 1.0 : 0.0);
-        else
-            v = (r == c - NB) ? 1.0 : 0.0;
-        sA[c][r] = v;
-    }
-    // this CTA's share of the pivot-column copy
-    for (int u = t; u < W * NB; u += 128) {
-        const int r = j0 + u / NB, l = u % NB;
-        if (r < f.p) cpan[f.cpan + (int64_t)r * NB + l] = l < kb ? M[(int64_t)r * f.ld + k0 + l] : 0.0;
-    }
-    __syncthreads();
-    const double rel = block_invert(sA, kb, tol, s_red);
-    if (blockIdx.y == 0 && t == 0) {
-        if (rel < 0.0) atomicExch(err, 1);
-        else atomic_min_pos(minpiv, rel);
-    }
-    constexpr int PER = NB * W / 128;                 // rows of T per thread
-    const int j = j0 + t % W, g = t / W;
-    if (j < f.ld) {
-        const bool own = j >= k0 && j < k0 + kb;
-        double m[NB];
+    const int kb = min(KB, f.p - k0), t = threadIdx.x, j = t & 31, g = t >> 5;
+    const double *M = buf + f.off + (int64_t)k0 * f.ld + k0;
 #pragma unroll
-        for (int l = 0; l < NB; l++) m[l] = l < kb ? M[(int64_t)(k0 + l) * f.ld + j] : 0.0;
-        double *T = tpan + f.tpan + j;
+    for (int r = g; r < KB; r += 4) sW[r][j] = (r < kb && j < kb) ? M[(int64_t)r * f.ld + j] : 0.0;
+    for (int s = 0; s < kb; s += NB) {
+        const int b = min(NB, kb - s), o = NB - s;
+        __syncthreads();
+        for (int u = t; u < 2 * NB * NB; u += 128) {
+            const int c = u / NB, r = u % NB;
+            sA[c][r] = c < NB ? ((r < b && c < b) ? sW[s + r][s + c] : (r == c ? 1.0 : 0.0)) : (r == c - NB ? 1.0 : 0.0);
+        }
+        __syncthreads();
+        const double rel = block_invert(sA, b, tol, s_red);
+        if (t == 0) {
+            if (rel < 0.0) atomicCAS(err, 0, 1);
+            else atomic_min_pos(minpiv, rel);
+        }
+        // T = D16^-1 W[16 rows,:], thread = (column, four rows)
+        double acc[4] = {};
+        const bool own = j >= s && j < s + NB;
+        if (own) {
 #pragma unroll
-        for (int q = 0; q < PER; q++) {
-            const int k = g * PER + q;
-            double acc = 0.0;
-            if (own) {
-                acc = sA[NB + j - k0][k];
-            } else {
+            for (int u = 0; u < 4; u++) acc[u] = sA[NB + j - s][g * 4 + u];
+        } else {
 #pragma unroll
-                for (int l = 0; l < NB; l++) acc = fma(sA[NB + l][k], m[l], acc);
+            for (int l = 0; l < NB; l++) {
+                const double m = sW[s + l][j];
+#pragma unroll
+                for (int u = 0; u < 4; u++) acc[u] = fma(sA[NB + l][g * 4 + u], m, acc[u]);
             }
-            T[(int64_t)k * f.ld] = acc;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) sT[g * 4 + u][j] = acc[u];
+        __syncthreads();
+        // the other 16 rows less C T (their columns s .. s + 15 are C), then T
+#pragma unroll
+        for (int u = 0; u < 4; u++) acc[u] = own ? 0.0 : sW[o + g * 4 + u][j];
+#pragma unroll
+        for (int l = 0; l < NB; l++) {
+            const double v = sT[l][j];
+#pragma unroll
+            for (int u = 0; u < 4; u++) acc[u] = fma(-sW[o + g * 4 + u][s + l], v, acc[u]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            sW[o + g * 4 + u][j] = acc[u];
+            sW[s + g * 4 + u][j] = sT[g * 4 + u][j];
         }
     }
+    __syncthreads();
+    double *D = dinv + (int64_t)blockIdx.x * KB * KB;
+#pragma unroll
+    for (int k = g; k < KB; k += 4) D[k * KB + j] = (k < kb && j < kb) ? sW[j][k] : 0.0;
 }
 
-constexpr int TILE = 64;   // rows and columns of a CTA's tile, 8 warps of 16 x 32
-
-// acc[a][b] += sum over 16 k of A[k][row a] B[k][col b] for a warp's 16 x 32
-// part of the tile: lane = (row quad, column pair), columns 2 apart by 16
-__device__ __forceinline__ void tile_fma(double (&acc)[4][4], const double (*sa)[TILE + 2],
-                                         const double (*sb)[TILE], int r, int c)
+// T = D^-1 M[K,:] for 128 columns, as the product of M[K,:]^T and D^-T; columns
+// K of T hold D^-1.  And 128 rows of the copy C = M[P,K].
+__global__ void __launch_bounds__(split::SHORT_THREADS, 2)
+k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
+        const double *__restrict__ dinv, double *__restrict__ cpan, double *__restrict__ tpan, int *err)
 {
+    extern __shared__ __align__(1024) char s_stage[];
+    const Front f = fr[perm[blockIdx.x]];
+    const int j0 = blockIdx.y * split::TM;
+    if (j0 >= f.n) return;
+    const int kb = min(KB, f.p - k0), t = threadIdx.x;
+    const double *M = buf + f.off, *D = dinv + (int64_t)blockIdx.x * KB * KB;
+    for (int u = t; u < split::TM * KB; u += split::SHORT_THREADS) {
+        const int r = j0 + u / KB, l = u % KB;
+        if (r < f.p) cpan[f.cpan + (int64_t)r * KB + l] = l < kb ? M[(int64_t)r * f.ld + k0 + l] : 0.0;
+    }
+    const int m = min(split::TM, f.n - j0);
+    const bool ok = split::short_product<KB, true>(
+        s_stage, m, kb,
+        [&](int j, int k, double (&x)[8]) {
 #pragma unroll
-    for (int l = 0; l < NB; l++) {
-        double a[4], b[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) a[u] = sa[l][r + u];
-        const double2 b0 = *reinterpret_cast<const double2 *>(&sb[l][c]);
-        const double2 b1 = *reinterpret_cast<const double2 *>(&sb[l][c + 16]);
-        b[0] = b0.x; b[1] = b0.y; b[2] = b1.x; b[3] = b1.y;
-#pragma unroll
-        for (int u = 0; u < 4; u++)
-#pragma unroll
-            for (int v = 0; v < 4; v++) acc[u][v] = fma(a[u], b[v], acc[u][v]);
+            for (int u = 0; u < 8; u++)
+                if (k + u < kb) x[u] = M[(int64_t)(k0 + k + u) * f.ld + j0 + j];
+        },
+        [&](int k, int r) { return D[k * KB + r]; });
+    if (!ok) {
+        if (t == 0) atomicExch(err, 2);
+        return;
+    }
+    const double *out = reinterpret_cast<const double *>(s_stage);
+    for (int u = t; u < KB * split::TM; u += split::SHORT_THREADS) {
+        const int r = u / split::TM, c = u % split::TM, j = j0 + c;
+        if (r < kb && c < m)
+            tpan[f.tpan + (int64_t)r * f.ld + j] = j >= k0 && j < k0 + kb ? D[(j - k0) * KB + r] : out[c * (KB + 1) + r];
     }
 }
 
 // M[i,:] -= C_i T for the pivot rows outside K, M[K,:] = T (in place: C and T
 // are copies, an entry is read and written by its own thread)
-__global__ void __launch_bounds__(256, 2)
+__global__ void __launch_bounds__(split::SHORT_THREADS, 2)
 k_update(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, int ntc,
-         const double *__restrict__ cpan, const double *__restrict__ tpan, double *__restrict__ buf)
+         const double *__restrict__ cpan, const double *__restrict__ tpan, double *__restrict__ buf, int *err)
 {
-    __shared__ double sa[NB][TILE + 2];
-    __shared__ __align__(16) double sb[NB][TILE];
+    extern __shared__ __align__(1024) char s_stage[];
     const Front f = fr[perm[blockIdx.x]];
-    const int i0 = (blockIdx.y / ntc) * TILE, j0 = (blockIdx.y % ntc) * TILE;
-    if (i0 >= f.p || j0 >= f.ld) return;
-    const int t = threadIdx.x;
-    for (int u = t; u < TILE * NB; u += 256) {
-        const int r = u / NB, l = u % NB;
-        sa[l][r] = i0 + r < f.p ? cpan[f.cpan + (int64_t)(i0 + r) * NB + l] : 0.0;
-        const int k = u / TILE, c = u % TILE;
-        sb[k][c] = j0 + c < f.ld ? tpan[f.tpan + (int64_t)k * f.ld + j0 + c] : 0.0;
+    const int i0 = (blockIdx.y / ntc) * split::TM, j0 = (blockIdx.y % ntc) * split::TN;
+    if (i0 >= f.p || j0 >= f.n) return;
+    const int kb = min(KB, f.p - k0), t = threadIdx.x;
+    const int m = min(split::TM, f.p - i0), n = min(split::TN, f.n - j0);
+    const double *C = cpan + f.cpan + (int64_t)i0 * KB, *T = tpan + f.tpan + j0;
+    const bool copy = i0 >= k0 && i0 + m <= k0 + kb;  // only rows K
+    if (!copy && !split::short_product<split::TN, false>(
+                     s_stage, m, n,
+                     [&](int r, int k, double (&x)[8]) {
+                         if (i0 + r >= k0 && i0 + r < k0 + kb) return;
+#pragma unroll
+                         for (int u = 0; u < 8; u += 2) {
+                             const double2 v = *reinterpret_cast<const double2 *>(C + r * KB + k + u);
+                             x[u] = v.x;
+                             x[u + 1] = v.y;
+                         }
+                     },
+                     [&](int k, int c) { return k < kb ? T[(int64_t)k * f.ld + c] : 0.0; })) {
+        if (t == 0) atomicExch(err, 2);
+        return;
     }
-    __syncthreads();
-    const int w = t >> 5, lane = t & 31;
-    const int wr = (w >> 1) * 16, wc = (w & 1) * 32;
-    if (i0 + wr >= f.p || j0 + wc >= f.ld) return;
-    const int r = wr + (lane >> 3) * 4, c = wc + (lane & 7) * 2;
-    const int kb = min(NB, f.p - k0);
-    double acc[4][4] = {};
-    const bool copy = i0 + wr == k0;                  // the warp's rows are K
-    if (!copy) tile_fma(acc, sa, sb, r, c);
-#pragma unroll
-    for (int u = 0; u < 4; u++) {
-        const int i = i0 + r + u;
-        if (i >= f.p) continue;
-        double *row = buf + f.off + (int64_t)i * f.ld + j0;
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int cc = c + 16 * h, j = j0 + cc;
-            if (j >= f.ld) continue;
-            double2 v;
-            if (copy) {
-                v = *reinterpret_cast<const double2 *>(&sb[i - k0][cc]);
-            } else {
-                v = *reinterpret_cast<const double2 *>(row + cc);
-                if (j >= k0 && j < k0 + kb) v.x = 0.0;
-                if (j + 1 >= k0 && j + 1 < k0 + kb) v.y = 0.0;
-                v.x -= acc[u][2 * h];
-                v.y -= acc[u][2 * h + 1];
-            }
-            *reinterpret_cast<double2 *>(row + cc) = v;
-        }
+    const double *out = reinterpret_cast<const double *>(s_stage);
+    double *A = buf + f.off + (int64_t)i0 * f.ld + j0;
+    for (int u = t; u < m * split::TN; u += split::SHORT_THREADS) {
+        const int r = u / split::TN, c = u % split::TN;
+        if (c >= n) continue;
+        const int i = i0 + r, j = j0 + c;
+        double v;
+        if (i >= k0 && i < k0 + kb)
+            v = T[(int64_t)(i - k0) * f.ld + c];
+        else
+            v = (j >= k0 && j < k0 + kb ? 0.0 : A[(int64_t)r * f.ld + c]) - out[r * split::OUT_LD + c];
+        A[(int64_t)r * f.ld + c] = v;
     }
 }
 
@@ -280,8 +298,8 @@ k_split_outer(const Front *__restrict__ fr, const int32_t *__restrict__ perm, co
 }
 
 // M[F,F] -= M[F,P] M[P,F] on the tensor cores, for every p: fronts with fewer
-// than 16, 32 or 64 pivots left to a tiled FP64 product made 20,000 quads 0.2,
-// 2.1 and 9.4 ms slower.  Bound by the cutting of the operands
+// than 16, 32 or 64 pivots left to a tiled FP64 product made 20,000 quads 77.4,
+// 79.3 and 86.6 ms in place of 77.2.  Bound by the cutting of the operands
 // (integer instructions) and, in the deepest levels, by a tile's fixed cost.
 __global__ void __launch_bounds__(split::THREADS, 1)
 k_schur(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int ntc, const int32_t *__restrict__ e0,
@@ -420,7 +438,7 @@ struct Guard {
 struct Level {
     int first, count;           // fronts, and their places in perm (most pivots first)
     int nmax, pmax, qmax, ldmax;
-    std::vector<int> active;    // fronts with more than 16 s pivots, per step s
+    std::vector<int> active;    // fronts with more than 32 s pivots, per step s
     std::vector<int> ld_active; // largest leading dimension among them
 };
 
@@ -434,7 +452,7 @@ struct vefem_tree {
     Front *fr = nullptr;
     int32_t *perm = nullptr, *ids = nullptr, *src0 = nullptr, *src1 = nullptr;
     int32_t *e0 = nullptr, *e1 = nullptr;   // exponents of the split products
-    double *cpan = nullptr, *tpan = nullptr;
+    double *cpan = nullptr, *tpan = nullptr, *dinv = nullptr;
     double *y = nullptr, *b = nullptr, *x = nullptr;
     int *err = nullptr;
     unsigned long long *minpiv = nullptr;
@@ -546,7 +564,7 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
     std::vector<Front> fr(nfront);
     std::vector<int32_t> perm(nfront);
     std::iota(perm.begin(), perm.end(), 0);
-    int64_t cmax = 0, tmax = 0;
+    int64_t cmax = 0, tmax = 0, dmax = 0;
     for (int l = 0; l < nlevel; l++) {
         Level v{level_ptr[l], level_ptr[l + 1] - level_ptr[l], 0, 0, 0, 0, {}, {}};
         std::stable_sort(perm.begin() + v.first, perm.begin() + v.first + v.count,
@@ -555,19 +573,20 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
         for (int k = v.first; k < v.first + v.count; k++) {
             const int t = perm[k];
             fr[t] = Front{off[t], cp, tp, (int32_t)idx_off[t], n[t], p[t], ld[t], {child[2 * t], child[2 * t + 1]}};
-            cp += (int64_t)p[t] * NB;
-            tp += (int64_t)ld[t] * NB;
+            cp += (int64_t)p[t] * KB;
+            tp += (int64_t)ld[t] * KB;
             v.nmax = std::max(v.nmax, n[t]);
             v.pmax = std::max(v.pmax, p[t]);
             v.qmax = std::max(v.qmax, n[t] - p[t]);
             v.ldmax = std::max(v.ldmax, ld[t]);
         }
-        for (int k0 = 0; k0 < v.pmax; k0 += NB) {
+        for (int k0 = 0; k0 < v.pmax; k0 += KB) {
             int a = 0, m = 0;
             while (a < v.count && p[perm[v.first + a]] > k0) m = std::max(m, (int)ld[perm[v.first + a++]]);
             v.active.push_back(a);
             v.ld_active.push_back(m);
         }
+        dmax = std::max<int64_t>(dmax, (int64_t)v.count * KB * KB);
         cmax = std::max(cmax, cp);
         tmax = std::max(tmax, tp);
         f->pmax = std::max(f->pmax, v.pmax);
@@ -587,11 +606,14 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
         put(&f->perm, perm.data(), perm.size()) && put(&f->ids, ids32.data(), ids32.size()) &&
         put(&f->src0, src, (size_t)tot) && put(&f->src1, src + tot, (size_t)tot) &&
         put(&f->e0, (const int32_t *)nullptr, (size_t)tot) && put(&f->e1, (const int32_t *)nullptr, (size_t)tot) && put(&f->cpan, none, (size_t)cmax) &&
-        put(&f->tpan, none, (size_t)tmax) && put(&f->y, none, (size_t)tot) && put(&f->b, none, (size_t)N) &&
+        put(&f->tpan, none, (size_t)tmax) && put(&f->dinv, none, (size_t)dmax) && put(&f->y, none, (size_t)tot) && put(&f->b, none, (size_t)N) &&
         put(&f->x, none, (size_t)N) && put(&f->err, (const int *)nullptr, 1) &&
         put(&f->minpiv, (const unsigned long long *)nullptr, 1);
     const int sm_p = f->pmax * (int)sizeof(double), sm_q = f->qmax * (int)sizeof(double);
     if (!ok ||
+        cudaFuncSetAttribute(k_pivot, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SHORT_SMEM<KB>) != cudaSuccess ||
+        cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SHORT_SMEM<split::TN>) !=
+            cudaSuccess ||
         cudaFuncSetAttribute(k_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SMEM) != cudaSuccess ||
         (sm_p > 48 * 1024 &&
                 (cudaFuncSetAttribute(k_tree_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess ||
@@ -625,15 +647,13 @@ extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_
             k_assemble<<<dim3(l.count, up(l.nmax, AS_ROWS)), dim3(32, AS_ROWS), 0, s>>>(f->fr, perm, f->src0, f->src1,
                                                                                        buf);
         for (size_t st = 0; st < l.active.size(); st++) {
-            const int k0 = (int)st * NB, a = l.active[st], ld = l.ld_active[st];
-            if ((int64_t)a * up(ld, 128) >= 4 * f->sms)
-                k_pivot<128><<<dim3(a, up(ld, 128)), 128, 0, s>>>(f->fr, perm, k0, buf, f->cpan, f->tpan, f->err,
-                                                                  f->minpiv, tol);
-            else
-                k_pivot<32><<<dim3(a, up(ld, 32)), 128, 0, s>>>(f->fr, perm, k0, buf, f->cpan, f->tpan, f->err,
-                                                                f->minpiv, tol);
-            const int ntc = (int)up(ld, TILE);
-            k_update<<<dim3(a, ntc * up(l.pmax, TILE)), 256, 0, s>>>(f->fr, perm, k0, ntc, f->cpan, f->tpan, buf);
+            const int k0 = (int)st * KB, a = l.active[st], ld = l.ld_active[st];
+            k_invert<<<a, 128, 0, s>>>(f->fr, perm, k0, buf, f->dinv, f->err, f->minpiv, tol);
+            k_pivot<<<dim3(a, up(ld, split::TM)), split::SHORT_THREADS, split::SHORT_SMEM<KB>, s>>>(
+                f->fr, perm, k0, buf, f->dinv, f->cpan, f->tpan, f->err);
+            const int ntc = (int)up(ld, split::TN);
+            k_update<<<dim3(a, ntc * up(l.pmax, split::TM)), split::SHORT_THREADS, split::SHORT_SMEM<split::TN>, s>>>(
+                f->fr, perm, k0, ntc, f->cpan, f->tpan, buf, f->err);
         }
         if (l.qmax > 0 && l.pmax > 0) {
             const int ntc = (int)up(l.qmax, split::TN);
@@ -698,7 +718,7 @@ extern "C" void vefem_tree_destroy(vefem_tree *f)
         Guard g(f->device);
         if (f->graph) cudaGraphExecDestroy(f->graph);
         if (f->cs) cudaStreamDestroy(f->cs);
-        void *p[] = {f->fr, f->perm, f->ids, f->src0, f->src1, f->e0, f->e1, f->cpan, f->tpan, f->y, f->b, f->x, f->err, f->minpiv};
+        void *p[] = {f->fr, f->perm, f->ids, f->src0, f->src1, f->e0, f->e1, f->cpan, f->tpan, f->dinv, f->y, f->b, f->x, f->err, f->minpiv};
         for (void *q : p) cudaFree(q);
     }
     delete f;
