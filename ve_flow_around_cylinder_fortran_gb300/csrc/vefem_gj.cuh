@@ -15,18 +15,30 @@ __device__ void atomic_min_pos(unsigned long long *addr, double v)
     atomicMin(addr, (unsigned long long)__double_as_longlong(v));
 }
 
-// 1/x: a single-precision seed refined by two steps of Newton's iteration for
-// the reciprocal, r <- r + r (1 - x r) (quadratic convergence: ~2^-23 ->
-// ~2^-46 -> rounding level).  A handful of FP64 instructions instead of a full
-// IEEE division, which matters on the critical path of the pivot-block
-// inversion (a warp issues an FP64 instruction every few tens of clocks on this
-// GPU).  Values outside the single-precision range take the IEEE division.
+// 1/x: the hardware's approximation (20 bits) refined by two steps of Newton's
+// iteration for the reciprocal, r <- r + r (1 - x r) (quadratic convergence: 20
+// -> 40 -> rounding level).  Four FP64 instructions instead of a full IEEE
+// division, which matters on the critical path of a pivot block's inversion (a
+// warp issues an FP64 instruction every few tens of clocks on this GPU, and a
+// conversion to and from a single-precision seed counts as two).  Values whose
+// reciprocal comes near the ends of the range take the IEEE division.
+__device__ __forceinline__ bool plain_exponent(double x)
+{
+    const int ex = (__double2hiint(x) >> 20) & 0x7ff;
+    return ex >= 64 && ex <= 1982;
+}
+
+__device__ __forceinline__ double approximate_reciprocal(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+
 __device__ __forceinline__ double recip(double x)
 {
-    const float xf = (float)x;
-    const float rf = __frcp_rn(xf);
-    if (!(fabsf(rf) < 3.0e38f) || rf == 0.0f || !(fabsf(xf) < 3.0e38f)) return 1.0 / x;
-    double r = (double)rf;
+    if (!plain_exponent(x)) return 1.0 / x;
+    double r = approximate_reciprocal(x);
     double e = fma(-x, r, 1.0);
     r = fma(r, e, r);
     e = fma(-x, r, 1.0);

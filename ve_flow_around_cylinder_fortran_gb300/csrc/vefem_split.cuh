@@ -25,8 +25,7 @@
 // One tcgen05.mma takes a digit of A (128 x 16) against several digits of B,
 // laid out as one operand of up to 256 columns: 14 instructions per 16 k.
 // Operands are cut by the CTA's 16 warps straight into the core-matrix layout
-// (8 rows x 16 bytes, no swizzle), two stages of 32 k, so the tensor core works
-// on one while the next is cut; the nine accumulators take 432 of the SM's 512
+// (8 rows x 16 bytes, no swizzle), 32 k a stage; the nine accumulators take 432 of the SM's 512
 // tensor memory columns, which is why a tile has 48 columns and not 64.
 #pragma once
 
@@ -47,9 +46,8 @@ constexpr int LBO_A = ND * TM * 16;    // bytes between k-neighbouring core matr
 constexpr int LBO_B = ND * TN * 16;
 constexpr int STAGE_A = (KS / 8) * LBO_A, STAGE_B = (KS / 8) * LBO_B;
 constexpr int STAGE = STAGE_A + STAGE_B;
-constexpr int SMEM = 2 * STAGE;
 constexpr int OUT_LD = TN + 1;         // the result tile, in the stages' place
-static_assert(TM * OUT_LD * 8 <= SMEM, "result tile");
+static_assert(TM * OUT_LD * 8 <= STAGE, "result tile");
 constexpr int NOT_FINITE = 1 << 20;    // exponent of a row or column with an infinity or NaN
 constexpr int EMPTY = -(1 << 20);      // ... of one with zeros only
 
@@ -83,12 +81,11 @@ __device__ __forceinline__ uint64_t fixed_point(double x, int s, int top)
                        (uint32_t)__double2loint(x);
     const int sh = min(max(top - (field_of(hi) + s), 0), 63);
     const uint64_t v = (((m << 10) >> sh) + 1) >> 1;
-    return (hi < 0 ? 0 - v : v) + 0x8080808080808080ull;
+    return hi < 0 ? 0x8080808080808080ull - v : 0x8080808080808080ull + v;
 }
 
-// the digits of eight k of one row, 16 bytes per digit
-template <int ROWS>
-__device__ __forceinline__ void put_digits(char *dst, const uint64_t (&w)[8])
+// the digits of eight k of one row, 16 bytes per digit, digits a stride apart
+__device__ __forceinline__ void put_digits(char *dst, int stride, const uint64_t (&w)[8])
 {
 #pragma unroll
     for (int a = 0; a < ND; a++) {
@@ -101,7 +98,7 @@ __device__ __forceinline__ void put_digits(char *dst, const uint64_t (&w)[8])
             const float f1 = __uint_as_float(__byte_perm(w1, 0x4b000000u, 0x7440u | (3 - (a & 3)))) - 8388736.0f;
             r[u] = __byte_perm(__float_as_uint(f0), __float_as_uint(f1), 0x7632);
         }
-        *reinterpret_cast<uint4 *>(dst + a * ROWS * 16) = make_uint4(r[0], r[1], r[2], r[3]);
+        *reinterpret_cast<uint4 *>(dst + a * stride) = make_uint4(r[0], r[1], r[2], r[3]);
     }
 }
 
@@ -136,50 +133,43 @@ __device__ __forceinline__ bool wait(uint32_t bar, uint32_t parity)
     return false;
 }
 
-// W columns of a warp's 32 rows, as integers
-template <int W>
-__device__ __forceinline__ void tmem_load(uint32_t addr, int (&v)[W])
+// four columns of a warp's 32 rows; the values are there after tmem_wait
+__device__ __forceinline__ void tmem_load(uint32_t addr, uint32_t (&r)[4])
 {
-    static_assert(W == 4 || W == 8, "columns");
-    uint32_t r[8];
-    if constexpr (W == 8)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                     : "r"(addr));
-    else
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                     : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                     : "r"(addr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < W; i++) v[i] = __float2int_rn(__uint_as_float(r[i]));
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(addr));
 }
+__device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// hi 2^40 + lo += W columns of the nine accumulators, N columns apart (the one
-// of a + b = d is at most (d + 1) 2^21 in size, and 2^24)
-template <int N, int W>
+// hi 2^40 + lo += four columns of the nine accumulators, N columns apart (the
+// one of a + b = d is at most (d + 1) 2^21 in size, and 2^24).  Five and four
+// loads in flight: a wait after each made a tile's rounding wait 27 times.
+template <int N>
 __device__ __forceinline__ void add_sums(uint32_t addr, int64_t *hi, int64_t *lo)
 {
-    int p[W], v[W];
-    tmem_load<W>(addr, p);
-    tmem_load<W>(addr + N, v);
+    uint32_t r[5][4];
+    auto at = [&](int d, int i) { return __float2int_rn(__uint_as_float(r[d][i])); };
 #pragma unroll
-    for (int i = 0; i < W; i++) hi[i] += (int64_t)(p[i] * 256 + v[i]) * 65536;
-    tmem_load<W>(addr + 2 * N, p);
-    tmem_load<W>(addr + 3 * N, v);
+    for (int d = 0; d < 4; d++) tmem_load(addr + d * N, r[d]);
+    tmem_wait();
 #pragma unroll
-    for (int i = 0; i < W; i++) hi[i] += (int64_t)(p[i] * 256 + v[i]);
-    tmem_load<W>(addr + 4 * N, p);
-    tmem_load<W>(addr + 5 * N, v);
+    for (int d = 0; d < 4; d++)
 #pragma unroll
-    for (int i = 0; i < W; i++) lo[i] += ((int64_t)p[i] * 256 + v[i]) * 16777216;
-    tmem_load<W>(addr + 6 * N, p);
-    tmem_load<W>(addr + 7 * N, v);
+        for (int i = 0; i < 4; i++) asm volatile("" : "+r"(r[d][i]));  // not read before the wait
 #pragma unroll
-    for (int i = 0; i < W; i++) lo[i] += ((int64_t)p[i] * 256 + v[i]) * 256;
-    tmem_load<W>(addr + 8 * N, p);
+    for (int i = 0; i < 4; i++)
+        hi[i] += (int64_t)(at(0, i) * 256 + at(1, i)) * 65536 + (at(2, i) * 256 + at(3, i));
 #pragma unroll
-    for (int i = 0; i < W; i++) lo[i] += p[i];
+    for (int d = 0; d < 5; d++) tmem_load(addr + (d + 4) * N, r[d]);
+    tmem_wait();
+#pragma unroll
+    for (int d = 0; d < 5; d++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) asm volatile("" : "+r"(r[d][i]));
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        lo[i] += ((int64_t)at(0, i) * 256 + at(1, i)) * 16777216 + ((int64_t)at(2, i) * 256 + at(3, i)) * 256 + at(4, i);
 }
 
 // (hi 2^40 + lo) 2^e rounded to a double, e from the largest exponents of row
@@ -191,30 +181,59 @@ __device__ __forceinline__ double rounded(int64_t hi, int64_t lo, int ta, int tb
     const int e = ta + tb - (2 * 1084 - 48);
     int64_t top = hi + (lo >> 40);                                 // with rem, a fraction of 64 bits
     uint64_t rem = (uint64_t)lo << 24;
-    const bool neg = top < 0;
-    if (neg) {
-        rem = 0 - rem;
-        top = ~top + (rem == 0);
+    const uint64_t neg = (uint64_t)(top >> 63);
+    top ^= neg;                                                    // less 2^-64 if negative: rounded away
+    rem ^= neg;
+    // the leading 64 bits, from words
+    uint32_t w2 = (uint32_t)((uint64_t)top >> 32), w1 = (uint32_t)top, w0 = (uint32_t)(rem >> 32);
+    int n = 0;
+    if (w2 == 0) {
+        w2 = w1;
+        w1 = w0;
+        w0 = (uint32_t)rem;
+        n = 32;
+        if (w2 == 0) {                                             // 2^46 below the largest possible
+            if ((w1 | w0) == 0) return 0.0;
+            if (w1 == 0) {
+                w1 = w0;
+                w0 = 0;
+                n = 64;
+            }
+            w2 = w1;
+            w1 = w0;
+            w0 = 0;
+            n += 32;
+        }
     }
-    uint64_t y;
-    int n;
-    if (top != 0) {
-        n = __clzll(top);
-        y = ((uint64_t)top << n) | (rem >> (64 - n));
-    } else {
-        if (rem == 0) return 0.0;
-        n = __clzll((long long)rem);
-        y = rem << n;
-        n += 64;
-    }
-    const uint64_t mant = (y >> 11) + ((y >> 10) & 1);             // 2^52 .. 2^53, times 2^(51 - n + e)
+    const int z = __clz((int)w2);
+    n += z;
+    const uint32_t y1 = __funnelshift_l(w1, w2, z), y0 = __funnelshift_l(w0, w1, z);
+    const uint64_t y = ((uint64_t)y1 << 32) | y0;
+    const uint64_t mant = (y >> 11) + ((y0 >> 10) & 1);            // 2^52 .. 2^53, times 2^(51 - n + e)
     const int be = e + 51 - n + 52 + 1023;
-    double v;
-    if (be >= 1 && be < 2046)
-        v = __longlong_as_double((long long)(((uint64_t)(be - 1) << 52) + mant));
-    else
-        v = ldexp((double)mant, e + 51 - n);
-    return neg ? -v : v;
+    if (be < 1 || be >= 2046) {
+        const double v = ldexp((double)mant, e + 51 - n);
+        return neg ? -v : v;
+    }
+    return __longlong_as_double((long long)((((uint64_t)(be - 1) << 52) + mant) | (neg << 63)));
+}
+
+// count columns (a multiple of 4) of a warp's rows, from c0, rounded into out
+template <int N, class TB>
+__device__ __forceinline__ void round_columns(uint32_t tmem, int c0, int count, bool in, int ta, TB tb, double *out)
+{
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+    for (int c = c0; c < c0 + count; c += 4) {
+        int64_t hi[4], lo[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) hi[i] = lo[i] = 0;
+        add_sums<N>(tmem + c, hi, lo);
+        if (in)
+#pragma unroll
+            for (int i = 0; i < 4; i++) out[c + i] = rounded(hi[i], lo[i], ta, tb(c + i));
+        __syncwarp();
+    }
 }
 
 // 16 k: every digit of A with the digits of B it meets, N columns per digit.
@@ -257,93 +276,105 @@ struct Operands {
 };
 
 // out[row * OUT_LD + column] (shared) = the tile of A B; false (to all threads)
-// if a wait ran out.  smem: SMEM bytes, 1024-byte aligned; all 512 threads call.
+// if a wait ran out.  All THREADS threads call; smem: BUFFERS * STAGE bytes.
+//
+// Two stages, one CTA on an SM, for long products: the tensor core multiplies
+// one stage while the next is cut.  One stage, two CTAs on an SM, for k <=
+// EXACT_K: most of such a tile is its loads, its rounding and its update of the
+// result, which the other CTA's share then covers; the tensor memory is taken
+// after the first stage is cut.  512 threads (16 warps a CTA at 64 registers):
+// with 256 at 128 a scheduler issued every fourth clock, 44.5 ms for 40.3.
+template <int BUFFERS>
 __device__ __forceinline__ bool product(char *smem, const Operands &o)
 {
     __shared__ uint32_t s_tmem;
-    __shared__ __align__(8) uint64_t s_bar[2];
+    __shared__ __align__(8) uint64_t s_bar[BUFFERS];
+    constexpr int GROUPS = THREADS / TM;               // 8-k groups of A in one go
+    constexpr int PART = TN / GROUPS;                  // columns of a warp's share
+    constexpr bool LONG = BUFFERS > 1;
     const int t = threadIdx.x, warp = t >> 5;
     const uint32_t bar0 = smem_addr(&s_bar[0]);
-    if (warp == 0) tmem_alloc(&s_tmem);
+    if (LONG && warp == 0) tmem_alloc(&s_tmem);
     if (t == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8) : "memory");
+#pragma unroll
+        for (int i = 0; i < BUFFERS; i++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * i) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = s_tmem;
+    uint32_t tmem = LONG ? s_tmem : 0;
 
-    const int ra = t & (TM - 1), ga = t / TM;          // row and 8-k group of A (4 groups)
+    const int ra = t & (TM - 1), g0 = t / TM;          // row and first 8-k group of A
     const int cb = t % TN, gb = t / TN;                // column and group of B (the first threads)
     const int top_a = ra < o.m ? o.ta[ra] : EMPTY, top_b = cb < o.n ? o.tb[cb] : EMPTY;
     const double *pa = o.a + (int64_t)min(ra, o.m - 1) * o.lda;
-    constexpr int PART = TN / 4;                       // columns of a warp's share
-    int64_t hi[PART], lo[PART];
+    int64_t hi[LONG ? PART : 1], lo[LONG ? PART : 1];
 #pragma unroll
-    for (int i = 0; i < PART; i++) hi[i] = lo[i] = 0;
-    const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * PART);
+    for (int i = 0; i < (LONG ? PART : 1); i++) hi[i] = lo[i] = 0;
     auto drain = [&]() {
+        const uint32_t mine = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * PART);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        add_sums<TN, 8>(mine, hi, lo);
-        add_sums<TN, 4>(mine + 8, hi + 8, lo + 8);
+#pragma unroll
+        for (int c = 0; c < PART; c += 4) add_sums<TN>(mine + c, hi + c, lo + c);
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     };
+    auto buffer = [&](int st) { return LONG ? st & 1 : 0; };
+    auto parity = [&](int st) { return (uint32_t)((LONG ? st >> 1 : st) & 1); };
 
     const int steps = (o.k + KS - 1) / KS;
     bool ok = true;
     int sent = 0;                                      // stages handed to the tensor core
     for (int st = 0; st < steps; st++) {
-        char *const stage = smem + (st & 1) * STAGE;
-        if (st >= 2) ok = wait(bar0 + 8 * (st & 1), ((st - 2) >> 1) & 1);
-        if (ra < o.m) {                                // rows beyond m stay undefined, and unread
-            const int k0 = st * KS + ga * 8;
+        char *const stage = smem + buffer(st) * STAGE;
+        if (st >= BUFFERS) ok = wait(bar0 + 8 * buffer(st), parity(st - BUFFERS));
+        // the thread's groups of A and then its group of B, by one copy of the
+        // code: unrolled, a tile streamed 90 KB of instructions through their
+        // cache and waited for them half of the time.  Rows beyond m and
+        // columns beyond n stay undefined, and unread.
+#pragma unroll 1
+        for (int i = 0; i <= KS / 8 / GROUPS; i++) {
+            const bool is_b = i == KS / 8 / GROUPS;
+            if (is_b ? t >= TN * (KS / 8) || cb >= o.n : ra >= o.m) continue;
+            const int g = is_b ? gb : g0 + i * GROUPS, k0 = st * KS + g * 8;
+            const double *from = is_b ? o.b + (int64_t)k0 * o.ldb + cb : pa + k0;
+            const int64_t step = is_b ? o.ldb : 1;
             double x[8];
             int e[8];
-            if (k0 + 8 <= o.k) {
+            if (!is_b && k0 + 8 <= o.k) {
 #pragma unroll
                 for (int u = 0; u < 4; u++) {
-                    const double2 v = __ldg(reinterpret_cast<const double2 *>(pa + k0) + u);
+                    const double2 v = __ldg(reinterpret_cast<const double2 *>(from) + u);
                     x[2 * u] = v.x;
                     x[2 * u + 1] = v.y;
                 }
-#pragma unroll
-                for (int u = 0; u < 8; u++) e[u] = __ldg(o.s + k0 + u);
             } else {
 #pragma unroll
-                for (int u = 0; u < 8; u++) {
-                    const bool in = k0 + u < o.k;
-                    x[u] = in ? pa[k0 + u] : 0.0;
-                    e[u] = in ? o.s[k0 + u] : 0;
-                }
+                for (int u = 0; u < 8; u++) x[u] = k0 + u < o.k ? __ldg(from + u * step) : 0.0;
             }
-            uint64_t w[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) w[u] = fixed_point(x[u], e[u], top_a);
-            put_digits<TM>(stage + ga * LBO_A + ra * 16, w);
-        }
-        if (t < TN * (KS / 8) && cb < o.n) {
-            const int k0 = st * KS + gb * 8;
+            for (int u = 0; u < 8; u++) e[u] = k0 + u < o.k ? __ldg(o.s + k0 + u) : 0;
             uint64_t w[8];
+            const int top = is_b ? top_b : top_a;
 #pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const bool in = k0 + u < o.k;
-                const double x = in ? o.b[(int64_t)(k0 + u) * o.ldb + cb] : 0.0;
-                w[u] = fixed_point(x, in ? -o.s[k0 + u] : 0, top_b);
-            }
-            put_digits<TN>(stage + STAGE_A + gb * LBO_B + cb * 16, w);
+            for (int u = 0; u < 8; u++) w[u] = fixed_point(x[u], is_b ? -e[u] : e[u], top);
+            put_digits(stage + (is_b ? STAGE_A + g * LBO_B + cb * 16 : g * LBO_A + ra * 16), is_b ? TN * 16 : TM * 16, w);
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        if (st > 0 && st % (EXACT_K / KS) == 0) {      // the exact sums are full
-            ok = wait(bar0 + 8 * ((st - 1) & 1), ((st - 1) >> 1) & 1) && ok;
+        if constexpr (LONG) if (st > 0 && st % (EXACT_K / KS) == 0) {  // the exact sums are full
+            ok = wait(bar0 + 8 * buffer(st - 1), parity(st - 1)) && ok;
             __syncwarp();
             if (__all_sync(0xffffffffu, ok)) drain();
+        }
+        if (!LONG && st == 0) {
+            if (warp == 0) tmem_alloc(&s_tmem);
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         }
         if (__syncthreads_or(!ok)) {
             ok = false;
             break;
         }
+        if (!LONG) tmem = s_tmem;
         if (t == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t sa = smem_addr(stage), sb = sa + STAGE_A;
@@ -352,27 +383,29 @@ __device__ __forceinline__ bool product(char *smem, const Operands &o)
                 mma_step<TN>(tmem, sa + h * 2 * LBO_A, sb + h * 2 * LBO_B, LBO_A, LBO_B,
                              (st % (EXACT_K / KS) != 0 || h > 0) ? 1u : 0u);
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             bar0 + 8 * (st & 1))
+                             bar0 + 8 * buffer(st))
                          : "memory");
         }
         __syncwarp();
         sent = st + 1;
     }
-    // the last two stages' products (also after a failed wait, again bounded)
+    // the last stages' products (also after a failed wait, again bounded)
     bool done = true;
-    if (sent > 1) done = wait(bar0 + 8 * ((sent - 2) & 1), ((sent - 2) >> 1) & 1);
-    if (sent > 0) done = wait(bar0 + 8 * ((sent - 1) & 1), ((sent - 1) >> 1) & 1) && done;
+    if (LONG && sent > 1) done = wait(bar0 + 8 * buffer(sent - 2), parity(sent - 2));
+    if (sent > 0) done = wait(bar0 + 8 * buffer(sent - 1), parity(sent - 1)) && done;
     ok = !__syncthreads_or(!(ok && done));
-    if (ok) {
-        drain();
-        double *out = reinterpret_cast<double *>(smem);
-        const int row = (warp & 3) * 32 + (t & 31), col = (warp >> 2) * PART;
-        const int ta = row < o.m ? o.ta[row] : EMPTY;
+    double *out = reinterpret_cast<double *>(smem);
+    const int row = (warp & 3) * 32 + (t & 31), col = (warp >> 2) * PART;
+    const int ta = row < o.m ? o.ta[row] : EMPTY;
+    if constexpr (LONG) {
+        if (ok) drain();
+        if (ok && row < o.m)
 #pragma unroll
-        for (int i = 0; i < PART; i++) {
-            const int tb = col + i < o.n ? o.tb[col + i] : EMPTY;
-            out[row * OUT_LD + col + i] = rounded(hi[i], lo[i], ta, tb);
-        }
+            for (int i = 0; i < PART; i++)
+                out[row * OUT_LD + col + i] = rounded(hi[i], lo[i], ta, col + i < o.n ? o.tb[col + i] : EMPTY);
+    } else if (ok) {
+        round_columns<TN>(tmem + ((uint32_t)((warp & 3) * 32) << 16), col, PART, row < o.m, ta,
+                          [&](int c) { return c < o.n ? __ldg(o.tb + c) : EMPTY; }, out + row * OUT_LD);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
@@ -382,7 +415,6 @@ __device__ __forceinline__ bool product(char *smem, const Operands &o)
 
 // ---- products of up to 32 inner indices: one stage, exponents found by the CTA
 
-constexpr int SHORT_THREADS = 256;
 template <int N>
 constexpr int SHORT_SMEM = (KS / 8) * ND * (TM + N) * 16;
 
@@ -409,30 +441,31 @@ __device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, F
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const int ra = t & (TM - 1), ga = t / TM;          // row, and 8-k groups ga and ga + 2 of A
+    constexpr int GROUPS = THREADS / TM, SLOTS = KS / 8 / GROUPS;
+    const int ra = t & (TM - 1), ga = t / TM;          // row, and every GROUPS-th 8-k group of A
     // columns 16 to a half warp, so that one maximum per half warp is one k's
     const int hw = t / 16, gb = hw / (N / 16), cb = hw % (N / 16) * 16 + (t & 15);
     const bool in_a = ra < m, in_b = gb < KS / 8 && cb < n;
-    double xa[2][8], xb[8];
+    double x[SLOTS + 1][8];                            // groups of A, and one of B
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
+    for (int h = 0; h < SLOTS; h++) {
 #pragma unroll
-        for (int u = 0; u < 8; u++) xa[h][u] = 0.0;
-        if (in_a) fa(ra, (ga + 2 * h) * 8, xa[h]);
+        for (int u = 0; u < 8; u++) x[h][u] = 0.0;
+        if (in_a) fa(ra, (ga + GROUPS * h) * 8, x[h]);
     }
 #pragma unroll
-    for (int u = 0; u < 8; u++) xb[u] = in_b ? fb(gb * 8 + u, cb) : 0.0;
+    for (int u = 0; u < 8; u++) x[SLOTS][u] = in_b ? fb(gb * 8 + u, cb) : 0.0;
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 8; u++) {
         if (EVEN_A) {
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int r = __reduce_max_sync(0xffffffffu, finite_high(xa[h][u]));
-                if (lane == 0) atomicMax(&s_k[(ga + 2 * h) * 8 + u], r);
+            for (int h = 0; h < SLOTS; h++) {
+                const int r = __reduce_max_sync(0xffffffffu, finite_high(x[h][u]));
+                if (lane == 0) atomicMax(&s_k[(ga + GROUPS * h) * 8 + u], r);
             }
         } else {
-            const int r = __reduce_max_sync(0xffffu << (lane & 16), finite_high(xb[u]));
+            const int r = __reduce_max_sync(0xffffu << (lane & 16), finite_high(x[SLOTS][u]));
             if ((t & 15) == 0 && gb < KS / 8) atomicMax(&s_k[gb * 8 + u], r);
         }
     }
@@ -442,28 +475,28 @@ __device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, F
 #pragma unroll
     for (int u = 0; u < 8; u++) {
 #pragma unroll
-        for (int h = 0; h < 2; h++) ta = max(ta, scaled_exponent(xa[h][u], inner((ga + 2 * h) * 8 + u)));
-        if (in_b) tb = max(tb, scaled_exponent(xb[u], -inner(gb * 8 + u)));
+        for (int h = 0; h < SLOTS; h++) ta = max(ta, scaled_exponent(x[h][u], inner((ga + GROUPS * h) * 8 + u)));
+        if (in_b) tb = max(tb, scaled_exponent(x[SLOTS][u], -inner(gb * 8 + u)));
     }
     if (in_a) atomicMax(&s_ta[ra], ta);
     if (in_b) atomicMax(&s_tb[cb], tb);
     __syncthreads();
-    uint64_t w[8];
-    if (in_a) {
-        ta = s_ta[ra];
+    // one copy of the code for all groups, which move up
+#pragma unroll 1
+    for (int i = 0; i <= SLOTS; i++) {
+        const bool is_b = i == SLOTS;
+        if (is_b ? in_b : in_a) {
+            const int g = is_b ? gb : ga + GROUPS * i, tp = is_b ? s_tb[cb] : s_ta[ra];
+            uint64_t w[8];
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int g = ga + 2 * h;
-#pragma unroll
-            for (int u = 0; u < 8; u++) w[u] = fixed_point(xa[h][u], inner(g * 8 + u), ta);
-            put_digits<TM>(smem + g * LA + ra * 16, w);
+            for (int u = 0; u < 8; u++) w[u] = fixed_point(x[0][u], is_b ? -inner(g * 8 + u) : inner(g * 8 + u), tp);
+            put_digits(smem + (is_b ? (KS / 8) * LA + g * LB + cb * 16 : g * LA + ra * 16), is_b ? N * 16 : TM * 16, w);
         }
-    }
-    if (in_b) {
-        tb = s_tb[cb];
 #pragma unroll
-        for (int u = 0; u < 8; u++) w[u] = fixed_point(xb[u], -inner(gb * 8 + u), tb);
-        put_digits<N>(smem + (KS / 8) * LA + gb * LB + cb * 16, w);
+        for (int u = 0; u < 8; u++) {
+#pragma unroll
+            for (int h = 0; h < SLOTS; h++) x[h][u] = x[h + 1][u];
+        }
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 0) tmem_alloc(&s_tmem);
@@ -481,21 +514,9 @@ __device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, F
     if (!ok) ok = wait(bar, 0);
     ok = !__syncthreads_or(!ok);
     if (ok) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        double *out = reinterpret_cast<double *>(smem);
-        const int row = (warp & 3) * 32 + lane, c0 = (warp >> 2) * (N / 2);
-        ta = s_ta[row];
-#pragma unroll 1
-        for (int c = c0; c < c0 + N / 2; c += 8) {
-            int64_t hi[8], lo[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) hi[i] = lo[i] = 0;
-            add_sums<N, 8>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c, hi, lo);
-            if (row < m)
-#pragma unroll
-                for (int i = 0; i < 8; i++) out[row * (N + 1) + c + i] = rounded(hi[i], lo[i], ta, s_tb[c + i]);
-            __syncwarp();
-        }
+        const int row = (warp & 3) * 32 + lane;
+        round_columns<N>(tmem + ((uint32_t)((warp & 3) * 32) << 16), (warp >> 2) * (N / GROUPS), N / GROUPS, row < m, s_ta[row],
+                         [&](int c) { return s_tb[c]; }, reinterpret_cast<double *>(smem) + row * (N + 1));
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

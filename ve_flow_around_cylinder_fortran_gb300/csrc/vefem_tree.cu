@@ -29,7 +29,8 @@
 // over the whole front.  Measured, factorise and solve, 20,000 and 2,000 quads:
 // panels 1,185 and 89.9 ms; the tree on the FP64 pipe, 16 pivots a step, 127 and
 // 10.6; Schur complements in digits 76 and 8.1; all products in digits, 32
-// pivots a step, 55.8 and 7.0.  A solve checked to 1e-14 went from 43.6 to 1.6
+// pivots a step, 55.8 and 7.0; with two short tiles to an SM and
+// the pivot blocks inverted in registers 38.9 and 5.2.  A solve checked to 1e-14 went from 43.6 to 1.6
 // ms at 20,000 (2,500 panels are 5,000 dependent launches, the tree 41): one
 // sweep leaves a residual of 1e-15, where the panels' longer chain of pivots
 // left 1e-12 and took a refinement.
@@ -100,77 +101,115 @@ k_assemble(const Front *__restrict__ fr, const int32_t *__restrict__ perm, const
 }
 
 constexpr int KB = 2 * NB;   // pivots per step
+constexpr int BATCH = 6;    // entries a thread of a product reads before it writes them back
 
-// The inverse of D = M[K,K], K = [k0, k0 + kb), transposed to dinv: blocked
-// Gauss-Jordan in two steps of 16 pivots, a CTA per front.  Bound by its own
-// chain, 2 x 16 pivots, where the fronts are few, and by the FP64 pipe (32^3
-// multiply-adds) where they are many.
-__global__ void __launch_bounds__(128)
+// The inverse of D = M[K,K], K = [k0, k0 + kb), transposed to dinv: in-place
+// Gauss-Jordan without pivoting, a CTA per front, thread = (column, four rows)
+// with its entries in registers; the warp that holds the next pivot's row
+// updates and divides it first and passes it on, with the pivot's column,
+// through shared memory.  A pivot is measured against the largest entry of its
+// 16 x 16 block as the block is reached.  Bound by the chain of 32 pivots, each
+// four dependent FP64 instructions and a barrier (0.8 us), and where the fronts
+// are many by the FP64 pipe (32^3 multiply-adds, 8.6 us on an SM); comparisons
+// are made on the bit patterns, which order like the numbers, to keep them off
+// that pipe.  In two blocked steps of 16 pivots with the division at each
+// pivot: 8.2 ms of a factorisation of 20,000 quads, so 4.1.
+constexpr int IV_THREADS = 8 * KB;
+__global__ void __launch_bounds__(IV_THREADS)
 k_invert(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
          double *__restrict__ dinv, int *err, unsigned long long *minpiv, double tol)
 {
-    __shared__ double sW[KB][KB + 1], sT[NB][KB + 1], sA[2 * NB][NB + 1];
-    __shared__ double s_red[4];
+    __shared__ double s_row[2][KB], s_col[2][KB], s_out[KB][KB + 1];
+    __shared__ unsigned long long s_max[2];
     const Front f = fr[perm[blockIdx.x]];
     const int kb = min(KB, f.p - k0), t = threadIdx.x, j = t & 31, g = t >> 5;
     const double *M = buf + f.off + (int64_t)k0 * f.ld + k0;
+    constexpr unsigned long long MAGN = 0x7fffffffffffffffull, INF = 0x7ff0000000000000ull;
+    auto magn = [](double x) { return (unsigned long long)__double_as_longlong(x) & MAGN; };
+    double a[4];
 #pragma unroll
-    for (int r = g; r < KB; r += 4) sW[r][j] = (r < kb && j < kb) ? M[(int64_t)r * f.ld + j] : 0.0;
-    for (int s = 0; s < kb; s += NB) {
-        const int b = min(NB, kb - s), o = NB - s;
-        __syncthreads();
-        for (int u = t; u < 2 * NB * NB; u += 128) {
-            const int c = u / NB, r = u % NB;
-            sA[c][r] = c < NB ? ((r < b && c < b) ? sW[s + r][s + c] : (r == c ? 1.0 : 0.0)) : (r == c - NB ? 1.0 : 0.0);
-        }
-        __syncthreads();
-        const double rel = block_invert(sA, b, tol, s_red);
-        if (t == 0) {
-            if (rel < 0.0) atomicCAS(err, 0, 1);
-            else atomic_min_pos(minpiv, rel);
-        }
-        // T = D16^-1 W[16 rows,:], thread = (column, four rows)
-        double acc[4] = {};
-        const bool own = j >= s && j < s + NB;
-        if (own) {
-#pragma unroll
-            for (int u = 0; u < 4; u++) acc[u] = sA[NB + j - s][g * 4 + u];
+    for (int u = 0; u < 4; u++) a[u] = (g * 4 + u < kb && j < kb) ? M[(int64_t)(g * 4 + u) * f.ld + j] : 0.0;
+    if (t < 2) s_max[t] = 0;
+    unsigned long long largest[2] = {INF, INF}, smallest[2] = {INF, INF}, floor_ = 0;
+    bool bad = false;
+    // row q (the warp's row u) divided by its pivot, and the pivot.  v / piv from
+    // the hardware's reciprocal r (20 bits, e = 1 - piv r): v r (1 + e + e^2), the
+    // next term is 2^-60; three dependent FP64 instructions.
+    auto publish = [&](int q, int u) {
+        const double piv = __shfl_sync(0xffffffffu, a[u], q), v = j == q ? 1.0 : a[u];
+        if (plain_exponent(piv)) {
+            const double r = approximate_reciprocal(piv), e = fma(-piv, r, 1.0), y = v * r;
+            s_row[q & 1][j] = fma(y, fma(e, e, e), y);
         } else {
+            s_row[q & 1][j] = v * (1.0 / piv);
+        }
+        if (j == q) s_col[q & 1][q] = piv;
+    };
+    if (g == 0) publish(0, 0);
+    if (j == 0)
 #pragma unroll
-            for (int l = 0; l < NB; l++) {
-                const double m = sW[s + l][j];
+        for (int u = 0; u < 4; u++)
+            if (g * 4 + u != 0) s_col[0][g * 4 + u] = a[u];
+    for (int p0 = 0; p0 < kb; p0 += 4) {
+        if (p0 % NB == 0) {                            // a 16 x 16 block begins
+            unsigned long long m = 0;
+            if (g * 4 / NB == p0 / NB && j / NB == p0 / NB)
 #pragma unroll
-                for (int u = 0; u < 4; u++) acc[u] = fma(sA[NB + l][g * 4 + u], m, acc[u]);
+                for (int u = 0; u < 4; u++) m = max(m, magn(a[u]));
+#pragma unroll
+            for (int o = NB / 2; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+            __syncthreads();
+            if (m && j % NB == 0) atomicMax(&s_max[p0 / NB], m);
+            __syncthreads();
+            m = s_max[p0 / NB];
+            largest[p0 / NB] = m;
+            floor_ = magn(tol * __longlong_as_double((long long)m));
+            bad = bad || m == 0 || m >= INF;
+        }
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            const int p = p0 + w, q = p + 1;
+            if (p >= kb) break;
+            const int b = w & 1, un = (w + 1) & 3;     // row q is its warp's row un
+            __syncthreads();
+            const double v = s_row[b][j];
+            // the next pivot's row first, so that its reciprocal's chain runs
+            // beside the other rows' updates
+            const bool next = q < kb && g == q / 4;
+            if (next) {
+                a[un] = fma(-s_col[b][q], v, j == p ? 0.0 : a[un]);
+                publish(q, un);
             }
-        }
 #pragma unroll
-        for (int u = 0; u < 4; u++) sT[g * 4 + u][j] = acc[u];
-        __syncthreads();
-        // the other 16 rows less C T (their columns s .. s + 15 are C), then T
+            for (int u = 0; u < 4; u++) {
+                const int r = g * 4 + u;
+                if (!(next && u == un)) a[u] = r == p ? v : fma(-s_col[b][r], v, j == p ? 0.0 : a[u]);
+            }
+            if (j == q)
 #pragma unroll
-        for (int u = 0; u < 4; u++) acc[u] = own ? 0.0 : sW[o + g * 4 + u][j];
-#pragma unroll
-        for (int l = 0; l < NB; l++) {
-            const double v = sT[l][j];
-#pragma unroll
-            for (int u = 0; u < 4; u++) acc[u] = fma(-sW[o + g * 4 + u][s + l], v, acc[u]);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            sW[o + g * 4 + u][j] = acc[u];
-            sW[s + g * 4 + u][j] = sT[g * 4 + u][j];
+                for (int u = 0; u < 4; u++)
+                    if (g * 4 + u != q) s_col[b ^ 1][g * 4 + u] = a[u];
+            const unsigned long long piv = magn(s_col[b][p]);
+            smallest[p0 / NB] = min(smallest[p0 / NB], piv);
+            bad = bad || piv <= floor_ || piv >= INF;
         }
     }
+#pragma unroll
+    for (int u = 0; u < 4; u++) s_out[g * 4 + u][j] = a[u];
     __syncthreads();
     double *D = dinv + (int64_t)blockIdx.x * KB * KB;
 #pragma unroll
-    for (int k = g; k < KB; k += 4) D[k * KB + j] = (k < kb && j < kb) ? sW[j][k] : 0.0;
+    for (int k = g; k < KB; k += 8) D[k * KB + j] = (k < kb && j < kb) ? s_out[j][k] : 0.0;
+    if (t == 0) {
+        if (bad) atomicCAS(err, 0, 1);
+        for (int h = 0; h * NB < kb && !bad; h++)
+            atomic_min_pos(minpiv, __longlong_as_double((long long)smallest[h]) / __longlong_as_double((long long)largest[h]));
+    }
 }
 
 // T = D^-1 M[K,:] for 128 columns, as the product of M[K,:]^T and D^-T; columns
 // K of T hold D^-1.  And 128 rows of the copy C = M[P,K].
-__global__ void __launch_bounds__(split::SHORT_THREADS, 2)
+__global__ void __launch_bounds__(split::THREADS, 2)
 k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
         const double *__restrict__ dinv, double *__restrict__ cpan, double *__restrict__ tpan, int *err)
 {
@@ -180,7 +219,8 @@ k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, 
     if (j0 >= f.n) return;
     const int kb = min(KB, f.p - k0), t = threadIdx.x;
     const double *M = buf + f.off, *D = dinv + (int64_t)blockIdx.x * KB * KB;
-    for (int u = t; u < split::TM * KB; u += split::SHORT_THREADS) {
+#pragma unroll 8
+    for (int u = t; u < split::TM * KB; u += split::THREADS) {
         const int r = j0 + u / KB, l = u % KB;
         if (r < f.p) cpan[f.cpan + (int64_t)r * KB + l] = l < kb ? M[(int64_t)r * f.ld + k0 + l] : 0.0;
     }
@@ -198,7 +238,7 @@ k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, 
         return;
     }
     const double *out = reinterpret_cast<const double *>(s_stage);
-    for (int u = t; u < KB * split::TM; u += split::SHORT_THREADS) {
+    for (int u = t; u < KB * split::TM; u += split::THREADS) {
         const int r = u / split::TM, c = u % split::TM, j = j0 + c;
         if (r < kb && c < m)
             tpan[f.tpan + (int64_t)r * f.ld + j] = j >= k0 && j < k0 + kb ? D[(j - k0) * KB + r] : out[c * (KB + 1) + r];
@@ -207,7 +247,7 @@ k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, 
 
 // M[i,:] -= C_i T for the pivot rows outside K, M[K,:] = T (in place: C and T
 // are copies, an entry is read and written by its own thread)
-__global__ void __launch_bounds__(split::SHORT_THREADS, 2)
+__global__ void __launch_bounds__(split::THREADS, 2)
 k_update(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, int ntc,
          const double *__restrict__ cpan, const double *__restrict__ tpan, double *__restrict__ buf, int *err)
 {
@@ -236,16 +276,24 @@ k_update(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0,
     }
     const double *out = reinterpret_cast<const double *>(s_stage);
     double *A = buf + f.off + (int64_t)i0 * f.ld + j0;
-    for (int u = t; u < m * split::TN; u += split::SHORT_THREADS) {
-        const int r = u / split::TN, c = u % split::TN;
-        if (c >= n) continue;
-        const int i = i0 + r, j = j0 + c;
-        double v;
-        if (i >= k0 && i < k0 + kb)
-            v = T[(int64_t)(i - k0) * f.ld + c];
-        else
-            v = (j >= k0 && j < k0 + kb ? 0.0 : A[(int64_t)r * f.ld + c]) - out[r * split::OUT_LD + c];
-        A[(int64_t)r * f.ld + c] = v;
+    for (int u0 = t; u0 < m * split::TN; u0 += BATCH * split::THREADS) {
+        double v[BATCH];
+#pragma unroll
+        for (int h = 0; h < BATCH; h++) {
+            const int u = u0 + h * split::THREADS, r = u / split::TN, c = u % split::TN, i = i0 + r, j = j0 + c;
+            v[h] = 0.0;
+            if (r >= m || c >= n) continue;
+            if (i >= k0 && i < k0 + kb)
+                v[h] = T[(int64_t)(i - k0) * f.ld + c];
+            else if (j < k0 || j >= k0 + kb)
+                v[h] = A[(int64_t)r * f.ld + c];
+        }
+#pragma unroll
+        for (int h = 0; h < BATCH; h++) {
+            const int u = u0 + h * split::THREADS, r = u / split::TN, c = u % split::TN, i = i0 + r;
+            if (r >= m || c >= n) continue;
+            A[(int64_t)r * f.ld + c] = i >= k0 && i < k0 + kb ? v[h] : v[h] - out[r * split::OUT_LD + c];
+        }
     }
 }
 
@@ -297,13 +345,15 @@ k_split_outer(const Front *__restrict__ fr, const int32_t *__restrict__ perm, co
     }
 }
 
-// M[F,F] -= M[F,P] M[P,F] on the tensor cores, for every p: fronts with fewer
-// than 16, 32 or 64 pivots left to a tiled FP64 product made 20,000 quads 77.4,
-// 79.3 and 86.6 ms in place of 77.2.  Bound by the cutting of the operands
-// (integer instructions) and, in the deepest levels, by a tile's fixed cost.
-__global__ void __launch_bounds__(split::THREADS, 1)
+// M[F,F] -= M[F,P] M[P,F], for every p: fronts with fewer than 16, 32 or 64
+// pivots left to a tiled FP64 product made 20,000 quads 0.2, 2.1 and 9.4 ms
+// slower.  Two stages for fronts of more than EXACT_K pivots, whose sums are
+// emptied into registers; one for the others: 43.5 ms with two stages for all,
+// 40.6 with the line at 64, 40.0 at 128.
+template <int BUFFERS>
+__global__ void __launch_bounds__(split::THREADS, 3 - BUFFERS)
 k_schur(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int ntc, const int32_t *__restrict__ e0,
-              const int32_t *__restrict__ e1, double *__restrict__ buf, int *err)
+        const int32_t *__restrict__ e1, double *__restrict__ buf, int *err)
 {
     extern __shared__ __align__(1024) char s_stage[];
     const Front f = fr[perm[blockIdx.x]];
@@ -321,15 +371,24 @@ k_schur(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int ntc,
     o.s = e0 + f.base;
     o.ta = e0 + f.base + f.p + i0;
     o.tb = e1 + f.base + f.p + j0;
-    if (!split::product(s_stage, o)) {
+    if (!split::product<BUFFERS>(s_stage, o)) {
         if (threadIdx.x == 0) atomicExch(err, 2);
         return;
     }
     const double *out = reinterpret_cast<const double *>(s_stage);
     double *S = M + (int64_t)(f.p + i0) * f.ld + f.p + j0;
-    for (int u = threadIdx.x; u < o.m * split::TN; u += split::THREADS) {
-        const int r = u / split::TN, c = u % split::TN;
-        if (c < o.n) S[(int64_t)r * f.ld + c] -= out[r * split::OUT_LD + c];
+    for (int u0 = threadIdx.x; u0 < o.m * split::TN; u0 += BATCH * split::THREADS) {
+        double v[BATCH];
+#pragma unroll
+        for (int h = 0; h < BATCH; h++) {
+            const int u = u0 + h * split::THREADS, r = u / split::TN, c = u % split::TN;
+            v[h] = r < o.m && c < o.n ? S[(int64_t)r * f.ld + c] : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < BATCH; h++) {
+            const int u = u0 + h * split::THREADS, r = u / split::TN, c = u % split::TN;
+            if (r < o.m && c < o.n) S[(int64_t)r * f.ld + c] = v[h] - out[r * split::OUT_LD + c];
+        }
     }
 }
 
@@ -440,6 +499,7 @@ struct Level {
     int nmax, pmax, qmax, ldmax;
     std::vector<int> active;    // fronts with more than 32 s pivots, per step s
     std::vector<int> ld_active; // largest leading dimension among them
+    int many;                   // fronts whose Schur product is a long one
 };
 
 }  // namespace
@@ -566,7 +626,7 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
     std::iota(perm.begin(), perm.end(), 0);
     int64_t cmax = 0, tmax = 0, dmax = 0;
     for (int l = 0; l < nlevel; l++) {
-        Level v{level_ptr[l], level_ptr[l + 1] - level_ptr[l], 0, 0, 0, 0, {}, {}};
+        Level v{level_ptr[l], level_ptr[l + 1] - level_ptr[l], 0, 0, 0, 0, {}, {}, 0};
         std::stable_sort(perm.begin() + v.first, perm.begin() + v.first + v.count,
                          [&](int a, int c) { return p[a] > p[c]; });
         int64_t cp = 0, tp = 0;
@@ -586,6 +646,7 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
             v.active.push_back(a);
             v.ld_active.push_back(m);
         }
+        while (v.many < v.count && p[perm[v.first + v.many]] > split::EXACT_K) v.many++;
         dmax = std::max<int64_t>(dmax, (int64_t)v.count * KB * KB);
         cmax = std::max(cmax, cp);
         tmax = std::max(tmax, tp);
@@ -614,7 +675,10 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
         cudaFuncSetAttribute(k_pivot, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SHORT_SMEM<KB>) != cudaSuccess ||
         cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SHORT_SMEM<split::TN>) !=
             cudaSuccess ||
-        cudaFuncSetAttribute(k_schur, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(k_schur<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             2 * split::STAGE) != cudaSuccess ||
+        cudaFuncSetAttribute(k_schur<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, split::STAGE) !=
+            cudaSuccess ||
         (sm_p > 48 * 1024 &&
                 (cudaFuncSetAttribute(k_tree_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess ||
                  cudaFuncSetAttribute(k_tree_up, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess)) ||
@@ -648,19 +712,24 @@ extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_
                                                                                        buf);
         for (size_t st = 0; st < l.active.size(); st++) {
             const int k0 = (int)st * KB, a = l.active[st], ld = l.ld_active[st];
-            k_invert<<<a, 128, 0, s>>>(f->fr, perm, k0, buf, f->dinv, f->err, f->minpiv, tol);
-            k_pivot<<<dim3(a, up(ld, split::TM)), split::SHORT_THREADS, split::SHORT_SMEM<KB>, s>>>(
+            k_invert<<<a, IV_THREADS, 0, s>>>(f->fr, perm, k0, buf, f->dinv, f->err, f->minpiv, tol);
+            k_pivot<<<dim3(a, up(ld, split::TM)), split::THREADS, split::SHORT_SMEM<KB>, s>>>(
                 f->fr, perm, k0, buf, f->dinv, f->cpan, f->tpan, f->err);
             const int ntc = (int)up(ld, split::TN);
-            k_update<<<dim3(a, ntc * up(l.pmax, split::TM)), split::SHORT_THREADS, split::SHORT_SMEM<split::TN>, s>>>(
+            k_update<<<dim3(a, ntc * up(l.pmax, split::TM)), split::THREADS, split::SHORT_SMEM<split::TN>, s>>>(
                 f->fr, perm, k0, ntc, f->cpan, f->tpan, buf, f->err);
         }
         if (l.qmax > 0 && l.pmax > 0) {
             const int ntc = (int)up(l.qmax, split::TN);
             k_split_inner<<<dim3(l.count, up(l.pmax, 32)), 256, 0, s>>>(f->fr, perm, buf, f->e0);
             k_split_outer<<<dim3(l.count, up(l.qmax, 32)), 256, 0, s>>>(f->fr, perm, buf, f->e0, f->e1);
-            k_schur<<<dim3(l.count, ntc * up(l.qmax, split::TM)), split::THREADS, split::SMEM, s>>>(
-                f->fr, perm, ntc, f->e0, f->e1, buf, f->err);
+            const unsigned tiles = ntc * up(l.qmax, split::TM);
+            if (l.many > 0)
+                k_schur<2><<<dim3(l.many, tiles), split::THREADS, 2 * split::STAGE, s>>>(
+                    f->fr, perm, ntc, f->e0, f->e1, buf, f->err);
+            if (l.many < l.count)
+                k_schur<1><<<dim3(l.count - l.many, tiles), split::THREADS, split::STAGE, s>>>(
+                    f->fr, perm + l.many, ntc, f->e0, f->e1, buf, f->err);
         }
     }
     TCK(cudaGetLastError());
