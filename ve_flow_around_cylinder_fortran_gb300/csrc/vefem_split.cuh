@@ -413,22 +413,29 @@ __device__ __forceinline__ bool product(char *smem, const Operands &o)
     return ok;
 }
 
+// programmatic launches: let the next kernel of the stream start, wait for the
+// one before
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---- products of up to 32 inner indices: one stage, exponents found by the CTA
 
 template <int N>
 constexpr int SHORT_SMEM = (KS / 8) * ND * (TM + N) * 16;
 
-// out[row * (N + 1) + column] (shared) = sum over k < 32 of A[row, k] fb(k, column)
-// for m rows and n columns; fa(row, k, x) gives A[row, k .. k + 7], and fa and
-// fb give 0 for k outside.  EVEN_A: the columns of A, not the rows of B, are the
-// ones evened (the transpose of a product evens its right factor so).  The tensor memory
-// is taken after the operands are cut: with two CTAs on an SM one cuts while
-// the other multiplies.
-template <int N, bool EVEN_A, class FA, class FB>
-__device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, FB fb)
+// out[row * (N + 1) + column] (shared) = sum over k < 32 of A[row, k] B[k, column]
+// for m rows and n columns; fa(row, k, x) and fb(column, k, x) give eight
+// entries from k on, 0 for k outside.  EVEN_A: the columns of A, not the rows of
+// B, are the ones evened (the transpose of a product evens its right factor so),
+// and A is cut before b_ready() is called and B read.  The tensor memory is
+// taken after the operands are cut: with two CTAs on an SM one cuts while the
+// other multiplies.
+template <int N, bool EVEN_A, class FA, class FB, class Ready>
+__device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, FB fb, Ready b_ready)
 {
     constexpr int LA = ND * TM * 16, LB = ND * N * 16;
     static_assert(TM * (N + 1) * 8 <= SHORT_SMEM<N>, "result tile");
+    static_assert(THREADS == TM * (KS / 8), "a group of A per thread");
     __shared__ uint32_t s_tmem;
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ int s_k[KS], s_ta[TM], s_tb[N];
@@ -441,62 +448,80 @@ __device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, F
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    constexpr int GROUPS = THREADS / TM, SLOTS = KS / 8 / GROUPS;
-    const int ra = t & (TM - 1), ga = t / TM;          // row, and every GROUPS-th 8-k group of A
+    const int ra = t & (TM - 1), ga = t / TM;          // row and 8-k group of A
     // columns 16 to a half warp, so that one maximum per half warp is one k's
     const int hw = t / 16, gb = hw / (N / 16), cb = hw % (N / 16) * 16 + (t & 15);
     const bool in_a = ra < m, in_b = gb < KS / 8 && cb < n;
-    double x[SLOTS + 1][8];                            // groups of A, and one of B
-#pragma unroll
-    for (int h = 0; h < SLOTS; h++) {
-#pragma unroll
-        for (int u = 0; u < 8; u++) x[h][u] = 0.0;
-        if (in_a) fa(ra, (ga + GROUPS * h) * 8, x[h]);
-    }
-#pragma unroll
-    for (int u = 0; u < 8; u++) x[SLOTS][u] = in_b ? fb(gb * 8 + u, cb) : 0.0;
-    __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 8; u++) {
-        if (EVEN_A) {
-#pragma unroll
-            for (int h = 0; h < SLOTS; h++) {
-                const int r = __reduce_max_sync(0xffffffffu, finite_high(x[h][u]));
-                if (lane == 0) atomicMax(&s_k[(ga + GROUPS * h) * 8 + u], r);
-            }
-        } else {
-            const int r = __reduce_max_sync(0xffffu << (lane & 16), finite_high(x[SLOTS][u]));
-            if ((t & 15) == 0 && gb < KS / 8) atomicMax(&s_k[gb * 8 + u], r);
-        }
-    }
-    __syncthreads();
+    double x[8], y[8];
     auto inner = [&](int k) { return EVEN_A ? -inner_exponent(s_k[k]) : inner_exponent(s_k[k]); };
-    int ta = EMPTY, tb = EMPTY;
+    auto load_a = [&]() {
 #pragma unroll
-    for (int u = 0; u < 8; u++) {
+        for (int u = 0; u < 8; u++) x[u] = 0.0;
+        if (in_a) fa(ra, ga * 8, x);
+    };
+    auto load_b = [&]() {
 #pragma unroll
-        for (int h = 0; h < SLOTS; h++) ta = max(ta, scaled_exponent(x[h][u], inner((ga + GROUPS * h) * 8 + u)));
-        if (in_b) tb = max(tb, scaled_exponent(x[SLOTS][u], -inner(gb * 8 + u)));
-    }
-    if (in_a) atomicMax(&s_ta[ra], ta);
-    if (in_b) atomicMax(&s_tb[cb], tb);
-    __syncthreads();
-    // one copy of the code for all groups, which move up
+        for (int u = 0; u < 8; u++) y[u] = 0.0;
+        if (in_b) fb(cb, gb * 8, y);
+    };
+    auto top_a = [&]() {
+        int top = EMPTY;
+#pragma unroll
+        for (int u = 0; u < 8; u++) top = max(top, scaled_exponent(x[u], inner(ga * 8 + u)));
+        if (in_a) atomicMax(&s_ta[ra], top);
+    };
+    auto top_b = [&]() {
+        int top = EMPTY;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (in_b) top = max(top, scaled_exponent(y[u], -inner(gb * 8 + u)));
+        if (in_b) atomicMax(&s_tb[cb], top);
+    };
+    // one copy of the code cuts both operands
+    auto cut = [&](int first, int last) {
 #pragma unroll 1
-    for (int i = 0; i <= SLOTS; i++) {
-        const bool is_b = i == SLOTS;
-        if (is_b ? in_b : in_a) {
-            const int g = is_b ? gb : ga + GROUPS * i, tp = is_b ? s_tb[cb] : s_ta[ra];
-            uint64_t w[8];
+        for (int i = first; i <= last; i++) {
+            if (i ? in_b : in_a) {
+                const int g = i ? gb : ga, top = i ? s_tb[cb] : s_ta[ra];
+                uint64_t w[8];
 #pragma unroll
-            for (int u = 0; u < 8; u++) w[u] = fixed_point(x[0][u], is_b ? -inner(g * 8 + u) : inner(g * 8 + u), tp);
-            put_digits(smem + (is_b ? (KS / 8) * LA + g * LB + cb * 16 : g * LA + ra * 16), is_b ? N * 16 : TM * 16, w);
+                for (int u = 0; u < 8; u++) w[u] = fixed_point(i ? y[u] : x[u], i ? -inner(g * 8 + u) : inner(g * 8 + u), top);
+                put_digits(smem + (i ? (KS / 8) * LA + g * LB + cb * 16 : g * LA + ra * 16), i ? N * 16 : TM * 16, w);
+            }
         }
+    };
+    if constexpr (EVEN_A) {
+        load_a();
+        __syncthreads();
 #pragma unroll
         for (int u = 0; u < 8; u++) {
-#pragma unroll
-            for (int h = 0; h < SLOTS; h++) x[h][u] = x[h + 1][u];
+            const int r = __reduce_max_sync(0xffffffffu, finite_high(x[u]));
+            if (lane == 0) atomicMax(&s_k[ga * 8 + u], r);
         }
+        __syncthreads();
+        top_a();
+        __syncthreads();
+        cut(0, 0);
+        b_ready();
+        load_b();
+        top_b();
+        __syncthreads();
+        cut(1, 1);
+    } else {
+        b_ready();
+        load_a();
+        load_b();
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int r = __reduce_max_sync(0xffffu << (lane & 16), finite_high(y[u]));
+            if ((t & 15) == 0 && gb < KS / 8) atomicMax(&s_k[gb * 8 + u], r);
+        }
+        __syncthreads();
+        top_a();
+        top_b();
+        __syncthreads();
+        cut(0, 1);
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (warp == 0) tmem_alloc(&s_tmem);
@@ -515,7 +540,7 @@ __device__ __forceinline__ bool short_product(char *smem, int m, int n, FA fa, F
     ok = !__syncthreads_or(!ok);
     if (ok) {
         const int row = (warp & 3) * 32 + lane;
-        round_columns<N>(tmem + ((uint32_t)((warp & 3) * 32) << 16), (warp >> 2) * (N / GROUPS), N / GROUPS, row < m, s_ta[row],
+        round_columns<N>(tmem + ((uint32_t)((warp & 3) * 32) << 16), (warp >> 2) * (N / 4), N / 4, row < m, s_ta[row],
                          [&](int c) { return s_tb[c]; }, reinterpret_cast<double *>(smem) + row * (N + 1));
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

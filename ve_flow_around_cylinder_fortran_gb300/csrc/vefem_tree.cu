@@ -29,11 +29,12 @@
 // over the whole front.  Measured, factorise and solve, 20,000 and 2,000 quads:
 // panels 1,185 and 89.9 ms; the tree on the FP64 pipe, 16 pivots a step, 127 and
 // 10.6; Schur complements in digits 76 and 8.1; all products in digits, 32
-// pivots a step, 55.8 and 7.0; with two short tiles to an SM and
-// the pivot blocks inverted in registers 38.9 and 5.2.  A solve checked to 1e-14 went from 43.6 to 1.6
-// ms at 20,000 (2,500 panels are 5,000 dependent launches, the tree 41): one
-// sweep leaves a residual of 1e-15, where the panels' longer chain of pivots
-// left 1e-12 and took a refinement.
+// pivots a step, 55.8 and 7.0; with two short tiles to an SM and the pivot
+// blocks inverted in registers 38.9 and 5.2; the kernels of a step started
+// before the last one's end 38.0 and 4.7.  A solve checked to 1e-14 went from
+// 43.6 to 1.6 ms at 20,000 (2,500 panels are 5,000 dependent launches, the tree
+// 41): one sweep leaves a residual of 1e-15, where the panels' longer chain of
+// pivots left 1e-12 and took a refinement.
 //
 // Solve: per depth, deepest first, y_P = A^-1 b_P and the update -C y_P a
 // front hands to its parent; then, root first, x_P = y_P - X x_F.  A row's dot
@@ -116,12 +117,14 @@ constexpr int BATCH = 6;    // entries a thread of a product reads before it wri
 // pivot: 8.2 ms of a factorisation of 20,000 quads, so 4.1.
 constexpr int IV_THREADS = 8 * KB;
 __global__ void __launch_bounds__(IV_THREADS)
-k_invert(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
-         double *__restrict__ dinv, int *err, unsigned long long *minpiv, double tol)
+k_invert(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *buf, double *dinv,
+         int *err, unsigned long long *minpiv, double tol)
 {
     __shared__ double s_row[2][KB], s_col[2][KB], s_out[KB][KB + 1];
     __shared__ unsigned long long s_max[2];
     const Front f = fr[perm[blockIdx.x]];
+    split::wait_previous();
+    split::launch_next();
     const int kb = min(KB, f.p - k0), t = threadIdx.x, j = t & 31, g = t >> 5;
     const double *M = buf + f.off + (int64_t)k0 * f.ld + k0;
     constexpr unsigned long long MAGN = 0x7fffffffffffffffull, INF = 0x7ff0000000000000ull;
@@ -208,12 +211,15 @@ k_invert(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0,
 }
 
 // T = D^-1 M[K,:] for 128 columns, as the product of M[K,:]^T and D^-T; columns
-// K of T hold D^-1.  And 128 rows of the copy C = M[P,K].
+// K of T hold D^-1.  And 128 rows of the copy C = M[P,K].  Starts while k_invert
+// runs, whose blocks have all waited for the kernel before it: M is as that one
+// left it.  D^-1 is read after the wait.
 __global__ void __launch_bounds__(split::THREADS, 2)
 k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
-        const double *__restrict__ dinv, double *__restrict__ cpan, double *__restrict__ tpan, int *err)
+        const double *dinv, double *__restrict__ cpan, double *__restrict__ tpan, int *err)
 {
     extern __shared__ __align__(1024) char s_stage[];
+    split::launch_next();
     const Front f = fr[perm[blockIdx.x]];
     const int j0 = blockIdx.y * split::TM;
     if (j0 >= f.n) return;
@@ -232,7 +238,11 @@ k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, 
             for (int u = 0; u < 8; u++)
                 if (k + u < kb) x[u] = M[(int64_t)(k0 + k + u) * f.ld + j0 + j];
         },
-        [&](int k, int r) { return D[k * KB + r]; });
+        [&](int r, int k, double (&y)[8]) {
+#pragma unroll
+            for (int u = 0; u < 8; u++) y[u] = D[(k + u) * KB + r];
+        },
+        [] { split::wait_previous(); });
     if (!ok) {
         if (t == 0) atomicExch(err, 2);
         return;
@@ -249,12 +259,14 @@ k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, 
 // are copies, an entry is read and written by its own thread)
 __global__ void __launch_bounds__(split::THREADS, 2)
 k_update(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, int ntc,
-         const double *__restrict__ cpan, const double *__restrict__ tpan, double *__restrict__ buf, int *err)
+         const double *cpan, const double *tpan, double *buf, int *err)
 {
     extern __shared__ __align__(1024) char s_stage[];
+    split::launch_next();
     const Front f = fr[perm[blockIdx.x]];
     const int i0 = (blockIdx.y / ntc) * split::TM, j0 = (blockIdx.y % ntc) * split::TN;
     if (i0 >= f.p || j0 >= f.n) return;
+    split::wait_previous();
     const int kb = min(KB, f.p - k0), t = threadIdx.x;
     const int m = min(split::TM, f.p - i0), n = min(split::TN, f.n - j0);
     const double *C = cpan + f.cpan + (int64_t)i0 * KB, *T = tpan + f.tpan + j0;
@@ -270,7 +282,12 @@ k_update(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0,
                              x[u + 1] = v.y;
                          }
                      },
-                     [&](int k, int c) { return k < kb ? T[(int64_t)k * f.ld + c] : 0.0; })) {
+                     [&](int c, int k, double (&y)[8]) {
+#pragma unroll
+                         for (int u = 0; u < 8; u++)
+                             if (k + u < kb) y[u] = T[(int64_t)(k + u) * f.ld + c];
+                     },
+                     [] {})) {
         if (t == 0) atomicExch(err, 2);
         return;
     }
@@ -540,6 +557,24 @@ int tfail(vefem_tree *f, int code, const std::string &m)
 
 unsigned up(int a, int b) { return (unsigned)((a + b - 1) / b); }
 
+// programmatic launch: the kernel starts when every block of the one before it
+// has let it, and waits itself for what it reads
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute early[1];
+    early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = early;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // rows per CTA of a sweep launch: one CTA per front where the fronts fill the
 // GPU twice over, else as many as spread the rows over it
 int rows_per_cta(const vefem_tree *f, int fronts, int rmax)
@@ -712,12 +747,12 @@ extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_
                                                                                        buf);
         for (size_t st = 0; st < l.active.size(); st++) {
             const int k0 = (int)st * KB, a = l.active[st], ld = l.ld_active[st];
-            k_invert<<<a, IV_THREADS, 0, s>>>(f->fr, perm, k0, buf, f->dinv, f->err, f->minpiv, tol);
-            k_pivot<<<dim3(a, up(ld, split::TM)), split::THREADS, split::SHORT_SMEM<KB>, s>>>(
-                f->fr, perm, k0, buf, f->dinv, f->cpan, f->tpan, f->err);
             const int ntc = (int)up(ld, split::TN);
-            k_update<<<dim3(a, ntc * up(l.pmax, split::TM)), split::THREADS, split::SHORT_SMEM<split::TN>, s>>>(
-                f->fr, perm, k0, ntc, f->cpan, f->tpan, buf, f->err);
+            TCK(launch_early(k_invert, dim3(a), IV_THREADS, 0, s, f->fr, perm, k0, buf, f->dinv, f->err, f->minpiv, tol));
+            TCK(launch_early(k_pivot, dim3(a, up(ld, split::TM)), split::THREADS, split::SHORT_SMEM<KB>, s, f->fr, perm, k0,
+                             buf, f->dinv, f->cpan, f->tpan, f->err));
+            TCK(launch_early(k_update, dim3(a, ntc * up(l.pmax, split::TM)), split::THREADS, split::SHORT_SMEM<split::TN>, s,
+                             f->fr, perm, k0, ntc, f->cpan, f->tpan, buf, f->err));
         }
         if (l.qmax > 0 && l.pmax > 0) {
             const int ntc = (int)up(l.qmax, split::TN);
