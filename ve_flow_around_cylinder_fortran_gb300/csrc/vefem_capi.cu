@@ -129,39 +129,60 @@ void gauss_tables_host(GaussTables *t)
         }
 }
 
-// edge contributions, sequential over edges (setEquationsEdge runs after the bulk)
+// edge contributions, sequential over edges (setEquationsEdge runs after the
+// bulk): edges share the nodes of their corners, and an entry takes its edges in
+// order.  Bound by the chain of an edge's loads; the places and contributions of
+// the next edge are therefore fetched before this one's are added.
+constexpr int GE_THREADS = 1024, GE_ITEMS = 54 + 2916 + 54, GE_PER = (GE_ITEMS + GE_THREADS - 1) / GE_THREADS;
 template <class V>
-__global__ void k_gather_edges(int nedge, int nex, const int64_t *rowptr, const int32_t *conn,
-                               int nel, const int32_t *edge_elem, const int32_t *edge_row,
-                               const int32_t *edge_off, const double *rs, const double *es,
-                               const double *as, double *b, V *vals, int want_jac)
+__global__ void __launch_bounds__(GE_THREADS)
+k_gather_edges(int nedge, int nex, const int64_t *__restrict__ rowptr, const int32_t *__restrict__ conn, int nel,
+               const int32_t *__restrict__ edge_elem, const int32_t *__restrict__ edge_row,
+               const int32_t *__restrict__ edge_off, const double *__restrict__ rs, const double *__restrict__ es,
+               const double *__restrict__ as, double *b, V *vals, int want_jac)
 {
-    for (int k = 0; k < nedge; k++) {
+    // the place in b (t < 54) or vals of item t of edge k, or -1, and what to add
+    auto locate = [&](int k, int t, int64_t &at, double &x) {
+        at = -1;
+        if (k >= nedge || t >= GE_ITEMS) return;
         const int e = edge_elem[k];
-        for (int t = threadIdx.x; t < 54 + 2916 + 54; t += blockDim.x) {
-            if (t < 54) {
-                if (!b) continue;
-                const int jnod = t / 6, jeq = t - 6 * (t / 6);
-                const int64_t row = (int64_t)conn[jnod * nel + e] * 6 + jeq;
-                b[row] = b[row] + rs[(int64_t)k * 54 + t];
-            } else if (t < 54 + 2916) {
-                if (!want_jac) continue;
-                const int r = t - 54;
-                const int blk = r / 36, q = r - 36 * (r / 36);
-                const int jeq = q / 6, ieq = q - 6 * (q / 6);
-                const int64_t slot = rowptr[(int64_t)edge_row[k * 81 + blk] * 6 + jeq] +
-                                     edge_off[k * 81 + blk] + ieq;
-                vals[slot] = vals[slot] + (V)es[(int64_t)k * 2916 + r];
-            } else {
-                if (!want_jac || nex == 0) continue;
-                const int r = t - 54 - 2916;
-                const int jnod = r / 6, jeq = r - 6 * (r / 6);
-                const int64_t row = (int64_t)conn[jnod * nel + e] * 6 + jeq;
-                const int64_t slot = rowptr[row + 1] - 1;
-                vals[slot] = vals[slot] + (V)as[(int64_t)k * 54 + r];
-            }
+        if (t < 54) {
+            if (!b) return;
+            at = (int64_t)conn[t / 6 * nel + e] * 6 + t % 6;
+            x = rs[(int64_t)k * 54 + t];
+        } else if (t < 54 + 2916) {
+            if (!want_jac) return;
+            const int r = t - 54, blk = r / 36, q = r % 36;
+            at = rowptr[(int64_t)edge_row[k * 81 + blk] * 6 + q / 6] + edge_off[k * 81 + blk] + q % 6;
+            x = es[(int64_t)k * 2916 + r];
+        } else {
+            if (!want_jac || nex == 0) return;
+            const int r = t - 54 - 2916;
+            at = rowptr[(int64_t)conn[r / 6 * nel + e] * 6 + r % 6 + 1] - 1;
+            x = as[(int64_t)k * 54 + r];
+        }
+    };
+    int64_t at[GE_PER], next[GE_PER];
+    double x[GE_PER], y[GE_PER];
+#pragma unroll
+    for (int u = 0; u < GE_PER; u++) locate(0, threadIdx.x + u * GE_THREADS, at[u], x[u]);
+    for (int k = 0; k < nedge; k++) {
+#pragma unroll
+        for (int u = 0; u < GE_PER; u++) locate(k + 1, threadIdx.x + u * GE_THREADS, next[u], y[u]);
+#pragma unroll
+        for (int u = 0; u < GE_PER; u++) {
+            if (at[u] < 0) continue;
+            if (threadIdx.x + u * GE_THREADS < 54)
+                b[at[u]] = b[at[u]] + x[u];
+            else
+                vals[at[u]] = vals[at[u]] + (V)x[u];
         }
         __syncthreads();
+#pragma unroll
+        for (int u = 0; u < GE_PER; u++) {
+            at[u] = next[u];
+            x[u] = y[u];
+        }
     }
 }
 
@@ -393,6 +414,7 @@ extern "C" int vefem_create(const vefem_mesh *mesh, const vefem_csr *pat,
     if (ce == cudaSuccess) ce = cudaStreamCreateWithFlags(&ctx->stream2, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming);
+    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ctx->join_edges, cudaEventDisableTiming);
     if (ce != cudaSuccess) {
         std::string m = std::string("cudaStreamCreate: ") + cudaGetErrorString(ce);
         delete ctx;
@@ -564,24 +586,45 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     ea.rs = ctx->d_rs;
     ea.es = ctx->d_es;
     ea.as = ctx->d_as;
+    const bool side = jmode != VEFEM_JAC_FD64 && want_res && want_jac;
+    if (side || edges) {
+        CK(cudaEventRecord(ctx->fork, s));
+        CK(cudaStreamWaitEvent(ctx->stream2, ctx->fork, 0));
+    }
+    if (side) {
+        // The FP64 residual and an exact Jacobian are independent until the
+        // scatter: the residual runs on a second stream, so the FP64 pipe works
+        // on it while the exact kernel keeps the FP32 pipes busy.
+        CK(launch_residual64(ea, ctx->prm, ctx->stream2));
+        CK(cudaEventRecord(ctx->join, ctx->stream2));
+        ctx->launches++;
+    }
+    if (edges) {
+        // so do the outlet edges, a few blocks with a long serial chain each
+        // (145 us in FP64 columns), until they are added at the end
+        EdgeArgs eg;
+        eg.nedge = ctx->nedge;
+        eg.nel = ctx->nel;
+        eg.nnodes = ctx->nnodes;
+        eg.edge_elem = ctx->d_edge_elem;
+        eg.edge_id = ctx->d_edge_id;
+        eg.conn = ctx->d_conn;
+        eg.xy = ctx->d_xy;
+        eg.TL = dTL;
+        eg.EU = dEU;
+        eg.rs = ctx->d_ers;
+        eg.es = ctx->d_ees;
+        eg.as = ctx->d_eas;
+        CK(launch_edge64(eg, ctx->prm, want_jac ? 1 : 0, ctx->stream2));
+        CK(cudaEventRecord(ctx->join_edges, ctx->stream2));
+    }
     if (jmode == VEFEM_JAC_FD64) {
         CK(launch_residual64(ea, ctx->prm, s));    // the columns' base residual
         CK(launch_fd64(ea, ctx->prm, s));
         ctx->launches += 2;
     } else {
-        // The FP64 residual and an exact Jacobian are independent until the
-        // scatter: the residual runs on a second stream, so the FP64 pipe works
-        // on it while the exact kernel keeps the FP32 pipes busy.
-        const bool side = want_res && want_jac;
-        if (want_res) {
-            if (side) {
-                CK(cudaEventRecord(ctx->fork, s));
-                CK(cudaStreamWaitEvent(ctx->stream2, ctx->fork, 0));
-                CK(launch_residual64(ea, ctx->prm, ctx->stream2));
-                CK(cudaEventRecord(ctx->join, ctx->stream2));
-            } else {
-                CK(launch_residual64(ea, ctx->prm, s));
-            }
+        if (want_res && !side) {
+            CK(launch_residual64(ea, ctx->prm, s));
             ctx->launches++;
         }
         if (jmode == VEFEM_JAC_EXACT64 || jac32) {
@@ -645,27 +688,14 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     }
     if (timing) CK(cudaEventRecord(ctx->ev[4], s));
     if (edges) {
-        EdgeArgs eg;
-        eg.nedge = ctx->nedge;
-        eg.nel = ctx->nel;
-        eg.nnodes = ctx->nnodes;
-        eg.edge_elem = ctx->d_edge_elem;
-        eg.edge_id = ctx->d_edge_id;
-        eg.conn = ctx->d_conn;
-        eg.xy = ctx->d_xy;
-        eg.TL = dTL;
-        eg.EU = dEU;
-        eg.rs = ctx->d_ers;
-        eg.es = ctx->d_ees;
-        eg.as = ctx->d_eas;
-        CK(launch_edge64(eg, ctx->prm, want_jac ? 1 : 0, s));
+        CK(cudaStreamWaitEvent(s, ctx->join_edges, 0));
         if (jac32)
-            k_gather_edges<float><<<1, 1024, 0, s>>>(
+            k_gather_edges<float><<<1, GE_THREADS, 0, s>>>(
                 ctx->nedge, ctx->nex, ctx->d_rowptr, ctx->d_conn, ctx->nel, ctx->d_edge_elem,
                 ctx->d_edge_row, ctx->d_edge_off, ctx->d_ers, ctx->d_ees, ctx->d_eas,
                 want_res ? db : nullptr, dvals32, 1);
         else
-            k_gather_edges<double><<<1, 1024, 0, s>>>(
+            k_gather_edges<double><<<1, GE_THREADS, 0, s>>>(
                 ctx->nedge, ctx->nex, ctx->d_rowptr, ctx->d_conn, ctx->nel, ctx->d_edge_elem,
                 ctx->d_edge_row, ctx->d_edge_off, ctx->d_ers, ctx->d_ees, ctx->d_eas,
                 want_res ? db : nullptr, want_jac ? dvals : nullptr, want_jac ? 1 : 0);
@@ -769,6 +799,7 @@ extern "C" int vefem_destroy(vefem_ctx *ctx)
     if (ctx->stream2) cudaStreamSynchronize(ctx->stream2);
     if (ctx->fork) cudaEventDestroy(ctx->fork);
     if (ctx->join) cudaEventDestroy(ctx->join);
+    if (ctx->join_edges) cudaEventDestroy(ctx->join_edges);
     if (ctx->stream2) cudaStreamDestroy(ctx->stream2);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;

@@ -20,7 +20,7 @@ struct vefem_ctx {
     vefem::KParams prm{};
     cudaStream_t stream = nullptr;
     cudaStream_t stream2 = nullptr;          // FP64 residual beside an exact Jacobian
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, join_edges = nullptr;
     cudaEvent_t ev[8] = {};
     float timing[5] = {0, 0, 0, 0, 0};
     int launches = 0;
