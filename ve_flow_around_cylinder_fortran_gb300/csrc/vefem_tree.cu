@@ -32,7 +32,7 @@
 // pivots a step, 55.8 and 7.0; with two short tiles to an SM and the pivot
 // blocks inverted in registers 38.9 and 5.2; the kernels of a step started
 // before the last one's end 38.0 and 4.7.  A solve checked to 1e-14 went from
-// 43.6 to 1.6 ms at 20,000 (2,500 panels are 5,000 dependent launches, the tree
+// 43.6 to 1.4 ms at 20,000 (2,500 panels are 5,000 dependent launches, the tree
 // 41): one sweep leaves a residual of 1e-15, where the panels' longer chain of
 // pivots left 1e-12 and took a refinement.
 //
@@ -575,12 +575,13 @@ cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, int smem,
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
-// rows per CTA of a sweep launch: one CTA per front where the fronts fill the
-// GPU twice over, else as many as spread the rows over it
+// Rows per CTA of a sweep launch: one pass of its 32 groups of lanes, unless
+// that makes more than 32 CTAs an SM.  A pass is mostly the latency of its rows'
+// loads: with passes in turn wherever the fronts fill the GPU twice a sweep of
+// 20,000 quads took 1.49 ms, of 2,000 0.33, now 1.31 and 0.27.
 int rows_per_cta(const vefem_tree *f, int fronts, int rmax)
 {
-    if (fronts >= 2 * f->sms) return std::max(SV_ROWS, rmax);
-    const int parts = std::max(1, 4 * f->sms / fronts);
+    const int parts = std::max(1, 32 * f->sms / fronts);
     return std::max(SV_ROWS, (int)up((int)up(rmax, parts), SV_ROWS) * SV_ROWS);
 }
 
