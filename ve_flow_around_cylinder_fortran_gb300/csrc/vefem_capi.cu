@@ -587,7 +587,27 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     ea.es = ctx->d_es;
     ea.as = ctx->d_as;
     const bool side = jmode != VEFEM_JAC_FD64 && want_res && want_jac;
-    if (side || edges) {
+    // The outlet edges are a few blocks with a long serial chain each (145 us in
+    // FP64 columns), independent of the elements until they are added at the end:
+    // on the second stream beside the element kernels, 2,746 -> 2,607 us for a host
+    // call on 2,000 quads.  Not beside a forward difference that fills every SM
+    // in one wave: its displaced blocks would start when an edge's block ends
+    // (1,300 -> 1,870 us on a few hundred quads).
+    const bool beside = edges && !(jmode == VEFEM_JAC_FD64 && fd64_one_wave(ctx->nel));
+    EdgeArgs eg;
+    eg.nedge = ctx->nedge;
+    eg.nel = ctx->nel;
+    eg.nnodes = ctx->nnodes;
+    eg.edge_elem = ctx->d_edge_elem;
+    eg.edge_id = ctx->d_edge_id;
+    eg.conn = ctx->d_conn;
+    eg.xy = ctx->d_xy;
+    eg.TL = dTL;
+    eg.EU = dEU;
+    eg.rs = ctx->d_ers;
+    eg.es = ctx->d_ees;
+    eg.as = ctx->d_eas;
+    if (side || beside) {
         CK(cudaEventRecord(ctx->fork, s));
         CK(cudaStreamWaitEvent(ctx->stream2, ctx->fork, 0));
     }
@@ -599,22 +619,7 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
         CK(cudaEventRecord(ctx->join, ctx->stream2));
         ctx->launches++;
     }
-    if (edges) {
-        // so do the outlet edges, a few blocks with a long serial chain each
-        // (145 us in FP64 columns), until they are added at the end
-        EdgeArgs eg;
-        eg.nedge = ctx->nedge;
-        eg.nel = ctx->nel;
-        eg.nnodes = ctx->nnodes;
-        eg.edge_elem = ctx->d_edge_elem;
-        eg.edge_id = ctx->d_edge_id;
-        eg.conn = ctx->d_conn;
-        eg.xy = ctx->d_xy;
-        eg.TL = dTL;
-        eg.EU = dEU;
-        eg.rs = ctx->d_ers;
-        eg.es = ctx->d_ees;
-        eg.as = ctx->d_eas;
+    if (beside) {
         CK(launch_edge64(eg, ctx->prm, want_jac ? 1 : 0, ctx->stream2));
         CK(cudaEventRecord(ctx->join_edges, ctx->stream2));
     }
@@ -688,7 +693,10 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     }
     if (timing) CK(cudaEventRecord(ctx->ev[4], s));
     if (edges) {
-        CK(cudaStreamWaitEvent(s, ctx->join_edges, 0));
+        if (beside)
+            CK(cudaStreamWaitEvent(s, ctx->join_edges, 0));
+        else
+            CK(launch_edge64(eg, ctx->prm, want_jac ? 1 : 0, s));
         if (jac32)
             k_gather_edges<float><<<1, GE_THREADS, 0, s>>>(
                 ctx->nedge, ctx->nex, ctx->d_rowptr, ctx->d_conn, ctx->nel, ctx->d_edge_elem,

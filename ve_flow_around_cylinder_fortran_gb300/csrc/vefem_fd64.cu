@@ -120,8 +120,8 @@ constexpr int FS_COLS = 28, FU_COLS = 18, FP_COLS = 9;
 
 // Elements per CTA by kind (stress, velocity, pressure, residue check)
 template <int THREADS> struct FdRun;
-template <> struct FdRun<256> { static constexpr int S = 9, U = 14, P = 28, R = 64; };
-template <> struct FdRun<64> { static constexpr int S = 2, U = 3, P = 7, R = 16; };
+template <> struct FdRun<256> { static constexpr int S = 9, U = 14, P = 28, R = 4; };
+template <> struct FdRun<64> { static constexpr int S = 2, U = 3, P = 7, R = 1; };
 constexpr int FD_RUN = 252;       // elements of a group of 256-thread CTAs
 
 template <int EL>
@@ -154,8 +154,8 @@ struct FdPressureSmem {
 
 template <int THREADS>
 struct FdResidueSmem {
-    double tl[THREADS / 64][3][54];   // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
-    int list[FdRun<THREADS>::R], n;
+    double tl[FdRun<THREADS>::R][3][54];   // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
+    int any[FdRun<THREADS>::R];
 };
 
 template <int FORM, int THREADS>
@@ -473,72 +473,60 @@ __device__ __forceinline__ void fd_pressure(const ElemArgs &a, const KParams &pr
 }
 
 // Elements with a restore residue: all 55 columns, each a full evaluation of the
-// state the sequential loop would have, 64 threads an element.
+// state the sequential loop would have, 4 elements (1 in a CTA of 64 threads) on
+// 220 (55) lanes.  Values below eps that are not zero leave one, so a converged
+// flow has them wherever a component vanishes: 4 elements to a CTA and not 64 in
+// turn, which took 22 ms for 500 quads with residues in half of them, 1.4 now
+// (FD_RES_FIGURES).  A CTA without any costs its look at the state, 2 us.
 template <int FORM, int SPEC, int THREADS>
 __device__ __forceinline__ void fd_residue(const ElemArgs &a, const KParams &prm, int e0, FdResidueSmem<THREADS> &sm)
 {
-    const int t = threadIdx.x, ne = min(FdRun<THREADS>::R, a.nel - e0);
-    if (t == 0) sm.n = 0;
+    constexpr int R = FdRun<THREADS>::R;
+    static_assert(R * 55 <= THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(R, a.nel - e0);
+    if (t < R) sm.any[t] = 0;
     __syncthreads();
-    const double eps = prm.eps;
-    for (int el = t >> 2; el < ne; el += THREADS >> 2) {
-        bool any = false;
-        for (int pos = t & 3; pos < 54; pos += 4) {
-            const int inod = pos / 6, f = pos - 6 * inod;
-            const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e0 + el]];
-            any |= __double_as_longlong((v + eps) - eps) != __double_as_longlong(v);
-        }
-        const unsigned quad = 0xfu << (threadIdx.x & 28);
-        any = __any_sync(quad, any);
-        if (any && (t & 3) == 0) sm.list[atomicAdd(&sm.n, 1)] = e0 + el;
+    if (t < ne * 54) {
+        const int el = t / 54, k = t - 54 * el, inod = k / 6, f = k - 6 * inod;
+        const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e0 + el]];
+        const double vp = v + prm.eps, back = vp - prm.eps;
+        sm.tl[el][0][k] = v;
+        sm.tl[el][2][k] = vp;
+        sm.tl[el][1][k] = back;
+        if (__double_as_longlong(back) != __double_as_longlong(v)) sm.any[el] = 1;
     }
     __syncthreads();
-    const int count = sm.n, grp = t >> 6, k = t & 63;
-    for (int i = 0; i < count; i += THREADS / 64) {
-        const bool live = i + grp < count;
-        const int e = live ? sm.list[i + grp] : 0;
-        if (live && k < 54) {
-            const int inod = k / 6, f = k - 6 * inod;
-            const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e]];
-            const double vp = v + eps;
-            sm.tl[grp][0][k] = v;
-            sm.tl[grp][2][k] = vp;
-            sm.tl[grp][1][k] = vp - eps;
-        }
-        __syncthreads();
-        const bool ac = k == 54;
-        if (live && (k < 54 || (ac && prm.nex > 0))) {
-            FdView V;
-            V.orig = sm.tl[grp][0];
-            V.rest = sm.tl[grp][1];
-            V.pert = sm.tl[grp][2];
-            V.kk = k;
-            double WiN = prm.WiN;
-            if (prm.nex > 0) {
-                const double eu = a.EU[prm.nex - 1];
-                WiN = prm.Wi0 * (ac ? eu + eps : eu);
-            }
-            double res[54];
+    const int el = t / 55, k = t - 55 * el, e = e0 + el;
+    const bool ac = k == 54;
+    if (el >= ne || !sm.any[el] || (ac && prm.nex == 0)) return;
+    FdView V;
+    V.orig = sm.tl[el][0];
+    V.rest = sm.tl[el][1];
+    V.pert = sm.tl[el][2];
+    V.kk = k;
+    double WiN = prm.WiN;
+    if (prm.nex > 0) {
+        const double eu = a.EU[prm.nex - 1];
+        WiN = prm.Wi0 * (ac ? eu + prm.eps : eu);
+    }
+    double res[54];
 #pragma unroll
-            for (int q = 0; q < 54; q++) res[q] = 0.0;
+    for (int q = 0; q < 54; q++) res[q] = 0.0;
 #pragma unroll 1
-            for (int ig = 0; ig < 9; ig++) {
-                const double *geo = a.geo + ((size_t)e * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
-                const Interp<double> I = interpolate(V, c_bfn[ig], dFx, dFy, geo + 18, geo + 27);
-                double dotU[9];
-                const GpCoef<double> g = gauss_point<FORM, SPEC>(I, prm, WiN, geo[36], dFx, dFy, dotU);
+    for (int ig = 0; ig < 9; ig++) {
+        const double *geo = a.geo + ((size_t)e * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
+        const Interp<double> I = interpolate(V, c_bfn[ig], dFx, dFy, geo + 18, geo + 27);
+        double dotU[9];
+        const GpCoef<double> g = gauss_point<FORM, SPEC>(I, prm, WiN, geo[36], dFx, dFy, dotU);
 #pragma unroll
-                for (int n = 0; n < 9; n++) {
-                    double o[6];
-                    test_node<FORM, SPEC>(g, prm, c_bfn[ig][n], dFx[n], dFy[n], dotU[n], geo[37], o);
+        for (int n = 0; n < 9; n++) {
+            double o[6];
+            test_node<FORM, SPEC>(g, prm, c_bfn[ig][n], dFx[n], dFy[n], dotU[n], geo[37], o);
 #pragma unroll
-                    for (int w = 0; w < 6; w++) res[n * 6 + w] = res[n * 6 + w] + o[w];
-                }
-            }
-            store_column(a, prm, e, ac ? 0 : k / 6, ac ? 6 : k - 6 * (k / 6), res);
+            for (int w = 0; w < 6; w++) res[n * 6 + w] = res[n * 6 + w] + o[w];
         }
-        __syncthreads();
     }
+    store_column(a, prm, e, ac ? 0 : k / 6, ac ? 6 : k - 6 * (k / 6), res);
 }
 
 template <int FORM, int SPEC, int THREADS>
@@ -572,7 +560,7 @@ __global__ void __launch_bounds__(THREADS, 256 / THREADS) k_fd64(const ElemArgs 
 // mesh's table (11% of the instructions, once per mesh instead of per call).
 // The 54 terms of a Gauss point go through shared memory three test nodes at a
 // time, which keeps a CTA at 31 KB, 6 or 7 of them per SM.  40,000 elements:
-// 2.43 ms -> RES_MS_AFTER.
+// 2.43 -> 1.63 ms.
 constexpr int RS_EPB = RES_EPB;
 constexpr int RS_THREADS = 64;
 constexpr int RS_MIN_CTAS = 6;
@@ -856,6 +844,8 @@ static cudaError_t go_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, k_fd64<FORM, SPEC, THREADS>, a, p, groups, run);
 }
+
+bool fd64_one_wave(int nel) { return nel <= FD_NARROW_MAX; }
 
 cudaError_t launch_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
 {

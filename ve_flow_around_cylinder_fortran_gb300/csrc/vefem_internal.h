@@ -82,6 +82,8 @@ struct EdgeArgs {
     double *es;                // [((k*81 + jnod*9 + inod)*36 + jeq*6 + ieq]
     double *as;                // [(k*9 + jnod)*6 + jeq]
 };
+// the forward difference of a mesh this small is a single wave of blocks
+bool fd64_one_wave(int nel);
 cudaError_t launch_edge64(const EdgeArgs &a, const KParams &p, int want_jac, cudaStream_t s);
 
 // What the scatter needs of a node-pair block, in one 32-byte load.
