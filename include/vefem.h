@@ -257,8 +257,10 @@ int vefem_frontal_solve_path(const vefem_frontal *f);
  * Every unknown is a pivot of exactly one front.  All of these are host arrays,
  * read by create only.
  * vefem_tree_factor: vals [nnz] (device) go to buf[dest[k]] (device, int64,
- * distinct), everything else in buf [buf_len] starts from zero; the elimination
- * leaves A^-1 and A^-1 B in the pivot rows.  tol, min_pivot and
+ * distinct), everything else in buf [buf_len] (16-byte aligned) starts from
+ * zero; the elimination leaves A^-1 and A^-1 B in the pivot rows.  Its products
+ * are formed from 63-bit fixed-point operands on the tensor cores and rounded
+ * once (an infinity or NaN makes its row or column of a product NaN).  tol, min_pivot and
  * VEFEM_ERR_SINGULAR as in vefem_frontal_factor.  Synchronises the stream.
  * vefem_tree_solve: x = A^-1 b, device vectors of N doubles; asynchronous on
  * the stream, vefem_tree_launches kernels replayed from a CUDA graph. */
@@ -322,7 +324,8 @@ int vefem_assemble_batched(vefem_batch *bt, const double *const *TL, const doubl
  * c clamped to 0..VEFEM_BATCH_CLASSES-1).  vefem_batch_autotune times every
  * candidate tile of every class present on the live GPU (reps launches each,
  * device-resident buffers of its own) and keeps the fastest; tiles_out
- * (may be NULL) receives the chosen tiles. */
+ * (may be NULL) receives the chosen tiles.  A tile is rounded up to whole groups
+ * of the elements the Jacobian kernel takes at a time (4 in FP32, 3 in FP64). */
 #define VEFEM_BATCH_CLASSES 6
 int vefem_batch_autotune(vefem_batch *bt, int flags, int reps, int *tiles_out);
 int vefem_batch_set_tiles(vefem_batch *bt, const int *tiles);
@@ -356,7 +359,7 @@ int vefem_mlp_forward(vefem_mlp *m, const float *X, int n, float *Y);
 /* loss = mean((net(X) - T)^2) and its gradient in the parameter layout */
 int vefem_mlp_loss_grad(vefem_mlp *m, const float *X, const float *T, int n, float *loss,
                         float *grad);
-/* iters Adam iterations at learning rate lr (one CUDA graph per iteration);
+/* iters Adam iterations at learning rate lr (CUDA graphs of eight iterations and of one);
  * final_loss (may be NULL) receives the loss of the last iteration's forward */
 int vefem_mlp_train(vefem_mlp *m, const float *X, const float *T, int n, int iters, float lr,
                     float *final_loss);

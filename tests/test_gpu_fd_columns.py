@@ -66,3 +66,8 @@ def test_models(model, ve, rtol, form, re, df):
 @pytest.mark.parametrize("residue", [1, 5, 60])
 def test_restore_residue_beside_clean_elements(form, residue):
     _check(13, 7, S.oldroyd_b(0.5, 0.59, form, nex=1), residue=residue)
+
+
+@pytest.mark.parametrize("residue", [3, 700])
+def test_restore_residue_on_a_mesh_of_several_waves(residue):
+    _check(31, 20, S.oldroyd_b(0.5, 0.59, "SQRT", nex=1), residue=residue)

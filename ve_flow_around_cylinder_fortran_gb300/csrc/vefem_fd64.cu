@@ -107,7 +107,8 @@ struct FdView {
 // so that every lane of a warp runs the same code; 28 + 18 + 9 CTAs cover the
 // same 252 elements, next to each other in the grid, so their parts of an
 // element's rows meet in L2.  Small meshes take 64-thread CTAs (2, 3, 7 elements;
-// 56, 54, 63 lanes), which spread over more SMs.  The base residual is k_res64's (launched before).
+// 56, 54, 63 lanes), which spread over more SMs, the smallest k_fd64_element.
+// The base residual is k_res64's (launched before).
 // An element with a restore residue ((x + eps) - eps differs from x, so later
 // columns see a changed state) is left to the last kind of CTA, which
 // evaluates it in full.
@@ -473,11 +474,11 @@ __device__ __forceinline__ void fd_pressure(const ElemArgs &a, const KParams &pr
 }
 
 // Elements with a restore residue: all 55 columns, each a full evaluation of the
-// state the sequential loop would have, 4 elements (1 in a CTA of 64 threads) on
-// 220 (55) lanes.  Values below eps that are not zero leave one, so a converged
-// flow has them wherever a component vanishes: 4 elements to a CTA and not 64 in
-// turn, which took 22 ms for 500 quads with residues in half of them, 1.4 now
-// (FD_RES_FIGURES).  A CTA without any costs its look at the state, 2 us.
+// state the sequential loop would have, 4 elements on 220 lanes.  Values below
+// eps that are not zero leave one, so a converged flow has them wherever a
+// component vanishes: 4 elements to a CTA and not 64 in turn, SQRT form, 20,000
+// quads with residues in all of them 75 -> 46.6 ms, in half 65 -> 39.8.  A CTA
+// without any costs its look at the state, 2 us.
 template <int FORM, int SPEC, int THREADS>
 __device__ __forceinline__ void fd_residue(const ElemArgs &a, const KParams &prm, int e0, FdResidueSmem<THREADS> &sm)
 {
@@ -527,6 +528,81 @@ __device__ __forceinline__ void fd_residue(const ElemArgs &a, const KParams &prm
         }
     }
     store_column(a, prm, e, ac ? 0 : k / 6, ac ? 6 : k - 6 * (k / 6), res);
+}
+
+// All columns of one element, 55 of 64 lanes, for a mesh whose elements fit the
+// GPU at once, up to three to an SM: its time is one column's chain of FP64
+// instructions, which keeping the other fields' part does not shorten (a
+// thread first waits for it), and the warps spread better over the SMs' pipes.
+// SQRT form, 300 quads: 765 us, 850 with residues (columns split by field 972 and
+// 1,243, all columns of four elements in 224 threads 1,255 and 1,440).
+struct FdElementSmem {
+    double tl[3][54];            // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
+    Interp<double> base[9];
+    int any;
+};
+
+template <int FORM, int SPEC>
+__global__ void __launch_bounds__(64, 4) k_fd64_element(const ElemArgs a, const KParams prm)
+{
+    __shared__ __align__(16) unsigned char raw[sizeof(FdElementSmem)];
+    FdElementSmem &sm = *reinterpret_cast<FdElementSmem *>(raw);
+    const int t = threadIdx.x, e = blockIdx.x, inod = t / 6, f = t - 6 * inod;
+    if (t == 0) sm.any = 0;
+    __syncthreads();
+    if (t < 54) {
+        const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e]];
+        const double vp = v + prm.eps, back = vp - prm.eps;
+        sm.tl[0][t] = v;
+        sm.tl[2][t] = vp;
+        sm.tl[1][t] = back;
+        if (__double_as_longlong(back) != __double_as_longlong(v)) sm.any = 1;
+    }
+    __syncthreads();
+    const bool clean = !sm.any;
+    if (clean && t < 9) {
+        const double *geo = a.geo + ((size_t)e * 9 + t) * GEO_REC;
+        SmemView V{sm.tl[0]};
+        sm.base[t] = interpolate(V, c_bfn[t], geo, geo + 9, geo + 18, geo + 27);
+    }
+    __syncthreads();
+    const bool ac = t == 54;
+    if (t > 54 || (ac && prm.nex == 0)) return;
+    double WiN = prm.WiN;
+    if (prm.nex > 0) {
+        const double eu = a.EU[prm.nex - 1];
+        WiN = prm.Wi0 * (ac ? eu + prm.eps : eu);
+    }
+    double res[54];
+#pragma unroll
+    for (int q = 0; q < 54; q++) res[q] = 0.0;
+#pragma unroll 1
+    for (int ig = 0; ig < 9; ig++) {
+        const double *geo = a.geo + ((size_t)e * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
+        Interp<double> I;
+        if (clean) {
+            I = sm.base[ig];
+            FdCleanView V{sm.tl[0], sm.tl[2], t};
+            if (!ac) interpolate_field(V, f, c_bfn[ig], dFx, dFy, geo + 18, geo + 27, I);
+        } else {
+            FdView V;
+            V.orig = sm.tl[0];
+            V.rest = sm.tl[1];
+            V.pert = sm.tl[2];
+            V.kk = t;
+            I = interpolate(V, c_bfn[ig], dFx, dFy, geo + 18, geo + 27);
+        }
+        double dotU[9];
+        const GpCoef<double> g = gauss_point<FORM, SPEC>(I, prm, WiN, geo[36], dFx, dFy, dotU);
+#pragma unroll
+        for (int n = 0; n < 9; n++) {
+            double o[6];
+            test_node<FORM, SPEC>(g, prm, c_bfn[ig][n], dFx[n], dFy[n], dotU[n], geo[37], o);
+#pragma unroll
+            for (int w = 0; w < 6; w++) res[n * 6 + w] = res[n * 6 + w] + o[w];
+        }
+    }
+    store_column(a, prm, e, ac ? 0 : inod, ac ? 6 : f, res);
 }
 
 template <int FORM, int SPEC, int THREADS>
@@ -820,11 +896,27 @@ int residual_batched_ctas_per_sm(int form, int spec)
     return n;
 }
 
-template <int FORM, int SPEC, int THREADS>
-static cudaError_t go_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
+template <class... P>
+static cudaError_t launch_fd(void (*kernel)(P...), int grid, int threads, int smem, bool early, cudaStream_t s, P... args)
 {
-    // a small mesh is one group: all stress CTAs, the longest, are placed first
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <int FORM, int SPEC, int THREADS>
+static cudaError_t go_columns(const ElemArgs &a, const KParams &p, bool early, cudaStream_t s)
+{
     typedef FdRun<THREADS> Run;
+    // a small mesh is one group: all stress CTAs, the longest, are placed first
     const int run = THREADS == 64 ? a.nel : FD_RUN, groups = (a.nel + run - 1) / run;
     const int per = (run + Run::S - 1) / Run::S + (run + Run::U - 1) / Run::U + (run + Run::P - 1) / Run::P;
     const int residue = (a.nel + Run::R - 1) / Run::R;
@@ -832,17 +924,19 @@ static cudaError_t go_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
     const cudaError_t e =
         cudaFuncSetAttribute(k_fd64<FORM, SPEC, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(groups * per + residue));
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_fd64<FORM, SPEC, THREADS>, a, p, groups, run);
+    return launch_fd<ElemArgs, KParams, int, int>(k_fd64<FORM, SPEC, THREADS>, groups * per + residue, THREADS, smem, early, s,
+                                                  a, p, groups, run);
+}
+
+// One wave of blocks does not start beside the residual kernel: its blocks would
+// go where the residual's leave first, four to an SM on some (300 quads, SQRT
+// form, 765 us in order and 1,368 early).
+template <int FORM, int SPEC>
+static cudaError_t go_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
+{
+    if (a.nel <= FD_ELEMENT_MAX) return launch_fd<ElemArgs, KParams>(k_fd64_element<FORM, SPEC>, a.nel, 64, 0, false, s, a, p);
+    if (a.nel <= FD_NARROW_MAX) return go_columns<FORM, SPEC, 64>(a, p, false, s);
+    return go_columns<FORM, SPEC, 256>(a, p, true, s);
 }
 
 bool fd64_one_wave(int nel) { return nel <= FD_NARROW_MAX; }
@@ -850,7 +944,7 @@ bool fd64_one_wave(int nel) { return nel <= FD_NARROW_MAX; }
 cudaError_t launch_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
 {
     if (a.nel <= 0) return cudaSuccess;
-#define GO(F, SP) return a.nel <= FD_NARROW_MAX ? go_fd64<F, SP, 64>(a, p, s) : go_fd64<F, SP, 256>(a, p, s)
+#define GO(F, SP) return go_fd64<F, SP>(a, p, s)
     RES_DISPATCH(p.form, spec_of(p), GO);
 #undef GO
     return cudaSuccess;

@@ -19,10 +19,12 @@ constexpr int RES_EPB = 7;
 // 1, 51 / 65 / 65 / 65 with 3, 98 throughout with k_res64; one wave more costs
 // 94 (1, 800 quads) and 96 us (3, 1,000).
 constexpr int RES_WIDE1_MAX = 4 * 152, RES_WIDE3_MAX = 6 * 152;
-// Forward-difference kernel: meshes up to this size take 64-thread CTAs, four
-// of which are resident on each of 152 SMs.  SQRT form, 64 against 256 threads:
-// 0.69 / 1.33 ms on 200 quads, 1.30 / 1.35 on 600, 1.56 / 1.36 on 700; T form
-// 0.44 / 0.79 on 200, even on 500, 1.13 / 0.90 on 700.
+// Forward-difference kernel.  Up to three elements per SM a CTA of 64 threads
+// takes an element's columns, up to four CTAs per SM of 64 threads take columns by
+// field, then CTAs of 256.  SQRT form on 210 / 300 / 400 / 500 / 600 quads: elements
+// 760 / 765 / 1,076 / 1,406 / 1,408 us, by field in 64 threads 693 / 972 / 1,086 / 1,289 /
+// 1,291, in 256 threads 1,330 to 1,350; 700 quads 1,560 (64) and 1,345 (256).
+constexpr int FD_ELEMENT_MAX = 3 * 152;
 constexpr int FD_NARROW_MAX = 4 * 152;
 // doubles per Gauss point of a mesh's geometry table
 constexpr int GEO_REC = 38;

@@ -731,7 +731,7 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
 extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_t *dest, int64_t nnz, double *buf,
                                  int64_t buf_len, void *stream, double tol, double *min_pivot)
 {
-    if (!f || !vals || !dest || nnz <= 0 || !buf) return VEFEM_ERR_ARG;
+    if (!f || !vals || !dest || nnz <= 0 || !buf || reinterpret_cast<uintptr_t>(buf) % 16) return VEFEM_ERR_ARG;
     Guard g(f->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const double one = 1.0;

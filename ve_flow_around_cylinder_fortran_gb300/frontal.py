@@ -13,8 +13,9 @@ Two orderings of the fronts:
 
 * Nested dissection (the default on a CUDA device): the fronts of a binary
   tree of element sets (``dissection.py``), all fronts of one depth at a time
-  in the library's kernels (``csrc/vefem_tree.cu``).  50 G multiply-adds and
-  260 dependent steps for 20,000 quads.
+  in the library's kernels (``csrc/vefem_tree.cu``), the products on the
+  tensor cores in exact digits (``csrc/vefem_split.cuh``).  50 G multiply-adds
+  and 133 dependent steps for 20,000 quads.
 * Panels (``panel`` given, the pivoted method, the CPU): elements are swept
   downstream in order of their centroid x and grouped into panels of ``G``
   elements.  A node is *fully summed* after the last panel that touches it;
@@ -42,7 +43,7 @@ Solve of the pivoted method: forward y_P = LU_q^-1 b_P, b_F -= M_q[F, P] y_P;
 backward x_P = y_P - X_q x_F.  Each solve is checked against the CSR matrix
 (FP64 SpMV) and refined (x += solve(b - A x)) up to ``refine`` times; a zero
 pivot or a solve that stays inaccurate hands the matrix to the host SuperLU
-(``linsolve.SparseLU``) for that factorisation.  Everything is FP64.
+(``linsolve.SparseLU``) for that factorisation.  Values, factors and vectors are FP64.
 """
 from __future__ import annotations
 
