@@ -375,6 +375,9 @@ class FrontalLU:
             # a copy: the caller's buffer is overwritten by the next assembly
             # while this factorisation is still in use
             v = vals.to(device=self.dev, dtype=torch.float64, copy=True)
+        if v.shape != self.dest.shape:
+            # the library takes the count from here and the places from dest
+            raise RuntimeError(f"{tuple(v.shape)} AIJ values for a pattern of {self.dest.numel()}")
         self.vals = v
         self._since_factor = 0
         self._needs_checks = False
