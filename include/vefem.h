@@ -257,10 +257,11 @@ int vefem_frontal_solve_path(const vefem_frontal *f);
  * Every unknown is a pivot of exactly one front.  All of these are host arrays,
  * read by create only.
  * vefem_tree_factor: vals [nnz] (device) go to buf[dest[k]] (device, int64,
- * distinct), everything else in buf [buf_len] (16-byte aligned) starts from
- * zero; the elimination leaves A^-1 and A^-1 B in the pivot rows.  Its products
- * are formed from 63-bit fixed-point operands on the tensor cores and rounded
- * once (an infinity or NaN makes its row or column of a product NaN).  tol, min_pivot and
+ * distinct), everything else in buf [buf_len] (16-byte aligned, at least
+ * off[nfront] long or VEFEM_ERR_ARG) starts from zero; the elimination leaves
+ * A^-1 and A^-1 B in the pivot rows.  Its products are formed from 63-bit
+ * fixed-point operands on the tensor cores and rounded once (an infinity or NaN
+ * makes its row or column of a product NaN).  tol, min_pivot and
  * VEFEM_ERR_SINGULAR as in vefem_frontal_factor.  Synchronises the stream.
  * vefem_tree_solve: x = A^-1 b, device vectors of N doubles; asynchronous on
  * the stream, vefem_tree_launches kernels replayed from a CUDA graph. */

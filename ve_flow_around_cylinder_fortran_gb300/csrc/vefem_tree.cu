@@ -523,7 +523,7 @@ struct Level {
 
 struct vefem_tree {
     int device = 0, nfront = 0, sms = 0;
-    int64_t N = 0, total = 0;
+    int64_t N = 0, total = 0, buf_len = 0;  // buf_len: doubles that the fronts take
     std::vector<Level> levels;
     int pmax = 0, qmax = 0;
     Front *fr = nullptr;
@@ -621,7 +621,7 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
         !src || N <= 0 || N >= INT32_MAX || idx_off[nfront] >= INT32_MAX)
         return VEFEM_ERR_ARG;
     *out = nullptr;
-    if (level_ptr[0] != 0 || level_ptr[nlevel] != nfront) return VEFEM_ERR_ARG;
+    if (level_ptr[0] != 0 || level_ptr[nlevel] != nfront || off[0] < 0) return VEFEM_ERR_ARG;
     const int64_t tot = idx_off[nfront];
     // every unknown a pivot once; every map inside its child's boundary; children one level below
     std::vector<int> level(nfront);
@@ -657,6 +657,7 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
     f->nfront = nfront;
     f->N = N;
     f->total = tot;
+    f->buf_len = off[nfront];
     std::vector<Front> fr(nfront);
     std::vector<int32_t> perm(nfront);
     std::iota(perm.begin(), perm.end(), 0);
@@ -731,7 +732,8 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
 extern "C" int vefem_tree_factor(vefem_tree *f, const double *vals, const int64_t *dest, int64_t nnz, double *buf,
                                  int64_t buf_len, void *stream, double tol, double *min_pivot)
 {
-    if (!f || !vals || !dest || nnz <= 0 || !buf || reinterpret_cast<uintptr_t>(buf) % 16) return VEFEM_ERR_ARG;
+    if (!f || !vals || !dest || nnz <= 0 || !buf || reinterpret_cast<uintptr_t>(buf) % 16 || buf_len < f->buf_len)
+        return VEFEM_ERR_ARG;
     Guard g(f->device);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const double one = 1.0;
