@@ -51,3 +51,23 @@ def test_short_buffer_is_refused(short):
     assert bool((buf == 7.0).all())
     assert factor(need) == 0
     lib.vefem_tree_destroy(h)
+
+
+def test_handles_of_different_sizes():
+    """Fronts beyond 48 KB of staged vector: the smaller handle's creation does
+    not lower what the larger one's sweeps may take."""
+    lib = V.load()
+    N = 7000
+    big, need = _one_front(N)
+    small, _ = _one_front(6400)
+    buf = torch.zeros(N, need // N, dtype=torch.float64, device="cuda")
+    buf[torch.arange(N), torch.arange(N)] = 2.0                              # in place of an inverse
+    b = torch.arange(N, dtype=torch.float64, device="cuda")
+    x = torch.zeros_like(b)
+    torch.cuda.synchronize()
+    assert lib.vefem_tree_solve(big, ct.c_void_p(buf.data_ptr()), ct.c_void_p(b.data_ptr()),
+                                ct.c_void_p(x.data_ptr()), ct.c_void_p(0)) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(x, 2.0 * b)
+    lib.vefem_tree_destroy(small)
+    lib.vefem_tree_destroy(big)

@@ -707,20 +707,24 @@ extern "C" int vefem_tree_create(int device, int nfront, int nlevel, const int32
         put(&f->tpan, none, (size_t)tmax) && put(&f->dinv, none, (size_t)dmax) && put(&f->y, none, (size_t)tot) && put(&f->b, none, (size_t)N) &&
         put(&f->x, none, (size_t)N) && put(&f->err, (const int *)nullptr, 1) &&
         put(&f->minpiv, (const unsigned long long *)nullptr, 1);
-    const int sm_p = f->pmax * (int)sizeof(double), sm_q = f->qmax * (int)sizeof(double);
-    if (!ok ||
+    // The sweeps stage a vector of pivots or boundary unknowns.  The limit of a
+    // kernel's dynamic shared memory is the device's, not this handle's: beyond
+    // the default it is set to all there is, so that no handle lowers another's.
+    const int64_t staged = (int64_t)std::max(f->pmax, f->qmax) * (int64_t)sizeof(double);
+    int most = 0;
+    bool fits = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) == cudaSuccess &&
+                staged <= most;
+    if (fits && staged > 48 * 1024)
+        fits = cudaFuncSetAttribute(k_tree_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tree_up, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tree_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
+    if (!ok || !fits ||
         cudaFuncSetAttribute(k_pivot, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SHORT_SMEM<KB>) != cudaSuccess ||
         cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize, split::SHORT_SMEM<split::TN>) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_schur<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              2 * split::STAGE) != cudaSuccess ||
-        cudaFuncSetAttribute(k_schur<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, split::STAGE) !=
-            cudaSuccess ||
-        (sm_p > 48 * 1024 &&
-                (cudaFuncSetAttribute(k_tree_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess ||
-                 cudaFuncSetAttribute(k_tree_up, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_p) != cudaSuccess)) ||
-        (sm_q > 48 * 1024 &&
-         cudaFuncSetAttribute(k_tree_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, sm_q) != cudaSuccess)) {
+        cudaFuncSetAttribute(k_schur<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, split::STAGE) != cudaSuccess) {
         cudaGetLastError();
         vefem_tree_destroy(f);
         return VEFEM_ERR_NOMEM;
