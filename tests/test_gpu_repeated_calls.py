@@ -1,0 +1,44 @@
+"""Calls whose input buffers are overwritten from one call to the next, many
+times over: every result has the bits of the first call on the same values.  A
+kernel that begins while its predecessors run may not read what they, or those
+before them, left in a cache."""
+import numpy as np
+import pytest
+import torch
+
+from ve_flow_around_cylinder_fortran_gb300 import build as B
+from ve_flow_around_cylinder_fortran_gb300 import mesh as M
+from ve_flow_around_cylinder_fortran_gb300 import pattern as P
+from ve_flow_around_cylinder_fortran_gb300 import state as S
+from ve_flow_around_cylinder_fortran_gb300 import vefem as V
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _built():
+    B.build()
+    V.load()
+
+
+@pytest.mark.parametrize("nel", [300, 520, 700, 2000])
+def test_forward_difference(nel):
+    mesh = M.build_cylinder_mesh(nel, exact=False)
+    phys = S.oldroyd_b(0.5, 0.59, "SQRT", nex=1)
+    rp, ci = P.build_pattern(mesh.element_nodes(), mesh.nnodes, 1)
+    asm = V.BulkAssembler(mesh, phys, rp, ci)
+    states = [torch.from_numpy(S.seeded_state(mesh.xyz, phys, s)[0]).cuda() for s in (1, 2, 3)]
+    TL, EU = torch.empty_like(states[0]), torch.ones(1, dtype=torch.float64, device="cuda")
+    first = {}
+    for call in range(24):
+        k = call * 7 % 3
+        TL.copy_(states[k])
+        EU.fill_(1.0 + 0.25 * k)
+        b = torch.zeros(asm.N, dtype=torch.float64, device="cuda")
+        v = torch.zeros(asm.nnz, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        asm.assemble(TL, EU, V.VEFEM_RESIDUAL | V.VEFEM_JAC_FD64 | V.VEFEM_ZERO_FIRST, b, v, on_device=True)
+        torch.cuda.synchronize()
+        fb, fv = first.setdefault(k, (b, v))
+        assert torch.equal(b, fb) and torch.equal(v, fv)
+    asm.close()
