@@ -107,8 +107,8 @@ struct FdView {
 //    9 pressure columns                        x 28 elements (252)
 // so that every lane of a warp runs the same code; 28 + 18 + 9 CTAs cover the
 // same 252 elements, next to each other in the grid, so their parts of an
-// element's rows meet in L2.  Small meshes take 64-thread CTAs (2, 3, 7 elements;
-// 56, 54, 63 lanes), which spread over more SMs, the smallest k_fd64_element.
+// element's rows meet in L2.  Meshes of up to four elements per SM take
+// k_fd64_element.
 // The base residual is k_res64's (launched before).
 // An element with a restore residue ((x + eps) - eps differs from x, so later
 // columns see a changed state) is left to the last kind of CTA, which
@@ -120,52 +120,48 @@ struct FdView {
 // T form 50.9 -> 40.8 on 40,000.
 constexpr int FS_COLS = 28, FU_COLS = 18, FP_COLS = 9;
 
-// Elements per CTA by kind (stress, velocity, pressure, residue check)
-template <int THREADS> struct FdRun;
-template <> struct FdRun<256> { static constexpr int S = 9, U = 14, P = 28, R = 4; };
-template <> struct FdRun<64> { static constexpr int S = 2, U = 3, P = 7, R = 1; };
-constexpr int FD_RUN = 252;       // elements of a group of 256-thread CTAs
+constexpr int FD_THREADS = 256;
+// elements per CTA by kind (stress, velocity, pressure, residue check)
+constexpr int FD_S = 9, FD_U = 14, FD_P = 28, FD_R = 4;
+constexpr int FD_RUN = 252;       // elements of a group of CTAs
 
-template <int EL>
 struct FdStressSmem {
-    double tl[EL][2][54];        // 0: original, 1: perturbed x + eps
-    Interp<double> base[EL][9];
-    FlowPart<double> flow[EL][9];
-    double dotU[EL][9][9];
-    int residue[EL];
+    double tl[FD_S][2][54];        // 0: original, 1: perturbed x + eps
+    Interp<double> base[FD_S][9];
+    FlowPart<double> flow[FD_S][9];
+    double dotU[FD_S][9][9];
+    int residue[FD_S];
 };
 
-template <int FORM, int EL>
+template <int FORM>
 struct FdFlowSmem {
-    double tl[EL][2][54];
-    Interp<double> base[EL][9];
-    StressPart<double> stress[EL][9];
-    double test[EL][9][9][FORM == FORM_SQRT ? 11 : 3];       // TestStress (T form: grad S . grad phi only)
-    int residue[EL];
+    double tl[FD_U][2][54];
+    Interp<double> base[FD_U][9];
+    StressPart<double> stress[FD_U][9];
+    double test[FD_U][9][9][FORM == FORM_SQRT ? 11 : 3];       // TestStress (T form: grad S . grad phi only)
+    int residue[FD_U];
 };
 
-template <int EL>
 struct FdPressureSmem {
-    double tl[EL][54];
-    double pert[EL][9];
-    GpCoef<double> g[EL][9];
-    double keep[EL][9][6];       // stress + BvN G without p, div T, BvN Laplacian
-    TestPressure<double> test[EL][9];                         // of the current Gauss point
-    int residue[EL];
+    double tl[FD_P][54];
+    double pert[FD_P][9];
+    GpCoef<double> g[FD_P][9];
+    double keep[FD_P][9][6];       // stress + BvN G without p, div T, BvN Laplacian
+    TestPressure<double> test[FD_P][9];                         // of the current Gauss point
+    int residue[FD_P];
 };
 
-template <int THREADS>
 struct FdResidueSmem {
-    double tl[FdRun<THREADS>::R][3][54];   // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
-    int any[FdRun<THREADS>::R];
+    double tl[FD_R][3][54];      // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
+    int any[FD_R];
 };
 
-template <int FORM, int THREADS>
+template <int FORM>
 union FdSmem {
-    FdStressSmem<FdRun<THREADS>::S> s;
-    FdFlowSmem<FORM, FdRun<THREADS>::U> u;
-    FdPressureSmem<FdRun<THREADS>::P> p;
-    FdResidueSmem<THREADS> r;
+    FdStressSmem s;
+    FdFlowSmem<FORM> u;
+    FdPressureSmem p;
+    FdResidueSmem r;
 };
 
 // x / y with r the rounded reciprocal of y: div_r's steps, infinities and NaN
@@ -224,13 +220,13 @@ __device__ __forceinline__ void store_column(const ElemArgs &a, const KParams &p
 }
 
 // stage the states of elements e0 .. e0 + ne, and mark those with a restore residue
-template <int EL, int THREADS>
+template <int EL>
 __device__ __forceinline__ void stage_states(const ElemArgs &a, const KParams &prm, int e0, int ne,
                                              double (*tl)[2][54], int *residue)
 {
-    for (int i = threadIdx.x; i < EL; i += THREADS) residue[i] = 0;
+    for (int i = threadIdx.x; i < EL; i += FD_THREADS) residue[i] = 0;
     __syncthreads();
-    for (int i = threadIdx.x; i < ne * 54; i += THREADS) {
+    for (int i = threadIdx.x; i < ne * 54; i += FD_THREADS) {
         const int el = i / 54, pos = i - 54 * el, inod = pos / 6, f = pos - 6 * inod;
         const double v = early_state(a, f, inod, e0 + el);
         const double vp = v + prm.eps, back = vp - prm.eps;
@@ -267,14 +263,14 @@ __device__ __forceinline__ void perturbed(const FdCleanView &V, int f, const dou
     }
 }
 
-template <int FORM, int SPEC, int EL, int THREADS>
-__device__ __forceinline__ void fd_stress(const ElemArgs &a, const KParams &prm, int e0, FdStressSmem<EL> &sm)
+template <int FORM, int SPEC>
+__device__ __forceinline__ void fd_stress(const ElemArgs &a, const KParams &prm, int e0, FdStressSmem &sm)
 {
-    static_assert(EL * FS_COLS <= THREADS, "a thread per column");
-    const int t = threadIdx.x, ne = min(EL, a.nel - e0);
+    static_assert(FD_S * FS_COLS <= FD_THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(FD_S, a.nel - e0);
     if (ne <= 0) return;
-    stage_states<EL, THREADS>(a, prm, e0, ne, sm.tl, sm.residue);
-    for (int i = t; i < ne * 9; i += THREADS) {
+    stage_states<FD_S>(a, prm, e0, ne, sm.tl, sm.residue);
+    for (int i = t; i < ne * 9; i += FD_THREADS) {
         const int el = i / 9, ig = i - 9 * el;
         const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
         SmemView V{sm.tl[el][0]};
@@ -325,15 +321,15 @@ __device__ __forceinline__ void fd_stress(const ElemArgs &a, const KParams &prm,
     store_column(a, prm, e, inod, ac ? 6 : f, res);
 }
 
-template <int FORM, int SPEC, int EL, int THREADS>
-__device__ __forceinline__ void fd_flow(const ElemArgs &a, const KParams &prm, int e0, FdFlowSmem<FORM, EL> &sm)
+template <int FORM, int SPEC>
+__device__ __forceinline__ void fd_flow(const ElemArgs &a, const KParams &prm, int e0, FdFlowSmem<FORM> &sm)
 {
-    static_assert(EL * FU_COLS <= THREADS, "a thread per column");
-    const int t = threadIdx.x, ne = min(EL, a.nel - e0);
+    static_assert(FD_U * FU_COLS <= FD_THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(FD_U, a.nel - e0);
     if (ne <= 0) return;
     const double WiN = early_wi(a, prm);
-    stage_states<EL, THREADS>(a, prm, e0, ne, sm.tl, sm.residue);
-    for (int i = t; i < ne * 9; i += THREADS) {
+    stage_states<FD_U>(a, prm, e0, ne, sm.tl, sm.residue);
+    for (int i = t; i < ne * 9; i += FD_THREADS) {
         const int el = i / 9, ig = i - 9 * el;
         const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
         SmemView V{sm.tl[el][0]};
@@ -342,7 +338,7 @@ __device__ __forceinline__ void fd_flow(const ElemArgs &a, const KParams &prm, i
         sm.stress[el][ig] = stress_part<FORM>(I, prm, WiN, geo[36]);
     }
     __syncthreads();
-    for (int i = t; i < ne * 81; i += THREADS) {
+    for (int i = t; i < ne * 81; i += FD_THREADS) {
         const int el = i / 81, ig = (i / 9) % 9, n = i % 9;
         const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
         const StressPart<double> &p = sm.stress[el][ig];
@@ -396,16 +392,16 @@ __device__ __forceinline__ void fd_flow(const ElemArgs &a, const KParams &prm, i
     store_column(a, prm, e, inod, f, res);
 }
 
-template <int FORM, int SPEC, int EL, int THREADS>
-__device__ __forceinline__ void fd_pressure(const ElemArgs &a, const KParams &prm, int e0, FdPressureSmem<EL> &sm)
+template <int FORM, int SPEC>
+__device__ __forceinline__ void fd_pressure(const ElemArgs &a, const KParams &prm, int e0, FdPressureSmem &sm)
 {
-    static_assert(EL * FP_COLS <= THREADS, "a thread per column");
-    const int t = threadIdx.x, ne = min(EL, a.nel - e0);
+    static_assert(FD_P * FP_COLS <= FD_THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(FD_P, a.nel - e0);
     if (ne <= 0) return;
     const double WiN = early_wi(a, prm);
-    for (int i = t; i < EL; i += THREADS) sm.residue[i] = 0;
+    for (int i = t; i < FD_P; i += FD_THREADS) sm.residue[i] = 0;
     __syncthreads();
-    for (int i = t; i < ne * 54; i += THREADS) {
+    for (int i = t; i < ne * 54; i += FD_THREADS) {
         const int el = i / 54, pos = i - 54 * el, inod = pos / 6, f = pos - 6 * inod;
         const double v = early_state(a, f, inod, e0 + el);
         const double vp = v + prm.eps, back = vp - prm.eps;
@@ -414,7 +410,7 @@ __device__ __forceinline__ void fd_pressure(const ElemArgs &a, const KParams &pr
         if (__double_as_longlong(back) != __double_as_longlong(v)) sm.residue[el] = 1;
     }
     __syncthreads();
-    for (int i = t; i < ne * 9; i += THREADS) {
+    for (int i = t; i < ne * 9; i += FD_THREADS) {
         const int el = i / 9, ig = i - 9 * el;
         const double *geo = a.geo + ((size_t)(e0 + el) * 9 + ig) * GEO_REC;
         SmemView V{sm.tl[el]};
@@ -492,13 +488,12 @@ __device__ __forceinline__ void fd_pressure(const ElemArgs &a, const KParams &pr
 // component vanishes: 4 elements to a CTA and not 64 in turn, SQRT form, 20,000
 // quads with residues in all of them 75 -> 46.6 ms, in half 65 -> 39.8.  A CTA
 // without any costs its look at the state, 2 us.
-template <int FORM, int SPEC, int THREADS>
-__device__ __forceinline__ void fd_residue(const ElemArgs &a, const KParams &prm, int e0, FdResidueSmem<THREADS> &sm)
+template <int FORM, int SPEC>
+__device__ __forceinline__ void fd_residue(const ElemArgs &a, const KParams &prm, int e0, FdResidueSmem &sm)
 {
-    constexpr int R = FdRun<THREADS>::R;
-    static_assert(R * 55 <= THREADS, "a thread per column");
-    const int t = threadIdx.x, ne = min(R, a.nel - e0);
-    if (t < R) sm.any[t] = 0;
+    static_assert(FD_R * 55 <= FD_THREADS, "a thread per column");
+    const int t = threadIdx.x, ne = min(FD_R, a.nel - e0);
+    if (t < FD_R) sm.any[t] = 0;
     __syncthreads();
     if (t < ne * 54) {
         const int el = t / 54, k = t - 54 * el, inod = k / 6, f = k - 6 * inod;
@@ -539,44 +534,54 @@ __device__ __forceinline__ void fd_residue(const ElemArgs &a, const KParams &prm
     store_column(a, prm, e, ac ? 0 : k / 6, ac ? 6 : k - 6 * (k / 6), res);
 }
 
-// All columns of one element, 55 of 64 lanes, for a mesh whose elements fit the
-// GPU at once, up to three to an SM: its time is one column's chain of FP64
-// instructions, which keeping the other fields' part does not shorten (a
-// thread first waits for it), and the warps spread better over the SMs' pipes.
-// SQRT form, 300 quads: 765 us, 850 with residues (columns split by field 972 and
-// 1,243, all columns of four elements in 224 threads 1,255 and 1,440).
+// All columns of an element in one CTA, for a mesh whose CTAs fit the GPU at once:
+// its time is one column's chain of FP64 instructions, which keeping the other
+// fields' part does not shorten (a thread first waits for it).  One element, 55
+// of 64 lanes, where there are up to three to an SM: SQRT form, 300 quads, 765
+// us, 850 with residues (four elements 1,255 and 1,440).  Four, 220 of 224 lanes,
+// up to four to an SM, where a CTA of one would be the fourth on some of them:
+// SQRT form, 460 / 500 / 606 quads, 1,240 / 1,241 / 1,244 us, with residues in half
+// of the elements 1,413 / 1,415 / 1,425; T form 757 to 759 and 932 to 943.  Columns
+// by field in CTAs of 64 threads took 1,220 / 1,288 / 1,289 and 1,443 / 1,626 /
+// 1,819 there, in the T form 775 to 786 and 995 to 1,283.
+template <int EL>
 struct FdElementSmem {
-    double tl[3][54];            // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
-    Interp<double> base[9];
-    int any;
+    double tl[EL][3][54];        // 0: original, 1: restored (x+eps)-eps, 2: perturbed x+eps
+    Interp<double> base[EL][9];
+    int any[EL];
 };
 
-template <int FORM, int SPEC>
-__global__ void __launch_bounds__(64, 4) k_fd64_element(const ElemArgs a, const KParams prm)
+constexpr int FE_COLS = 55;
+template <int EL> constexpr int FE_THREADS = (EL * FE_COLS + 31) / 32 * 32;
+
+template <int FORM, int SPEC, int EL>
+__global__ void __launch_bounds__(FE_THREADS<EL>, EL == 1 ? 4 : 1) k_fd64_element(const ElemArgs a, const KParams prm)
 {
-    __shared__ __align__(16) unsigned char raw[sizeof(FdElementSmem)];
-    FdElementSmem &sm = *reinterpret_cast<FdElementSmem *>(raw);
-    const int t = threadIdx.x, e = blockIdx.x, inod = t / 6, f = t - 6 * inod;
-    if (t == 0) sm.any = 0;
+    __shared__ __align__(16) unsigned char raw[sizeof(FdElementSmem<EL>)];
+    FdElementSmem<EL> &sm = *reinterpret_cast<FdElementSmem<EL> *>(raw);
+    const int el = threadIdx.x / FE_COLS, t = threadIdx.x - FE_COLS * el, e = blockIdx.x * EL + el;
+    const bool in = el < EL && e < a.nel;
+    const int inod = t / 6, f = t - 6 * inod;
+    if (threadIdx.x < EL) sm.any[threadIdx.x] = 0;
     __syncthreads();
-    if (t < 54) {
+    if (in && t < 54) {
         const double v = a.TL[(size_t)f * a.nnodes + a.conn[inod * a.nel + e]];
         const double vp = v + prm.eps, back = vp - prm.eps;
-        sm.tl[0][t] = v;
-        sm.tl[2][t] = vp;
-        sm.tl[1][t] = back;
-        if (__double_as_longlong(back) != __double_as_longlong(v)) sm.any = 1;
+        sm.tl[el][0][t] = v;
+        sm.tl[el][2][t] = vp;
+        sm.tl[el][1][t] = back;
+        if (__double_as_longlong(back) != __double_as_longlong(v)) sm.any[el] = 1;
     }
     __syncthreads();
-    const bool clean = !sm.any;
+    const bool clean = in && !sm.any[el];
     if (clean && t < 9) {
         const double *geo = a.geo + ((size_t)e * 9 + t) * GEO_REC;
-        SmemView V{sm.tl[0]};
-        sm.base[t] = interpolate(V, c_bfn[t], geo, geo + 9, geo + 18, geo + 27);
+        SmemView V{sm.tl[el][0]};
+        sm.base[el][t] = interpolate(V, c_bfn[t], geo, geo + 9, geo + 18, geo + 27);
     }
     __syncthreads();
     const bool ac = t == 54;
-    if (t > 54 || (ac && prm.nex == 0)) return;
+    if (!in || (ac && prm.nex == 0)) return;
     double WiN = prm.WiN;
     if (prm.nex > 0) {
         const double eu = a.EU[prm.nex - 1];
@@ -590,14 +595,14 @@ __global__ void __launch_bounds__(64, 4) k_fd64_element(const ElemArgs a, const 
         const double *geo = a.geo + ((size_t)e * 9 + ig) * GEO_REC, *dFx = geo, *dFy = geo + 9;
         Interp<double> I;
         if (clean) {
-            I = sm.base[ig];
-            FdCleanView V{sm.tl[0], sm.tl[2], t};
+            I = sm.base[el][ig];
+            FdCleanView V{sm.tl[el][0], sm.tl[el][2], t};
             if (!ac) interpolate_field(V, f, c_bfn[ig], dFx, dFy, geo + 18, geo + 27, I);
         } else {
             FdView V;
-            V.orig = sm.tl[0];
-            V.rest = sm.tl[1];
-            V.pert = sm.tl[2];
+            V.orig = sm.tl[el][0];
+            V.rest = sm.tl[el][1];
+            V.pert = sm.tl[el][2];
             V.kk = t;
             I = interpolate(V, c_bfn[ig], dFx, dFy, geo + 18, geo + 27);
         }
@@ -614,26 +619,26 @@ __global__ void __launch_bounds__(64, 4) k_fd64_element(const ElemArgs a, const 
     store_column(a, prm, e, ac ? 0 : inod, ac ? 6 : f, res);
 }
 
-template <int FORM, int SPEC, int THREADS>
-__global__ void __launch_bounds__(THREADS, 256 / THREADS) k_fd64(const ElemArgs a, const KParams prm, int groups, int run)
+template <int FORM, int SPEC>
+__global__ void __launch_bounds__(FD_THREADS, 1) k_fd64(const ElemArgs a, const KParams prm, int groups)
 {
-    typedef FdRun<THREADS> Run;
     extern __shared__ __align__(16) unsigned char fd_raw[];
-    FdSmem<FORM, THREADS> &sm = *reinterpret_cast<FdSmem<FORM, THREADS> *>(fd_raw);
-    // CTAs of each kind in a group of `run` elements, in this order
-    const int S = (run + Run::S - 1) / Run::S, U = (run + Run::U - 1) / Run::U, P = (run + Run::P - 1) / Run::P;
+    FdSmem<FORM> &sm = *reinterpret_cast<FdSmem<FORM> *>(fd_raw);
+    // CTAs of each kind in a group, in this order
+    constexpr int S = FD_RUN / FD_S, U = FD_RUN / FD_U, P = FD_RUN / FD_P;
+    static_assert(S * FD_S == FD_RUN && U * FD_U == FD_RUN && P * FD_P == FD_RUN, "whole CTAs in a group");
     const int grp = blockIdx.x / (S + U + P);
     if (grp >= groups) {
-        fd_residue<FORM, SPEC, THREADS>(a, prm, (blockIdx.x - groups * (S + U + P)) * Run::R, sm.r);
+        fd_residue<FORM, SPEC>(a, prm, (blockIdx.x - groups * (S + U + P)) * FD_R, sm.r);
         return;
     }
-    const int b = blockIdx.x - grp * (S + U + P), e0 = grp * run;
+    const int b = blockIdx.x - grp * (S + U + P), e0 = grp * FD_RUN;
     if (b < S)
-        fd_stress<FORM, SPEC, Run::S, THREADS>(a, prm, e0 + b * Run::S, sm.s);
+        fd_stress<FORM, SPEC>(a, prm, e0 + b * FD_S, sm.s);
     else if (b < S + U)
-        fd_flow<FORM, SPEC, Run::U, THREADS>(a, prm, e0 + (b - S) * Run::U, sm.u);
+        fd_flow<FORM, SPEC>(a, prm, e0 + (b - S) * FD_U, sm.u);
     else
-        fd_pressure<FORM, SPEC, Run::P, THREADS>(a, prm, e0 + (b - S - U) * Run::P, sm.p);
+        fd_pressure<FORM, SPEC>(a, prm, e0 + (b - S - U) * FD_P, sm.p);
 }
 
 // ---------------------------------------------------------------------------
@@ -905,50 +910,38 @@ int residual_batched_ctas_per_sm(int form, int spec)
     return n;
 }
 
-template <class... P>
-static cudaError_t launch_fd(void (*kernel)(P...), int grid, int threads, int smem, bool early, cudaStream_t s, P... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = early ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, args...);
-}
-
-template <int FORM, int SPEC, int THREADS>
-static cudaError_t go_columns(const ElemArgs &a, const KParams &p, bool early, cudaStream_t s)
-{
-    typedef FdRun<THREADS> Run;
-    // a small mesh is one group: all stress CTAs, the longest, are placed first
-    const int run = THREADS == 64 ? a.nel : FD_RUN, groups = (a.nel + run - 1) / run;
-    const int per = (run + Run::S - 1) / Run::S + (run + Run::U - 1) / Run::U + (run + Run::P - 1) / Run::P;
-    const int residue = (a.nel + Run::R - 1) / Run::R;
-    const int smem = (int)sizeof(FdSmem<FORM, THREADS>);
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_fd64<FORM, SPEC, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    return launch_fd<ElemArgs, KParams, int, int>(k_fd64<FORM, SPEC, THREADS>, groups * per + residue, THREADS, smem, early, s,
-                                                  a, p, groups, run);
-}
-
-// One wave of blocks does not start beside the residual kernel: its blocks would
-// go where the residual's leave first, four to an SM on some (300 quads, SQRT
-// form, 765 us in order and 1,368 early).
+// The columns by field start beside the residual kernel; one wave of blocks does
+// not: its blocks would go where the residual's leave first, four to an SM on
+// some (300 quads, SQRT form, 765 us in order and 1,368 early).
 template <int FORM, int SPEC>
 static cudaError_t go_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
 {
-    if (a.nel <= FD_ELEMENT_MAX) return launch_fd<ElemArgs, KParams>(k_fd64_element<FORM, SPEC>, a.nel, 64, 0, false, s, a, p);
-    if (a.nel <= FD_NARROW_MAX) return go_columns<FORM, SPEC, 64>(a, p, false, s);
-    return go_columns<FORM, SPEC, 256>(a, p, true, s);
+    if (a.nel <= FD_ELEMENT_MAX) {
+        k_fd64_element<FORM, SPEC, 1><<<a.nel, FE_THREADS<1>, 0, s>>>(a, p);
+        return cudaGetLastError();
+    }
+    if (a.nel <= FD_FOUR_MAX) {
+        k_fd64_element<FORM, SPEC, 4><<<(a.nel + 3) / 4, FE_THREADS<4>, 0, s>>>(a, p);
+        return cudaGetLastError();
+    }
+    const int groups = (a.nel + FD_RUN - 1) / FD_RUN, residue = (a.nel + FD_R - 1) / FD_R;
+    const int per = FD_RUN / FD_S + FD_RUN / FD_U + FD_RUN / FD_P, smem = (int)sizeof(FdSmem<FORM>);
+    const cudaError_t e = cudaFuncSetAttribute(k_fd64<FORM, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute early[1];
+    early[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(groups * per + residue));
+    cfg.blockDim = dim3(FD_THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cfg.attrs = early;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_fd64<FORM, SPEC>, a, p, groups);
 }
 
-bool fd64_one_wave(int nel) { return nel <= FD_NARROW_MAX; }
+bool fd64_one_wave(int nel) { return nel <= FD_FOUR_MAX; }
 
 cudaError_t launch_fd64(const ElemArgs &a, const KParams &p, cudaStream_t s)
 {

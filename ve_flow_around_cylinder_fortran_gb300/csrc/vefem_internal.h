@@ -19,13 +19,12 @@ constexpr int RES_EPB = 7;
 // 1, 51 / 65 / 65 / 65 with 3, 98 throughout with k_res64; one wave more costs
 // 94 (1, 800 quads) and 96 us (3, 1,000).
 constexpr int RES_WIDE1_MAX = 4 * 152, RES_WIDE3_MAX = 6 * 152;
-// Forward-difference kernel.  Up to three elements per SM a CTA of 64 threads
-// takes an element's columns, up to four CTAs per SM of 64 threads take columns by
-// field, then CTAs of 256.  SQRT form on 210 / 300 / 400 / 500 / 600 quads: elements
-// 760 / 765 / 1,076 / 1,406 / 1,408 us, by field in 64 threads 693 / 972 / 1,086 / 1,289 /
-// 1,291, in 256 threads 1,330 to 1,350; 700 quads 1,560 (64) and 1,345 (256).
+// Forward-difference kernel: up to three elements per SM a CTA takes an element,
+// up to four four of them, beyond that columns by field.  SQRT form, us on 300 /
+// 450 / 460 / 500 / 606 / 700 quads: one element 764 / 1,077 / 1,400 and up; four 1,255
+// / 1,256 / 1,240 / 1,241 / 1,244 / two waves; by field 1,330 to 1,350.
 constexpr int FD_ELEMENT_MAX = 3 * 152;
-constexpr int FD_NARROW_MAX = 4 * 152;
+constexpr int FD_FOUR_MAX = 4 * 152;
 // doubles per Gauss point of a mesh's geometry table
 constexpr int GEO_REC = 38;
 
