@@ -7,6 +7,7 @@ import pytest
 import torch
 
 from ve_flow_around_cylinder_fortran_gb300 import build as B
+from ve_flow_around_cylinder_fortran_gb300 import frontal as FR
 from ve_flow_around_cylinder_fortran_gb300 import mesh as M
 from ve_flow_around_cylinder_fortran_gb300 import pattern as P
 from ve_flow_around_cylinder_fortran_gb300 import state as S
@@ -42,3 +43,24 @@ def test_forward_difference(nel):
         fb, fv = first.setdefault(k, (b, v))
         assert torch.equal(b, fb) and torch.equal(v, fv)
     asm.close()
+
+
+@pytest.mark.parametrize("nel", [300, 1150])
+def test_factorisation(nel):
+    from test_gpu_tree import _system
+    mesh, rp, ci, vals, b, _ = _system(nel, 1, nel)
+    lu = FR.FrontalLU(rp, ci, mesh)
+    matrices = [torch.from_numpy(vals).cuda()]
+    for scale in (1.5, -0.75):
+        matrices.append(matrices[0].clone())
+        matrices[-1][:int(rp[-2])] *= scale
+    rhs = torch.from_numpy(b).cuda()
+    v, first = torch.empty_like(matrices[0]), {}
+    for call in range(45):
+        k = call * 7 % 3
+        v.copy_(matrices[k])
+        lu.factor(v)
+        x = lu._sweep(rhs)
+        factors, fx = first.setdefault(k, (lu.buf.clone(), x))
+        assert lu.mode == "native" and torch.equal(lu.buf, factors) and torch.equal(x, fx)
+    lu.close()

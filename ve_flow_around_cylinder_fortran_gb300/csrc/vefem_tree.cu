@@ -52,6 +52,7 @@
 #include <vector>
 
 #include "vefem.h"
+#include "vefem_early.cuh"
 #include "vefem_gj.cuh"
 #include "vefem_split.cuh"
 
@@ -213,9 +214,12 @@ k_invert(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0,
 // T = D^-1 M[K,:] for 128 columns, as the product of M[K,:]^T and D^-T; columns
 // K of T hold D^-1.  And 128 rows of the copy C = M[P,K].  Starts while k_invert
 // runs, whose blocks have all waited for the kernel before it: M is as that one
-// left it.  D^-1 is read after the wait.
+// left it, and is read with load_early (vefem_early.cuh), which costs no more
+// than plain loads (4.18 and 35.9 ms per factorisation of 2,000 and 20,000 quads
+// with either; 4.37 and 36.4 with all loads after the wait).  D^-1 is read after
+// the wait.
 __global__ void __launch_bounds__(split::THREADS, 2)
-k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *__restrict__ buf,
+k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, const double *buf,
         const double *dinv, double *__restrict__ cpan, double *__restrict__ tpan, int *err)
 {
     extern __shared__ __align__(1024) char s_stage[];
@@ -228,7 +232,7 @@ k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, 
 #pragma unroll 8
     for (int u = t; u < split::TM * KB; u += split::THREADS) {
         const int r = j0 + u / KB, l = u % KB;
-        if (r < f.p) cpan[f.cpan + (int64_t)r * KB + l] = l < kb ? M[(int64_t)r * f.ld + k0 + l] : 0.0;
+        if (r < f.p) cpan[f.cpan + (int64_t)r * KB + l] = l < kb ? load_early(M + (int64_t)r * f.ld + k0 + l) : 0.0;
     }
     const int m = min(split::TM, f.n - j0);
     const bool ok = split::short_product<KB, true>(
@@ -236,7 +240,7 @@ k_pivot(const Front *__restrict__ fr, const int32_t *__restrict__ perm, int k0, 
         [&](int j, int k, double (&x)[8]) {
 #pragma unroll
             for (int u = 0; u < 8; u++)
-                if (k + u < kb) x[u] = M[(int64_t)(k0 + k + u) * f.ld + j0 + j];
+                if (k + u < kb) x[u] = load_early(M + (int64_t)(k0 + k + u) * f.ld + j0 + j);
         },
         [&](int r, int k, double (&y)[8]) {
 #pragma unroll
