@@ -64,3 +64,20 @@ def test_factorisation(nel):
         factors, fx = first.setdefault(k, (lu.buf.clone(), x))
         assert lu.mode == "native" and torch.equal(lu.buf, factors) and torch.equal(x, fx)
     lu.close()
+
+
+@pytest.mark.parametrize("rows", [3, 40, 300])
+def test_training(rows):
+    """The predictor's network: iterations of one call, whose kernels begin while
+    others run, and one call per iteration."""
+    rng = np.random.default_rng(rows)
+    X = rng.standard_normal((rows, 98)).astype(np.float32)
+    T = rng.standard_normal((rows, 32)).astype(np.float32)
+    one, many = (V.MLP(98, 32, width=256, hidden=3, seed=1) for _ in range(2))
+    for iters in (64, 21):
+        a = one.train(X, T, iters, 1e-3)
+        for _ in range(iters):
+            b = many.train(X, T, 1, 1e-3)
+        assert a == b and np.array_equal(one.get_params(), many.get_params())
+    one.close()
+    many.close()

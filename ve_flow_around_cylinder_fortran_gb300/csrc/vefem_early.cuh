@@ -21,3 +21,10 @@ __device__ __forceinline__ double load_early(const double *p)
     asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
+
+__device__ __forceinline__ __nv_bfloat16 load_early(const __nv_bfloat16 *p)
+{
+    unsigned short v;
+    asm volatile("ld.relaxed.gpu.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return __ushort_as_bfloat16(v);
+}

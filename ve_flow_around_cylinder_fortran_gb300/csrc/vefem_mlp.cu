@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "vefem.h"
+#include "vefem_early.cuh"
 #include "vefem_internal.h"
 
 namespace {
@@ -96,7 +97,10 @@ enum { LIN_FWD = 0, LIN_BWD_X = 1, LIN_BWD_W = 2 };
 // Programmatic dependent launch inside an iteration.  A kernel first waits for
 // its predecessor (at once, without a programmatic dependency), then lets its
 // successor start; so whatever runs before a kernel's wait may read what the
-// predecessor's own predecessors wrote, but nothing of the predecessor's.
+// predecessor's own predecessors wrote, with load_early (vefem_early.cuh), but
+// nothing of the predecessor's.  What it reads after the wait was written while
+// it was resident: no operand is const __restrict__, whose loads are for data
+// that does not change while a kernel runs.
 __device__ __forceinline__ void pdl_link()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -109,7 +113,7 @@ __device__ __forceinline__ void pdl_link()
 //   weights  gW = dZ^T X: A(m, k) = dZ[k][m]  (out x n), B(k, c) = X[k][c], and
 //                         column c = in the constant 1 (its output is gb)
 template <int MODE>
-__device__ __forceinline__ float load_a(const float *__restrict__ A, int M, int K, int lda, int m, int k)
+__device__ __forceinline__ float load_a(const float *A, int M, int K, int lda, int m, int k)
 {
     if (m >= M || k >= K) return 0.0f;
     return MODE == LIN_BWD_W ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
@@ -133,10 +137,8 @@ constexpr int MMA_AHEAD = 4;
 // BWD_W: out0 weight gradient, out2 bias gradient.
 template <int MODE>
 __global__ void __launch_bounds__(MMA_WARPS * 32)
-k_linear_mma(int M, int N, int K, const float *__restrict__ A, int lda,
-             const __nv_bfloat16 *__restrict__ Wb, const float *__restrict__ Bf, int ldb,
-             const float *__restrict__ bias, const float *__restrict__ aux, float *__restrict__ out0,
-             float *__restrict__ out1, float *__restrict__ out2, int ldo, int gelu, int early)
+k_linear_mma(int M, int N, int K, const float *A, int lda, const __nv_bfloat16 *Wb, const float *Bf, int ldb,
+             const float *bias, const float *aux, float *out0, float *out1, float *out2, int ldo, int gelu, int early)
 {
     __shared__ float s_part[MMA_WARPS - 1][32][4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -155,7 +157,7 @@ k_linear_mma(int M, int N, int K, const float *__restrict__ A, int lda,
             for (int u = 0; u < 4; u++) {
                 const int k = (ks + h) * 16 + 2 * t + (u & 1) + 8 * (u >> 1);
                 const bool in = ks + h < ks1 && c < N && k < K;
-                wb[h][u] = in ? (MODE == LIN_FWD ? Wb[(size_t)c * ldb + k] : Wb[(size_t)k * ldb + c])
+                wb[h][u] = in ? load_early(MODE == LIN_FWD ? Wb + (size_t)c * ldb + k : Wb + (size_t)k * ldb + c)
                               : __float2bfloat16_rn(0.0f);
             }
     };
