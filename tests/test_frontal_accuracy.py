@@ -11,7 +11,7 @@ from test_linsolve import _jacobian
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("tol,refine,steps", [(1e-14, 3, 1), (1e-12, 1, 1), (1e-11, 3, 1), (1e-14, 0, 0), (1e-10, 3, 0),
+@pytest.mark.parametrize("tol,refine,steps", [(1e-14, 3, 1), (1e-12, 1, 1), (9e-11, 3, 1), (1e-14, 0, 0), (1e-10, 3, 0),
                                               (1e-8, 3, 0)])
 @pytest.mark.parametrize("tree", [True, False])
 def test_refinement_by_tolerance(monkeypatch, tree, tol, refine, steps):

@@ -55,14 +55,15 @@ import numpy as np
 from . import dissection
 
 
-# A sweep of the tree leaves a residual of 3e-16 to 2e-13 (20 bordered Jacobians of
-# 300 to 20,000 quads, Wi 0.1 to 0.6), a sweep of the panels 2e-15 to 2e-11.  So a
-# caller with a tolerance below 2e-11 had the panels' solution refined, to an error
-# of 3e-14 to 6e-13 in x at 2,000 quads and more, and would have the tree's as it
-# is, with one of 4e-14 to 2e-11: below this tolerance the tree's is refined too, to
-# the same error (3e-14 to 6e-13).  Tolerances from here on (the drivers' 1e-10 and
-# 1e-8) accepted the panels' sweep, whose error is the larger one at every size.
-REFINE_BELOW = 2.0e-11
+# A sweep of the tree leaves a residual of 3e-16 to 4e-13 (40 bordered Jacobians of
+# 300 to 20,000 quads, Wi 0.1 to 0.6, eight right-hand sides each), a sweep of the
+# panels 2e-15 to 5e-11.  So a caller with a tolerance below the default had the
+# panels' solution refined, to an error of 1e-14 to 9e-13 in x on 2,000 quads and
+# more, and would have the tree's as it is, with one of 4e-14 to 9e-11: below this
+# tolerance the tree's is refined too, to 1e-14 to 7e-13.  From here on (the
+# drivers' 1e-10 and 1e-8) the panels' sweep was accepted as it was, and its error
+# was larger than the tree's on all but one of the matrices.
+REFINE_BELOW = 1.0e-10
 
 
 def default_panel(nel: int) -> int:
