@@ -264,7 +264,10 @@ int vefem_frontal_solve_path(const vefem_frontal *f);
  * makes its row or column of a product NaN).  tol, min_pivot and
  * VEFEM_ERR_SINGULAR as in vefem_frontal_factor.  Synchronises the stream.
  * vefem_tree_solve: x = A^-1 b, device vectors of N doubles; asynchronous on
- * the stream, vefem_tree_launches kernels replayed from a CUDA graph. */
+ * the stream, vefem_tree_launches kernels replayed from a CUDA graph.  A handle
+ * holds the scratch of one factorisation or solve: calls on one handle are made
+ * in order, by one thread and on one stream (or streams that the caller orders);
+ * different handles share nothing.  vefem_frontal handles are the same in this. */
 typedef struct vefem_tree vefem_tree;
 
 int vefem_tree_create(int device, int nfront, int nlevel, const int32_t *level_ptr,

@@ -20,10 +20,15 @@
 // complements of a 2,000-quad Jacobian the error against extended precision is a
 // quarter of an FP64 product's (all its fronts and rows no larger); with the
 // pairs a + b <= 7 alone, or A's columns evened too, single rows were 2 to 14
-// times worse and the residual of a solve grew by 40%.
+// times worse and the residual of a solve grew by 40%.  FP64 is the better one
+// for entries that spread inside a row or column by more than powers of two of
+// rows, columns and inner indices even: an entry 2^-10 of the largest in the
+// scaled row keeps fewer than 53 bits, one below 2^-62 of it none.  What that does
+// to a solve stands at the elimination (vefem_tree.cu).
 //
 // One tcgen05.mma takes a digit of A (128 x 16) against several digits of B,
-// laid out as one operand of up to 256 columns: 14 instructions per 16 k.
+// laid out as one operand of up to 256 columns: 13 instructions per 16 k with 48
+// columns, 9 with 32.
 // Operands are cut by the CTA's 16 warps straight into the core-matrix layout
 // (8 rows x 16 bytes, no swizzle), 32 k a stage; the nine accumulators take 432 of the SM's 512
 // tensor memory columns, which is why a tile has 48 columns and not 64.

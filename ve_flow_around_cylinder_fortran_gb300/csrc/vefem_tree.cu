@@ -31,10 +31,20 @@
 // 10.6; Schur complements in digits 76 and 8.1; all products in digits, 32
 // pivots a step, 55.8 and 7.0; with two short tiles to an SM and the pivot
 // blocks inverted in registers 38.9 and 5.2; the kernels of a step started
-// before the last one's end 38.0 and 4.7.  A solve checked to 1e-14 went from
-// 43.6 to 1.4 ms at 20,000 (2,500 panels are 5,000 dependent launches, the tree
-// 41): one sweep leaves a residual of 1e-15, where the panels' longer chain of
-// pivots left 1e-12 and took a refinement.
+// before the last one's end 38.0 and 4.7 (36.0 and 4.2 without the solve).  A
+// sweep went from 21 to 1.31 ms at 20,000 (2,500 panels are 5,000 dependent
+// launches, the tree 41).
+//
+// What one sweep leaves, 32 bordered Jacobians of 2,000 to 20,000 quads (Wi 0.1 to
+// 0.6, two states each), eight right-hand sides each, geometric means against a
+// solution refined in twice the precision: with the same elimination on the FP64
+// pipe a residual of 3e-16 to 1e-13; with all products in digits 0.96 times that
+// and 0.79 times its error in x; with the pivot blocks inverted in registers (one
+// elimination of 32 pivots instead of two of 16) 1.06 and 1.11 times (at 20,000
+// quads 0.82 and 1.95, single matrices up to 7 and 3.5 times).  Dividing by the
+// pivots in full there gives 0.90 and 1.00 times for 4% to 11% more time, a step
+// of Newton's iteration on the inverse 0.88 and 5 times.  The panels leave a
+// residual of 3e-15 to 2e-11 and errors 0.6 to 35,000 times as large.
 //
 // Solve: per depth, deepest first, y_P = A^-1 b_P and the update -C y_P a
 // front hands to its parent; then, root first, x_P = y_P - X x_F.  A row's dot
