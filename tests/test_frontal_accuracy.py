@@ -1,7 +1,8 @@
 """Accuracy that ``FrontalLU.solve`` owes to the tolerance it is given.  The sweep
 of the tree elimination leaves so small a residual that a check alone asks for
 no refinement; a caller with a tolerance near rounding level gets one all the
-same, as the panel elimination's sweeps needed it to pass."""
+same where the panel elimination's sweeps needed it to pass, on all but the
+smallest meshes."""
 import numpy as np
 import pytest
 
@@ -11,11 +12,12 @@ from test_linsolve import _jacobian
 torch = pytest.importorskip("torch")
 
 
-@pytest.mark.parametrize("tol,refine,steps", [(1e-14, 3, 1), (1e-12, 1, 1), (9e-11, 3, 1), (1e-14, 0, 0), (1e-10, 3, 0),
-                                              (1e-8, 3, 0)])
+@pytest.mark.parametrize("nel,tol,refine,steps", [(270, 1e-14, 3, 1), (270, 1e-12, 1, 1), (270, 9e-11, 3, 1),
+                                                  (270, 1e-14, 0, 0), (270, 1e-10, 3, 0), (270, 1e-8, 3, 0),
+                                                  (60, 1.9e-15, 3, 1), (60, 1e-14, 3, 0), (60, 1e-10, 3, 0)])
 @pytest.mark.parametrize("tree", [True, False])
-def test_refinement_by_tolerance(monkeypatch, tree, tol, refine, steps):
-    mesh, rp, ci, v, b = _jacobian(60, 1)
+def test_refinement_by_tolerance(monkeypatch, tree, nel, tol, refine, steps):
+    mesh, rp, ci, v, b = _jacobian(nel, 1)
     N = len(rp) - 1
     rows = np.repeat(np.arange(N), np.diff(rp))
     v = np.where(rows == ci, 8.0, 0.0) + 0.01 * np.random.default_rng(1).standard_normal(len(v))

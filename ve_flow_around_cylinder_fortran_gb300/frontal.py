@@ -64,6 +64,11 @@ from . import dissection
 # drivers' 1e-10 and 1e-8) the panels' sweep was accepted as it was, and its error
 # was larger than the tree's on all but one of the matrices.
 REFINE_BELOW = 1.0e-10
+# On 40 to 250 quads (up to 6,601 unknowns, 18 matrices each of six sizes) the
+# panels' sweeps left residuals of at most 1.6e-15 and were accepted at 1e-14, with
+# the errors that the tree's leave (2e-14 to 5e-14 on average, either way): there
+# the line lies below that.  A refinement costs four times the sweep on 40 quads.
+SMALL, REFINE_BELOW_SMALL = 7000, 2.0e-15
 
 
 def default_panel(nel: int) -> int:
@@ -560,7 +565,8 @@ class FrontalLU:
         backward error of an unpivoted elimination is a property of its
         factors, so a factorisation that passes on its first right-hand side
         passes on the next ones.  With a ``check_tol`` below ``REFINE_BELOW``
-        every solve of the tree is refined at least once, and checked."""
+        (``REFINE_BELOW_SMALL`` up to ``SMALL`` unknowns) every solve of the
+        tree is refined at least once, and checked."""
         torch = self.torch
         host = isinstance(b, np.ndarray)
         if self._host is not None:
@@ -577,7 +583,8 @@ class FrontalLU:
         else:
             bt = b.to(device=self.dev, dtype=torch.float64)
         x = self._sweep(bt)
-        tight = self.tree and self.mode == "native" and self.refine > 0 and self.check_tol < REFINE_BELOW
+        line = REFINE_BELOW if self.N > SMALL else REFINE_BELOW_SMALL
+        tight = self.tree and self.mode == "native" and self.refine > 0 and self.check_tol < line
         check = tight or (self._since_factor % self.check_every == 0) or self._needs_checks
         self._since_factor += 1
         if check:
