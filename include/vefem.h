@@ -329,7 +329,8 @@ int vefem_assemble_batched(vefem_batch *bt, const double *const *TL, const doubl
  * candidate tile of every class present on the live GPU (reps launches each,
  * device-resident buffers of its own) and keeps the fastest; tiles_out
  * (may be NULL) receives the chosen tiles.  A tile is rounded up to whole groups
- * of the elements the Jacobian kernel takes at a time (4 in FP32, 3 in FP64). */
+ * of the elements the Jacobian kernel takes at a time (4 in FP32; 3 in FP64, fewer
+ * for batches of up to two elements per SM). */
 #define VEFEM_BATCH_CLASSES 6
 int vefem_batch_autotune(vefem_batch *bt, int flags, int reps, int *tiles_out);
 int vefem_batch_set_tiles(vefem_batch *bt, const int *tiles);

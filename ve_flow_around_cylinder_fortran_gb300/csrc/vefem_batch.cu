@@ -166,11 +166,11 @@ int bfail(vefem_batch *b, int code, const std::string &msg)
 
 int spec_of(const KParams &p) { return (p.ReN == 0.0 ? SPEC_RE0 : 0) | (p.DfN == 0.0 ? SPEC_DF0 : 0); }
 
-// a run of `tile` elements holds whole groups of the elements the Jacobian
-// kernel works on at a time: a smaller tile would leave its lanes idle
-int whole_tile(int tile, int elem_size)
+// a run of `tile` elements holds whole groups of the elements that an item of the
+// Jacobian kernel does: a smaller tile would leave its lanes idle
+int whole_tile(const vefem_batch *bt, int tile, int elem_size)
 {
-    const int ne = exact_elements_at_a_time(elem_size);
+    const int ne = exact_elements_per_item(elem_size, bt->total_el, bt->sms);
     return (tile + ne - 1) / ne * ne;
 }
 
@@ -181,7 +181,7 @@ int build_work(vefem_batch *bt)
         const int nel = bt->ctx[i]->nel;
         for (int e0 = 0; e0 < nel; e0 += RES_EPB) rw.push_back({i, e0, std::min(RES_EPB, nel - e0), 0});
         for (int k = 0; k < 2; k++) {
-            const int tile = whole_tile(bt->tiles[size_class(nel)], k == 0 ? 4 : 8);
+            const int tile = whole_tile(bt, bt->tiles[size_class(nel)], k == 0 ? 4 : 8);
             for (int e0 = 0; e0 < nel; e0 += tile) xw[k].push_back({i, e0, std::min(tile, nel - e0), 0});
         }
     }
@@ -596,7 +596,7 @@ extern "C" int vefem_batch_autotune(vefem_batch *bt, int flags, int reps, int *t
         float best = 1e30f;
         int tried = 0;
         for (int tile : EX_TILES) {
-            const int run = whole_tile(tile, (int)vsize);
+            const int run = whole_tile(bt, tile, (int)vsize);
             if (run == tried) continue;      // the same work items as a smaller tile's
             tried = run;
             std::vector<WorkItem> w;

@@ -415,6 +415,7 @@ extern "C" int vefem_create(const vefem_mesh *mesh, const vefem_csr *pat,
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ctx->join, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&ctx->join_edges, cudaEventDisableTiming);
+    if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device);
     if (ce != cudaSuccess) {
         std::string m = std::string("cudaStreamCreate: ") + cudaGetErrorString(ce);
         delete ctx;
@@ -586,7 +587,13 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
     ea.rs = ctx->d_rs;
     ea.es = ctx->d_es;
     ea.as = ctx->d_as;
-    const bool side = jmode != VEFEM_JAC_FD64 && want_res && want_jac;
+    // The residual beside an exact Jacobian, but for an FP64 one of up to three
+    // elements per SM: both are bound by the FP64 pipe, and residual blocks that
+    // came first crowd the Jacobian's onto fewer SMs (T form, 150 / 300 / 450 quads,
+    // three elements to an item: 343 / 346 / 352 us beside, 204 / 209 / 215 in order;
+    // on 600 quads 362 and 368).
+    const bool side = jmode != VEFEM_JAC_FD64 && want_res && want_jac &&
+                      !(jmode == VEFEM_JAC_EXACT64 && ctx->nel <= 3 * ctx->sms);
     // The outlet edges are a few blocks with a long serial chain each (145 us in
     // FP64 columns), independent of the elements until they are added at the end:
     // on the second stream beside the element kernels, 2,746 -> 2,607 us for a host
@@ -633,11 +640,8 @@ extern "C" int vefem_assemble(vefem_ctx *ctx, const double *TL, const double *EU
             ctx->launches++;
         }
         if (jmode == VEFEM_JAC_EXACT64 || jac32) {
-            if (!ctx->d_self) {
-                CK(cudaMalloc((void **)&ctx->d_self, sizeof(BatchInst)));
-                CK(cudaDeviceGetAttribute(&ctx->sms, cudaDevAttrMultiProcessorCount, ctx->device));
-            }
-            const int ne = exact_elements_at_a_time(jac32 ? 4 : 8), nwork = ((int)nel + ne - 1) / ne;
+            if (!ctx->d_self) CK(cudaMalloc((void **)&ctx->d_self, sizeof(BatchInst)));
+            const int ne = exact_elements_per_item(jac32 ? 4 : 8, nel, ctx->sms), nwork = ((int)nel + ne - 1) / ne;
             WorkItem *&d_work = ctx->d_work[jac32 ? 0 : 1];
             if (!d_work) {
                 std::vector<WorkItem> w(nwork);

@@ -36,6 +36,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "vefem_dual.cuh"
 #include "vefem_internal.h"
 #include "vefem_physics.cuh"
@@ -559,7 +561,17 @@ static cudaError_t go_exact_batched(const BatchInst *insts, const WorkItem *work
     return cudaGetLastError();
 }
 
-int exact_elements_at_a_time(int elem_size) { return elem_size == 4 ? ExCfg<float>::NE : ExCfg<double>::NE; }
+// Elements per work item of nel elements in all (a mesh, a batch).  In FP64 a mesh
+// of a few elements per SM takes as long as one SM does, most of it the FP64 pipe's
+// time for the SM's elements, so they are spread evenly.  Residual, then Jacobian,
+// T form, 150 / 300 / 450 quads: 145 / 213 / 372 us with one element to an item,
+// 184 / 189 / 316 with two, 204 / 209 / 215 with three (a kernel of one element at a
+// time took 222 / 347 / 471).  FP32 gains nothing by it (40 to 900 quads within 5%).
+int exact_elements_per_item(int elem_size, int64_t nel, int sms)
+{
+    if (elem_size == 4) return ExCfg<float>::NE;
+    return (int)std::min<int64_t>(ExCfg<double>::NE, std::max<int64_t>(1, (nel + sms - 1) / std::max(1, sms)));
+}
 
 template <class T>
 cudaError_t launch_exact_batched(const BatchInst *insts, const WorkItem *work, int nwork,

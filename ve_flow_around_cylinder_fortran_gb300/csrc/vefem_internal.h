@@ -173,9 +173,9 @@ cudaError_t launch_residual64_batched(const BatchInst *insts, const WorkItem *wo
 template <class T>
 cudaError_t launch_exact_batched(const BatchInst *insts, const WorkItem *work, int nwork,
                                  int form, int spec, int grid, cudaStream_t s);
-// elements the exact-Jacobian kernel works on at a time (element size 4 or 8 bytes):
-// its work items hold a multiple of it
-int exact_elements_at_a_time(int elem_size);
+// elements of a work item of the exact-Jacobian kernel for nel elements in all
+// (element size 4 or 8 bytes): as many as it works on at a time, or fewer
+int exact_elements_per_item(int elem_size, int64_t nel, int sms);
 // occupancy of the persistent kernels (resident CTAs per SM)
 int exact_batched_ctas_per_sm(int elem_size, int form, int spec);
 int residual_batched_ctas_per_sm(int form, int spec);
