@@ -16,7 +16,8 @@ Two orderings of the fronts:
   in the library's kernels (``csrc/vefem_tree.cu``), the products on the
   tensor cores in exact digits (``csrc/vefem_split.cuh``).  50 G multiply-adds
   and 133 dependent steps for 20,000 quads.
-* Panels (``panel`` given, the pivoted method, the CPU): elements are swept
+* Panels (``panel`` given, the pivoted method, the CPU, a pattern with entries
+  that the dissection's fronts do not hold): elements are swept
   downstream in order of their centroid x and grouped into panels of ``G``
   elements.  A node is *fully summed* after the last panel that touches it;
   the *front* after panel q is the set of nodes touched by panels <= q and by a
@@ -79,6 +80,10 @@ def default_panel(nel: int) -> int:
     a quarter column measured fastest of the panel sizes on GB300 at 20,000 and
     40,000 quads."""
     return max(4, int(round(math.sqrt(nel / 20.0) / 4.0)))
+
+
+class OutsideFront(RuntimeError):
+    """A matrix entry whose two unknowns no front holds together."""
 
 
 class FrontalLU:
@@ -150,9 +155,15 @@ class FrontalLU:
     def _analyse(self, en):
         """Symbolic phase (mesh and pattern only) and the native handle."""
         if self.tree:
-            self._symbolic_tree(en)
-            self._create_tree()
-            return
+            try:
+                self._symbolic_tree(en)
+            except OutsideFront:
+                # entries between nodes that share no element: the panels' fronts,
+                # where more nodes meet, may hold them
+                self.tree, self.G = False, default_panel(en.shape[0])
+            else:
+                self._create_tree()
+                return
         self._symbolic(en, self.mesh.xyz[0][en].mean(axis=1))
         if self.method == "native":
             self._create_native()
@@ -178,7 +189,7 @@ class FrontalLU:
             k = f * N + u
             i = torch.clamp(torch.searchsorted(keys, k), max=len(keys) - 1)
             if not bool((keys[i] == k).all()):
-                raise RuntimeError("frontal symbolic phase: an entry outside its front")
+                raise OutsideFront("frontal symbolic phase: an entry outside its front")
             return pos_sorted[i]
 
         # each CSR entry goes to the deeper (larger heap id) of its unknowns' fronts
@@ -300,7 +311,7 @@ class FrontalLU:
             i = torch.searchsorted(keys_t, k)
             i = torch.clamp(i, max=len(keys_t) - 1)
             if not bool((keys_t[i] == k).all()):
-                raise RuntimeError("frontal symbolic phase: an entry outside its panel")
+                raise OutsideFront("frontal symbolic phase: an entry outside its panel")
             return pos_t[i]
 
         # each CSR entry goes to panel min(last(row), last(col))
